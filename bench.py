@@ -316,7 +316,7 @@ def main():
                     help="force a DOM sweep path (fs_dom_set_sweep_mode); 0 picks automatically")
     ap.add_argument("--dom-kernel", type=int, default=0,
                     help="path 8's sweep kernel (fs_dom_set_sweep_kernel): 0 automatic, "
-                         "1 pencil per thread, 2 lane column")
+                         "1 pencil per thread, 2 lane column, 3 register patch")
     ap.add_argument("--batch", type=int, default=0,
                     help="instead of the headline line: N cases of the batched sweep of uneven "
                          "domains (Nx 200-600) stepped concurrently, against the same cases "
@@ -513,7 +513,8 @@ def kernel_roofline(solver, kt, steps, form, peak, peak_src):
         if lib.fs_dom_launch_shape(solver.dom, shape) == 0:
             out["dom_cluster"] = dict(zip(("ctas", "rows", "threads", "smem_bytes", "groups"),
                                           list(shape)))
-            out["dom_cluster"]["kernel"] = {1: "pencil per thread", 2: "lane column"}.get(
+            out["dom_cluster"]["kernel"] = {1: "pencil per thread", 2: "lane column",
+                                          3: "register patch"}.get(
                 int(lib.fs_dom_sweep_kernel(solver.dom)), "none")
     if dom_k == "dom_sweep":
         out["fused_sweep_bytes_per_launch"] = fused_dom

@@ -27,6 +27,8 @@
 //     octant's partial G and ground flux and never stores intensities.  The
 //     cluster shape is planned so that all clusters are resident at once
 //     where the part allows it.
+//     Kernels: the pencil-per-thread one, the lane-column one, and, where path
+//     and kernel are automatic, the register-patch one (dom_patch.cuh).
 //   3 (any quadrature) one launch per hyperplane over all ordinates, with the
 //     full intensity field stored; G summed over ordinates in ordinate order.
 // Path 8 sums G within each octant in ordinate order and then over octants in
@@ -65,6 +67,12 @@ struct DomCtx {
   size_t cl_smem;
   int sweep_kernel;           // requested path-8 kernel: 0/1 pencil per thread, 2 lane column
   int cl_lane;                // resolved: 1 = the lane-column kernel
+  // the register-patch kernel (resolved: rp = 1): skewed (kappa, kappa*B) and
+  // ground intensity, FP64 or FP32 by fp32; |ordinate components| of an octant
+  int rp, rp_pair, rp_zs;
+  void *kb4[4], *igA, *igB;
+  double* om;
+  double rp_dz0;
   int begun;                  // dom_begin done, dom_end due
   double pend_I_amb;          // ambient intensity of the begun solve
   int down_slot[8];
@@ -185,37 +193,80 @@ template <> struct Vec2Of<double> { using type = double2; };
 template <> struct Vec2Of<float> { using type = float2; };
 
 // ---- set-up: absorption, emission, ground ------------------------------------
-__global__ void k_dom_setup(GridDev g, const double* __restrict__ Ts, const double* __restrict__ Tg,
-                            const double* __restrict__ as, const double* __restrict__ om,
-                            const double* __restrict__ YH, const double* __restrict__ rho,
-                            const double* __restrict__ Mloc, double sigma, double Tamb4,
-                            double kgmax, double* ks, double* kg, double* ksafe, double* B,
-                            double2* kb, float2* kb32) {
-  int64_t n = ncells_dev(g);
-  int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (c >= n) return;
-  double ksol = sigma * as[c];
-  if (Mloc) ksol = ksol * (1.0 + 5.0 * Mloc[c]);
-  double of = clip01(om[c] / 1.0e-3);
-  double tf = clip01((Tg[c] - 600.0) / 400.0);
+// x^4 from the square and its rounding error, within about half an ulp; a
+// fraction of pow's cost, which was most of the set-up's arithmetic
+__device__ __forceinline__ double fourth_power(double x) {
+  const double s = __dmul_rn(x, x), e = __fma_rn(x, x, -s);
+  return __fma_rn(s, s, __dmul_rn(2.0 * s, e));
+}
+struct DomSetupArgs {
+  const double *Ts, *Tg, *as, *om, *YH, *rho, *Mloc;
+  double sigma, Tamb4, kgmax;
+};
+// one cell: the absorption coefficients (solid, gas, their sum floored) and
+// the emission B
+__device__ __forceinline__ void dom_setup_cell(const DomSetupArgs& s, int64_t c, double* ks,
+                                               double* kg, double* ksafe, double* B, double& ksf,
+                                               double& Bc) {
+  double ksol = s.sigma * s.as[c];
+  if (s.Mloc) ksol = ksol * __fma_rn(5.0, s.Mloc[c], 1.0);
+  double of = clip01(s.om[c] / 1.0e-3);
+  double tf = clip01((s.Tg[c] - 600.0) / 400.0);
   double mx = (of >= tf || of != of) ? of : tf;
-  double kgas = kgmax * mx;
-  if (YH && rho) kgas = kgas + 30.0 * rho[c] * YH[c];
+  double kgas = s.kgmax * mx;
+  if (s.YH && s.rho) kgas = __fma_rn(__dmul_rn(30.0, s.rho[c]), s.YH[c], kgas);
   double kap = ksol + kgas;
-  double ksf = (kap >= 1.0e-3 || kap != kap) ? kap : 1.0e-3;
+  ksf = (kap >= 1.0e-3 || kap != kap) ? kap : 1.0e-3;
   double T4;
   if (kap > 1.0e-9) {
-    T4 = (ksol * pow(Ts[c], 4.0) + kgas * pow(Tg[c], 4.0)) / ksf;
+    // (explicit rounding: the same numbers whichever kernel this is part of)
+    T4 = __fma_rn(ksol, fourth_power(s.Ts[c]), __dmul_rn(kgas, fourth_power(s.Tg[c]))) / ksf;
   } else {
-    T4 = Tamb4;
+    T4 = s.Tamb4;
   }
-  const double Bc = SIGMA_SB_D * T4 / PI_D;
+  Bc = SIGMA_SB_D * T4 / PI_D;
   ks[c] = ksol;
   kg[c] = kgas;
   ksafe[c] = ksf;
   B[c] = Bc;
+}
+
+__global__ void k_dom_setup(GridDev g, DomSetupArgs s, double* ks, double* kg, double* ksafe,
+                            double* B, double2* kb, float2* kb32) {
+  int64_t n = ncells_dev(g);
+  int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (c >= n) return;
+  double ksf, Bc;
+  dom_setup_cell(s, c, ks, kg, ksafe, B, ksf, Bc);
   if (kb) kb[c] = make_double2(ksf, ksf * Bc);
   if (kb32) kb32[c] = make_float2((float)ksf, (float)(ksf * Bc));
+}
+
+// The convergence test's maxima, as order-preserving keys: G and |G - G_prev|
+// are not negative, NaN maps above +inf.
+__device__ __forceinline__ void dom_G_keys(double s, double gp, unsigned long long& bg,
+                                           unsigned long long& bd) {
+  const double d = fabs(s - gp);
+  const unsigned long long ks =
+      (s != s) ? 0x7ff8000000000000ull
+               : (unsigned long long)__double_as_longlong(s > 0.0 ? s : 0.0);
+  const unsigned long long kd =
+      (d != d) ? 0x7ff8000000000000ull : (unsigned long long)__double_as_longlong(d);
+  bg = ks > bg ? ks : bg;
+  bd = kd > bd ? kd : bd;
+}
+__device__ __forceinline__ void dom_G_max(unsigned long long bg, unsigned long long bd,
+                                          unsigned long long* keys) {
+  for (int o = 16; o > 0; o >>= 1) {
+    unsigned long long y = __shfl_xor_sync(0xffffffffu, bg, o);
+    bg = y > bg ? y : bg;
+    y = __shfl_xor_sync(0xffffffffu, bd, o);
+    bd = y > bd ? y : bd;
+  }
+  if ((threadIdx.x & 31) == 0) {
+    atomicMax(keys, bg);
+    atomicMax(keys + 1, bd);
+  }
 }
 
 __global__ void k_dom_ground_init(int n2, const double* __restrict__ Tsoil, double eps_w,
@@ -291,25 +342,9 @@ __global__ void k_dom_G(int64_t N, int M, const double* __restrict__ w,
     double s = 0.0;
     for (int n = 0; n < M; ++n) s += w[n] * I[(int64_t)n * N + c];
     G[c] = s;
-    double d = fabs(s - Gp[c]);
-    // keys for non-negative doubles (NaN maps above +inf)
-    unsigned long long ks = (s != s) ? 0x7ff8000000000000ull
-                                     : (unsigned long long)__double_as_longlong(s > 0.0 ? s : 0.0);
-    unsigned long long kd = (d != d) ? 0x7ff8000000000000ull
-                                     : (unsigned long long)__double_as_longlong(d);
-    bg = ks > bg ? ks : bg;
-    bd = kd > bd ? kd : bd;
+    dom_G_keys(s, Gp[c], bg, bd);
   }
-  for (int o = 16; o > 0; o >>= 1) {
-    unsigned long long y = __shfl_xor_sync(0xffffffffu, bg, o);
-    bg = y > bg ? y : bg;
-    y = __shfl_xor_sync(0xffffffffu, bd, o);
-    bd = y > bd ? y : bd;
-  }
-  if ((threadIdx.x & 31) == 0) {
-    atomicMax(keys, bg);
-    atomicMax(keys + 1, bd);
-  }
+  dom_G_max(bg, bd, keys);
 }
 
 // q_in at the ground, new ground intensity with under-relaxation
@@ -822,6 +857,8 @@ __global__ void __launch_bounds__(PPT == 1 ? CL_MAX_THREADS_1 : CL_MAX_THREADS_2
   cluster_wait_acquire();
 }
 
+#include "dom_patch.cuh"
+
 // ---- path 8, lane-column form ------------------------------------------------
 // The same sweep (cluster per octant, CTAs splitting the k' rows, the ring
 // hand-off between CTAs, the same inputs, outputs and arithmetic, so the same
@@ -1150,24 +1187,9 @@ __global__ void k_dom_G_oct(int64_t N, int nparts, const T* __restrict__ Goct, d
     double s = 0.0;
     for (int o = 0; o < nparts; ++o) s += (double)Goct[(int64_t)o * N + c];
     G[c] = s;
-    double d = fabs(s - Gp[c]);
-    unsigned long long ks = (s != s) ? 0x7ff8000000000000ull
-                                     : (unsigned long long)__double_as_longlong(s > 0.0 ? s : 0.0);
-    unsigned long long kd = (d != d) ? 0x7ff8000000000000ull
-                                     : (unsigned long long)__double_as_longlong(d);
-    bg = ks > bg ? ks : bg;
-    bd = kd > bd ? kd : bd;
+    dom_G_keys(s, Gp[c], bg, bd);
   }
-  for (int o = 16; o > 0; o >>= 1) {
-    unsigned long long y = __shfl_xor_sync(0xffffffffu, bg, o);
-    bg = y > bg ? y : bg;
-    y = __shfl_xor_sync(0xffffffffu, bd, o);
-    bd = y > bd ? y : bd;
-  }
-  if ((threadIdx.x & 31) == 0) {
-    atomicMax(keys, bg);
-    atomicMax(keys + 1, bd);
-  }
+  dom_G_max(bg, bd, keys);
 }
 
 // q_in at the ground from the downward octants' partial fluxes; ground
@@ -1263,6 +1285,9 @@ void* dom_create(const GridDev& g, int M, const double* ox, const double* oy, co
   D->withhold_plane = -1;
   D->fp32 = 0; D->cl_ppt = 1; D->cl_waves = 0; D->begun = 0; D->pend_I_amb = 0.0;
   D->sweep_kernel = 0; D->cl_lane = 0;
+  D->rp = 0; D->rp_pair = 0;
+  for (int q = 0; q < 4; ++q) D->kb4[q] = nullptr;
+  D->igA = nullptr; D->igB = nullptr; D->om = nullptr;
   cudaMalloc(&D->G, sizeof(double) * N); cudaMalloc(&D->Gp, sizeof(double) * N);
   cudaMemsetAsync(D->G, 0, sizeof(double) * N, ss.s);
   cudaMemsetAsync(D->Gp, 0, sizeof(double) * N, ss.s);
@@ -1294,6 +1319,8 @@ void dom_destroy(void* h) {
   if (!D) return;
   cudaFree(D->ox); cudaFree(D->oy); cudaFree(D->oz); cudaFree(D->w); cudaFree(D->I);
   cudaFree(D->kb); cudaFree(D->Goct); cudaFree(D->Qoct); cudaFree(D->wrap);
+  for (int q = 0; q < 4; ++q) cudaFree(D->kb4[q]);
+  cudaFree(D->igA); cudaFree(D->igB); cudaFree(D->om);
   cudaFree(D->G); cudaFree(D->Gp); cudaFree(D->ks); cudaFree(D->kg); cudaFree(D->ksafe);
   cudaFree(D->B); cudaFree(D->Ig_out); cudaFree(D->Isoil); cudaFree(D->qin); cudaFree(D->keys);
   cudaFreeHost(D->h_keys);
@@ -1438,11 +1465,151 @@ static bool plan_lc(DomCtx* D) {
   return true;
 }
 
+// The register-patch kernel's launch shape: octant-major ordinates whose
+// components and weights are the same numbers in every octant (one table per
+// launch), 3, 6 or 10 of them in the level-symmetric point order, on a grid
+// whose rows fit.  The cluster size is the one with the least waves x steps x
+// time per step: about a thousand cycles of latency (barrier, exchange through
+// shared memory, the update's dependency chain) and the busiest scheduler's
+// arithmetic, and every CTA of the chain adds the steps by which it trails the
+// one before it.  Measured at 97 x 41 x 23, S4: 158, 117, 114 and 111 us a sweep
+// with 2, 4, 6 and 8 CTAs; 400 x 120 x 60, S8: 907 us with 10, 1514 with 15 (two
+// waves of clusters).
+static const void* octant_rp_ptr(bool fp32, int Mo, bool pair) {
+#define RPP(T, M, P) (const void*)k_dom_octant_rp<T, M, P>
+  switch (Mo) {
+    case 3: return fp32 ? RPP(float, 3, false) : (pair ? RPP(double, 3, true) : RPP(double, 3, false));
+    case 6: return fp32 ? RPP(float, 6, false) : (pair ? RPP(double, 6, true) : RPP(double, 6, false));
+    case 10: return fp32 ? RPP(float, 10, false) : (pair ? RPP(double, 10, true) : RPP(double, 10, false));
+  }
+#undef RPP
+  return nullptr;
+}
+
+template <int MO>
+static bool rp_points_match(const DomCtx* D) {
+  using PT = RpPoints<MO>;
+  double X[PT::NL], W[PT::NW];
+  for (int m = 0; m < MO; ++m) {
+    X[rp_digit(PT::X, m)] = fabs(D->hox[m]);
+    W[rp_digit(PT::W, m)] = D->hw[m];
+  }
+  for (int m = 0; m < MO; ++m)
+    if (fabs(D->hox[m]) != X[rp_digit(PT::X, m)] || fabs(D->hoy[m]) != X[rp_digit(PT::Y, m)] ||
+        fabs(D->hoz[m]) != X[rp_digit(PT::Z, m)] || D->hw[m] != W[rp_digit(PT::W, m)])
+      return false;
+  return true;
+}
+
+static bool plan_rp(DomCtx* D, int force_C) {
+  const GridDev& g = D->g;
+  const int Mo = D->M / 8;
+  if (Mo != 3 && Mo != 6 && Mo != 10) return false;
+  for (int n = Mo; n < D->M; ++n) {
+    const int m = n % Mo;
+    if (fabs(D->hox[n]) != fabs(D->hox[m]) || fabs(D->hoy[n]) != fabs(D->hoy[m]) ||
+        fabs(D->hoz[n]) != fabs(D->hoz[m]) || D->hw[n] != D->hw[m])
+      return false;
+  }
+  // the level-symmetric point order; pairs with x and y components swapped
+  // have equal denominators when dx == dy
+  const bool ls = Mo == 10 ? rp_points_match<10>(D) : Mo == 6 ? rp_points_match<6>(D)
+                                                             : rp_points_match<3>(D);
+  if (!ls) return false;
+  D->rp_pair = g.dx == g.dy;
+  const int rk = Mo == 10 ? RpShape<10>::RK : Mo == 6 ? RpShape<6>::RK : RpShape<3>::RK;
+  const int maxw = Mo == 10 ? RpShape<10>::MAXW : Mo == 6 ? RpShape<6>::MAXW : RpShape<3>::MAXW;
+  const int tsize = D->fp32 ? (int)sizeof(float) : (int)sizeof(double);
+  const void* fn = octant_rp_ptr(D->fp32 != 0, Mo, D->rp_pair != 0);
+  int dev = 0, optin = 0, smem_sm = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+  cudaDeviceGetAttribute(&smem_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev);
+  cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+  cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, optin);
+  double best = 1e300;
+  bool found = false;
+  for (int C = 16; C >= 1; --C) {
+    if (force_C > 0 && C != force_C) continue;
+    const int rows = (g.nz + C - 1) / C;
+    if ((g.nz + rows - 1) / rows != C) continue;
+    const int warps = ((g.ny + 31) / 32) * ((rows + rk - 1) / rk);
+    if (warps > maxw) continue;
+    int zs = RP_ZS_MAX;
+    while (zs > 4 && rp_layout(tsize, Mo, rows, g.ny, zs).total > (size_t)optin) zs /= 2;
+    const size_t need = rp_layout(tsize, Mo, rows, g.ny, zs).total;
+    const size_t pad = (size_t)smem_sm / 2 + 1024;  // no two CTAs on one SM
+    const size_t smem = need > pad ? need : pad;
+    if (smem > (size_t)optin) continue;
+    const int threads = 32 * warps;
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = C; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
+    cfg.gridDim = dim3(8 * C); cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem; cfg.attrs = at; cfg.numAttrs = 1;
+    int active = 0;
+    if (cudaOccupancyMaxActiveClusters(&active, fn, &cfg) != cudaSuccess) {
+      cudaGetLastError();
+      active = 0;
+    }
+    if (active < 1) continue;
+    const int waves = (8 + active - 1) / active;
+    const double step = 1000.0 + (double)((warps + 3) / 4) * rk * Mo * (D->fp32 ? 18 : 24);
+    const double cost = waves * step * (g.nx + g.ny + g.nz + 2.0 * C);
+    if (cost < best) {
+      best = cost; found = true;
+      D->cl_C = C; D->cl_rows = rows; D->cl_threads = threads; D->cl_smem = smem;
+      D->cl_ppt = 1; D->groups = 1; D->cl_waves = waves;
+      D->rp_zs = zs;
+    }
+  }
+  return found;
+}
+
 static int dom_prepare(DomCtx* D, cudaStream_t st) {
   if (D->mode != 0) return FS_OK;
   const GridDev& g = D->g;
   const int64_t N = ncells(g), n2 = (int64_t)g.nx * g.ny;
   const int want = D->mode_req;
+  const size_t ts = D->fp32 ? sizeof(float) : sizeof(double);
+  // the register-patch kernel where path and kernel are automatic, or on request
+  if ((D->sweep_kernel == 3 && want != 3) || (D->sweep_kernel == 0 && want == 0)) {
+    if (D->force_groups < 2 && octant_grouping(D) && plan_rp(D, D->force_C)) {
+      D->mode = 8;
+      D->rp = 1;
+      D->Mo = D->M / 8;
+      int slot = 0;
+      for (int o = 0; o < 8; ++o) D->down_slot[o] = D->hoz[o * D->Mo] < 0.0 ? slot++ : -1;
+      const int64_t plane = (int64_t)(g.nx + g.ny - 1) * rp_pitch(g.ny);
+      const int64_t all = (int64_t)(g.nx + g.ny + g.nz - 2) * g.nz * rp_pitch(g.ny);
+      const int64_t wn = 8ll * rp_pad((int)ts, D->Mo) * g.nz * (g.nx + g.nz - 1);
+      for (int q = 0; q < 4; ++q) cudaMalloc(&D->kb4[q], 2 * ts * all);
+      cudaMalloc(&D->igA, ts * plane);
+      cudaMalloc(&D->igB, ts * plane);
+      cudaMalloc(&D->Goct, ts * 8 * g.nz * plane);
+      cudaMalloc(&D->Qoct, ts * 8 * plane);
+      cudaMalloc(&D->wrap, ts * wn);
+      cudaMemsetAsync(D->wrap, 0, ts * wn, st);
+      std::vector<double> om(3 * D->Mo);
+      for (int m = 0; m < D->Mo; ++m) {
+        om[m] = fabs(D->hox[m]);
+        om[D->Mo + m] = fabs(D->hoy[m]);
+        om[2 * D->Mo + m] = fabs(D->hoz[m]);
+      }
+      cudaMalloc(&D->om, sizeof(double) * om.size());
+      cudaMemcpyAsync(D->om, om.data(), sizeof(double) * om.size(), cudaMemcpyHostToDevice, st);
+      // the height the launch constants are for; every CTA compares its levels
+      cudaMemcpyAsync(&D->rp_dz0, g.dz, sizeof(double), cudaMemcpyDeviceToHost, st);
+      if (fs_stream_wait(st) != FS_OK) return FS_ECUDA;
+      return cuda_status();
+    }
+    if (D->sweep_kernel == 3) {
+      fs_set_error("the register-patch sweep kernel is not built for this shape (3, 6 or 10 "
+                   "ordinates per octant, the same in every octant; rows that fit a CTA)");
+      return FS_EARG;
+    }
+  }
   const bool oct = (want == 0 || want == 8) && octant_grouping(D) && plan_cl(D, D->force_C);
   if (oct && D->sweep_kernel == 2 && !plan_lc(D)) {
     fs_set_error("the lane-column sweep kernel is not built for this shape (ten ordinates per "
@@ -1454,7 +1621,6 @@ static int dom_prepare(DomCtx* D, cudaStream_t st) {
     D->Mo = D->M / 8;
     int slot = 0;
     for (int o = 0; o < 8; ++o) D->down_slot[o] = D->hoz[o * D->Mo] < 0.0 ? slot++ : -1;
-    const size_t ts = D->fp32 ? sizeof(float) : sizeof(double);
     cudaMalloc(&D->kb, 2 * ts * N);
     cudaMalloc(&D->Goct, ts * 8 * D->groups * N);
     cudaMalloc(&D->Qoct, ts * 8 * D->groups * n2);
@@ -1495,8 +1661,9 @@ int dom_set_mode(void* h, int mode, int cluster_ctas) {
 
 int dom_set_sweep_kernel(void* h, int kernel) {
   DomCtx* D = (DomCtx*)h;
-  if (kernel < 0 || kernel > 2) {
-    fs_set_error("sweep kernel %d: 0 (automatic), 1 (pencil per thread), 2 (lane column)", kernel);
+  if (kernel < 0 || kernel > 3) {
+    fs_set_error("sweep kernel %d: 0 (automatic), 1 (pencil per thread), 2 (lane column), "
+                 "3 (register patch)", kernel);
     return FS_EARG;
   }
   if (D->mode != 0) {
@@ -1508,7 +1675,7 @@ int dom_set_sweep_kernel(void* h, int kernel) {
 }
 int dom_sweep_kernel(void* h) {
   const DomCtx* D = (const DomCtx*)h;
-  return D->mode != 8 ? 0 : (D->cl_lane ? 2 : 1);
+  return D->mode != 8 ? 0 : (D->rp ? 3 : (D->cl_lane ? 2 : 1));
 }
 
 int dom_mode(void* h) { return ((DomCtx*)h)->mode; }
@@ -1551,13 +1718,31 @@ int dom_set_precision(void* h, int fp32) {
   return FS_OK;
 }
 
+static RpOct rp_octants(const DomCtx* D) {
+  RpOct o8;
+  for (int o = 0; o < 8; ++o) {
+    const int n = o * (D->M / 8);
+    o8.fx[o] = D->hox[n] >= 0.0; o8.fy[o] = D->hoy[n] >= 0.0; o8.fz[o] = D->hoz[n] >= 0.0;
+    o8.slot[o] = (signed char)D->down_slot[o];
+  }
+  return o8;
+}
+
 int dom_load_intensity(void* h, const double* I_full, cudaStream_t st) {
   DomCtx* D = (DomCtx*)h;
   int rc = dom_prepare(D, st);
   if (rc != FS_OK) return rc;
   const GridDev& g = D->g;
   const int64_t tot = (int64_t)D->M * g.nz * g.nx;
-  if (D->mode == 8) {
+  if (D->rp) {
+    double* rows = nullptr;  // M x Nz x Nx, then into the kernel's order
+    if (cudaMallocAsync(&rows, sizeof(double) * tot, st) != cudaSuccess) return cuda_status();
+    k_dom_extract_wrap<double><<<blocks_for(tot, 256), 256, 0, st>>>(g, D->M, D->oy, I_full, rows);
+    fs_count_launch();
+    rc = dom_set_wrap(h, rows, st);
+    cudaFreeAsync(rows, st);
+    if (rc != FS_OK) return rc;
+  } else if (D->mode == 8) {
     if (D->fp32)
       k_dom_extract_wrap<float><<<blocks_for(tot, 256), 256, 0, st>>>(g, D->M, D->oy, I_full,
                                                                      (float*)D->wrap);
@@ -1584,7 +1769,16 @@ int dom_get_wrap(void* h, double* dst, cudaStream_t st) {
   int rc = dom_prepare(D, st);
   if (rc != FS_OK) return rc;
   const int64_t tot = dom_wrap_size(h);
-  if (D->mode == 8 && D->fp32) {
+  if (D->rp) {
+    const int mow = rp_pad(D->fp32 ? 4 : 8, D->Mo);
+    if (D->fp32)
+      k_dom_wrap_copy<float, double><<<blocks_for(tot, 256), 256, 0, st>>>(
+          D->g, rp_octants(D), D->M, D->Mo, mow, (const float*)D->wrap, dst, 0);
+    else
+      k_dom_wrap_copy<double, double><<<blocks_for(tot, 256), 256, 0, st>>>(
+          D->g, rp_octants(D), D->M, D->Mo, mow, (const double*)D->wrap, dst, 0);
+    fs_count_launch();
+  } else if (D->mode == 8 && D->fp32) {
     k_convert<float, double><<<blocks_for(tot, 256), 256, 0, st>>>(tot, (const float*)D->wrap,
                                                                    dst);
     fs_count_launch();
@@ -1603,7 +1797,16 @@ int dom_set_wrap(void* h, const double* src, cudaStream_t st) {
   int rc = dom_prepare(D, st);
   if (rc != FS_OK) return rc;
   const int64_t tot = dom_wrap_size(h);
-  if (D->mode == 8 && D->fp32) {
+  if (D->rp) {
+    const int mow = rp_pad(D->fp32 ? 4 : 8, D->Mo);
+    if (D->fp32)
+      k_dom_wrap_copy<double, float><<<blocks_for(tot, 256), 256, 0, st>>>(
+          D->g, rp_octants(D), D->M, D->Mo, mow, src, (float*)D->wrap, 1);
+    else
+      k_dom_wrap_copy<double, double><<<blocks_for(tot, 256), 256, 0, st>>>(
+          D->g, rp_octants(D), D->M, D->Mo, mow, src, (double*)D->wrap, 1);
+    fs_count_launch();
+  } else if (D->mode == 8 && D->fp32) {
     k_convert<double, float><<<blocks_for(tot, 256), 256, 0, st>>>(tot, src, (float*)D->wrap);
     fs_count_launch();
   } else if (D->mode == 8) {
@@ -1636,6 +1839,13 @@ static double key_to_double(unsigned long long k) {
   double d;
   memcpy(&d, &k, sizeof(double));
   return d;
+}
+
+template <typename T2>
+static RpKb<T2> rp_kb(const DomCtx* D) {
+  RpKb<T2> o;
+  for (int q = 0; q < 4; ++q) o.kb[q] = (T2*)D->kb4[q];
+  return o;
 }
 
 static int launch_cl_sweep(DomCtx* D, const ClArgs& a, cudaStream_t st) {
@@ -1680,6 +1890,77 @@ static int launch_cl_sweep(DomCtx* D, const ClArgs& a, cudaStream_t st) {
   return e == cudaSuccess ? FS_OK : FS_ECUDA;
 }
 
+template <typename T, int MO, bool PAIR>
+static int launch_rp(DomCtx* D, const ClArgs& c, cudaStream_t st) {
+  using T2 = typename Vec2Of<T>::type;
+  using PT = RpPoints<MO>;
+  const GridDev& g = D->g;
+  RpArgs<T, MO> a{};
+  for (int q = 0; q < 4; ++q) a.kb[q] = (const T2*)D->kb4[q];
+  a.igA = (const T*)D->igA; a.igB = (const T*)D->igB;
+  a.Goct = (T*)D->Goct; a.Qoct = (T*)D->Qoct; a.wrap = (T*)D->wrap;
+  a.om = D->om;
+  a.dz0 = D->rp_dz0; a.zs = D->rp_zs;
+  a.I_amb = c.I_amb;
+  for (int m = 0; m < MO; ++m) {
+    const double ax = fabs(D->hox[m]) / g.dx, ay = fabs(D->hoy[m]) / g.dy;
+    const double az = fabs(D->hoz[m]) / D->rp_dz0;
+    a.ax[rp_digit(PT::X, m)] = (T)ax;
+    a.ay[rp_digit(PT::Y, m)] = (T)ay;
+    a.az[rp_digit(PT::Z, m)] = (T)az;
+    a.as[m] = (T)(ax + ay + az);
+    a.w[rp_digit(PT::W, m)] = (T)D->hw[m];
+    a.wq[m] = (T)(D->hw[m] * fabs(D->hoz[m]));
+  }
+  a.C = D->cl_C; a.rows = D->cl_rows; a.pitch = rp_pitch(g.ny);
+  const RpOct o8 = rp_octants(D);
+  for (int o = 0; o < 8; ++o) {
+    a.fx[o] = o8.fx[o]; a.fy[o] = o8.fy[o]; a.fz[o] = o8.fz[o]; a.slot[o] = o8.slot[o];
+  }
+  a.done = c.done; a.err = c.err; a.withhold = c.withhold;
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = D->cl_C; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
+  cfg.gridDim = dim3(8 * D->cl_C); cfg.blockDim = dim3(D->cl_threads);
+  cfg.dynamicSmemBytes = D->cl_smem; cfg.stream = st; cfg.attrs = at; cfg.numAttrs = 1;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, k_dom_octant_rp<T, MO, PAIR>, g, a);
+  fs_count_launch();
+  return e == cudaSuccess ? FS_OK : FS_ECUDA;
+}
+
+static int launch_rp_sweep(DomCtx* D, const ClArgs& c, cudaStream_t st) {
+  const bool f = D->fp32 != 0, p = D->rp_pair != 0;
+  switch (D->Mo) {
+    case 3: return f ? launch_rp<float, 3, false>(D, c, st)
+                     : p ? launch_rp<double, 3, true>(D, c, st) : launch_rp<double, 3, false>(D, c, st);
+    case 6: return f ? launch_rp<float, 6, false>(D, c, st)
+                     : p ? launch_rp<double, 6, true>(D, c, st) : launch_rp<double, 6, false>(D, c, st);
+    default: return f ? launch_rp<float, 10, false>(D, c, st)
+                      : p ? launch_rp<double, 10, true>(D, c, st) : launch_rp<double, 10, false>(D, c, st);
+  }
+}
+
+// the ground exchange on the skewed layouts (start: the solve's first intensity)
+static void launch_rp_ground(DomCtx* D, int start, double refl, const int* done, cudaStream_t st) {
+  const GridDev& g = D->g;
+  const unsigned nb = blocks_for((int64_t)g.nx * g.ny, 128);
+  const int pitch = rp_pitch(g.ny);
+  if (D->fp32)
+    k_dom_ground_skew<float><<<nb, 128, 0, st>>>(g, rp_octants(D), start, (const float*)D->Qoct,
+                                                 pitch, D->Isoil, refl, D->relax, D->Ig_out, D->qin,
+                                                 (float*)D->igA, (float*)D->igB, done);
+  else
+    k_dom_ground_skew<double><<<nb, 128, 0, st>>>(g, rp_octants(D), start, (const double*)D->Qoct,
+                                                  pitch, D->Isoil, refl, D->relax, D->Ig_out,
+                                                  D->qin, (double*)D->igA, (double*)D->igB, done);
+  fs_count_launch();
+}
+
+static dim3 rp_tiles(const GridDev& g) {
+  return dim3((g.nx + RP_T - 1) / RP_T, (g.ny + RP_T - 1) / RP_T, g.nz);
+}
+
 int dom_begin(void* h, const double* Ts, const double* Tg, const double* as, const double* om,
               double sigma, double T_amb, const double* Tsoil0, const double* YH,
               const double* rho, const double* Mloc, cudaStream_t st) {
@@ -1689,16 +1970,26 @@ int dom_begin(void* h, const double* Ts, const double* Tg, const double* as, con
   const GridDev& g = D->g;
   const int64_t N = ncells(g), n2 = (int64_t)g.nx * g.ny;
   const double Tamb4 = pow(T_amb, 4.0);
-  double2* kb = (D->mode == 8 && !D->fp32) ? (double2*)D->kb : nullptr;
-  float2* kb32 = (D->mode == 8 && D->fp32) ? (float2*)D->kb : nullptr;
-  k_dom_setup<<<blocks_for(N, 256), 256, 0, st>>>(g, Ts, Tg, as, om, YH, rho, Mloc, sigma, Tamb4,
-                                                  D->kgmax, D->ks, D->kg, D->ksafe, D->B, kb,
-                                                  kb32);
+  const DomSetupArgs sa{Ts, Tg, as, om, YH, rho, Mloc, sigma, Tamb4, D->kgmax};
+  if (D->rp) {
+    const int pitch = rp_pitch(g.ny);
+    if (D->fp32)
+      k_dom_setup_skew<float><<<rp_tiles(g), 256, 0, st>>>(
+          g, sa, D->ks, D->kg, D->ksafe, D->B, rp_kb<float2>(D), pitch);
+    else
+      k_dom_setup_skew<double><<<rp_tiles(g), 256, 0, st>>>(
+          g, sa, D->ks, D->kg, D->ksafe, D->B, rp_kb<double2>(D), pitch);
+  } else {
+    double2* kb = (D->mode == 8 && !D->fp32) ? (double2*)D->kb : nullptr;
+    float2* kb32 = (D->mode == 8 && D->fp32) ? (float2*)D->kb : nullptr;
+    k_dom_setup<<<blocks_for(N, 256), 256, 0, st>>>(g, sa, D->ks, D->kg, D->ksafe, D->B, kb, kb32);
+  }
   fs_count_launch();
   const double I_amb = SIGMA_SB_D * Tamb4 / PI_D;
   k_dom_ground_init<<<blocks_for(n2, 128), 128, 0, st>>>((int)n2, Tsoil0, D->eps_w, I_amb, D->Isoil,
                                                         D->Ig_out);
   fs_count_launch();
+  if (D->rp) launch_rp_ground(D, 1, 0.0, nullptr, st);
   D->pend_I_amb = I_amb;
   D->begun = 1;
   return cuda_status();
@@ -1751,11 +2042,21 @@ static int dom_iterate_dev(DomCtx* D, const ClArgs& base, int nslots, double ref
       ClArgs ca = base;
       ca.done = D->dstate;
       ca.err = D->dstate + 3;
-      int rc = launch_cl_sweep(D, ca, st);
+      int rc = D->rp ? launch_rp_sweep(D, ca, st) : launch_cl_sweep(D, ca, st);
       if (rc != FS_OK) return rc;
       if (D->timing) cudaEventRecord(D->ev1[queued], st);
       cudaMemsetAsync(D->keys, 0, sizeof(unsigned long long) * 2, st);
-      if (D->fp32) {
+      if (D->rp) {
+        if (D->fp32)
+          k_dom_G_skew<float><<<rp_tiles(g), 32 * RP_GW, 0, st>>>(g, rp_octants(D), (const float*)D->Goct,
+                                                           rp_pitch(g.ny), D->G, D->Gp, D->keys,
+                                                           D->dstate);
+        else
+          k_dom_G_skew<double><<<rp_tiles(g), 32 * RP_GW, 0, st>>>(g, rp_octants(D),
+                                                            (const double*)D->Goct, rp_pitch(g.ny),
+                                                            D->G, D->Gp, D->keys, D->dstate);
+        launch_rp_ground(D, 0, refl, D->dstate, st);
+      } else if (D->fp32) {
         k_dom_G_oct<float><<<nb, 256, 0, st>>>(N, nparts, (const float*)D->Goct, D->G, D->Gp,
                                                D->keys, D->dstate);
         k_dom_ground_oct<float><<<blocks_for(n2, 128), 128, 0, st>>>(

@@ -436,13 +436,18 @@ int fs_dom_set_sweep_mode(void* handle, int mode, int cluster_ctas);
 int fs_dom_set_octant_groups(void* handle, int groups);
 /* The path in use (0 before the first solve or intensity load). */
 int fs_dom_sweep_mode(void* handle);
-/* Path 8's kernel: 1 one pencil per thread (a hyperplane's intensities pass
- * through shared memory, one barrier over all pencil warps; the default, also
- * for 0), 2 lane column (a lane owns one y column of all of the CTA's k' rows
- * and keeps their intensities in registers, y-neighbours by warp shuffles;
- * built for ten ordinates per cluster, 4 to 8 rows per CTA and ny <= 128;
- * FS_EARG at the first solve for other shapes).  Both give the same results
- * bit for bit; the lane-column kernel is the slower one on the S8 workload
+/* Path 8's kernel: 0 automatic: 3 where the sweep path is automatic too (mode
+ * 0, one cluster per octant) and its shape fits, else 1; 1 one pencil per
+ * thread (a hyperplane's intensities pass through shared memory, one barrier
+ * over all pencil warps); 3 register patch (a thread keeps its pencils'
+ * intensities in registers, inputs and outputs lie by hyperplane; 3, 6 or 10
+ * ordinates per octant, the same level-symmetric set in every octant; FS_EARG at
+ * the first solve for other shapes): 0.91 ms per FP64 sweep of the S8 workload
+ * at 400 x 120 x 60 against kernel 1's 1.81; 2 lane column (a lane owns one y
+ * column of all of the CTA's k' rows and keeps their intensities in registers,
+ * y-neighbours by warp shuffles; built for ten ordinates per cluster, 4 to 8 rows per CTA and ny <= 128;
+ * FS_EARG at the first solve for other shapes).  All give the same results
+ * bit for bit; the lane-column kernel is the slowest one on the S8 workload
  * (3.85 ms per FP64 sweep at 400 x 120 x 60, about twice the other).  Only before the
  * first solve or intensity load.  fs_dom_sweep_kernel: the kernel in use (0
  * before the path is resolved or on path 3). */

@@ -509,7 +509,7 @@ def test_dom_s8_matches_reference(fp32):
 
 
 def _dom_solves(mode, fp32, nz, ny, nx, seed, calls=2, order=8, cluster_ctas=0, groups=0,
-                kernel=0, want_kernel=None):
+                kernel=0, want_kernel=None, want_mode=None):
     """q_rad_solid, q_rad_gas, q_in_soil after each of ``calls`` solves of an
     S_order DOM on seeded random fields (the y-inflow rows persist between calls);
     ``kernel`` picks path 8's sweep kernel (0 automatic, 1 pencil per thread,
@@ -546,7 +546,7 @@ def _dom_solves(mode, fp32, nz, ny, nx, seed, calls=2, order=8, cluster_ctas=0, 
             call("fs_dom_solve", h, ptr(Ts), ptr(Tg), ptr(a), ptr(omg), 5000.0, 300.0,
                  ptr(Tsoil), ptr(YH), ptr(rho), ptr(M), ptr(qs), ptr(qg), ptr(qsoil), stream())
             out.append((host(qs), host(qg), host(qsoil), lib().fs_dom_iterations(h)))
-        assert lib().fs_dom_sweep_mode(h) == mode
+        assert lib().fs_dom_sweep_mode(h) == (mode if want_mode is None else want_mode)
         if want_kernel is not None:
             assert lib().fs_dom_sweep_kernel(h) == want_kernel
     finally:
@@ -572,6 +572,28 @@ def test_dom_lane_column_kernel_equals_pencil_kernel(fp32, shape):
         assert ia == ib
         assert np.array_equal(qa, qb) and np.array_equal(ga, gb) and np.array_equal(sa, sb)
     assert np.array_equal(c[0][0], a[0][0])
+
+
+@pytest.mark.parametrize("fp32", [0, 1])
+@pytest.mark.parametrize("case", [((60, 120, 24), 8, 0), ((37, 70, 33), 8, 0), ((13, 7, 21), 8, 0),
+                                  ((29, 40, 48), 6, 5), ((23, 41, 97), 4, 0), ((2, 3, 5), 4, 0),
+                                  ((12, 33, 2), 6, 1), ((64, 128, 9), 8, 16)])
+def test_dom_register_patch_kernel_equals_pencil_kernel(fp32, case):
+    """Path 8's register-patch kernel (the automatic choice) gives the
+    pencil-per-thread kernel's results bit for bit, with the same source
+    iterations over three solves: full and partial last CTAs, warps and
+    patches, odd extents, rows shorter than the prefetch depth, one CTA per
+    octant and sixteen, levels of unequal height."""
+    (nz, ny, nx), order, cc = case
+    # one cluster per octant on both sides (two would sum G in halves)
+    a = _dom_solves(8, fp32, nz, ny, nx, seed=21, calls=3, order=order, groups=1, kernel=1,
+                    want_kernel=1)
+    mode = 8 if cc else 0
+    b = _dom_solves(mode, fp32, nz, ny, nx, seed=21, calls=3, order=order, cluster_ctas=cc,
+                    kernel=3 if cc else 0, want_kernel=3, want_mode=8)
+    for (qa, ga, sa, ia), (qb, gb, sb, ib) in zip(a, b):
+        assert ia == ib
+        assert np.array_equal(qa, qb) and np.array_equal(ga, gb) and np.array_equal(sa, sb)
 
 
 @pytest.mark.parametrize("fp32", [0, 1])
