@@ -32,8 +32,8 @@
 #define MG_OMEGA_DEFAULT 0.9  // damping of the V-cycle's smoothing sweeps
 #define MG_NU_DEFAULT 4
 #define MG_COARSE_MAX 48
-// blocks of the reducing CG kernels (8 per SM of the 148: enough loads in
-// flight to stream HBM); their partials are added in block order
+// blocks of the pointwise reducing kernels (8 per SM of the 148: enough loads in
+// flight to stream HBM)
 #define RED_BLOCKS 1184
 #define RED_THREADS 256
 // Device scalar slots: 0 rz, 1 pq, 2 rz_new, 4 ||b_A||^2, 5 ||r_A||^2,
@@ -58,12 +58,29 @@ inline Dims dims_make(int nx, int ny, int nz) {
   return D;
 }
 
+// The operator of a level >= 1: face conductances and the per-cell term.
+template <typename T>
+struct OpA {
+  const T *gx, *gy, *gz, *e;
+};
+// Level 0's, from the reciprocal density alone: a face conductance is a factor
+// of its direction and level times the sum of the two cells' 1/rho, so a sweep
+// reads one field where the stored form read four.  tab: OP_TAB factors a level
+// (x face, y face, z face above and below, the shift, the outlet and top faces).
+#define OP_TAB 8
+template <typename T>
+struct OpI {
+  const T *ir, *tab;
+};
+
 template <typename T>
 struct MGLevelT {
   int nx, ny, nz;
   Dims dims;
   int64_t n;
-  T *gx, *gy, *gz, *e, *dinv;  // conductances, per-cell term, 1/diag
+  // conductances and per-cell term (levels >= 1; level 0 only when it is the
+  // coarsest), 1/diag
+  T *gx, *gy, *gz, *e, *dinv;
   T *x, *b, *t, *s;            // correction, rhs, temps
 };
 using MGLevel = MGLevelT<double>;
@@ -76,13 +93,16 @@ struct ProjCtx {
   double* pc_r;       // PCG residual (level 0)
   double* pc_z;
   double* pc_p;
+  double* pc_p2;      // the directions of odd iterations
   double* pc_q;
   double* rhs;        // b_S
-  double* partial;    // block partial sums [RED_BLOCKS * 4]
+  double* partial;    // block partial sums
   double* scal;       // device scalars
   double* h_scal;     // pinned host mirror
   double* p_prev;     // warm start / solution (owned)
   double* ir;         // 1/max(rho, 0.01)
+  double* tab;        // level 0's factors (OP_TAB per level)
+  float *ir32, *tab32;
   int have_prev;
   int last_iters;     // CG iterations of the previous solve (batch size hint)
   cudaStream_t cs;    // private stream for graph capture
@@ -116,54 +136,65 @@ struct ProjCtx {
 };
 
 // ---------------------------------------------------------------------------
-__global__ void k_proj_level0(GridDev g, const double* __restrict__ rho, double* ir, double* gx,
-                              double* gy, double* gz, double* e, double dx2, double dy2) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  int j = blockIdx.y * blockDim.y + threadIdx.y;
-  int k = blockIdx.z;
-  if (i >= g.nx || j >= g.ny) return;
-  const int nx = g.nx, ny = g.ny, nz = g.nz;
-  const int64_t sy = nx, sz = (int64_t)nx * ny;
-  int64_t c = cidx(g, k, j, i);
-  auto IR = [&](int64_t q) {
-    double r = rho[q];
-    double m = (r >= 0.01 || r != r) ? r : 0.01;
-    return 1.0 / m;
-  };
-  double irc = IR(c);
-  ir[c] = irc;
-  const double dzk = g.dz[k];
-  const double idz = 1.0 / dzk;
-  double ee = -dzk * PROJ_EPS;
-  // x faces
-  if (i < nx - 1) {
-    gx[c] = dzk * ((0.5 * (irc + IR(c + 1))) / dx2);
-  } else {
-    gx[c] = 0.0;
-    ee += dzk * ((2.0 * irc) / dx2);
+// 1/rho (floored) and, by the first block, level 0's factors
+template <typename T>
+__global__ void k_proj_ir(GridDev g, const double* __restrict__ rho, double* ir, T* irT, double* tab,
+                          T* tabT, double dx2, double dy2) {
+  const int64_t n = ncells_dev(g);
+  const int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (blockIdx.x == 0) {
+    for (int k = threadIdx.x; k < g.nz; k += blockDim.x) {
+      const double dz = g.dz[k];
+      const double v[OP_TAB] = {dz * (0.5 / dx2), dz * (0.5 / dy2), 0.5 / g.da[k],
+                                k > 0 ? 0.5 / g.da[k - 1] : 0.0, -dz * PROJ_EPS, dz * (2.0 / dx2),
+                                2.0 / dz, 0.0};
+      for (int q = 0; q < OP_TAB; ++q) {
+        tab[k * OP_TAB + q] = v[q];
+        if (tabT) tabT[k * OP_TAB + q] = (T)v[q];
+      }
+    }
   }
-  // y faces (periodic); Ny == 1 has no y coupling (projection_3d.py:128)
-  if (ny > 1) {
-    int jp = j + 1 < ny ? j + 1 : 0;
-    gy[c] = dzk * ((0.5 * (irc + IR(c - (int64_t)j * sy + (int64_t)jp * sy))) / dy2);
-  } else {
-    gy[c] = 0.0;
-  }
-  // z faces
-  if (k < nz - 1) {
-    gz[c] = dzk * (((0.5 * (irc + IR(c + sz))) * idz) / g.da[k]);
-  } else {
-    gz[c] = 0.0;
-    ee += dzk * (((2.0 * irc) * idz) * idz);
-  }
-  e[c] = ee;
+  if (c >= n) return;
+  const double r = rho[c];
+  const double m = (r >= 0.01 || r != r) ? r : 0.01;
+  const double v = 1.0 / m;
+  ir[c] = v;
+  if (irT) irT[c] = (T)v;
 }
 
-// diagonal of a face-conductance operator -> 1/diag
+// the operator's parts: conductance of the face towards +x, +y, +z of cell c
+// (0 where there is none) and the per-cell term
 template <typename T>
-__global__ void k_mg_diag(Dims D, const T* __restrict__ gx,
-                          const T* __restrict__ gy, const T* __restrict__ gz,
-                          const T* __restrict__ e, T* dinv) {
+__device__ __forceinline__ T op_fx(const OpA<T>& o, int64_t c, int, int, int) { return o.gx[c]; }
+template <typename T>
+__device__ __forceinline__ T op_fy(const OpA<T>& o, int64_t c, int64_t, int) { return o.gy[c]; }
+template <typename T>
+__device__ __forceinline__ T op_fz(const OpA<T>& o, int64_t c, int64_t, int, int) { return o.gz[c]; }
+template <typename T>
+__device__ __forceinline__ T op_e(const OpA<T>& o, int64_t c, int, int, int, int) { return o.e[c]; }
+template <typename T>
+__device__ __forceinline__ T op_fx(const OpI<T>& o, int64_t c, int i, int k, int nx) {
+  return i < nx - 1 ? o.tab[k * OP_TAB] * (o.ir[c] + o.ir[c + 1]) : T(0);
+}
+template <typename T>
+__device__ __forceinline__ T op_fy(const OpI<T>& o, int64_t c, int64_t cp, int k) {
+  return o.tab[k * OP_TAB + 1] * (o.ir[c] + o.ir[cp]);
+}
+template <typename T>
+__device__ __forceinline__ T op_fz(const OpI<T>& o, int64_t c, int64_t sz, int k, int nz) {
+  return k < nz - 1 ? o.tab[k * OP_TAB + 2] * (o.ir[c] + o.ir[c + sz]) : T(0);
+}
+template <typename T>
+__device__ __forceinline__ T op_e(const OpI<T>& o, int64_t c, int i, int k, int nx, int nz) {
+  T e = o.tab[k * OP_TAB + 4];
+  if (i == nx - 1) e += o.tab[k * OP_TAB + 5] * o.ir[c];
+  if (k == nz - 1) e += o.tab[k * OP_TAB + 6] * o.ir[c];
+  return e;
+}
+
+// diagonal of the operator -> 1/diag
+template <typename T, typename Op>
+__global__ void k_mg_diag(Dims D, Op o, T* dinv) {
   const int nx = D.nx, ny = D.ny, nz = D.nz;
   int64_t n = (int64_t)nx * ny * nz;
   int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
@@ -171,48 +202,114 @@ __global__ void k_mg_diag(Dims D, const T* __restrict__ gx,
   int i, j, k;
   split_cell((uint32_t)c, D.fnx, D.fny, i, j, k);
   int64_t sy = nx, sz = (int64_t)nx * ny;
-  T d = e[c] + gx[c] + gy[c] + gz[c];
-  if (i > 0) d += gx[c - 1];
+  T d = op_e(o, c, i, k, nx, nz) + op_fx(o, c, i, k, nx);
   if (ny > 1) {
-    int jm = j > 0 ? j - 1 : ny - 1;
-    d += gy[c - (int64_t)j * sy + (int64_t)jm * sy];
+    int jp = j + 1 < ny ? j + 1 : 0, jm = j > 0 ? j - 1 : ny - 1;
+    const int64_t r = c - (int64_t)j * sy;
+    d += op_fy(o, c, r + (int64_t)jp * sy, k);
+    d += op_fy(o, r + (int64_t)jm * sy, c, k);
   }
-  if (k > 0) d += gz[c - sz];
+  d += op_fz(o, c, sz, k, nz);
+  if (i > 0) d += op_fx(o, c - 1, i - 1, k, nx);
+  if (k > 0) d += op_fz(o, c - sz, sz, k - 1, nz);
   dinv[c] = T(1) / d;
 }
 
-// (S x)_c for a face-conductance operator
+// level 0's operator as arrays (only where level 0 is the coarsest level)
 template <typename T>
-__device__ __forceinline__ T mg_apply(int nx, int ny, int nz, const T* __restrict__ gx,
-                                           const T* __restrict__ gy,
-                                           const T* __restrict__ gz,
-                                           const T* __restrict__ e,
-                                           const T* __restrict__ x, int64_t c, int i, int j,
-                                           int k) {
-  const int64_t sy = nx, sz = (int64_t)nx * ny;
-  const T xc = x[c];
-  T y = e[c] * xc;
-  if (i < nx - 1) y += gx[c] * (xc - x[c + 1]);
-  if (i > 0) y += gx[c - 1] * (xc - x[c - 1]);
+__global__ void k_op_arrays(Dims D, OpI<T> o, T* gx, T* gy, T* gz, T* e) {
+  const int64_t n = (int64_t)D.nx * D.ny * D.nz, sz = (int64_t)D.nx * D.ny;
+  const int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (c >= n) return;
+  int i, j, k;
+  split_cell((uint32_t)c, D.fnx, D.fny, i, j, k);
+  const int jp = j + 1 < D.ny ? j + 1 : 0;
+  gx[c] = op_fx(o, c, i, k, D.nx);
+  gy[c] = D.ny > 1 ? op_fy(o, c, c + (int64_t)(jp - j) * D.nx, k) : T(0);
+  gz[c] = op_fz(o, c, sz, k, D.nz);
+  e[c] = op_e(o, c, i, k, D.nx, D.nz);
+}
+
+__device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
+__device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, b); }
+
+// A vector the operator is applied to, cell by cell: stored; the first sweep's
+// iterate from x = 0, w b / d; an iterate plus the prolonged coarse correction
+// (piecewise constant).  The latter two are formed where they are read, so
+// neither the first sweep nor the prolongation is a pass of its own.
+template <typename T>
+struct VecX {
+  const T* x;
+  __device__ __forceinline__ T at(int c, int, int, int) const { return x[c]; }
+};
+template <typename T>
+struct VecFirst {
+  const T *b, *dinv;
+  T w;
+  // (rounded as the stored value would be: no product left to contract)
+  __device__ __forceinline__ T at(int c, int, int, int) const {
+    return mul_rn(w * b[c], dinv[c]);
+  }
+};
+template <typename T>
+struct VecProl {
+  const T *x, *xc;
+  int cx, cy;
+  __device__ __forceinline__ T at(int c, int i, int j, int k) const {
+    return x[c] + xc[((k >> 1) * cy + (j >> 1)) * cx + (i >> 1)];
+  }
+};
+
+// (S x)_c; xc = x_c
+template <typename T, typename V>
+__device__ __forceinline__ T mg_apply(int nx, int ny, int nz, const OpA<T>& o, const V& x, T xc,
+                                      int c, int i, int j, int k) {
+  const int sy = nx, sz = nx * ny;
+  T y = o.e[c] * xc;
+  if (i < nx - 1) y += o.gx[c] * (xc - x.at(c + 1, i + 1, j, k));
+  if (i > 0) y += o.gx[c - 1] * (xc - x.at(c - 1, i - 1, j, k));
   if (ny > 1) {
     int jp = j + 1 < ny ? j + 1 : 0;
     int jm = j > 0 ? j - 1 : ny - 1;
-    int64_t cp = c - (int64_t)j * sy + (int64_t)jp * sy;
-    int64_t cm = c - (int64_t)j * sy + (int64_t)jm * sy;
-    y += gy[c] * (xc - x[cp]);
-    y += gy[cm] * (xc - x[cm]);
+    int cp = c + (jp - j) * sy;
+    int cm = c + (jm - j) * sy;
+    y += o.gy[c] * (xc - x.at(cp, i, jp, k));
+    y += o.gy[cm] * (xc - x.at(cm, i, jm, k));
   }
-  if (k < nz - 1) y += gz[c] * (xc - x[c + sz]);
-  if (k > 0) y += gz[c - sz] * (xc - x[c - sz]);
+  if (k < nz - 1) y += o.gz[c] * (xc - x.at(c + sz, i, j, k + 1));
+  if (k > 0) y += o.gz[c - sz] * (xc - x.at(c - sz, i, j, k - 1));
+  return y;
+}
+template <typename T, typename V>
+__device__ __forceinline__ T mg_apply(int nx, int ny, int nz, const OpI<T>& o, const V& x, T xc,
+                                      int c, int i, int j, int k) {
+  const int sy = nx, sz = nx * ny;
+  const T* __restrict__ ir = o.ir;
+  const T* __restrict__ tb = o.tab + k * OP_TAB;
+  const T r = ir[c], hx = tb[0], hy = tb[1];
+  T e = tb[4];
+  if (i == nx - 1) e += tb[5] * r;
+  if (k == nz - 1) e += tb[6] * r;
+  T y = e * xc;
+  if (i < nx - 1) y += hx * (r + ir[c + 1]) * (xc - x.at(c + 1, i + 1, j, k));
+  if (i > 0) y += hx * (r + ir[c - 1]) * (xc - x.at(c - 1, i - 1, j, k));
+  if (ny > 1) {
+    int jp = j + 1 < ny ? j + 1 : 0;
+    int jm = j > 0 ? j - 1 : ny - 1;
+    int cp = c + (jp - j) * sy;
+    int cm = c + (jm - j) * sy;
+    y += hy * (r + ir[cp]) * (xc - x.at(cp, i, jp, k));
+    y += hy * (r + ir[cm]) * (xc - x.at(cm, i, jm, k));
+  }
+  if (k < nz - 1) y += tb[2] * (r + ir[c + sz]) * (xc - x.at(c + sz, i, j, k + 1));
+  if (k > 0) y += tb[3] * (r + ir[c - sz]) * (xc - x.at(c - sz, i, j, k - 1));
   return y;
 }
 
 // Galerkin aggregation of level f into level c (coarse = scale * P^T S_f P)
-template <typename T>
-__global__ void k_mg_coarsen(int fx, int fy, int fz, const T* __restrict__ gxf,
-                             const T* __restrict__ gyf, const T* __restrict__ gzf,
-                             const T* __restrict__ ef, Dims DC, T* gxc,
-                             T* gyc, T* gzc, T* ec, double scale_) {
+template <typename T, typename Op>
+__global__ void k_mg_coarsen(int fx, int fy, int fz, Op o, Dims DC, T* gxc, T* gyc, T* gzc, T* ec,
+                             double scale_) {
   const int cx = DC.nx, cy = DC.ny, cz = DC.nz;
   int64_t n = (int64_t)cx * cy * cz;
   int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
@@ -226,18 +323,24 @@ __global__ void k_mg_coarsen(int fx, int fy, int fz, const T* __restrict__ gxf,
   T se = 0.0, sx = 0.0, sy = 0.0, sz = 0.0;
   for (int k = k0; k <= k1; ++k)
     for (int j = j0; j <= j1; ++j)
-      for (int i = i0; i <= i1; ++i) se += ef[(int64_t)k * fsz + (int64_t)j * fsy + i];
+      for (int i = i0; i <= i1; ++i)
+        se += op_e(o, (int64_t)k * fsz + (int64_t)j * fsy + i, i, k, fx, fz);
   if (I < cx - 1) {
     for (int k = k0; k <= k1; ++k)
-      for (int j = j0; j <= j1; ++j) sx += gxf[(int64_t)k * fsz + (int64_t)j * fsy + i1];
+      for (int j = j0; j <= j1; ++j)
+        sx += op_fx(o, (int64_t)k * fsz + (int64_t)j * fsy + i1, i1, k, fx);
   }
   if (cy > 1) {
+    const int jp = j1 + 1 < fy ? j1 + 1 : 0;
     for (int k = k0; k <= k1; ++k)
-      for (int i = i0; i <= i1; ++i) sy += gyf[(int64_t)k * fsz + (int64_t)j1 * fsy + i];
+      for (int i = i0; i <= i1; ++i)
+        sy += op_fy(o, (int64_t)k * fsz + (int64_t)j1 * fsy + i,
+                    (int64_t)k * fsz + (int64_t)jp * fsy + i, k);
   }
   if (K < cz - 1) {
     for (int j = j0; j <= j1; ++j)
-      for (int i = i0; i <= i1; ++i) sz += gzf[(int64_t)k1 * fsz + (int64_t)j * fsy + i];
+      for (int i = i0; i <= i1; ++i)
+        sz += op_fz(o, (int64_t)k1 * fsz + (int64_t)j * fsy + i, fsz, k1, fz);
   }
   const T scale = (T)scale_;
   gxc[q] = scale * sx;
@@ -254,9 +357,7 @@ __global__ void k_mg_coarse_inverse(int nx, int ny, int nz, const T* __restrict_
   __shared__ T M[MG_COARSE_MAX][2 * MG_COARSE_MAX + 1];
   const int n = nx * ny * nz;
   const int t = threadIdx.x;
-  for (int r = t; r < n; r += blockDim.x) {
-    for (int q = 0; q < 2 * n; ++q) M[r][q] = 0.0;
-  }
+  for (int e_ = t; e_ < n * 2 * n; e_ += blockDim.x) M[e_ / (2 * n)][e_ % (2 * n)] = 0.0;
   __syncthreads();
   if (t == 0) {
     const int sy = nx, sz = nx * ny;
@@ -277,21 +378,25 @@ __global__ void k_mg_coarse_inverse(int nx, int ny, int nz, const T* __restrict_
     }
   }
   __syncthreads();
+  // a warp takes whole rows (the columns are its lanes), so a pivot step is a few
+  // shared-memory operations deep; with a thread per row it was 2 n deep (149 us
+  // for 48 cells, 16 now)
+  const int lane = t & 31, wid = t >> 5, nwarps = blockDim.x >> 5;
   for (int piv = 0; piv < n; ++piv) {
-    T d = M[piv][piv];
+    const T d = M[piv][piv];
     __syncthreads();
     for (int q = t; q < 2 * n; q += blockDim.x) M[piv][q] /= d;
     __syncthreads();
-    for (int r = t; r < n; r += blockDim.x) {
+    for (int r = wid; r < n; r += nwarps) {
       if (r == piv) continue;
-      T f = M[r][piv];
+      const T f = M[r][piv];
+      __syncwarp();
       if (f != 0.0)
-        for (int q = 0; q < 2 * n; ++q) M[r][q] -= f * M[piv][q];
+        for (int q = lane; q < 2 * n; q += 32) M[r][q] -= f * M[piv][q];
     }
     __syncthreads();
   }
-  for (int r = t; r < n; r += blockDim.x)
-    for (int q = 0; q < n; ++q) Ainv[r * n + q] = M[r][n + q];
+  for (int e_ = t; e_ < n * n; e_ += blockDim.x) Ainv[e_] = M[e_ / n][n + e_ % n];
 }
 
 template <typename T>
@@ -305,37 +410,36 @@ __global__ void k_mg_coarse_solve(int n, const T* __restrict__ Ainv,
   x[r] = s;
 }
 
-// damped Jacobi sweep: xo = x + w (b - S x) / d ; x == null means x = 0
-template <typename T>
-__global__ void k_mg_jacobi(Dims D, const T* __restrict__ gx,
-                            const T* __restrict__ gy, const T* __restrict__ gz,
-                            const T* __restrict__ e, const T* __restrict__ dinv,
-                            const T* __restrict__ b, const T* __restrict__ x, T* xo,
-                            double w_, const double* done) {
+// damped Jacobi sweep: xo = x + w (b - S x) / d
+template <typename T, typename Op, typename V>
+__global__ void k_mg_jacobi(Dims D, Op o, const T* __restrict__ dinv, const T* __restrict__ b, V x,
+                            T* xo, double w_, const double* done) {
   PCG_SKIP(done);
   const int nx = D.nx, ny = D.ny, nz = D.nz;
   const T w = (T)w_;
   int64_t n = (int64_t)nx * ny * nz;
   int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (c >= n) return;
-  if (!x) {
-    xo[c] = w * b[c] * dinv[c];
-    return;
-  }
   int i, j, k;
   split_cell((uint32_t)c, D.fnx, D.fny, i, j, k);
-  T r = b[c] - mg_apply(nx, ny, nz, gx, gy, gz, e, x, c, i, j, k);
-  xo[c] = x[c] + w * r * dinv[c];
+  const T xc = x.at(c, i, j, k);
+  T r = b[c] - mg_apply(nx, ny, nz, o, x, xc, c, i, j, k);
+  xo[c] = xc + w * r * dinv[c];
+}
+// the first sweep from x = 0 alone (where it is the only one)
+template <typename T>
+__global__ void k_mg_first(int64_t n, const T* __restrict__ dinv, const T* __restrict__ b, T* xo,
+                           double w_, const double* done) {
+  PCG_SKIP(done);
+  int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (c < n) xo[c] = (T)w_ * b[c] * dinv[c];
 }
 
 // coarse rhs = sum over children of the fine residual (b - S x)
-template <typename T>
-__global__ void k_mg_restrict_residual(Dims DF, const T* __restrict__ gx,
-                                       const T* __restrict__ gy,
-                                       const T* __restrict__ gz,
-                                       const T* __restrict__ e, const T* __restrict__ b,
-                                       const T* __restrict__ x, Dims DC,
-                                       T* bc, const double* done) {
+template <typename T, typename Op>
+__global__ void k_mg_restrict_residual(Dims DF, Op o, const T* __restrict__ b,
+                                       const T* __restrict__ x, Dims DC, T* bc,
+                                       const double* done) {
   PCG_SKIP(done);
   const int fx = DF.nx, fy = DF.ny, fz = DF.nz;
   const int cx = DC.nx, cy = DC.ny, cz = DC.nz;
@@ -345,27 +449,21 @@ __global__ void k_mg_restrict_residual(Dims DF, const T* __restrict__ gx,
   int I, J, K;
   split_cell((uint32_t)q, DC.fnx, DC.fny, I, J, K);
   const int64_t fsy = fx, fsz = (int64_t)fx * fy;
+  const VecX<T> X{x};
   T s = 0.0;
-  for (int k = 2 * K; k <= min(2 * K + 1, fz - 1); ++k)
-    for (int j = 2 * J; j <= min(2 * J + 1, fy - 1); ++j)
-      for (int i = 2 * I; i <= min(2 * I + 1, fx - 1); ++i) {
-        int64_t c = (int64_t)k * fsz + (int64_t)j * fsy + i;
-        s += b[c] - mg_apply(fx, fy, fz, gx, gy, gz, e, x, c, i, j, k);
+#pragma unroll
+  for (int dk = 0; dk < 2; ++dk)
+#pragma unroll
+    for (int dj = 0; dj < 2; ++dj)
+#pragma unroll
+      for (int di = 0; di < 2; ++di) {
+        const int k = 2 * K + dk, j = 2 * J + dj, i = 2 * I + di;
+        if (k < fz && j < fy && i < fx) {
+          int64_t c = (int64_t)k * fsz + (int64_t)j * fsy + i;
+          s += b[c] - mg_apply(fx, fy, fz, o, X, x[c], c, i, j, k);
+        }
       }
   bc[q] = s;
-}
-
-// x_f += P x_c (piecewise constant)
-template <typename T>
-__global__ void k_mg_prolong(Dims DF, T* x, int cx, int cy,
-                             const T* __restrict__ xc, const double* done) {
-  PCG_SKIP(done);
-  int64_t n = (int64_t)DF.nx * DF.ny * DF.nz;
-  int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (c >= n) return;
-  int i, j, k;
-  split_cell((uint32_t)c, DF.fnx, DF.fny, i, j, k);
-  x[c] += xc[((int64_t)(k >> 1) * cy + (j >> 1)) * cx + (i >> 1)];
 }
 
 // ---------------------------------------------------------------------------
@@ -376,159 +474,366 @@ __device__ __forceinline__ double warp_sum(double v) {
   return v;
 }
 
-template <int NV>
-__device__ __forceinline__ void block_sums_store(double (&v)[NV], double* partial) {
-  __shared__ double sh[NV][32];
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-#pragma unroll
-  for (int q = 0; q < NV; ++q) {
-    double s = warp_sum(v[q]);
-    if (lane == 0) sh[q][wid] = s;
-  }
+// A kernel's sum: every block leaves its partial, and one small block adds them
+// in block order and does the scalar work that follows (post).  (Adding them in
+// the kernel's own last block, found by a ticket, took 25 us more at the 5850
+// blocks of level 0's tiles: the tickets queue at one address.)
+#define POST_NONE 0
+#define POST_DIR 1    // rz of this iteration becomes the old one (slot 0 = slot 2)
+#define POST_CHECK 2  // end of a PCG iteration: count it, ||r_A|| < rtol ||b_A||
+#define FIN_THREADS 1024
+__device__ __forceinline__ double block_sum(double v, double* sh) {
+  const int tid = (threadIdx.z * blockDim.y + threadIdx.y) * blockDim.x + threadIdx.x;
+  const int lane = tid & 31, wid = tid >> 5;
+  v = warp_sum(v);
+  if (lane == 0) sh[wid] = v;
   __syncthreads();
-  if (wid == 0) {
-#pragma unroll
-    for (int q = 0; q < NV; ++q) {
-      double s = lane < (blockDim.x >> 5) ? sh[q][lane] : 0.0;
-      s = warp_sum(s);
-      if (lane == 0) partial[q * RED_BLOCKS + blockIdx.x] = s;
+  double s = 0.0;
+  const int nw = (int)(blockDim.x * blockDim.y * blockDim.z) >> 5;
+  if (wid == 0) s = warp_sum(lane < nw ? sh[lane] : 0.0);
+  return s;  // in thread 0
+}
+__device__ __forceinline__ void store_partial(double v, double* partial) {
+  __shared__ double sh[32];
+  const double s = block_sum(v, sh);
+  if ((threadIdx.x | threadIdx.y | threadIdx.z) == 0)
+    partial[blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z)] = s;
+}
+__global__ void __launch_bounds__(FIN_THREADS)
+    k_finish_sum(const double* __restrict__ partial, int nb, double* scal, int slot, int post,
+                 const double* done) {
+  PCG_SKIP(done);
+  __shared__ double sh[32];
+  double t = 0.0;
+  for (int q = threadIdx.x; q < nb; q += FIN_THREADS) t += partial[q];
+  t = block_sum(t, sh);
+  if (threadIdx.x == 0) {
+    scal[slot] = t;
+    if (post == POST_DIR) scal[0] = scal[2];
+    if (post == POST_CHECK) {
+      scal[SC_IT] += 1.0;
+      if (t < scal[6]) scal[SC_DONE] = 1.0;
     }
   }
-}
-
-__global__ void k_finish_sums(const double* __restrict__ partial, int nv, double* out,
-                              const double* done) {
-  PCG_SKIP(done);
-  int q = threadIdx.x >> 5;
-  int lane = threadIdx.x & 31;
-  if (q >= nv) return;
-  double s = 0.0;
-  for (int b = lane; b < RED_BLOCKS; b += 32) s += partial[q * RED_BLOCKS + b];
-  s = warp_sum(s);
-  if (lane == 0) out[q] = s;
 }
 
 // rhs: b_S = -dz_k (div - target)/dt, plus ||(div - target)/dt||^2
 __global__ void k_proj_rhs(GridDev g, const double* __restrict__ u, const double* __restrict__ v,
                            const double* __restrict__ w, const double* __restrict__ u_in,
-                           const double* __restrict__ target, double dt, double* bS,
-                           double* partial) {
+                           const double* __restrict__ target, double inv_dx, double inv_dy,
+                           double inv_dt, double* bS, double* partial) {
   const int64_t n = ncells_dev(g);
   const int nx = g.nx, ny = g.ny;
   const int64_t sy = nx, sz = (int64_t)nx * ny;
-  double acc[1] = {0.0};
+  double acc = 0.0;
   for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < n;
-       c += (int64_t)RED_BLOCKS * blockDim.x) {
+       c += (int64_t)gridDim.x * blockDim.x) {
     int i, j, k;
     split_cell((uint32_t)c, g.fnx, g.fny, i, j, k);
-    double div;
-    if (i > 0) div = (u[c] - u[c - 1]) / g.dx;
-    else div = (u[c] - u_in[(int64_t)k * ny + j]) / g.dx;
+    const double dz = g.dz[k];
+    const double ul = i > 0 ? u[c - 1] : u_in[(int64_t)k * ny + j];
+    double div = (u[c] - ul) * inv_dx;
     if (ny > 1) {
       int jm = j > 0 ? j - 1 : ny - 1;
-      div += (v[c] - v[c - (int64_t)j * sy + (int64_t)jm * sy]) / g.dy;
+      div += (v[c] - v[c - (int64_t)j * sy + (int64_t)jm * sy]) * inv_dy;
     }
-    if (k > 0) div += (w[c] - w[c - sz]) / g.dz[k];
-    else div += (w[c] - 0.0) / g.dz[0];
+    div += (w[c] - (k > 0 ? w[c - sz] : 0.0)) / dz;
     if (target) div = div - target[c];
-    double rA = div / dt;
-    bS[c] = -g.dz[k] * rA;
-    acc[0] += rA * rA;
+    const double rA = div * inv_dt;
+    bS[c] = -dz * rA;
+    acc += rA * rA;
   }
-  block_sums_store<1>(acc, partial);
+  store_partial(acc, partial);
 }
 
-// q = S p and partial of p.q
-__global__ void k_pcg_matvec(Dims D, const double* __restrict__ gx,
-                             const double* __restrict__ gy, const double* __restrict__ gz,
-                             const double* __restrict__ e, const double* __restrict__ p, double* q,
-                             double* partial, const double* done) {
-  PCG_SKIP(done);
+// ---------------------------------------------------------------------------
+// Level 0's kernels: blocks of consecutive cells, W = 2 neighbours in x a thread
+// where nx is even (every row then starts on a pair), one where it is odd.  The
+// load/store unit bounds them: a sweep of single cells takes 57 wavefronts for
+// 32 cells and 31.7 us at 400 x 120 x 60; pairs loaded as one vector, with the
+// x-neighbours taken from the lanes beside, take as many for 64.
+// ---------------------------------------------------------------------------
+#define Z_THREADS 256
+template <typename T>
+struct alignas(2 * sizeof(T)) Two {
+  T a, b;
+};
+template <typename T>
+__device__ __forceinline__ Two<T> ld2(const T* p) {
+  return *(const Two<T>*)p;
+}
+template <typename T>
+__device__ __forceinline__ Two<T> at2(const VecX<T>& x, int c, int, int, int) {
+  return ld2(x.x + c);
+}
+template <typename T>
+__device__ __forceinline__ Two<T> at2(const VecFirst<T>& x, int c, int, int, int) {
+  const Two<T> b = ld2(x.b + c), d = ld2(x.dinv + c);
+  return {mul_rn(x.w * b.a, d.a), mul_rn(x.w * b.b, d.b)};
+}
+template <typename T>
+__device__ __forceinline__ Two<T> at2(const VecProl<T>& x, int c, int i, int j, int k) {
+  const Two<T> v = ld2(x.x + c);
+  const T e = x.xc[((k >> 1) * x.cy + (j >> 1)) * x.cx + (i >> 1)];
+  return {v.a + e, v.b + e};
+}
+// The search direction where it is read: z + beta p (p the last direction;
+// first iteration z).  Z: the type the preconditioner leaves z in.
+template <typename Z>
+struct VecDir {
+  const Z* z;
+  const double* p;
+  double beta;
+  __device__ __forceinline__ double at(int c, int, int, int) const {
+    return beta == 0.0 ? (double)z[c] : (double)z[c] + beta * p[c];
+  }
+};
+template <typename Z>
+__device__ __forceinline__ Two<double> at2(const VecDir<Z>& x, int c, int, int, int) {
+  const Two<Z> z = ld2(x.z + c);
+  if (x.beta == 0.0) return {(double)z.a, (double)z.b};
+  const Two<double> p = ld2(x.p + c);
+  return {(double)z.a + x.beta * p.a, (double)z.b + x.beta * p.b};
+}
+
+// a thread's W cells: the first of them (all threads get one, for the shuffles;
+// in: it is theirs)
+struct ZCell {
+  int c, i, j, k;
+  bool in;
+};
+template <int W>
+__device__ __forceinline__ ZCell z_cell(const Dims& D) {
+  const int n = D.nx * D.ny * D.nz;
+  ZCell z;
+  z.c = (int)(blockIdx.x * Z_THREADS + threadIdx.x) * W;
+  z.in = z.c < n;
+  if (!z.in) z.c = n - W;
+  split_cell((uint32_t)z.c, D.fnx, D.fny, z.i, z.j, z.k);
+  return z;
+}
+inline int z_width(const Dims& D) { return D.nx % 2 == 0 ? 2 : 1; }
+inline int z_blocks(const Dims& D) {
+  const int w = z_width(D);
+  return (int)(((int64_t)D.nx * D.ny * D.nz / w + Z_THREADS - 1) / Z_THREADS);
+}
+
+// x and S x at W cells
+template <int W, typename T, typename V>
+__device__ __forceinline__ void z_apply(const Dims& D, const OpI<T>& o, const V& x, int c, int i,
+                                        int j, int k, T (&xc)[W], T (&y)[W]) {
   const int nx = D.nx, ny = D.ny, nz = D.nz;
-  const int64_t n = (int64_t)nx * ny * nz;
-  double acc[1] = {0.0};
-  for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < n;
-       c += (int64_t)RED_BLOCKS * blockDim.x) {
-    int i, j, k;
-    split_cell((uint32_t)c, D.fnx, D.fny, i, j, k);
-    double y = mg_apply(nx, ny, nz, gx, gy, gz, e, p, c, i, j, k);
-    q[c] = y;
-    acc[0] += p[c] * y;
+  if constexpr (W == 1) {
+    xc[0] = x.at(c, i, j, k);
+    y[0] = mg_apply(nx, ny, nz, o, x, xc[0], c, i, j, k);
+  } else {
+    const int sy = nx, sz = nx * ny, lane = threadIdx.x & 31;
+    const T* __restrict__ ir = o.ir;
+    const T* __restrict__ tb = o.tab + k * OP_TAB;
+    const int jp = j + 1 < ny ? j + 1 : 0, jm = j > 0 ? j - 1 : ny - 1;
+    const int cp = c + (jp - j) * sy, cm = c + (jm - j) * sy;
+    const int kp = min(k + 1, nz - 1), km = max(k - 1, 0);
+    const int ch = c + (kp - k) * sz, cl = c - (k - km) * sz;
+    const Two<T> X = at2(x, c, i, j, k), R = ld2(ir + c);
+    const Two<T> xp = at2(x, cp, i, jp, k), rp = ld2(ir + cp);
+    const Two<T> xm = at2(x, cm, i, jm, k), rm = ld2(ir + cm);
+    const Two<T> xh = at2(x, ch, i, j, kp), rh = ld2(ir + ch);
+    const Two<T> xl = at2(x, cl, i, j, km), rl = ld2(ir + cl);
+    T xe = __shfl_down_sync(0xffffffffu, X.a, 1), re = __shfl_down_sync(0xffffffffu, R.a, 1);
+    T xw = __shfl_up_sync(0xffffffffu, X.b, 1), rw = __shfl_up_sync(0xffffffffu, R.b, 1);
+    if (lane == 31 && i + 2 < nx) { xe = x.at(c + 2, i + 2, j, k); re = ir[c + 2]; }
+    if (lane == 0 && i > 0) { xw = x.at(c - 1, i - 1, j, k); rw = ir[c - 1]; }
+    const T hx = tb[0], hy = tb[1], hh = tb[2], hl = tb[3];
+    T ea = tb[4], eb = ea;
+    if (i + 2 == nx) eb += tb[5] * R.b;
+    if (k == nz - 1) { ea += tb[6] * R.a; eb += tb[6] * R.b; }
+    T ya = ea * X.a, yb = eb * X.b;
+    ya += hx * (R.a + R.b) * (X.a - X.b);
+    if (i + 2 < nx) yb += hx * (R.b + re) * (X.b - xe);
+    if (i > 0) ya += hx * (R.a + rw) * (X.a - xw);
+    yb += hx * (R.b + R.a) * (X.b - X.a);
+    if (ny > 1) {
+      ya += hy * (R.a + rp.a) * (X.a - xp.a);
+      yb += hy * (R.b + rp.b) * (X.b - xp.b);
+      ya += hy * (R.a + rm.a) * (X.a - xm.a);
+      yb += hy * (R.b + rm.b) * (X.b - xm.b);
+    }
+    if (k < nz - 1) {
+      ya += hh * (R.a + rh.a) * (X.a - xh.a);
+      yb += hh * (R.b + rh.b) * (X.b - xh.b);
+    }
+    if (k > 0) {
+      ya += hl * (R.a + rl.a) * (X.a - xl.a);
+      yb += hl * (R.b + rl.b) * (X.b - xl.b);
+    }
+    xc[0] = X.a; xc[1] = X.b;
+    y[0] = ya; y[1] = yb;
   }
-  block_sums_store<1>(acc, partial);
+}
+template <int W, typename T>
+__device__ __forceinline__ void z_load(const T* p, int c, T (&v)[W]) {
+  if constexpr (W == 2) {
+    const Two<T> t = ld2(p + c);
+    v[0] = t.a; v[1] = t.b;
+  } else {
+    v[0] = p[c];
+  }
+}
+template <int W, typename T>
+__device__ __forceinline__ void z_store(T* p, int c, const T (&v)[W]) {
+  if constexpr (W == 2) *(Two<T>*)(p + c) = Two<T>{v[0], v[1]};
+  else p[c] = v[0];
 }
 
-// r = b - S x, partial of ||r_A||^2 with r_A = -r / dz_k
-__global__ void k_pcg_residual(GridDev g, const double* __restrict__ gx,
-                               const double* __restrict__ gy, const double* __restrict__ gz,
-                               const double* __restrict__ e, const double* __restrict__ b,
-                               const double* __restrict__ x, double* r, double* partial) {
-  const int nx = g.nx, ny = g.ny, nz = g.nz;
-  const int64_t n = (int64_t)nx * ny * nz;
-  double acc[1] = {0.0};
-  for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < n;
-       c += (int64_t)RED_BLOCKS * blockDim.x) {
-    int i, j, k;
-    split_cell((uint32_t)c, g.fnx, g.fny, i, j, k);
-    double rr = b[c] - mg_apply(nx, ny, nz, gx, gy, gz, e, x, c, i, j, k);
-    r[c] = rr;
-    double ra = rr / g.dz[k];
-    acc[0] += ra * ra;
+// damped Jacobi sweep; with DOT the sum of rd * (the new iterate) as well (the
+// V-cycle's last sweep: r.z)
+template <int W, typename T, typename V, bool DOT>
+__global__ void __launch_bounds__(Z_THREADS, 4)
+    k_z_jacobi(Dims D, OpI<T> o, const T* __restrict__ dinv, const T* __restrict__ b, V x, T* xo,
+               double w_, const double* __restrict__ rd, double* partial, const double* done) {
+  PCG_SKIP(done);
+  const ZCell z = z_cell<W>(D);
+  T bc[W], dc[W], xc[W], y[W], v[W];
+  z_load<W>(b, z.c, bc);
+  z_load<W>(dinv, z.c, dc);
+  z_apply<W>(D, o, x, z.c, z.i, z.j, z.k, xc, y);
+#pragma unroll
+  for (int q = 0; q < W; ++q) v[q] = xc[q] + (T)w_ * (bc[q] - y[q]) * dc[q];
+  if (z.in) z_store<W>(xo, z.c, v);
+  if (DOT) {
+    double acc = 0.0, rr[W];
+    z_load<W>(rd, z.c, rr);
+    if (z.in)
+#pragma unroll
+      for (int q = 0; q < W; ++q) acc += rr[q] * (double)v[q];
+    store_partial(acc, partial);
   }
-  block_sums_store<1>(acc, partial);
 }
 
-// x += alpha p ; r -= alpha q ; partial ||r_A||^2   (alpha = rz / pq from device scalars)
-__global__ void k_pcg_update(GridDev g, const double* __restrict__ scal, double* x, double* r,
-                             const double* __restrict__ p, const double* __restrict__ q,
+// coarse rhs = sum over children of the fine residual, a coarse cell a thread
+template <typename T>
+__global__ void __launch_bounds__(Z_THREADS, 4)
+    k_z_restrict(Dims D, OpI<T> o, const T* __restrict__ b, const T* __restrict__ x, Dims DC, T* bc,
+                 const double* done) {
+  PCG_SKIP(done);
+  const ZCell z = z_cell<1>(DC);
+  T s = T(0);
+#pragma unroll
+  for (int dk = 0; dk < 2; ++dk)
+#pragma unroll
+    for (int dj = 0; dj < 2; ++dj) {
+      const int k = min(2 * z.k + dk, D.nz - 1), j = min(2 * z.j + dj, D.ny - 1), i = 2 * z.i;
+      const int c = (k * D.ny + j) * D.nx + i;
+      T xc[2], y[2], r[2];
+      z_load<2>(b, c, r);
+      z_apply<2>(D, o, VecX<T>{x}, c, i, j, k, xc, y);
+      if (2 * z.k + dk < D.nz && 2 * z.j + dj < D.ny) {
+        s += r[0] - y[0];
+        s += r[1] - y[1];
+      }
+    }
+  if (z.in) bc[z.c] = s;
+}
+
+// q = S p and p.q, with p = z + beta p of the last iteration formed on the way
+// into the other of the two direction buffers
+template <int W, typename Z>
+__global__ void __launch_bounds__(Z_THREADS, 4)
+    k_z_matvec_dir(Dims D, OpI<double> o, const Z* __restrict__ zv, double* p0, double* p1,
+                   double* q, const double* __restrict__ scal, double* partial) {
+  PCG_SKIP(scal + SC_DONE);
+  const int it = (int)scal[SC_IT];
+  const VecDir<Z> x{zv, it & 1 ? p0 : p1, it == 0 ? 0.0 : scal[2] / scal[0]};
+  double* pn = it & 1 ? p1 : p0;
+  const ZCell z = z_cell<W>(D);
+  double pc[W], y[W], acc = 0.0;
+  z_apply<W>(D, o, x, z.c, z.i, z.j, z.k, pc, y);
+  if (z.in) {
+    z_store<W>(pn, z.c, pc);
+    z_store<W>(q, z.c, y);
+#pragma unroll
+    for (int e = 0; e < W; ++e) acc += pc[e] * y[e];
+  }
+  store_partial(acc, partial);
+}
+// q = S p and p.q of a stored vector (W = 1 for a caller's: any alignment)
+template <int W>
+__global__ void __launch_bounds__(Z_THREADS, 4)
+    k_z_matvec(Dims D, OpI<double> o, const double* __restrict__ p, double* q, double* partial,
+               const double* done) {
+  PCG_SKIP(done);
+  const ZCell z = z_cell<W>(D);
+  double pc[W], y[W], acc = 0.0;
+  z_apply<W>(D, o, VecX<double>{p}, z.c, z.i, z.j, z.k, pc, y);
+  if (z.in) {
+    z_store<W>(q, z.c, y);
+#pragma unroll
+    for (int e = 0; e < W; ++e) acc += pc[e] * y[e];
+  }
+  if (partial) store_partial(acc, partial);
+}
+
+// r = b - S x (also in FP32 where the preconditioner is), ||r_A||^2 with
+// r_A = -r / dz_k
+template <int W>
+__global__ void __launch_bounds__(Z_THREADS, 4)
+    k_z_residual(GridDev g, Dims D, OpI<double> o, const double* __restrict__ b,
+                 const double* __restrict__ x, double* r, float* r32, double* partial) {
+  const ZCell z = z_cell<W>(D);
+  double xc[W], y[W], v[W], acc = 0.0;
+  z_load<W>(b, z.c, v);
+  z_apply<W>(D, o, VecX<double>{x}, z.c, z.i, z.j, z.k, xc, y);
+  if (z.in) {
+    const double dz = g.dz[z.k];
+#pragma unroll
+    for (int e = 0; e < W; ++e) {
+      v[e] -= y[e];
+      if (r32) r32[z.c + e] = (float)v[e];
+      const double ra = v[e] / dz;
+      acc += ra * ra;
+    }
+    z_store<W>(r, z.c, v);
+  }
+  store_partial(acc, partial);
+}
+
+// x += alpha p ; r -= alpha q ; ||r_A||^2   (alpha = rz / pq from device scalars;
+// p: the buffer of this iteration's parity, or p0 with p1 null)
+__global__ void k_pcg_update(GridDev g, double* x, double* r, float* r32,
+                             const double* __restrict__ p0, const double* __restrict__ p1,
+                             const double* __restrict__ q, const double* __restrict__ scal,
                              double* partial) {
   PCG_SKIP(scal + SC_DONE);
   const int64_t n = ncells_dev(g);
   const double alpha = scal[0] / scal[1];
-  double acc[1] = {0.0};
+  const double* p = p1 && ((int)scal[SC_IT] & 1) ? p1 : p0;
+  double acc = 0.0;
   for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < n;
-       c += (int64_t)RED_BLOCKS * blockDim.x) {
+       c += (int64_t)gridDim.x * blockDim.x) {
     x[c] += alpha * p[c];
     double rr = r[c] - alpha * q[c];
     r[c] = rr;
+    if (r32) r32[c] = (float)rr;
     double ra = rr / g.dz[(int)fdiv(fdiv((uint32_t)c, g.fnx), g.fny)];
-    acc[0] += ra * ra;
+    acc += ra * ra;
   }
-  block_sums_store<1>(acc, partial);
+  store_partial(acc, partial);
 }
 
-// partial of r.z
+// a.b
 __global__ void k_dot(int64_t n, const double* __restrict__ a, const double* __restrict__ b,
                       double* partial, const double* done) {
   PCG_SKIP(done);
-  double acc[1] = {0.0};
+  double acc = 0.0;
   for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < n;
-       c += (int64_t)RED_BLOCKS * blockDim.x)
-    acc[0] += a[c] * b[c];
-  block_sums_store<1>(acc, partial);
-}
-
-// p = z + beta p, beta = rz_new / rz_old ; first iteration p = z
-__global__ void k_pcg_dir(int64_t n, const double* __restrict__ scal, const double* __restrict__ z,
-                          double* p) {
-  PCG_SKIP(scal + SC_DONE);
-  int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (c >= n) return;
-  if (scal[SC_IT] == 0.0) { p[c] = z[c]; return; }
-  double beta = scal[2] / scal[0];
-  p[c] = z[c] + beta * p[c];
+       c += (int64_t)gridDim.x * blockDim.x)
+    acc += a[c] * b[c];
+  store_partial(acc, partial);
 }
 
 __global__ void k_set_scal(double* scal, int dst, int src) {
   PCG_SKIP(scal + SC_DONE);
   scal[dst] = scal[src];
-}
-
-// end of an iteration: count it and test ||r_A|| < rtol ||b_A||
-__global__ void k_pcg_check(double* scal) {
-  if (scal[SC_DONE] != 0.0) return;
-  scal[SC_IT] += 1.0;
-  if (scal[5] < scal[6]) scal[SC_DONE] = 1.0;
 }
 
 // start of a solve: tolerance, initial test, iteration count; b == 0 -> x = 0
@@ -568,17 +873,15 @@ __global__ void k_fcg_alpha(double* scal) {
 
 // out = b - S x (level operator, any precision)
 template <typename T>
-__global__ void k_lp_residual(Dims D, const T* __restrict__ gx,
-                              const T* __restrict__ gy, const T* __restrict__ gz,
-                              const T* __restrict__ e, const T* __restrict__ b,
-                              const T* __restrict__ x, T* out) {
+__global__ void k_lp_residual(Dims D, OpI<T> o, const T* __restrict__ b, const T* __restrict__ x,
+                              T* out) {
   const int nx = D.nx, ny = D.ny, nz = D.nz;
   int64_t n = (int64_t)nx * ny * nz;
   int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (c >= n) return;
   int i, j, k;
   split_cell((uint32_t)c, D.fnx, D.fny, i, j, k);
-  out[c] = b[c] - mg_apply(nx, ny, nz, gx, gy, gz, e, x, c, i, j, k);
+  out[c] = b[c] - mg_apply(nx, ny, nz, o, VecX<T>{x}, x[c], c, i, j, k);
 }
 
 // e1 = float(e0) - t
@@ -679,9 +982,14 @@ void* proj_create(const GridDev& g) {
     MGLevel& lv = P->lev[L];
     lv.nx = nx; lv.ny = ny; lv.nz = nz; lv.n = (int64_t)nx * ny * nz;
     lv.dims = dims_make(nx, ny, nz);
-    lv.gx = dalloc(lv.n); lv.gy = dalloc(lv.n); lv.gz = dalloc(lv.n); lv.e = dalloc(lv.n);
-    lv.dinv = dalloc(lv.n); lv.x = dalloc(lv.n); lv.b = dalloc(lv.n); lv.t = dalloc(lv.n);
-    lv.s = dalloc(lv.n);
+    // level 0's operator is formed from 1/rho, its vectors are the solver's
+    const bool arr = L > 0 || lv.n <= MG_COARSE_MAX;
+    lv.gx = lv.gy = lv.gz = lv.e = lv.x = lv.b = nullptr;
+    if (arr) {
+      lv.gx = dalloc(lv.n); lv.gy = dalloc(lv.n); lv.gz = dalloc(lv.n); lv.e = dalloc(lv.n);
+      lv.x = dalloc(lv.n); lv.b = dalloc(lv.n);
+    }
+    lv.dinv = dalloc(lv.n); lv.t = dalloc(lv.n); lv.s = dalloc(lv.n);
     ++L;
     if (lv.n <= MG_COARSE_MAX || L >= 16) break;
     int cx = (nx + 1) / 2, cy = (ny + 1) / 2, cz = (nz + 1) / 2;
@@ -694,11 +1002,15 @@ void* proj_create(const GridDev& g) {
   P->Ainv = dalloc(nc <= MG_COARSE_MAX ? nc * nc : 1);
   P->pc_r = dalloc(n0); P->pc_z = dalloc(n0); P->pc_p = dalloc(n0); P->pc_q = dalloc(n0);
   P->rhs = dalloc(n0);
-  P->partial = dalloc(RED_BLOCKS * 4);
+  const int zb = z_blocks(P->lev[0].dims);
+  P->partial = dalloc(zb > RED_BLOCKS ? zb : RED_BLOCKS);
+  P->pc_p2 = dalloc(n0);
   P->scal = dalloc(16);
   cudaMallocHost(&P->h_scal, sizeof(double) * 16);
   P->p_prev = dalloc(n0);
   P->ir = dalloc(n0);
+  P->tab = dalloc((int64_t)OP_TAB * g.nz);
+  P->ir32 = nullptr; P->tab32 = nullptr;
   {
     // cleared before any solve is queued, on a private stream
     SetupStream ss;
@@ -750,8 +1062,9 @@ void proj_destroy(void* h) {
   if (P->iter_exec) cudaGraphExecDestroy(P->iter_exec);
   if (P->cs) cudaStreamDestroy(P->cs);
   cudaFree(P->Ainv); cudaFree(P->pc_r); cudaFree(P->pc_z); cudaFree(P->pc_p); cudaFree(P->pc_q);
+  cudaFree(P->pc_p2);
   cudaFree(P->rhs); cudaFree(P->partial); cudaFree(P->scal); cudaFreeHost(P->h_scal);
-  cudaFree(P->p_prev); cudaFree(P->ir);
+  cudaFree(P->p_prev); cudaFree(P->ir); cudaFree(P->tab); cudaFree(P->ir32); cudaFree(P->tab32);
   delete P;
 }
 
@@ -771,23 +1084,39 @@ __global__ void k_cvt_f2d(int64_t n, const float* __restrict__ a, double* b, con
 }
 
 template <typename T>
+static OpA<T> op_a(const MGLevelT<T>& f) {
+  return OpA<T>{f.gx, f.gy, f.gz, f.e};
+}
+static OpI<double> op_0(const ProjCtx* P, double) { return OpI<double>{P->ir, P->tab}; }
+static OpI<float> op_0(const ProjCtx* P, float) { return OpI<float>{P->ir32, P->tab32}; }
+
+template <typename T>
 static void rebuild_levels(ProjCtx* P, MGLevelT<T>* lev, T* Ainv, cudaStream_t st) {
+  const OpI<T> o0 = op_0(P, T(0));
   for (int l = 0; l < P->nlev; ++l) {
     MGLevelT<T>& f = lev[l];
     if (l > 0) {
       MGLevelT<T>& pf = lev[l - 1];
-      k_mg_coarsen<T><<<blocks_for(f.n, 128), 128, 0, st>>>(pf.nx, pf.ny, pf.nz, pf.gx, pf.gy,
-                                                           pf.gz, pf.e, f.dims, f.gx,
-                                                           f.gy, f.gz, f.e, 0.5);
+      if (l == 1)
+        k_mg_coarsen<T><<<blocks_for(f.n, 128), 128, 0, st>>>(pf.nx, pf.ny, pf.nz, o0, f.dims, f.gx,
+                                                             f.gy, f.gz, f.e, 0.5);
+      else
+        k_mg_coarsen<T><<<blocks_for(f.n, 128), 128, 0, st>>>(pf.nx, pf.ny, pf.nz, op_a(pf), f.dims,
+                                                             f.gx, f.gy, f.gz, f.e, 0.5);
       fs_count_launch();
+      k_mg_diag<T><<<blocks_for(f.n, 256), 256, 0, st>>>(f.dims, op_a(f), f.dinv);
+    } else {
+      k_mg_diag<T><<<blocks_for(f.n, 256), 256, 0, st>>>(f.dims, o0, f.dinv);
+      if (P->nlev == 1) {
+        k_op_arrays<T><<<blocks_for(f.n, 256), 256, 0, st>>>(f.dims, o0, f.gx, f.gy, f.gz, f.e);
+        fs_count_launch();
+      }
     }
-    k_mg_diag<T><<<blocks_for(f.n, 256), 256, 0, st>>>(f.dims, f.gx, f.gy, f.gz, f.e,
-                                                       f.dinv);
     fs_count_launch();
   }
   MGLevelT<T>& c = lev[P->nlev - 1];
   if (c.n <= MG_COARSE_MAX) {
-    k_mg_coarse_inverse<T><<<1, 64, 0, st>>>(c.nx, c.ny, c.nz, c.gx, c.gy, c.gz, c.e, Ainv);
+    k_mg_coarse_inverse<T><<<1, 1024, 0, st>>>(c.nx, c.ny, c.nz, c.gx, c.gy, c.gz, c.e, Ainv);
     fs_count_launch();
   }
 }
@@ -795,23 +1124,13 @@ static void rebuild_levels(ProjCtx* P, MGLevelT<T>* lev, T* Ainv, cudaStream_t s
 int proj_rebuild(void* h, const double* rho, cudaStream_t st) {
   ProjCtx* P = (ProjCtx*)h;
   const GridDev& g = P->g;
-  MGLevel& l0 = P->lev[0];
-  Launch3 L = launch_cells(g);
-  k_proj_level0<<<L.grid, L.block, 0, st>>>(g, rho, P->ir, l0.gx, l0.gy, l0.gz, l0.e,
-                                            g.dx * g.dx, g.dy * g.dy); fs_count_launch();
-  if (P->fp32) {
-    // the FP64 level-0 operator stays the CG's; the preconditioner gets an FP32 copy
-    MGLevelT<float>& f0 = P->lev32[0];
-    const double* src[4] = {l0.gx, l0.gy, l0.gz, l0.e};
-    float* dst[4] = {f0.gx, f0.gy, f0.gz, f0.e};
-    for (int q = 0; q < 4; ++q) {
-      k_cvt_d2f<<<blocks_for(l0.n, 256), 256, 0, st>>>(l0.n, src[q], dst[q], nullptr);
-      fs_count_launch();
-    }
-    rebuild_levels<float>(P, P->lev32, P->Ainv32, st);
-  } else {
-    rebuild_levels<double>(P, P->lev, P->Ainv, st);
-  }
+  const unsigned nb = blocks_for(P->lev[0].n, 256);
+  // the FP64 level-0 operator stays the CG's; the FP32 preconditioner has its own
+  k_proj_ir<float><<<nb, 256, 0, st>>>(g, rho, P->ir, P->fp32 ? P->ir32 : nullptr, P->tab,
+                                       P->fp32 ? P->tab32 : nullptr, g.dx * g.dx, g.dy * g.dy);
+  fs_count_launch();
+  if (P->fp32) rebuild_levels<float>(P, P->lev32, P->Ainv32, st);
+  else rebuild_levels<double>(P, P->lev, P->Ainv, st);
   return cuda_status();
 }
 
@@ -819,19 +1138,24 @@ int proj_set_precision(void* h, int fp32) {
   ProjCtx* P = (ProjCtx*)h;
   fp32 = fp32 ? 1 : 0;
   if (fp32 == P->fp32) return FS_OK;
-  if (fp32 && !P->lev32[0].gx) {
+  if (fp32 && !P->lev32[0].t) {
     for (int l = 0; l < P->nlev; ++l) {
       MGLevelT<float>& lv = P->lev32[l];
       const MGLevel& ld = P->lev[l];
       lv.nx = ld.nx; lv.ny = ld.ny; lv.nz = ld.nz; lv.n = ld.n; lv.dims = ld.dims;
       float** arrs[9] = {&lv.gx, &lv.gy, &lv.gz, &lv.e, &lv.dinv, &lv.x, &lv.b, &lv.t, &lv.s};
       for (float** a : arrs)
-        if (cudaMalloc(a, sizeof(float) * (size_t)(lv.n > 0 ? lv.n : 1)) != cudaSuccess)
+        // level 0: its operator is formed from 1/rho
+        if (!(l == 0 && P->nlev > 1 && (a == arrs[0] || a == arrs[1] || a == arrs[2] ||
+                                        a == arrs[3])) &&
+            cudaMalloc(a, sizeof(float) * (size_t)(lv.n > 0 ? lv.n : 1)) != cudaSuccess)
           return FS_ECUDA;
     }
     const int64_t nc = P->lev[P->nlev - 1].n;
     if (cudaMalloc(&P->Ainv32, sizeof(float) * (size_t)(nc <= MG_COARSE_MAX ? nc * nc : 1)) !=
             cudaSuccess ||
+        cudaMalloc(&P->ir32, sizeof(float) * P->lev[0].n) != cudaSuccess ||
+        cudaMalloc(&P->tab32, sizeof(float) * OP_TAB * P->lev[0].nz) != cudaSuccess ||
         cudaMalloc(&P->r32, sizeof(float) * P->lev[0].n) != cudaSuccess ||
         cudaMalloc(&P->z32, sizeof(float) * P->lev[0].n) != cudaSuccess)
       return FS_ECUDA;
@@ -1011,6 +1335,128 @@ __global__ void __launch_bounds__(MG_TAIL_THREADS, 1)
   for (int64_t c = threadIdx.x; c < L[0].n; c += blockDim.x) a.lev[0].x[c] = L[0].x[c];
 }
 
+// the sum of the partials that the kernel before left
+static void launch_finish(ProjCtx* P, int nb, int slot, int post, const double* done,
+                          cudaStream_t st) {
+  k_finish_sum<<<1, FIN_THREADS, 0, st>>>(P->partial, nb, P->scal, slot, post, done);
+}
+// a sweep and a restriction on level 0 and on the others (returns the launches)
+template <int W, typename T, typename V>
+static int launch_z_jacobi(ProjCtx* P, const Dims& D, const OpI<T>& o, const T* dinv, const T* b, V x,
+                           T* xo, double w, bool dot, const double* done, cudaStream_t st) {
+  const int nb = z_blocks(D);
+  if (!dot) {
+    k_z_jacobi<W, T, V, false><<<nb, Z_THREADS, 0, st>>>(D, o, dinv, b, x, xo, w, nullptr, nullptr,
+                                                         done);
+    return 1;
+  }
+  k_z_jacobi<W, T, V, true><<<nb, Z_THREADS, 0, st>>>(D, o, dinv, b, x, xo, w, P->pc_r, P->partial,
+                                                      done);
+  launch_finish(P, nb, 2, POST_NONE, done, st);  // rz_new
+  return 2;
+}
+template <typename T, typename V>
+static int launch_jacobi(ProjCtx* P, const Dims& D, const OpI<T>& o, const T* dinv, const T* b, V x,
+                         T* xo, double w, bool dot, const double* done, cudaStream_t st) {
+  return z_width(D) == 2 ? launch_z_jacobi<2>(P, D, o, dinv, b, x, xo, w, dot, done, st)
+                         : launch_z_jacobi<1>(P, D, o, dinv, b, x, xo, w, dot, done, st);
+}
+template <typename T, typename V>
+static int launch_jacobi(ProjCtx*, const Dims& D, const OpA<T>& o, const T* dinv, const T* b, V x,
+                          T* xo, double w, bool, const double* done, cudaStream_t st) {
+  k_mg_jacobi<T><<<blocks_for((int64_t)D.nx * D.ny * D.nz, 256), 256, 0, st>>>(D, o, dinv, b, x, xo,
+                                                                              w, done);
+  return 1;
+}
+template <typename T>
+static void launch_restrict(const Dims& D, const OpA<T>& o, const T* b, const T* x, const Dims& DC,
+                            T* bc, const double* done, cudaStream_t st) {
+  k_mg_restrict_residual<T><<<blocks_for((int64_t)DC.nx * DC.ny * DC.nz, 128), 128, 0, st>>>(
+      D, o, b, x, DC, bc, done);
+}
+template <typename T>
+static void launch_restrict(const Dims& D, const OpI<T>& o, const T* b, const T* x, const Dims& DC,
+                            T* bc, const double* done, cudaStream_t st) {
+  const unsigned nc = blocks_for((int64_t)DC.nx * DC.ny * DC.nz, Z_THREADS);
+  if (z_width(D) == 2)
+    k_z_restrict<T><<<nc, Z_THREADS, 0, st>>>(D, o, b, x, DC, bc, done);
+  else
+    k_mg_restrict_residual<T><<<nc, Z_THREADS, 0, st>>>(D, o, b, x, DC, bc, done);
+}
+template <typename Z>
+static void launch_matvec_dir(ProjCtx* P, const Z* z, cudaStream_t st) {
+  const Dims& D = P->lev[0].dims;
+  const int nb = z_blocks(D);
+  const OpI<double> o = op_0(P, 0.0);
+  if (z_width(D) == 2)
+    k_z_matvec_dir<2, Z><<<nb, Z_THREADS, 0, st>>>(D, o, z, P->pc_p, P->pc_p2, P->pc_q, P->scal,
+                                                   P->partial);
+  else
+    k_z_matvec_dir<1, Z><<<nb, Z_THREADS, 0, st>>>(D, o, z, P->pc_p, P->pc_p2, P->pc_q, P->scal,
+                                                   P->partial);
+  launch_finish(P, nb, 1, POST_DIR, P->scal + SC_DONE, st);  // p.q
+}
+// pc_r = rhs - S x and its norm
+static void launch_residual(ProjCtx* P, const double* x, float* r32, cudaStream_t st) {
+  const Dims& D = P->lev[0].dims;
+  const int nb = z_blocks(D);
+  const OpI<double> o = op_0(P, 0.0);
+  if (z_width(D) == 2)
+    k_z_residual<2><<<nb, Z_THREADS, 0, st>>>(P->g, D, o, P->rhs, x, P->pc_r, r32, P->partial);
+  else
+    k_z_residual<1><<<nb, Z_THREADS, 0, st>>>(P->g, D, o, P->rhs, x, P->pc_r, r32, P->partial);
+  launch_finish(P, nb, 5, POST_NONE, nullptr, st);
+}
+
+template <typename T>
+static int vcycle(ProjCtx* P, MGLevelT<T>* lev, const T* Ainv, int l, const T* b, T* x,
+                  const double* done, cudaStream_t st);
+
+// one level of the V-cycle in launches: the sweeps before (from x = 0, the first
+// two in one pass), the coarse correction, and the sweeps after (the
+// prolongation part of the first)
+template <typename T, typename Op>
+static int vcycle_level(ProjCtx* P, MGLevelT<T>* lev, const T* Ainv, int l, Op o, const T* b, T* x,
+                        const double* done, cudaStream_t st) {
+  MGLevelT<T>& f = lev[l];
+  MGLevelT<T>& cl = lev[l + 1];
+  const unsigned nb = blocks_for(f.n, 256);
+  const int nu = (l == 0 && P->nu0 > 0) ? P->nu0 : P->nu;
+  const double om = P->omega;
+  int nk = 0;
+  // pre-smoothing, ending in t: sweep i writes t when (nu-1-i) is even, else s
+  const T* src = nullptr;
+  if (nu == 1) {
+    k_mg_first<T><<<nb, 256, 0, st>>>(f.n, f.dinv, b, f.t, om, done);
+    ++nk;
+  }
+  for (int i = 1; i < nu; ++i) {
+    T* dst = ((nu - 1 - i) % 2 == 0) ? f.t : f.s;
+    if (i == 1)
+      nk += launch_jacobi(P, f.dims, o, f.dinv, b, VecFirst<T>{b, f.dinv, (T)om}, dst, om, false,
+                          done, st);
+    else
+      nk += launch_jacobi(P, f.dims, o, f.dinv, b, VecX<T>{src}, dst, om, false, done, st);
+    src = dst;
+  }
+  launch_restrict(f.dims, o, b, f.t, cl.dims, cl.b, done, st);
+  ++nk;
+  nk += vcycle<T>(P, lev, Ainv, l + 1, cl.b, cl.x, done, st);
+  // post-smoothing from t + P xc, ending in x:  s, t, s, ... then x
+  src = f.t;
+  for (int i = 0; i < nu; ++i) {
+    T* dst = (i == nu - 1) ? x : ((i % 2 == 0) ? f.s : f.t);
+    const bool dot = l == 0 && i == nu - 1;  // r.z with the last one
+    if (i == 0)
+      nk += launch_jacobi(P, f.dims, o, f.dinv, b, VecProl<T>{src, cl.x, cl.nx, cl.ny}, dst, om, dot,
+                          done, st);
+    else
+      nk += launch_jacobi(P, f.dims, o, f.dinv, b, VecX<T>{src}, dst, om, dot, done, st);
+    src = dst;
+  }
+  return nk;
+}
+
 template <typename T>
 static int vcycle(ProjCtx* P, MGLevelT<T>* lev, const T* Ainv, int l, const T* b, T* x,
                   const double* done, cudaStream_t st) {
@@ -1037,52 +1483,22 @@ static int vcycle(ProjCtx* P, MGLevelT<T>* lev, const T* Ainv, int l, const T* b
       ++nk;
     } else {
       // not coarsenable and too large for the dense solve: smoothing only
-      k_mg_jacobi<T><<<blocks_for(f.n, 256), 256, 0, st>>>(f.dims, f.gx, f.gy, f.gz,
-                                                          f.e, f.dinv, b, nullptr, x, MG_OMEGA,
-                                                          done);
+      const unsigned nb = blocks_for(f.n, 256);
+      k_mg_first<T><<<nb, 256, 0, st>>>(f.n, f.dinv, b, x, MG_OMEGA, done);
       ++nk;
       for (int s = 0; s < 8; ++s) {
         const T* src = (s & 1) ? f.t : x;
         T* dst = (s & 1) ? x : f.t;
-        k_mg_jacobi<T><<<blocks_for(f.n, 256), 256, 0, st>>>(f.dims, f.gx, f.gy, f.gz,
-                                                            f.e, f.dinv, b, src, dst, MG_OMEGA,
-                                                            done);
+        k_mg_jacobi<T><<<nb, 256, 0, st>>>(f.dims, op_a(f), f.dinv, b, VecX<T>{src}, dst, MG_OMEGA,
+                                           done);
         ++nk;
       }
     }
     return nk;
   }
-  MGLevelT<T>& cl = lev[l + 1];
-  unsigned nb = blocks_for(f.n, 256);
-  const int nu = (l == 0 && P->nu0 > 0) ? P->nu0 : P->nu;
-  const double om = P->omega;
-  // pre-smoothing from x = 0, ending in t:  sweep i writes t when (nu-1-i) is even, else s
-  const T* src = nullptr;
-  for (int i = 0; i < nu; ++i) {
-    T* dst = ((nu - 1 - i) % 2 == 0) ? f.t : f.s;
-    k_mg_jacobi<T><<<nb, 256, 0, st>>>(f.dims, f.gx, f.gy, f.gz, f.e, f.dinv, b, src,
-                                       dst, om, done);
-    src = dst;
-    ++nk;
-  }
-  k_mg_restrict_residual<T><<<blocks_for(cl.n, 128), 128, 0, st>>>(
-      f.dims, f.gx, f.gy, f.gz, f.e, b, f.t, cl.dims, cl.b, done);
-  ++nk;
-  nk += vcycle<T>(P, lev, Ainv, l + 1, cl.b, cl.x, done, st);
-  k_mg_prolong<T><<<nb, 256, 0, st>>>(f.dims, f.t, cl.nx, cl.ny, cl.x, done);
-  ++nk;
-  // post-smoothing from t, ending in x:  s, t, s, ... then x
-  src = f.t;
-  for (int i = 0; i < nu; ++i) {
-    T* dst = (i == nu - 1) ? x : ((i % 2 == 0) ? f.s : f.t);
-    k_mg_jacobi<T><<<nb, 256, 0, st>>>(f.dims, f.gx, f.gy, f.gz, f.e, f.dinv, b, src,
-                                       dst, om, done);
-    src = dst;
-    ++nk;
-  }
-  return nk;
+  return nk + (l == 0 ? vcycle_level<T>(P, lev, Ainv, l, op_0(P, T(0)), b, x, done, st)
+                      : vcycle_level<T>(P, lev, Ainv, l, op_a(f), b, x, done, st));
 }
-
 
 void proj_stats(void* h, double* out8) {
   ProjCtx* P = (ProjCtx*)h;
@@ -1131,26 +1547,27 @@ static int pcg_iteration(ProjCtx* P, double* x, cudaStream_t st) {
   const int64_t n = l0.n;
   const double* done = P->scal + SC_DONE;
   int nk;
-  if (P->fp32) {
-    k_cvt_d2f<<<blocks_for(n, 256), 256, 0, st>>>(n, P->pc_r, P->r32, done);
+  if (P->fp32)
     nk = vcycle<float>(P, P->lev32, P->Ainv32, 0, P->r32, P->z32, done, st);
-    k_cvt_f2d<<<blocks_for(n, 256), 256, 0, st>>>(n, P->z32, P->pc_z, done);
-    nk += 2;
-  } else {
+  else
     nk = vcycle<double>(P, P->lev, P->Ainv, 0, P->pc_r, P->pc_z, done, st);
+  if (P->nlev == 1) {  // no sweeps: r.z is a pass of its own
+    if (P->fp32) {
+      k_cvt_f2d<<<blocks_for(n, 256), 256, 0, st>>>(n, P->z32, P->pc_z, done);
+      ++nk;
+    }
+    k_dot<<<RED_BLOCKS, RED_THREADS, 0, st>>>(n, P->pc_r, P->pc_z, P->partial, done);
+    launch_finish(P, RED_BLOCKS, 2, POST_NONE, done, st);
+    nk += 2;
   }
-  k_dot<<<RED_BLOCKS, RED_THREADS, 0, st>>>(n, P->pc_r, P->pc_z, P->partial, done);
-  k_finish_sums<<<1, 32, 0, st>>>(P->partial, 1, P->scal + 2, done);  // rz_new
-  k_pcg_dir<<<blocks_for(n, 256), 256, 0, st>>>(n, P->scal, P->pc_z, P->pc_p);
-  k_set_scal<<<1, 1, 0, st>>>(P->scal, 0, 2);  // rz = rz_new
-  k_pcg_matvec<<<RED_BLOCKS, RED_THREADS, 0, st>>>(l0.dims, l0.gx, l0.gy, l0.gz,
-                                                   l0.e, P->pc_p, P->pc_q, P->partial, done);
-  k_finish_sums<<<1, 32, 0, st>>>(P->partial, 1, P->scal + 1, done);  // pq
-  k_pcg_update<<<RED_BLOCKS, RED_THREADS, 0, st>>>(P->g, P->scal, x, P->pc_r, P->pc_p, P->pc_q,
-                                                   P->partial);
-  k_finish_sums<<<1, 32, 0, st>>>(P->partial, 1, P->scal + 5, done);  // ||r_A||^2
-  k_pcg_check<<<1, 1, 0, st>>>(P->scal);
-  return nk + 10;
+  if (P->fp32)
+    launch_matvec_dir(P, P->z32, st);
+  else
+    launch_matvec_dir(P, P->pc_z, st);
+  k_pcg_update<<<RED_BLOCKS, RED_THREADS, 0, st>>>(P->g, x, P->pc_r, P->fp32 ? P->r32 : nullptr,
+                                                   P->pc_p, P->pc_p2, P->pc_q, P->scal, P->partial);
+  launch_finish(P, RED_BLOCKS, 5, POST_CHECK, done, st);  // ||r_A||^2
+  return nk + 4;
 }
 
 // Capture one iteration as a CUDA graph (on the context's private stream).
@@ -1214,13 +1631,15 @@ static void lp_presmooth(ProjCtx* P, cudaStream_t st) {
   const float* src = nullptr;
   for (int i = 0; i < P->nu; ++i) {
     float* dst = ((P->nu - 1 - i) % 2 == 0) ? f.t : f.s;
-    k_mg_jacobi<float><<<nb, 256, 0, st>>>(f.dims, f.gx, f.gy, f.gz, f.e, f.dinv,
-                                           P->r32, src, dst, P->omega, nullptr);
+    if (!src)
+      k_mg_first<float><<<nb, 256, 0, st>>>(f.n, f.dinv, P->r32, dst, P->omega, nullptr);
+    else
+      k_mg_jacobi<float><<<nb, 256, 0, st>>>(f.dims, op_0(P, 0.0f), f.dinv, P->r32,
+                                             VecX<float>{src}, dst, P->omega, nullptr);
     src = dst;
     fs_count_launch();
   }
-  k_lp_residual<float><<<nb, 256, 0, st>>>(f.dims, f.gx, f.gy, f.gz, f.e, P->r32, f.t,
-                                           f.b);
+  k_lp_residual<float><<<nb, 256, 0, st>>>(f.dims, op_0(P, 0.0f), P->r32, f.t, f.b);
   fs_count_launch();
 }
 
@@ -1241,8 +1660,8 @@ static int learned_precond(ProjCtx* P, cudaStream_t st) {
   const float* src = f.s;
   for (int i = 0; i < P->nu; ++i) {
     float* dst = (i == P->nu - 1) ? P->z32 : ((i % 2 == 0) ? f.t : f.x);
-    k_mg_jacobi<float><<<nb, 256, 0, st>>>(f.dims, f.gx, f.gy, f.gz, f.e, f.dinv,
-                                           P->r32, src, dst, P->omega, nullptr);
+    k_mg_jacobi<float><<<nb, 256, 0, st>>>(f.dims, op_0(P, 0.0f), f.dinv, P->r32, VecX<float>{src},
+                                           dst, P->omega, nullptr);
     src = dst;
     fs_count_launch();
   }
@@ -1280,22 +1699,24 @@ static int fcg_iteration(ProjCtx* P, double* x, int it, cudaStream_t st) {
   if (rc) return rc;
   if (it > 0) {
     k_dot<<<RED_BLOCKS, RED_THREADS, 0, st>>>(n, P->pc_z, P->pc_q, P->partial, done);
-    k_finish_sums<<<1, 32, 0, st>>>(P->partial, 1, P->scal + 10, done);  // z.q_prev
+    launch_finish(P, RED_BLOCKS, 10, POST_NONE, done, st);  // z.q_prev
     fs_count_launch(); fs_count_launch();
   }
   k_fcg_dir<<<blocks_for(n, 256), 256, 0, st>>>(n, P->scal, P->pc_z, P->pc_p);
-  k_pcg_matvec<<<RED_BLOCKS, RED_THREADS, 0, st>>>(l0.dims, l0.gx, l0.gy, l0.gz,
-                                                   l0.e, P->pc_p, P->pc_q, P->partial, done);
-  k_finish_sums<<<1, 32, 0, st>>>(P->partial, 1, P->scal + 1, done);  // p.q
+  const int nb = z_blocks(l0.dims);
+  if (z_width(l0.dims) == 2)
+    k_z_matvec<2><<<nb, Z_THREADS, 0, st>>>(l0.dims, op_0(P, 0.0), P->pc_p, P->pc_q, P->partial, done);
+  else
+    k_z_matvec<1><<<nb, Z_THREADS, 0, st>>>(l0.dims, op_0(P, 0.0), P->pc_p, P->pc_q, P->partial, done);
+  launch_finish(P, nb, 1, POST_NONE, done, st);  // p.q
   k_dot<<<RED_BLOCKS, RED_THREADS, 0, st>>>(n, P->pc_p, P->pc_r, P->partial, done);
-  k_finish_sums<<<1, 32, 0, st>>>(P->partial, 1, P->scal + 12, done);  // p.r
+  launch_finish(P, RED_BLOCKS, 12, POST_NONE, done, st);  // p.r
   k_fcg_alpha<<<1, 1, 0, st>>>(P->scal);  // alpha = p.r / p.q
-  k_pcg_update<<<RED_BLOCKS, RED_THREADS, 0, st>>>(P->g, P->scal, x, P->pc_r, P->pc_p, P->pc_q,
-                                                   P->partial);
-  k_finish_sums<<<1, 32, 0, st>>>(P->partial, 1, P->scal + 5, done);  // ||r_A||^2
   k_set_scal<<<1, 1, 0, st>>>(P->scal, 11, 1);
-  k_pcg_check<<<1, 1, 0, st>>>(P->scal);
-  for (int k = 0; k < 10; ++k) fs_count_launch();
+  k_pcg_update<<<RED_BLOCKS, RED_THREADS, 0, st>>>(P->g, x, P->pc_r, nullptr, P->pc_p, nullptr,
+                                                   P->pc_q, P->scal, P->partial);
+  launch_finish(P, RED_BLOCKS, 5, POST_CHECK, done, st);
+  for (int k = 0; k < 9; ++k) fs_count_launch();
   return cuda_status();
 }
 
@@ -1320,9 +1741,7 @@ static int fcg_solve(ProjCtx* P, double* x, int maxiter, int* learned, cudaStrea
       fall = !(f < P->stall);
     }
     if (fall) {
-      k_pcg_residual<<<RED_BLOCKS, RED_THREADS, 0, st>>>(g, l0.gx, l0.gy, l0.gz, l0.e, P->rhs, x,
-                                                         P->pc_r, P->partial);
-      k_finish_sums<<<1, 32, 0, st>>>(P->partial, 1, P->scal + 5, nullptr);
+      launch_residual(P, x, P->r32, st);
       k_fcg_restart<<<1, 1, 0, st>>>(P->scal);
       fs_count_launch(); fs_count_launch(); fs_count_launch();
       P->fcg[2] = 1.0;
@@ -1375,13 +1794,13 @@ int proj_project(void* h, double* u, double* v, double* w, const double* u_in,
   const auto t_start = Clock::now();
   for (int q = 0; q < 8; ++q) P->stats[q] = 0.0;
   *iters = 0;
-  k_proj_rhs<<<RED_BLOCKS, RED_THREADS, 0, st>>>(g, u, v, w, u_in, target, dt, P->rhs,
-                                                 P->partial); fs_count_launch();
-  k_finish_sums<<<1, 32, 0, st>>>(P->partial, 1, P->scal + 4, nullptr); fs_count_launch();
+  k_proj_rhs<<<RED_BLOCKS, RED_THREADS, 0, st>>>(g, u, v, w, u_in, target, 1.0 / g.dx, 1.0 / g.dy,
+                                                 1.0 / dt, P->rhs, P->partial);
+  launch_finish(P, RED_BLOCKS, 4, POST_NONE, nullptr, st);
+  fs_count_launch(); fs_count_launch();
   double* x = P->p_prev;
-  k_pcg_residual<<<RED_BLOCKS, RED_THREADS, 0, st>>>(g, l0.gx, l0.gy, l0.gz, l0.e, P->rhs, x,
-                                                     P->pc_r, P->partial); fs_count_launch();
-  k_finish_sums<<<1, 32, 0, st>>>(P->partial, 1, P->scal + 5, nullptr); fs_count_launch();
+  launch_residual(P, x, P->fp32 ? P->r32 : nullptr, st);
+  fs_count_launch(); fs_count_launch();
   k_pcg_init<<<1, 1, 0, st>>>(P->scal, rtol * rtol); fs_count_launch();
   k_zero_if_zero_rhs<<<blocks_for(n, 256), 256, 0, st>>>(n, P->scal, x); fs_count_launch();
   if (P->log_r0) {
@@ -1441,7 +1860,8 @@ int launch_div_resid_max(const GridDev& g, const double* u, const double* v, con
 int proj_apply(void* h, const double* x, double* y, cudaStream_t st) {
   ProjCtx* P = (ProjCtx*)h;
   MGLevel& l0 = P->lev[0];
-  k_pcg_matvec<<<RED_BLOCKS, RED_THREADS, 0, st>>>(l0.dims, l0.gx, l0.gy, l0.gz, l0.e,
-                                                   x, y, P->partial, nullptr); fs_count_launch();
+  k_z_matvec<1><<<blocks_for(l0.n, Z_THREADS), Z_THREADS, 0, st>>>(l0.dims, op_0(P, 0.0), x, y,
+                                                                  nullptr, nullptr);
+  fs_count_launch();
   return cuda_status();
 }

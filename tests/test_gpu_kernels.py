@@ -25,6 +25,7 @@ pytestmark = pytest.mark.gpu
 from gpu_helpers import Grid, call, dev, host, lib, stream  # noqa: E402
 from firewebapp_b200._lib import (FsBedParams, FsBedParticles, FsBedSegments,  # noqa: E402
                                   FsBedSources, dbl_array, ptr, ptr_array)
+from firewebapp_b200.solver import _DeviceBuffer  # noqa: E402
 
 TIGHT = 1e-13
 LIBM = 1e-11
@@ -803,6 +804,64 @@ def test_projection_coarse_tail_is_bit_identical(fp32):
     (ua, va, wa, ia), (ub, vb, wb, ib) = out
     assert ia == ib
     assert np.array_equal(ua, ub) and np.array_equal(va, vb) and np.array_equal(wa, wb)
+
+
+@pytest.mark.parametrize("fp32", [0, 1])
+@pytest.mark.parametrize("nx, ny, nz, nu", [
+    (2, 2, 5, 2),      # the dense coarsest level alone
+    (33, 1, 7, 2),     # single cells a thread, no y faces
+    (34, 1, 7, 1),     # pairs; one sweep
+    (66, 2, 5, 3),     # both y neighbours the same row; three sweeps
+    (65, 9, 6, 2), (70, 9, 9, 2), (34, 31, 12, 4)])
+def test_projection_solves_the_numpy_system(nx, ny, nz, nu, fp32):
+    """After a solve to 1e-6 the residual of the returned pressure, taken with
+    an operator assembled here in FP64, meets the tolerance.  Slack 1e-3 of it:
+    the recursively updated residual drifts from the true one by rounding,
+    some iterations x cond(S) x 2^-53 < 1e-9 relative.  A V-cycle with a wrong
+    part still lets CG converge, only slowly: 25 iterations at most (multigrid
+    reduces the residual by more than 2 an iteration: 20 for 1e-6)."""
+    rng = np.random.default_rng(nx + ny)
+    dz = 0.2 * 1.1 ** np.arange(nz)
+    da = np.append(0.5 * (dz[:-1] + dz[1:]), 0.5 * dz[-1])
+    db = np.append(0.5 * dz[0], da[:-1])
+    dx, dy, dt, eps = 0.3, 0.25, 0.01, 1e-6
+    g = Grid(nz, ny, nx, dx, dy, dz, da, db)
+    shape = (nz, ny, nx)
+    rho = 0.3 + rng.random(shape)
+    ir = 1.0 / rho
+    u0, v0, w0 = (rng.standard_normal(shape) for _ in range(3))
+    args = [dev(q) for q in (u0, v0, w0, np.full((nz, ny), 1.5), 0.01 * rng.standard_normal(shape))]
+    drho, b, x0 = dev(rho), dev(np.ones(shape)), dev(np.ones(shape))
+    h = C.c_void_p()
+    call("fs_proj_create", g.ref, C.byref(h))
+    try:
+        call("fs_proj_configure", h, nu, 0.9)
+        if fp32:
+            call("fs_proj_set_precision", h, 1)
+        call("fs_proj_set_log", h, ptr(b), ptr(x0))
+        call("fs_proj_rebuild", h, ptr(drho), stream())
+        its = C.c_int()
+        call("fs_proj_project", h, *(ptr(q) for q in args), dt, 1e-6, 200, C.byref(its), stream())
+        p = host(_DeviceBuffer(lib().fs_proj_pressure(h), nx * ny * nz, "cuda").tensor())
+    finally:
+        lib().fs_proj_destroy(h)
+    p, b = p.reshape(shape), host(b).reshape(shape)
+    assert not host(x0).any()
+    DZ = dz[:, None, None]
+    y = -DZ * 1e-6 * p
+    fx = DZ * 0.5 / dx**2 * (ir[:, :, 1:] + ir[:, :, :-1]) * (p[:, :, :-1] - p[:, :, 1:])
+    y[:, :, :-1] += fx
+    y[:, :, 1:] -= fx
+    y[:, :, -1] += dz[:, None] * 2.0 / dx**2 * ir[:, :, -1] * p[:, :, -1]
+    if ny > 1:
+        fy = DZ * 0.5 / dy**2 * (ir + np.roll(ir, -1, 1)) * (p - np.roll(p, -1, 1))
+        y += fy - np.roll(fy, 1, 1)
+    fz = 0.5 / da[:-1, None, None] * (ir[1:] + ir[:-1]) * (p[:-1] - p[1:])
+    y[:-1] += fz
+    y[1:] -= fz
+    y[-1] += 2.0 / dz[-1] * ir[-1] * p[-1]
+    assert np.linalg.norm((b - y) / DZ) <= 1.001e-6 * np.linalg.norm(b / DZ)
+    assert 1 <= its.value <= 25
 
 
 def test_level_set(vectors):
