@@ -73,6 +73,13 @@ struct OpI {
   const T *ir, *tab;
 };
 
+// Level 0's in FP32, stored (the FP64 operator rounded once): what the mixed
+// form's steps have always been preconditioned with.  Formed in FP32 from 1/rho it
+// gives another iterate within the solve's tolerance, and a step's extinction
+// thresholds then fall to the other side in some cells.
+template <typename T>
+struct OpZ : OpA<T> {};
+
 template <typename T>
 struct MGLevelT {
   int nx, ny, nz;
@@ -102,7 +109,6 @@ struct ProjCtx {
   double* p_prev;     // warm start / solution (owned)
   double* ir;         // 1/max(rho, 0.01)
   double* tab;        // level 0's factors (OP_TAB per level)
-  float *ir32, *tab32;
   int have_prev;
   int last_iters;     // CG iterations of the previous solve (batch size hint)
   cudaStream_t cs;    // private stream for graph capture
@@ -137,9 +143,8 @@ struct ProjCtx {
 
 // ---------------------------------------------------------------------------
 // 1/rho (floored) and, by the first block, level 0's factors
-template <typename T>
-__global__ void k_proj_ir(GridDev g, const double* __restrict__ rho, double* ir, T* irT, double* tab,
-                          T* tabT, double dx2, double dy2) {
+__global__ void k_proj_ir(GridDev g, const double* __restrict__ rho, double* ir, double* tab,
+                          double dx2, double dy2) {
   const int64_t n = ncells_dev(g);
   const int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (blockIdx.x == 0) {
@@ -148,18 +153,13 @@ __global__ void k_proj_ir(GridDev g, const double* __restrict__ rho, double* ir,
       const double v[OP_TAB] = {dz * (0.5 / dx2), dz * (0.5 / dy2), 0.5 / g.da[k],
                                 k > 0 ? 0.5 / g.da[k - 1] : 0.0, -dz * PROJ_EPS, dz * (2.0 / dx2),
                                 2.0 / dz, 0.0};
-      for (int q = 0; q < OP_TAB; ++q) {
-        tab[k * OP_TAB + q] = v[q];
-        if (tabT) tabT[k * OP_TAB + q] = (T)v[q];
-      }
+      for (int q = 0; q < OP_TAB; ++q) tab[k * OP_TAB + q] = v[q];
     }
   }
   if (c >= n) return;
   const double r = rho[c];
   const double m = (r >= 0.01 || r != r) ? r : 0.01;
-  const double v = 1.0 / m;
-  ir[c] = v;
-  if (irT) irT[c] = (T)v;
+  ir[c] = 1.0 / m;
 }
 
 // the operator's parts: conductance of the face towards +x, +y, +z of cell c
@@ -202,32 +202,31 @@ __global__ void k_mg_diag(Dims D, Op o, T* dinv) {
   int i, j, k;
   split_cell((uint32_t)c, D.fnx, D.fny, i, j, k);
   int64_t sy = nx, sz = (int64_t)nx * ny;
+  const int64_t r = c - (int64_t)j * sy;
+  const int jp = j + 1 < ny ? j + 1 : 0, jm = j > 0 ? j - 1 : ny - 1;
   T d = op_e(o, c, i, k, nx, nz) + op_fx(o, c, i, k, nx);
-  if (ny > 1) {
-    int jp = j + 1 < ny ? j + 1 : 0, jm = j > 0 ? j - 1 : ny - 1;
-    const int64_t r = c - (int64_t)j * sy;
-    d += op_fy(o, c, r + (int64_t)jp * sy, k);
-    d += op_fy(o, r + (int64_t)jm * sy, c, k);
-  }
+  if (ny > 1) d += op_fy(o, c, r + (int64_t)jp * sy, k);
   d += op_fz(o, c, sz, k, nz);
   if (i > 0) d += op_fx(o, c - 1, i - 1, k, nx);
+  if (ny > 1) d += op_fy(o, r + (int64_t)jm * sy, c, k);
   if (k > 0) d += op_fz(o, c - sz, sz, k - 1, nz);
   dinv[c] = T(1) / d;
 }
 
-// level 0's operator as arrays (only where level 0 is the coarsest level)
+// level 0's operator as arrays (in FP32; in FP64 only where level 0 is the
+// coarsest level)
 template <typename T>
-__global__ void k_op_arrays(Dims D, OpI<T> o, T* gx, T* gy, T* gz, T* e) {
+__global__ void k_op_arrays(Dims D, OpI<double> o, T* gx, T* gy, T* gz, T* e) {
   const int64_t n = (int64_t)D.nx * D.ny * D.nz, sz = (int64_t)D.nx * D.ny;
   const int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (c >= n) return;
   int i, j, k;
   split_cell((uint32_t)c, D.fnx, D.fny, i, j, k);
   const int jp = j + 1 < D.ny ? j + 1 : 0;
-  gx[c] = op_fx(o, c, i, k, D.nx);
-  gy[c] = D.ny > 1 ? op_fy(o, c, c + (int64_t)(jp - j) * D.nx, k) : T(0);
-  gz[c] = op_fz(o, c, sz, k, D.nz);
-  e[c] = op_e(o, c, i, k, D.nx, D.nz);
+  gx[c] = (T)op_fx(o, c, i, k, D.nx);
+  gy[c] = D.ny > 1 ? (T)op_fy(o, c, c + (int64_t)(jp - j) * D.nx, k) : T(0);
+  gz[c] = (T)op_fz(o, c, sz, k, D.nz);
+  e[c] = (T)op_e(o, c, i, k, D.nx, D.nz);
 }
 
 __device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
@@ -670,6 +669,50 @@ __device__ __forceinline__ void z_apply(const Dims& D, const OpI<T>& o, const V&
     y[0] = ya; y[1] = yb;
   }
 }
+template <int W, typename T, typename V>
+__device__ __forceinline__ void z_apply(const Dims& D, const OpA<T>& o, const V& x, int c, int i,
+                                        int j, int k, T (&xc)[W], T (&y)[W]) {
+  const int nx = D.nx, ny = D.ny, nz = D.nz;
+  if constexpr (W == 1) {
+    xc[0] = x.at(c, i, j, k);
+    y[0] = mg_apply(nx, ny, nz, o, x, xc[0], c, i, j, k);
+  } else {
+    const int sy = nx, sz = nx * ny, lane = threadIdx.x & 31;
+    const int jp = j + 1 < ny ? j + 1 : 0, jm = j > 0 ? j - 1 : ny - 1;
+    const int cp = c + (jp - j) * sy, cm = c + (jm - j) * sy;
+    const int kp = min(k + 1, nz - 1), km = max(k - 1, 0);
+    const int ch = c + (kp - k) * sz, cl = c - (k - km) * sz;
+    const Two<T> X = at2(x, c, i, j, k), gx = ld2(o.gx + c), e = ld2(o.e + c);
+    const Two<T> xp = at2(x, cp, i, jp, k), xm = at2(x, cm, i, jm, k);
+    const Two<T> xh = at2(x, ch, i, j, kp), xl = at2(x, cl, i, j, km);
+    const Two<T> gp = ld2(o.gy + c), gm = ld2(o.gy + cm), gh = ld2(o.gz + c), gl = ld2(o.gz + cl);
+    T xe = __shfl_down_sync(0xffffffffu, X.a, 1), xw = __shfl_up_sync(0xffffffffu, X.b, 1);
+    T gw = __shfl_up_sync(0xffffffffu, gx.b, 1);
+    if (lane == 31 && i + 2 < nx) xe = x.at(c + 2, i + 2, j, k);
+    if (lane == 0 && i > 0) { xw = x.at(c - 1, i - 1, j, k); gw = o.gx[c - 1]; }
+    T ya = e.a * X.a, yb = e.b * X.b;
+    ya += gx.a * (X.a - X.b);
+    if (i + 2 < nx) yb += gx.b * (X.b - xe);
+    if (i > 0) ya += gw * (X.a - xw);
+    yb += gx.a * (X.b - X.a);
+    if (ny > 1) {
+      ya += gp.a * (X.a - xp.a);
+      yb += gp.b * (X.b - xp.b);
+      ya += gm.a * (X.a - xm.a);
+      yb += gm.b * (X.b - xm.b);
+    }
+    if (k < nz - 1) {
+      ya += gh.a * (X.a - xh.a);
+      yb += gh.b * (X.b - xh.b);
+    }
+    if (k > 0) {
+      ya += gl.a * (X.a - xl.a);
+      yb += gl.b * (X.b - xl.b);
+    }
+    xc[0] = X.a; xc[1] = X.b;
+    y[0] = ya; y[1] = yb;
+  }
+}
 template <int W, typename T>
 __device__ __forceinline__ void z_load(const T* p, int c, T (&v)[W]) {
   if constexpr (W == 2) {
@@ -687,9 +730,9 @@ __device__ __forceinline__ void z_store(T* p, int c, const T (&v)[W]) {
 
 // damped Jacobi sweep; with DOT the sum of rd * (the new iterate) as well (the
 // V-cycle's last sweep: r.z)
-template <int W, typename T, typename V, bool DOT>
+template <int W, bool DOT, typename T, typename Op, typename V>
 __global__ void __launch_bounds__(Z_THREADS, 4)
-    k_z_jacobi(Dims D, OpI<T> o, const T* __restrict__ dinv, const T* __restrict__ b, V x, T* xo,
+    k_z_jacobi(Dims D, Op o, const T* __restrict__ dinv, const T* __restrict__ b, V x, T* xo,
                double w_, const double* __restrict__ rd, double* partial, const double* done) {
   PCG_SKIP(done);
   const ZCell z = z_cell<W>(D);
@@ -711,9 +754,9 @@ __global__ void __launch_bounds__(Z_THREADS, 4)
 }
 
 // coarse rhs = sum over children of the fine residual, a coarse cell a thread
-template <typename T>
+template <typename T, typename Op>
 __global__ void __launch_bounds__(Z_THREADS, 4)
-    k_z_restrict(Dims D, OpI<T> o, const T* __restrict__ b, const T* __restrict__ x, Dims DC, T* bc,
+    k_z_restrict(Dims D, Op o, const T* __restrict__ b, const T* __restrict__ x, Dims DC, T* bc,
                  const double* done) {
   PCG_SKIP(done);
   const ZCell z = z_cell<1>(DC);
@@ -873,7 +916,7 @@ __global__ void k_fcg_alpha(double* scal) {
 
 // out = b - S x (level operator, any precision)
 template <typename T>
-__global__ void k_lp_residual(Dims D, OpI<T> o, const T* __restrict__ b, const T* __restrict__ x,
+__global__ void k_lp_residual(Dims D, OpZ<T> o, const T* __restrict__ b, const T* __restrict__ x,
                               T* out) {
   const int nx = D.nx, ny = D.ny, nz = D.nz;
   int64_t n = (int64_t)nx * ny * nz;
@@ -1010,7 +1053,6 @@ void* proj_create(const GridDev& g) {
   P->p_prev = dalloc(n0);
   P->ir = dalloc(n0);
   P->tab = dalloc((int64_t)OP_TAB * g.nz);
-  P->ir32 = nullptr; P->tab32 = nullptr;
   {
     // cleared before any solve is queued, on a private stream
     SetupStream ss;
@@ -1064,7 +1106,7 @@ void proj_destroy(void* h) {
   cudaFree(P->Ainv); cudaFree(P->pc_r); cudaFree(P->pc_z); cudaFree(P->pc_p); cudaFree(P->pc_q);
   cudaFree(P->pc_p2);
   cudaFree(P->rhs); cudaFree(P->partial); cudaFree(P->scal); cudaFreeHost(P->h_scal);
-  cudaFree(P->p_prev); cudaFree(P->ir); cudaFree(P->tab); cudaFree(P->ir32); cudaFree(P->tab32);
+  cudaFree(P->p_prev); cudaFree(P->ir); cudaFree(P->tab);
   delete P;
 }
 
@@ -1088,11 +1130,18 @@ static OpA<T> op_a(const MGLevelT<T>& f) {
   return OpA<T>{f.gx, f.gy, f.gz, f.e};
 }
 static OpI<double> op_0(const ProjCtx* P, double) { return OpI<double>{P->ir, P->tab}; }
-static OpI<float> op_0(const ProjCtx* P, float) { return OpI<float>{P->ir32, P->tab32}; }
+static OpZ<float> op_0(const ProjCtx* P, float) {
+  return OpZ<float>{op_a(P->lev32[0])};
+}
 
 template <typename T>
 static void rebuild_levels(ProjCtx* P, MGLevelT<T>* lev, T* Ainv, cudaStream_t st) {
-  const OpI<T> o0 = op_0(P, T(0));
+  if (sizeof(T) == 4 || P->nlev == 1) {
+    MGLevelT<T>& f = lev[0];
+    k_op_arrays<T><<<blocks_for(f.n, 256), 256, 0, st>>>(f.dims, op_0(P, 0.0), f.gx, f.gy, f.gz, f.e);
+    fs_count_launch();
+  }
+  const auto o0 = op_0(P, T(0));
   for (int l = 0; l < P->nlev; ++l) {
     MGLevelT<T>& f = lev[l];
     if (l > 0) {
@@ -1107,10 +1156,6 @@ static void rebuild_levels(ProjCtx* P, MGLevelT<T>* lev, T* Ainv, cudaStream_t s
       k_mg_diag<T><<<blocks_for(f.n, 256), 256, 0, st>>>(f.dims, op_a(f), f.dinv);
     } else {
       k_mg_diag<T><<<blocks_for(f.n, 256), 256, 0, st>>>(f.dims, o0, f.dinv);
-      if (P->nlev == 1) {
-        k_op_arrays<T><<<blocks_for(f.n, 256), 256, 0, st>>>(f.dims, o0, f.gx, f.gy, f.gz, f.e);
-        fs_count_launch();
-      }
     }
     fs_count_launch();
   }
@@ -1126,8 +1171,7 @@ int proj_rebuild(void* h, const double* rho, cudaStream_t st) {
   const GridDev& g = P->g;
   const unsigned nb = blocks_for(P->lev[0].n, 256);
   // the FP64 level-0 operator stays the CG's; the FP32 preconditioner has its own
-  k_proj_ir<float><<<nb, 256, 0, st>>>(g, rho, P->ir, P->fp32 ? P->ir32 : nullptr, P->tab,
-                                       P->fp32 ? P->tab32 : nullptr, g.dx * g.dx, g.dy * g.dy);
+  k_proj_ir<<<nb, 256, 0, st>>>(g, rho, P->ir, P->tab, g.dx * g.dx, g.dy * g.dy);
   fs_count_launch();
   if (P->fp32) rebuild_levels<float>(P, P->lev32, P->Ainv32, st);
   else rebuild_levels<double>(P, P->lev, P->Ainv, st);
@@ -1145,17 +1189,12 @@ int proj_set_precision(void* h, int fp32) {
       lv.nx = ld.nx; lv.ny = ld.ny; lv.nz = ld.nz; lv.n = ld.n; lv.dims = ld.dims;
       float** arrs[9] = {&lv.gx, &lv.gy, &lv.gz, &lv.e, &lv.dinv, &lv.x, &lv.b, &lv.t, &lv.s};
       for (float** a : arrs)
-        // level 0: its operator is formed from 1/rho
-        if (!(l == 0 && P->nlev > 1 && (a == arrs[0] || a == arrs[1] || a == arrs[2] ||
-                                        a == arrs[3])) &&
-            cudaMalloc(a, sizeof(float) * (size_t)(lv.n > 0 ? lv.n : 1)) != cudaSuccess)
+        if (cudaMalloc(a, sizeof(float) * (size_t)(lv.n > 0 ? lv.n : 1)) != cudaSuccess)
           return FS_ECUDA;
     }
     const int64_t nc = P->lev[P->nlev - 1].n;
     if (cudaMalloc(&P->Ainv32, sizeof(float) * (size_t)(nc <= MG_COARSE_MAX ? nc * nc : 1)) !=
             cudaSuccess ||
-        cudaMalloc(&P->ir32, sizeof(float) * P->lev[0].n) != cudaSuccess ||
-        cudaMalloc(&P->tab32, sizeof(float) * OP_TAB * P->lev[0].nz) != cudaSuccess ||
         cudaMalloc(&P->r32, sizeof(float) * P->lev[0].n) != cudaSuccess ||
         cudaMalloc(&P->z32, sizeof(float) * P->lev[0].n) != cudaSuccess)
       return FS_ECUDA;
@@ -1341,22 +1380,20 @@ static void launch_finish(ProjCtx* P, int nb, int slot, int post, const double* 
   k_finish_sum<<<1, FIN_THREADS, 0, st>>>(P->partial, nb, P->scal, slot, post, done);
 }
 // a sweep and a restriction on level 0 and on the others (returns the launches)
-template <int W, typename T, typename V>
-static int launch_z_jacobi(ProjCtx* P, const Dims& D, const OpI<T>& o, const T* dinv, const T* b, V x,
+template <int W, typename T, typename Op, typename V>
+static int launch_z_jacobi(ProjCtx* P, const Dims& D, const Op& o, const T* dinv, const T* b, V x,
                            T* xo, double w, bool dot, const double* done, cudaStream_t st) {
   const int nb = z_blocks(D);
   if (!dot) {
-    k_z_jacobi<W, T, V, false><<<nb, Z_THREADS, 0, st>>>(D, o, dinv, b, x, xo, w, nullptr, nullptr,
-                                                         done);
+    k_z_jacobi<W, false, T><<<nb, Z_THREADS, 0, st>>>(D, o, dinv, b, x, xo, w, nullptr, nullptr, done);
     return 1;
   }
-  k_z_jacobi<W, T, V, true><<<nb, Z_THREADS, 0, st>>>(D, o, dinv, b, x, xo, w, P->pc_r, P->partial,
-                                                      done);
+  k_z_jacobi<W, true, T><<<nb, Z_THREADS, 0, st>>>(D, o, dinv, b, x, xo, w, P->pc_r, P->partial, done);
   launch_finish(P, nb, 2, POST_NONE, done, st);  // rz_new
   return 2;
 }
-template <typename T, typename V>
-static int launch_jacobi(ProjCtx* P, const Dims& D, const OpI<T>& o, const T* dinv, const T* b, V x,
+template <typename T, typename V, typename Op>
+static int launch_jacobi(ProjCtx* P, const Dims& D, const Op& o, const T* dinv, const T* b, V x,
                          T* xo, double w, bool dot, const double* done, cudaStream_t st) {
   return z_width(D) == 2 ? launch_z_jacobi<2>(P, D, o, dinv, b, x, xo, w, dot, done, st)
                          : launch_z_jacobi<1>(P, D, o, dinv, b, x, xo, w, dot, done, st);
@@ -1374,8 +1411,8 @@ static void launch_restrict(const Dims& D, const OpA<T>& o, const T* b, const T*
   k_mg_restrict_residual<T><<<blocks_for((int64_t)DC.nx * DC.ny * DC.nz, 128), 128, 0, st>>>(
       D, o, b, x, DC, bc, done);
 }
-template <typename T>
-static void launch_restrict(const Dims& D, const OpI<T>& o, const T* b, const T* x, const Dims& DC,
+template <typename T, typename Op>
+static void launch_restrict(const Dims& D, const Op& o, const T* b, const T* x, const Dims& DC,
                             T* bc, const double* done, cudaStream_t st) {
   const unsigned nc = blocks_for((int64_t)DC.nx * DC.ny * DC.nz, Z_THREADS);
   if (z_width(D) == 2)
