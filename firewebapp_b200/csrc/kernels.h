@@ -181,8 +181,7 @@ int launch_coldiag(const GridDev& g, const double* Ts, const double* om, const d
                    const double* Sd, double T_ign, double T_front, double scale, double* hrr_x,
                    void* scratch, cudaStream_t st);
 int launch_coldiag_keys(const void* scratch, double* out4, cudaStream_t st);
-// stencil kernels with TMA-staged inputs: the bounded-wait failure flag
-// (read, optionally cleared; -1 on a CUDA error) and the on/off switch
+// kept entry points of a former staged form (fs_stencil_status, fs_set_tma)
 int stencil_status(int clear);
 void set_tma(int on);
 int launch_edc_carry(int nb, const signed char* agg, signed char* carry, cudaStream_t st);

@@ -1,0 +1,139 @@
+// Z-marching stencils: a block owns a 32 (x) by 8 (y) tile of columns and
+// marches up a chunk of levels; the planes its stencil reads, with their x and
+// y halos, pass through a ring of shared-memory slots, each value fetched once
+// a block by cp.async while the levels before it compute.
+//
+// The copies are of single elements: rows need no alignment, the periodic wrap
+// in y is part of a thread's fixed offset, and any grid size takes this path.
+// Planes below the ground or above the top repeat the nearest one, columns
+// outside in x the nearest column (the stencils do not use them).
+#pragma once
+#include "common.cuh"
+
+#define MR_TX 32
+#define MR_TY 8
+#define MR_THREADS (MR_TX * MR_TY)
+#define MR_MAXK 64
+
+template <int BYTES>
+__device__ __forceinline__ void copy_async(uint32_t dst, const void* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(dst), "l"(src), "n"(BYTES)
+               : "memory");
+}
+__device__ __forceinline__ void copy_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+// all but the newest N groups have landed
+template <int N>
+__device__ __forceinline__ void copy_wait() {
+  asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
+
+// NF fields of element type T with a halo of R, SLOTS planes
+template <typename T, int NF, int R, int SLOTS>
+struct PlaneRing {
+  static constexpr int HX = MR_TX + 2 * R, HY = MR_TY + 2 * R, PLANE = HX * HY;
+  static constexpr int PER = (PLANE + MR_THREADS - 1) / MR_THREADS;
+  static constexpr int BYTES = SLOTS * NF * PLANE * (int)sizeof(T);
+  uint32_t dst;
+  int off[PER];  // of this thread's elements in a plane
+  int last;      // it has the last of them
+  __device__ __forceinline__ void init(T* base, const GridDev& g) {
+    const int tid = threadIdx.y * MR_TX + threadIdx.x;
+    dst = (uint32_t)__cvta_generic_to_shared(base) + tid * (int)sizeof(T);
+#pragma unroll
+    for (int q = 0; q < PER; ++q) {
+      const int e = tid + q * MR_THREADS;
+      const int i = (int)blockIdx.x * MR_TX - R + e % HX;
+      const int j = wrapj((int)blockIdx.y * MR_TY - R + e / HX, g.ny);
+      off[q] = j * g.nx + min(max(i, 0), g.nx - 1);
+    }
+    last = tid + (PER - 1) * MR_THREADS < PLANE;
+  }
+  // plane p of every field into a slot
+  __device__ __forceinline__ void load(const GridDev& g, const T* const (&f)[NF], int p, int slot) {
+    const int64_t pl = (int64_t)min(max(p, 0), g.nz - 1) * ((int64_t)g.nx * g.ny);
+    const uint32_t d = dst + slot * (NF * PLANE * (int)sizeof(T));
+#pragma unroll
+    for (int s = 0; s < NF; ++s)
+#pragma unroll
+      for (int q = 0; q < PER; ++q)
+        if (q < PER - 1 || last)
+          copy_async<(int)sizeof(T)>(d + (s * PLANE + q * MR_THREADS) * (int)sizeof(T),
+                                     f[s] + pl + off[q]);
+  }
+  // slot s + d (0 <= s < SLOTS, |d| < SLOTS), and its first element from base
+  static __device__ __forceinline__ int slot(int s, int d) {
+    const int t = s + d;
+    return t < 0 ? t + SLOTS : (t >= SLOTS ? t - SLOTS : t);
+  }
+  static __device__ __forceinline__ const T* at(const T* base, int s) {
+    return base + s * (NF * PLANE) + (threadIdx.y + R) * HX + threadIdx.x + R;
+  }
+};
+
+// Levels a block marches.  A block alone on its SM takes about twice the time
+// a level that it takes of a full one's, and two levels' worth before the first:
+// the chunk count with the least (blocks an SM + 1) x (levels + 2).  At
+// 400 x 120 x 60 that is 10 levels (momentum 104 us; 106 with 5, 110 with 15, 119
+// with 30), at 64 x 24 x 20 one.
+inline int march_levels(const GridDev& g) {
+  const int tiles = ((g.nx + MR_TX - 1) / MR_TX) * ((g.ny + MR_TY - 1) / MR_TY);
+  int best = 1;
+  int64_t least = INT64_MAX;
+  for (int kz = 1; kz <= g.nz && kz <= MR_MAXK; ++kz) {
+    const int64_t blocks = (int64_t)tiles * ((g.nz + kz - 1) / kz);
+    const int64_t cost = ((blocks + 147) / 148 + 1) * (kz + 2);
+    if (cost < least) {
+      least = cost;
+      best = kz;
+    }
+  }
+  return best;
+}
+inline dim3 march_grid(const GridDev& g, int kz) {
+  return dim3((g.nx + MR_TX - 1) / MR_TX, (g.ny + MR_TY - 1) / MR_TY, (g.nz + kz - 1) / kz);
+}
+
+// the shared memory a marching kernel may ask for (set on every call: the
+// attribute belongs to the current device)
+inline bool march_smem(const void* kernel, int bytes) {
+  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) ==
+         cudaSuccess;
+}
+
+// The reciprocal spacings of a chunk's levels, MR_RK a level: face above, face
+// below, cell, mean of the faces, and the vertical difference of the strain
+// and of the buoyancy (one-sided at the ground and the top).
+#define MR_RK 5
+template <typename T>
+__device__ __forceinline__ void march_spacings(const GridDev& g, int k0, int k1, T* rk) {
+  for (int q = threadIdx.y * MR_TX + threadIdx.x; q < k1 - k0; q += MR_THREADS) {
+    const int k = k0 + q;
+    const double da = g.da[k], db = g.db[k];
+    rk[q * MR_RK + 0] = (T)(1.0 / da);
+    rk[q * MR_RK + 1] = (T)(1.0 / db);
+    rk[q * MR_RK + 2] = (T)(1.0 / g.dz[k]);
+    rk[q * MR_RK + 3] = (T)(1.0 / (0.5 * (da + db)));
+    rk[q * MR_RK + 4] = (T)(1.0 / (k == 0 ? da : (k == g.nz - 1 ? db : da + db)));
+  }
+}
+
+// The smaller of two differences of one sign, else 0 (minmod)
+template <typename T>
+__device__ __forceinline__ T minmod_pair(T a, T b) {
+  const T m = (fabs(b) < fabs(a)) ? b : a;
+  return (a * b <= T(0)) ? T(0) : m;
+}
+// The difference of a cell's two MUSCL face values along one direction, over
+// the sign of the velocity: |uf| times it is uf (f+ - f-).  dp, dm: the
+// differences to the neighbours in + and - direction; N the upwind neighbour and
+// F the one beyond it.  Of the two limiters one is of dp and dm whichever way
+// the wind blows, so a cell needs three differences and two limiters where face
+// by face it took four to six differences and as many selections.
+template <typename T>
+__device__ __forceinline__ T muscl_diff(T dp, T dm, T C, T N, T F, bool up) {
+  const T h = up ? T(0.5) : T(-0.5);
+  const T d = up ? N - F : F - N;
+  const T a = C + h * minmod_pair(dp, dm);
+  const T b = N + h * minmod_pair(up ? dm : dp, d);
+  return a - b;
+}

@@ -14,6 +14,7 @@
 // clip), the turbulent diffusion sub-iteration (turbulence_3d.py:862-949)
 // and the Lagrangian-branch gas-energy update (spread_3d.py:3088-3146).
 #include "common.cuh"
+#include "substep_march.cuh"
 #include "kernels.h"
 
 // ---- conversions -------------------------------------------------------------
@@ -260,109 +261,12 @@ int launch_edc32(int64_t n, const float* rho, float* Tg, float* Yf, float* YO, c
   return cuda_status();
 }
 
-// ---- species step ------------------------------------------------------------
-// minmod and the MUSCL face value in float (the FP64 helpers' forms)
-__device__ __forceinline__ float minmod32(float a, float b) {
-  const float m = copysignf(fminf(fabsf(a), fabsf(b)), a);
-  return (a * b <= 0.0f) ? 0.0f : m;
-}
-
-__device__ __forceinline__ float muscl_face32(float pim1, float pi, float pip1, float pip2,
-                                              float uf) {
-  const bool up = uf >= 0.0f;
-  const float m = minmod32(pip1 - pi, up ? pi - pim1 : pip2 - pip1);
-  const float base = up ? pi : pip1;
-  const float half = up ? 0.5f : -0.5f;
-  return base + half * m;
-}
-
-#define S32_TX 32
-#define S32_TY 8
-struct Species32Args {
-  const float* Y[3];
-  float* Yo[3];
-  float Y_inlet[3];
-  const float *Sp, *Sd, *rho, *u, *v, *w;
-  float dt, D, inv_dx, inv_dy, inv_dx2, inv_dy2, o2_cap;
-};
-
-__global__ void __launch_bounds__(S32_TX * S32_TY, 4) k_species32(GridDev g, Species32Args a) {
-  __shared__ float rk[4];  // 1/da, 1/db, 1/dz, 1/hz of the block's level
-  const int nx = g.nx, ny = g.ny, nz = g.nz;
-  const int64_t sy = nx, sz = (int64_t)nx * ny;
-  const int k = blockIdx.z;
-  if (threadIdx.x == 0 && threadIdx.y == 0) {
-    const double da = g.da[k], db = g.db[k];
-    rk[0] = (float)(1.0 / da);
-    rk[1] = (float)(1.0 / db);
-    rk[2] = (float)(1.0 / g.dz[k]);
-    rk[3] = (float)(1.0 / (0.5 * (da + db)));
-  }
-  __syncthreads();
-  const int i = blockIdx.x * S32_TX + threadIdx.x;
-  const int j = blockIdx.y * S32_TY + threadIdx.y;
-  if (i >= nx || j >= ny) return;
-  const int64_t crow = (int64_t)k * sz + i;
-  const int64_t c = crow + (int64_t)j * sy;
-  const int jm2 = wrapj(j - 2, ny), jm1 = wrapj(j - 1, ny);
-  const int jp1 = wrapj(j + 1, ny), jp2 = wrapj(j + 2, ny);
-  const float ui = a.u[c], vi = a.v[c], wi = a.w[c];
-  const float inv_rho = 1.0f / a.rho[c];
-  const float inv_d_above = rk[0], inv_d_below = rk[1], inv_dz_k = rk[2], inv_hz = rk[3];
-  const float sp = a.Sp[c], sd = a.Sd[c];
-  const float stot = sp + sd;
-  const bool mx = (i >= 2 && i <= nx - 3);
-  const bool mz = (k >= 2 && k <= nz - 3);
-#pragma unroll
-  for (int s = 0; s < 3; ++s) {
-    const float* __restrict__ Y = a.Y[s];
-    const float Yi = Y[c];
-    const float YL_x = (i == 0) ? a.Y_inlet[s] : Y[c - 1];
-    const float YR_x = (i == nx - 1) ? Yi : Y[c + 1];
-    const float YL_z = (k == 0) ? Yi : Y[c - sz];
-    const float YR_z = (k == nz - 1) ? Yi : Y[c + sz];
-    float flux_x, flux_z;
-    if (mx) {
-      const float fxp = muscl_face32(Y[c - 1], Yi, Y[c + 1], Y[c + 2], ui);
-      const float fxm = muscl_face32(Y[c - 2], Y[c - 1], Yi, Y[c + 1], ui);
-      flux_x = ui * (fxp - fxm) * a.inv_dx;
-    } else {
-      flux_x = (ui >= 0.0f) ? ui * (Yi - YL_x) * a.inv_dx : ui * (YR_x - Yi) * a.inv_dx;
-    }
-    const float Yjm2 = Y[crow + jm2 * sy], Yjm1 = Y[crow + jm1 * sy];
-    const float Yjp1 = Y[crow + jp1 * sy], Yjp2 = Y[crow + jp2 * sy];
-    const float fyp = muscl_face32(Yjm1, Yi, Yjp1, Yjp2, vi);
-    const float fym = muscl_face32(Yjm2, Yjm1, Yi, Yjp1, vi);
-    const float flux_y = vi * (fyp - fym) * a.inv_dy;
-    if (mz) {
-      const float fzp = muscl_face32(Y[c - sz], Yi, Y[c + sz], Y[c + 2 * sz], wi);
-      const float fzm = muscl_face32(Y[c - 2 * sz], Y[c - sz], Yi, Y[c + sz], wi);
-      flux_z = wi * (fzp - fzm) * inv_hz;
-    } else {
-      flux_z = (wi >= 0.0f) ? wi * (Yi - YL_z) * inv_d_below : wi * (YR_z - Yi) * inv_d_above;
-    }
-    const float adv = -(flux_x + flux_y + flux_z);
-    const float d2x = (YR_x - 2.0f * Yi + YL_x) * a.inv_dx2;
-    const float d2y = (Yjp1 - 2.0f * Yi + Yjm1) * a.inv_dy2;
-    const float d2z = ((YR_z - Yi) * inv_d_above - (Yi - YL_z) * inv_d_below) * inv_dz_k;
-    const float diff = a.D * (d2x + d2y + d2z);
-    const float S = (s == 0) ? sp - Yi * stot : ((s == 1) ? -(Yi * stot) : sd - Yi * stot);
-    float nw = Yi + (adv + diff + S * inv_rho) * a.dt;
-    if (nw < 0.0f) nw = 0.0f;
-    else if (nw > 1.0f) nw = 1.0f;
-    if (s == 1) {
-      if (nw > a.o2_cap) nw = a.o2_cap;
-      if (nw < 0.0f) nw = 0.0f;
-    }
-    a.Yo[s][c] = nw;
-  }
-}
-
+// ---- species step and turbulent diffusion (the kernels: substep_march.cuh) -----
 int launch_species_step32(const GridDev& g, const float* const* Y, float* const* Yo,
                           const float* Sp, const float* Sd, const double* Y_inlet,
                           const float* rho, const float* u, const float* v, const float* w,
                           double dt, double D, double o2_cap, cudaStream_t st) {
-  Species32Args a{};
+  SpeciesArgs<float> a{};
   for (int s = 0; s < 3; ++s) {
     a.Y[s] = Y[s];
     a.Yo[s] = Yo[s];
@@ -372,94 +276,18 @@ int launch_species_step32(const GridDev& g, const float* const* Y, float* const*
   a.dt = (float)dt; a.D = (float)D; a.o2_cap = (float)o2_cap;
   a.inv_dx = (float)(1.0 / g.dx); a.inv_dy = (float)(1.0 / g.dy);
   a.inv_dx2 = (float)(1.0 / (g.dx * g.dx)); a.inv_dy2 = (float)(1.0 / (g.dy * g.dy));
-  const dim3 nb((g.nx + S32_TX - 1) / S32_TX, (g.ny + S32_TY - 1) / S32_TY, g.nz);
-  k_species32<<<nb, dim3(S32_TX, S32_TY), 0, st>>>(g, a);
-  fs_count_launch();
-  return cuda_status();
-}
-
-// ---- turbulent diffusion -----------------------------------------------------
-struct Diff32Args {
-  const float* f[4];
-  float* fo[4];
-  float lo[4], hi[4];
-  int clip;
-};
-
-// A block owns a 32 x 8 tile and marches up a chunk of z-levels (the FP64
-// kernel's scheme): the column's k-1, k, k+1 values stay in registers and
-// level k+2 is requested while level k computes.
-#define TD32_MAXKZ 64
-template <int NF>
-__global__ void __launch_bounds__(S32_TX * S32_TY, 4)
-    k_turb_diff32(GridDev g, Diff32Args a, const float* __restrict__ nu_t, float inv_sc,
-                  float dt_sub, float inv_dx2, float inv_dy2, int kz) {
-  __shared__ float rk[TD32_MAXKZ][3];
-  const int nx = g.nx, ny = g.ny, nz = g.nz;
-  const int64_t sy = nx, sz = (int64_t)nx * ny;
-  const int k0 = blockIdx.z * kz;
-  const int k1 = min(nz, k0 + kz);
-  const int tid = threadIdx.y * S32_TX + threadIdx.x;
-  for (int q = tid; q < k1 - k0; q += S32_TX * S32_TY) {
-    rk[q][0] = (float)(1.0 / g.dz[k0 + q]);
-    rk[q][1] = (float)(1.0 / g.da[k0 + q]);
-    rk[q][2] = (float)(1.0 / g.db[k0 + q]);
-  }
-  __syncthreads();
-  const int i = blockIdx.x * S32_TX + threadIdx.x;
-  const int j = blockIdx.y * S32_TY + threadIdx.y;
-  if (i >= nx || j >= ny || k0 >= nz) return;
-  const int64_t col = (int64_t)j * sy + i;
-  const int64_t cjp0 = (int64_t)wrapj(j + 1, ny) * sy + i, cjm0 = (int64_t)wrapj(j - 1, ny) * sy + i;
-  float fL[NF], fC[NF], fN[NF];
-#pragma unroll
-  for (int s = 0; s < NF; ++s) {
-    fC[s] = a.f[s][(int64_t)k0 * sz + col];
-    fL[s] = (k0 == 0) ? fC[s] : a.f[s][(int64_t)(k0 - 1) * sz + col];
-    fN[s] = (k0 == nz - 1) ? fC[s] : a.f[s][(int64_t)(k0 + 1) * sz + col];
-  }
-  float nu_c = nu_t[(int64_t)k0 * sz + col];
-  for (int k = k0; k < k1; ++k) {
-    const int64_t ks = (int64_t)k * sz;
-    const int64_t c = ks + col;
-    const bool more = k + 1 < k1;
-    float nu_n = 0.0f, fNN[NF];
-    if (more) nu_n = nu_t[c + sz];
-#pragma unroll
-    for (int s = 0; s < NF; ++s)
-      fNN[s] = (more && k + 2 < nz) ? a.f[s][c + 2 * sz] : fN[s];
-    const float D_t = nu_c * inv_sc;
-    const float r0 = rk[k - k0][0], r1 = rk[k - k0][1], r2 = rk[k - k0][2];
-#pragma unroll
-    for (int s = 0; s < NF; ++s) {
-      const float* __restrict__ f = a.f[s];
-      const float fc = fC[s];
-      const float fxL = (i == 0) ? fc : f[c - 1];
-      const float fxR = (i == nx - 1) ? fc : f[c + 1];
-      const float fzL = fL[s];
-      const float fzR = fN[s];
-      const float d2x = (fxR - 2.0f * fc + fxL) * inv_dx2;
-      const float d2y = (f[ks + cjp0] - 2.0f * fc + f[ks + cjm0]) * inv_dy2;
-      const float d2z = ((fzR - fc) * r1 - (fc - fzL) * r2) * r0;
-      float nv = fc + D_t * (d2x + d2y + d2z) * dt_sub;
-      if (a.clip) {
-        if (nv < a.lo[s]) nv = a.lo[s];
-        if (nv > a.hi[s]) nv = a.hi[s];
-      }
-      a.fo[s][c] = nv;
-      fL[s] = fc;
-      fC[s] = fzR;
-      fN[s] = fNN[s];
-    }
-    nu_c = nu_n;
-  }
+  return launch_species_march<float, 3, true>(g, a, st);
 }
 
 int launch_turb_diff32(const GridDev& g, int nfield, const float* const* f, float* const* fo,
                        const float* nu_t, double sc_t, double dt_sub, int clip, const double* lo,
                        const double* hi, cudaStream_t st) {
   if (nfield != 1 && nfield != 3) return FS_EARG;
-  Diff32Args a{};
+  DiffArgs<float> a{};
+  a.nu_t = nu_t;
+  a.inv_sc = (float)(1.0 / sc_t);
+  a.dt = (float)dt_sub;
+  a.inv_dx2 = (float)(1.0 / (g.dx * g.dx)); a.inv_dy2 = (float)(1.0 / (g.dy * g.dy));
   a.clip = clip;
   for (int s = 0; s < nfield; ++s) {
     a.f[s] = f[s];
@@ -467,26 +295,7 @@ int launch_turb_diff32(const GridDev& g, int nfield, const float* const* f, floa
     a.lo[s] = clip ? (float)lo[s] : 0.0f;
     a.hi[s] = clip ? (float)hi[s] : 0.0f;
   }
-  // z-chunks: about six blocks per SM of the 148, at least four levels each
-  const int tiles = ((g.nx + S32_TX - 1) / S32_TX) * ((g.ny + S32_TY - 1) / S32_TY);
-  int chunks = (6 * 148 + tiles - 1) / tiles;
-  if (chunks > g.nz) chunks = g.nz;
-  if (chunks < 1) chunks = 1;
-  int kz = (g.nz + chunks - 1) / chunks;
-  if (kz < 4) kz = g.nz < 4 ? g.nz : 4;
-  if (kz > TD32_MAXKZ) kz = TD32_MAXKZ;
-  chunks = (g.nz + kz - 1) / kz;
-  const dim3 nb((g.nx + S32_TX - 1) / S32_TX, (g.ny + S32_TY - 1) / S32_TY, chunks);
-  const dim3 tb(S32_TX, S32_TY);
-  const float ix2 = (float)(1.0 / (g.dx * g.dx)), iy2 = (float)(1.0 / (g.dy * g.dy));
-  if (nfield == 1)
-    k_turb_diff32<1><<<nb, tb, 0, st>>>(g, a, nu_t, (float)(1.0 / sc_t), (float)dt_sub, ix2, iy2,
-                                        kz);
-  else
-    k_turb_diff32<3><<<nb, tb, 0, st>>>(g, a, nu_t, (float)(1.0 / sc_t), (float)dt_sub, ix2, iy2,
-                                        kz);
-  fs_count_launch();
-  return cuda_status();
+  return nfield == 1 ? launch_turb_march<float, 1>(g, a, st) : launch_turb_march<float, 3>(g, a, st);
 }
 
 // ---- gas-energy update -------------------------------------------------------

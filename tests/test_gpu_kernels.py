@@ -13,6 +13,8 @@ compared the way the reference's own vectors intend: operator and divergence
 elementwise, the projected field through its divergence residual.
 """
 import ctypes as C
+import importlib.util
+import pathlib
 
 import numpy as np
 import pytest
@@ -862,6 +864,31 @@ def test_projection_solves_the_numpy_system(nx, ny, nz, nu, fp32):
     y[-1] += 2.0 / dz[-1] * ir[-1] * p[-1]
     assert np.linalg.norm((b - y) / DZ) <= 1.001e-6 * np.linalg.norm(b / DZ)
     assert 1 <= its.value <= 25
+
+
+@pytest.mark.parametrize("form", ["plain", "mixed"])
+@pytest.mark.parametrize("nx, ny, nz", [(33, 9, 12), (31, 1, 7), (64, 8, 4), (65, 2, 13),
+                                        (96, 24, 5), (98, 25, 17)])
+def test_marching_stencils_against_exact_forms(nx, ny, nz, form):
+    """The marching kernels (momentum, k-epsilon, gas energy; species and
+    turbulent diffusion in both precisions) on tiles that are full, ragged and
+    one column over, with periodic rows wrapped more than once (1 and 2 rows)
+    and chunks of one and several levels, against the FP64 tensor forms of the
+    workload cases.  About 200 operations a cell, each within 2^-53 (2^-24) of
+    terms no larger than 30 times the result: 1e-12 (5e-4 would be the FP32
+    worst case; independent roundings add as sqrt(200) x 30 x 2^-24 = 3e-5)."""
+    spec = importlib.util.spec_from_file_location(
+        "workload_cases", pathlib.Path(__file__).parents[1] / "perf" / "cases.py")
+    cases = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(cases)
+    kinds = ["substep"] + (["explicit"] if form == "plain" else [])
+    for kind in kinds:
+        case = dict(name=kind, kind=kind, nx=nx, ny=ny, nz=nz, order=4, form=form)
+        got = cases.run(cases.prepare(case, 11))
+        ref = cases.exact(case, 11)
+        for name, want in ref.items():
+            err = rel_l2(host(got[name]).astype(np.float64).ravel(), host(want).ravel())
+            assert err <= (1e-12 if form == "plain" else 3e-5), (kind, name, err)
 
 
 def test_level_set(vectors):
