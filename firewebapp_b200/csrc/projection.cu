@@ -43,6 +43,7 @@
 // Kernels of a PCG iteration return at once when the solve has converged,
 // so iterations queued past convergence change nothing.
 #define PCG_SKIP(done) \
+  FOLLOW();            \
   if ((done) && *(done) != 0.0) return;
 
 // a level's extents with the divisions that recover (i, j, k) from a flat index
@@ -143,8 +144,9 @@ struct ProjCtx {
 
 // ---------------------------------------------------------------------------
 // 1/rho (floored) and, by the first block, level 0's factors
-__global__ void k_proj_ir(GridDev g, const double* __restrict__ rho, double* ir, double* tab,
+__global__ void k_proj_ir(GridDev g, const double* rho, double* ir, double* tab,
                           double dx2, double dy2) {
+  FOLLOW();
   const int64_t n = ncells_dev(g);
   const int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (blockIdx.x == 0) {
@@ -195,6 +197,7 @@ __device__ __forceinline__ T op_e(const OpI<T>& o, int64_t c, int i, int k, int 
 // diagonal of the operator -> 1/diag
 template <typename T, typename Op>
 __global__ void k_mg_diag(Dims D, Op o, T* dinv) {
+  FOLLOW();
   const int nx = D.nx, ny = D.ny, nz = D.nz;
   int64_t n = (int64_t)nx * ny * nz;
   int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
@@ -217,6 +220,7 @@ __global__ void k_mg_diag(Dims D, Op o, T* dinv) {
 // coarsest level)
 template <typename T>
 __global__ void k_op_arrays(Dims D, OpI<double> o, T* gx, T* gy, T* gz, T* e) {
+  FOLLOW();
   const int64_t n = (int64_t)D.nx * D.ny * D.nz, sz = (int64_t)D.nx * D.ny;
   const int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (c >= n) return;
@@ -283,8 +287,8 @@ template <typename T, typename V>
 __device__ __forceinline__ T mg_apply(int nx, int ny, int nz, const OpI<T>& o, const V& x, T xc,
                                       int c, int i, int j, int k) {
   const int sy = nx, sz = nx * ny;
-  const T* __restrict__ ir = o.ir;
-  const T* __restrict__ tb = o.tab + k * OP_TAB;
+  const T* ir = o.ir;
+  const T* tb = o.tab + k * OP_TAB;
   const T r = ir[c], hx = tb[0], hy = tb[1];
   T e = tb[4];
   if (i == nx - 1) e += tb[5] * r;
@@ -309,6 +313,7 @@ __device__ __forceinline__ T mg_apply(int nx, int ny, int nz, const OpI<T>& o, c
 template <typename T, typename Op>
 __global__ void k_mg_coarsen(int fx, int fy, int fz, Op o, Dims DC, T* gxc, T* gyc, T* gzc, T* ec,
                              double scale_) {
+  FOLLOW();
   const int cx = DC.nx, cy = DC.ny, cz = DC.nz;
   int64_t n = (int64_t)cx * cy * cz;
   int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
@@ -316,30 +321,31 @@ __global__ void k_mg_coarsen(int fx, int fy, int fz, Op o, Dims DC, T* gxc, T* g
   int I, J, K;
   split_cell((uint32_t)q, DC.fnx, DC.fny, I, J, K);
   const int64_t fsy = fx, fsz = (int64_t)fx * fy;
-  int i0 = 2 * I, i1 = min(2 * I + 1, fx - 1);
-  int j0 = 2 * J, j1 = min(2 * J + 1, fy - 1);
-  int k0 = 2 * K, k1 = min(2 * K + 1, fz - 1);
+  const int i0 = 2 * I, i1 = min(2 * I + 1, fx - 1);
+  const int j0 = 2 * J, j1 = min(2 * J + 1, fy - 1);
+  const int k0 = 2 * K, k1 = min(2 * K + 1, fz - 1);
+  const int jp = j1 + 1 < fy ? j1 + 1 : 0;
   T se = 0.0, sx = 0.0, sy = 0.0, sz = 0.0;
-  for (int k = k0; k <= k1; ++k)
-    for (int j = j0; j <= j1; ++j)
-      for (int i = i0; i <= i1; ++i)
-        se += op_e(o, (int64_t)k * fsz + (int64_t)j * fsy + i, i, k, fx, fz);
-  if (I < cx - 1) {
-    for (int k = k0; k <= k1; ++k)
-      for (int j = j0; j <= j1; ++j)
-        sx += op_fx(o, (int64_t)k * fsz + (int64_t)j * fsy + i1, i1, k, fx);
+  // (every load at a clamped index and none behind a branch: all are in flight at
+  // once, where loops up to the extents took 9 to 12 us on the smallest levels)
+#pragma unroll
+  for (int d = 0; d < 8; ++d) {
+    const int k = min(k0 + (d >> 2), k1), j = min(j0 + ((d >> 1) & 1), j1), i = min(i0 + (d & 1), i1);
+    const T v = op_e(o, (int64_t)k * fsz + (int64_t)j * fsy + i, i, k, fx, fz);
+    if (k == k0 + (d >> 2) && j == j0 + ((d >> 1) & 1) && i == i0 + (d & 1)) se += v;
   }
-  if (cy > 1) {
-    const int jp = j1 + 1 < fy ? j1 + 1 : 0;
-    for (int k = k0; k <= k1; ++k)
-      for (int i = i0; i <= i1; ++i)
-        sy += op_fy(o, (int64_t)k * fsz + (int64_t)j1 * fsy + i,
-                    (int64_t)k * fsz + (int64_t)jp * fsy + i, k);
-  }
-  if (K < cz - 1) {
-    for (int j = j0; j <= j1; ++j)
-      for (int i = i0; i <= i1; ++i)
-        sz += op_fz(o, (int64_t)k1 * fsz + (int64_t)j * fsy + i, fsz, k1, fz);
+#pragma unroll
+  for (int d = 0; d < 4; ++d) {
+    const int a = d >> 1, b = d & 1;
+    const int ka = min(k0 + a, k1), ja = min(j0 + a, j1), jb = min(j0 + b, j1), ib = min(i0 + b, i1);
+    const int64_t ck = (int64_t)ka * fsz;
+    const T vx = op_fx(o, ck + (int64_t)jb * fsy + i1, i1, ka, fx);
+    const T vy = op_fy(o, ck + (int64_t)j1 * fsy + ib, ck + (int64_t)jp * fsy + ib, ka);
+    const T vz = op_fz(o, (int64_t)k1 * fsz + (int64_t)ja * fsy + ib, fsz, k1, fz);
+    const bool ka_in = ka == k0 + a, ja_in = ja == j0 + a, jb_in = jb == j0 + b, ib_in = ib == i0 + b;
+    if (I < cx - 1 && ka_in && jb_in) sx += vx;
+    if (cy > 1 && ka_in && ib_in) sy += vy;
+    if (K < cz - 1 && ja_in && ib_in) sz += vz;
   }
   const T scale = (T)scale_;
   gxc[q] = scale * sx;
@@ -350,9 +356,10 @@ __global__ void k_mg_coarsen(int fx, int fy, int fz, Op o, Dims DC, T* gxc, T* g
 
 // Dense inverse of the coarsest operator (Gauss-Jordan in shared memory, n <= 64).
 template <typename T>
-__global__ void k_mg_coarse_inverse(int nx, int ny, int nz, const T* __restrict__ gx,
-                                    const T* __restrict__ gy, const T* __restrict__ gz,
-                                    const T* __restrict__ e, T* Ainv) {
+__global__ void k_mg_coarse_inverse(int nx, int ny, int nz, const T* gx,
+                                    const T* gy, const T* gz,
+                                    const T* e, T* Ainv) {
+  FOLLOW();
   __shared__ T M[MG_COARSE_MAX][2 * MG_COARSE_MAX + 1];
   const int n = nx * ny * nz;
   const int t = threadIdx.x;
@@ -399,8 +406,8 @@ __global__ void k_mg_coarse_inverse(int nx, int ny, int nz, const T* __restrict_
 }
 
 template <typename T>
-__global__ void k_mg_coarse_solve(int n, const T* __restrict__ Ainv,
-                                  const T* __restrict__ b, T* x, const double* done) {
+__global__ void k_mg_coarse_solve(int n, const T* Ainv,
+                                  const T* b, T* x, const double* done) {
   PCG_SKIP(done);
   int r = threadIdx.x;
   if (r >= n) return;
@@ -411,7 +418,7 @@ __global__ void k_mg_coarse_solve(int n, const T* __restrict__ Ainv,
 
 // damped Jacobi sweep: xo = x + w (b - S x) / d
 template <typename T, typename Op, typename V>
-__global__ void k_mg_jacobi(Dims D, Op o, const T* __restrict__ dinv, const T* __restrict__ b, V x,
+__global__ void k_mg_jacobi(Dims D, Op o, const T* dinv, const T* b, V x,
                             T* xo, double w_, const double* done) {
   PCG_SKIP(done);
   const int nx = D.nx, ny = D.ny, nz = D.nz;
@@ -427,42 +434,45 @@ __global__ void k_mg_jacobi(Dims D, Op o, const T* __restrict__ dinv, const T* _
 }
 // the first sweep from x = 0 alone (where it is the only one)
 template <typename T>
-__global__ void k_mg_first(int64_t n, const T* __restrict__ dinv, const T* __restrict__ b, T* xo,
+__global__ void k_mg_first(int64_t n, const T* dinv, const T* b, T* xo,
                            double w_, const double* done) {
   PCG_SKIP(done);
   int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (c < n) xo[c] = (T)w_ * b[c] * dinv[c];
 }
 
-// coarse rhs = sum over children of the fine residual (b - S x)
+// the sum over the eight lanes of a coarse cell, in order (as one thread adds
+// the children up)
+template <typename T>
+__device__ __forceinline__ T octet_sum(T v) {
+  const int base = threadIdx.x & 24;
+  T s = T(0);
+#pragma unroll
+  for (int q = 0; q < 8; ++q) s += __shfl_sync(0xffffffffu, v, base + q);
+  return s;
+}
+
+// coarse rhs = sum over children of the fine residual (b - S x): a lane a child
+// (with a thread a coarse cell the eight children's loads came one after the
+// other: 11 to 14 us on levels of a few thousand cells)
 template <typename T, typename Op>
-__global__ void k_mg_restrict_residual(Dims DF, Op o, const T* __restrict__ b,
-                                       const T* __restrict__ x, Dims DC, T* bc,
+__global__ void k_mg_restrict_residual(Dims DF, Op o, const T* b, const T* x, Dims DC, T* bc,
                                        const double* done) {
   PCG_SKIP(done);
   const int fx = DF.nx, fy = DF.ny, fz = DF.nz;
-  const int cx = DC.nx, cy = DC.ny, cz = DC.nz;
-  int64_t n = (int64_t)cx * cy * cz;
-  int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (q >= n) return;
+  const int64_t n = (int64_t)DC.nx * DC.ny * DC.nz;
+  const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x, qu = t >> 3;
+  const int64_t q = qu < n ? qu : n - 1;
   int I, J, K;
   split_cell((uint32_t)q, DC.fnx, DC.fny, I, J, K);
-  const int64_t fsy = fx, fsz = (int64_t)fx * fy;
-  const VecX<T> X{x};
-  T s = 0.0;
-#pragma unroll
-  for (int dk = 0; dk < 2; ++dk)
-#pragma unroll
-    for (int dj = 0; dj < 2; ++dj)
-#pragma unroll
-      for (int di = 0; di < 2; ++di) {
-        const int k = 2 * K + dk, j = 2 * J + dj, i = 2 * I + di;
-        if (k < fz && j < fy && i < fx) {
-          int64_t c = (int64_t)k * fsz + (int64_t)j * fsy + i;
-          s += b[c] - mg_apply(fx, fy, fz, o, X, x[c], c, i, j, k);
-        }
-      }
-  bc[q] = s;
+  const int i = 2 * I + (t & 1), j = 2 * J + ((t >> 1) & 1), k = 2 * K + ((t >> 2) & 1);
+  T v = T(0);
+  if (k < fz && j < fy && i < fx) {
+    const int c = (k * fy + j) * fx + i;
+    v = b[c] - mg_apply(fx, fy, fz, o, VecX<T>{x}, x[c], c, i, j, k);
+  }
+  const T s = octet_sum(v);
+  if (qu < n && (t & 7) == 0) bc[q] = s;
 }
 
 // ---------------------------------------------------------------------------
@@ -499,7 +509,7 @@ __device__ __forceinline__ void store_partial(double v, double* partial) {
     partial[blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z)] = s;
 }
 __global__ void __launch_bounds__(FIN_THREADS)
-    k_finish_sum(const double* __restrict__ partial, int nb, double* scal, int slot, int post,
+    k_finish_sum(const double* partial, int nb, double* scal, int slot, int post,
                  const double* done) {
   PCG_SKIP(done);
   __shared__ double sh[32];
@@ -517,10 +527,11 @@ __global__ void __launch_bounds__(FIN_THREADS)
 }
 
 // rhs: b_S = -dz_k (div - target)/dt, plus ||(div - target)/dt||^2
-__global__ void k_proj_rhs(GridDev g, const double* __restrict__ u, const double* __restrict__ v,
-                           const double* __restrict__ w, const double* __restrict__ u_in,
-                           const double* __restrict__ target, double inv_dx, double inv_dy,
+__global__ void k_proj_rhs(GridDev g, const double* u, const double* v,
+                           const double* w, const double* u_in,
+                           const double* target, double inv_dx, double inv_dy,
                            double inv_dt, double* bS, double* partial) {
+  FOLLOW();
   const int64_t n = ncells_dev(g);
   const int nx = g.nx, ny = g.ny;
   const int64_t sy = nx, sz = (int64_t)nx * ny;
@@ -627,8 +638,8 @@ __device__ __forceinline__ void z_apply(const Dims& D, const OpI<T>& o, const V&
     y[0] = mg_apply(nx, ny, nz, o, x, xc[0], c, i, j, k);
   } else {
     const int sy = nx, sz = nx * ny, lane = threadIdx.x & 31;
-    const T* __restrict__ ir = o.ir;
-    const T* __restrict__ tb = o.tab + k * OP_TAB;
+    const T* ir = o.ir;
+    const T* tb = o.tab + k * OP_TAB;
     const int jp = j + 1 < ny ? j + 1 : 0, jm = j > 0 ? j - 1 : ny - 1;
     const int cp = c + (jp - j) * sy, cm = c + (jm - j) * sy;
     const int kp = min(k + 1, nz - 1), km = max(k - 1, 0);
@@ -732,8 +743,8 @@ __device__ __forceinline__ void z_store(T* p, int c, const T (&v)[W]) {
 // V-cycle's last sweep: r.z)
 template <int W, bool DOT, typename T, typename Op, typename V>
 __global__ void __launch_bounds__(Z_THREADS, 4)
-    k_z_jacobi(Dims D, Op o, const T* __restrict__ dinv, const T* __restrict__ b, V x, T* xo,
-               double w_, const double* __restrict__ rd, double* partial, const double* done) {
+    k_z_jacobi(Dims D, Op o, const T* dinv, const T* b, V x, T* xo,
+               double w_, const double* rd, double* partial, const double* done) {
   PCG_SKIP(done);
   const ZCell z = z_cell<W>(D);
   T bc[W], dc[W], xc[W], y[W], v[W];
@@ -756,7 +767,7 @@ __global__ void __launch_bounds__(Z_THREADS, 4)
 // coarse rhs = sum over children of the fine residual, a coarse cell a thread
 template <typename T, typename Op>
 __global__ void __launch_bounds__(Z_THREADS, 4)
-    k_z_restrict(Dims D, Op o, const T* __restrict__ b, const T* __restrict__ x, Dims DC, T* bc,
+    k_z_restrict(Dims D, Op o, const T* b, const T* x, Dims DC, T* bc,
                  const double* done) {
   PCG_SKIP(done);
   const ZCell z = z_cell<1>(DC);
@@ -782,8 +793,8 @@ __global__ void __launch_bounds__(Z_THREADS, 4)
 // into the other of the two direction buffers
 template <int W, typename Z>
 __global__ void __launch_bounds__(Z_THREADS, 4)
-    k_z_matvec_dir(Dims D, OpI<double> o, const Z* __restrict__ zv, double* p0, double* p1,
-                   double* q, const double* __restrict__ scal, double* partial) {
+    k_z_matvec_dir(Dims D, OpI<double> o, const Z* zv, double* p0, double* p1,
+                   double* q, const double* scal, double* partial) {
   PCG_SKIP(scal + SC_DONE);
   const int it = (int)scal[SC_IT];
   const VecDir<Z> x{zv, it & 1 ? p0 : p1, it == 0 ? 0.0 : scal[2] / scal[0]};
@@ -802,7 +813,7 @@ __global__ void __launch_bounds__(Z_THREADS, 4)
 // q = S p and p.q of a stored vector (W = 1 for a caller's: any alignment)
 template <int W>
 __global__ void __launch_bounds__(Z_THREADS, 4)
-    k_z_matvec(Dims D, OpI<double> o, const double* __restrict__ p, double* q, double* partial,
+    k_z_matvec(Dims D, OpI<double> o, const double* p, double* q, double* partial,
                const double* done) {
   PCG_SKIP(done);
   const ZCell z = z_cell<W>(D);
@@ -820,8 +831,9 @@ __global__ void __launch_bounds__(Z_THREADS, 4)
 // r_A = -r / dz_k
 template <int W>
 __global__ void __launch_bounds__(Z_THREADS, 4)
-    k_z_residual(GridDev g, Dims D, OpI<double> o, const double* __restrict__ b,
-                 const double* __restrict__ x, double* r, float* r32, double* partial) {
+    k_z_residual(GridDev g, Dims D, OpI<double> o, const double* b,
+                 const double* x, double* r, float* r32, double* partial) {
+  FOLLOW();
   const ZCell z = z_cell<W>(D);
   double xc[W], y[W], v[W], acc = 0.0;
   z_load<W>(b, z.c, v);
@@ -843,8 +855,8 @@ __global__ void __launch_bounds__(Z_THREADS, 4)
 // x += alpha p ; r -= alpha q ; ||r_A||^2   (alpha = rz / pq from device scalars;
 // p: the buffer of this iteration's parity, or p0 with p1 null)
 __global__ void k_pcg_update(GridDev g, double* x, double* r, float* r32,
-                             const double* __restrict__ p0, const double* __restrict__ p1,
-                             const double* __restrict__ q, const double* __restrict__ scal,
+                             const double* p0, const double* p1,
+                             const double* q, const double* scal,
                              double* partial) {
   PCG_SKIP(scal + SC_DONE);
   const int64_t n = ncells_dev(g);
@@ -864,7 +876,7 @@ __global__ void k_pcg_update(GridDev g, double* x, double* r, float* r32,
 }
 
 // a.b
-__global__ void k_dot(int64_t n, const double* __restrict__ a, const double* __restrict__ b,
+__global__ void k_dot(int64_t n, const double* a, const double* b,
                       double* partial, const double* done) {
   PCG_SKIP(done);
   double acc = 0.0;
@@ -881,20 +893,23 @@ __global__ void k_set_scal(double* scal, int dst, int src) {
 
 // start of a solve: tolerance, initial test, iteration count; b == 0 -> x = 0
 __global__ void k_pcg_init(double* scal, double rtol2) {
+  FOLLOW();
   scal[6] = rtol2 * scal[4];
   scal[SC_IT] = 0.0;
   scal[SC_DONE] = (scal[5] < scal[6] || scal[4] == 0.0) ? 1.0 : 0.0;
 }
 
-__global__ void k_zero_if_zero_rhs(int64_t n, const double* __restrict__ scal, double* x) {
+__global__ void k_zero_if_zero_rhs(int64_t n, const double* scal, double* x) {
+  FOLLOW();
   if (scal[4] != 0.0) return;
-  int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (c < n) x[c] = 0.0;
+  for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < n;
+       c += (int64_t)gridDim.x * blockDim.x)
+    x[c] = 0.0;
 }
 
 // Flexible CG (truncated to one previous direction): p = z - (z.q_prev / p.q_prev) p,
 // first iteration p = z.  Slots: 10 z.q_prev, 11 p.q of the previous iteration.
-__global__ void k_fcg_dir(int64_t n, const double* __restrict__ scal, const double* __restrict__ z,
+__global__ void k_fcg_dir(int64_t n, const double* scal, const double* z,
                           double* p) {
   PCG_SKIP(scal + SC_DONE);
   int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
@@ -908,6 +923,7 @@ __global__ void k_fcg_dir(int64_t n, const double* __restrict__ scal, const doub
 // (p.q = 0, e.g. a network output of 0) gives alpha = 0, so the residual
 // stalls and the solve falls back instead of dividing by zero
 __global__ void k_fcg_alpha(double* scal) {
+  FOLLOW();
   if (scal[SC_DONE] != 0.0) return;
   const bool ok = scal[1] > 0.0;
   scal[0] = ok ? scal[12] : 0.0;
@@ -916,8 +932,9 @@ __global__ void k_fcg_alpha(double* scal) {
 
 // out = b - S x (level operator, any precision)
 template <typename T>
-__global__ void k_lp_residual(Dims D, OpZ<T> o, const T* __restrict__ b, const T* __restrict__ x,
+__global__ void k_lp_residual(Dims D, OpZ<T> o, const T* b, const T* x,
                               T* out) {
+  FOLLOW();
   const int nx = D.nx, ny = D.ny, nz = D.nz;
   int64_t n = (int64_t)nx * ny * nz;
   int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
@@ -928,8 +945,9 @@ __global__ void k_lp_residual(Dims D, OpZ<T> o, const T* __restrict__ b, const T
 }
 
 // e1 = float(e0) - t
-__global__ void k_lp_err(int64_t n, const double* __restrict__ e0, const float* __restrict__ t,
+__global__ void k_lp_err(int64_t n, const double* e0, const float* t,
                          float* e1) {
+  FOLLOW();
   int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (c < n) e1[c] = (float)e0[c] - t[c];
 }
@@ -937,6 +955,7 @@ __global__ void k_lp_err(int64_t n, const double* __restrict__ e0, const float* 
 // restart as V-cycle PCG from the current iterate (the residual was just
 // recomputed into slot 5)
 __global__ void k_fcg_restart(double* scal) {
+  FOLLOW();
   scal[SC_IT] = 0.0;
   scal[SC_DONE] = (scal[5] < scal[6]) ? 1.0 : 0.0;
 }
@@ -945,8 +964,9 @@ __global__ void k_fcg_restart(double* scal) {
 // velocity correction (projection_3d.py:818-842)
 // ---------------------------------------------------------------------------
 __global__ void k_proj_correct(GridDev g, double* u, double* v, double* w,
-                               const double* __restrict__ p, const double* __restrict__ ir,
-                               double dt) {
+                               const double* p, const double* ir,
+                               double dt, double dt_dx, double dt_dy) {
+  FOLLOW();
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   int j = blockIdx.y * blockDim.y + threadIdx.y;
   int k = blockIdx.z;
@@ -956,13 +976,13 @@ __global__ void k_proj_correct(GridDev g, double* u, double* v, double* w,
   int64_t c = cidx(g, k, j, i);
   const double pc = p[c], irc = ir[c];
   if (nx > 2) {
-    if (i < nx - 1) u[c] -= dt * (p[c + 1] - pc) / g.dx * (0.5 * (irc + ir[c + 1]));
-    else u[c] += 2.0 * dt * pc / g.dx * irc;
+    if (i < nx - 1) u[c] -= dt_dx * (p[c + 1] - pc) * (0.5 * (irc + ir[c + 1]));
+    else u[c] += 2.0 * dt_dx * pc * irc;
   }
   if (ny > 1) {
     int jp = j + 1 < ny ? j + 1 : 0;
     int64_t cp = c - (int64_t)j * sy + (int64_t)jp * sy;
-    v[c] -= dt * (p[cp] - pc) / g.dy * (0.5 * (irc + ir[cp]));
+    v[c] -= dt_dy * (p[cp] - pc) * (0.5 * (irc + ir[cp]));
   }
   if (nz > 2) {
     if (k < nz - 1) w[c] -= dt * (p[c + sz] - pc) / g.da[k] * (0.5 * (irc + ir[c + sz]));
@@ -971,10 +991,12 @@ __global__ void k_proj_correct(GridDev g, double* u, double* v, double* w,
 }
 
 // max |div(u) - target| (projection_3d.py:847-892 plain branch)
-__global__ void k_div_resid_max(GridDev g, const double* __restrict__ u,
-                                const double* __restrict__ v, const double* __restrict__ w,
-                                const double* __restrict__ u_in, const double* __restrict__ target,
-                                double* div_out, unsigned long long* out_key) {
+__global__ void k_div_resid_max(GridDev g, const double* u,
+                                const double* v, const double* w,
+                                const double* u_in, const double* target,
+                                double inv_dx, double inv_dy, double* div_out,
+                                unsigned long long* out_key) {
+  FOLLOW();
   const int64_t n = ncells_dev(g);
   const int nx = g.nx, ny = g.ny;
   const int64_t sy = nx, sz = (int64_t)nx * ny;
@@ -985,11 +1007,11 @@ __global__ void k_div_resid_max(GridDev g, const double* __restrict__ u,
     int i, j, k;
     split_cell((uint32_t)c, g.fnx, g.fny, i, j, k);
     double div;
-    if (i > 0) div = (u[c] - u[c - 1]) / g.dx;
-    else div = (u[c] - u_in[(int64_t)k * ny + j]) / g.dx;
+    if (i > 0) div = (u[c] - u[c - 1]) * inv_dx;
+    else div = (u[c] - u_in[(int64_t)k * ny + j]) * inv_dx;
     if (ny > 1) {
       int jm = j > 0 ? j - 1 : ny - 1;
-      div += (v[c] - v[c - (int64_t)j * sy + (int64_t)jm * sy]) / g.dy;
+      div += (v[c] - v[c - (int64_t)j * sy + (int64_t)jm * sy]) * inv_dy;
     }
     if (k > 0) div += (w[c] - w[c - sz]) / g.dz[k];
     else div += (w[c] - 0.0) / g.dz[0];
@@ -1114,12 +1136,12 @@ double* proj_pressure(void* h) { return ((ProjCtx*)h)->p_prev; }
 const double* proj_inv_rho(void* h) { return ((ProjCtx*)h)->ir; }
 int proj_nlevels(void* h) { return ((ProjCtx*)h)->nlev; }
 
-__global__ void k_cvt_d2f(int64_t n, const double* __restrict__ a, float* b, const double* done) {
+__global__ void k_cvt_d2f(int64_t n, const double* a, float* b, const double* done) {
   PCG_SKIP(done);
   int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (c < n) b[c] = (float)a[c];
 }
-__global__ void k_cvt_f2d(int64_t n, const float* __restrict__ a, double* b, const double* done) {
+__global__ void k_cvt_f2d(int64_t n, const float* a, double* b, const double* done) {
   PCG_SKIP(done);
   int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (c < n) b[c] = (double)a[c];
@@ -1138,30 +1160,31 @@ template <typename T>
 static void rebuild_levels(ProjCtx* P, MGLevelT<T>* lev, T* Ainv, cudaStream_t st) {
   if (sizeof(T) == 4 || P->nlev == 1) {
     MGLevelT<T>& f = lev[0];
-    k_op_arrays<T><<<blocks_for(f.n, 256), 256, 0, st>>>(f.dims, op_0(P, 0.0), f.gx, f.gy, f.gz, f.e);
+    following(k_op_arrays<T>, blocks_for(f.n, 256), 256, 0, st)(f.dims, op_0(P, 0.0), f.gx, f.gy, f.gz, f.e);
     fs_count_launch();
   }
   const auto o0 = op_0(P, T(0));
+  typedef std::remove_const_t<decltype(o0)> Op0;
   for (int l = 0; l < P->nlev; ++l) {
     MGLevelT<T>& f = lev[l];
     if (l > 0) {
       MGLevelT<T>& pf = lev[l - 1];
       if (l == 1)
-        k_mg_coarsen<T><<<blocks_for(f.n, 128), 128, 0, st>>>(pf.nx, pf.ny, pf.nz, o0, f.dims, f.gx,
+        following(k_mg_coarsen<T, Op0>, blocks_for(f.n, 128), 128, 0, st)(pf.nx, pf.ny, pf.nz, o0, f.dims, f.gx,
                                                              f.gy, f.gz, f.e, 0.5);
       else
-        k_mg_coarsen<T><<<blocks_for(f.n, 128), 128, 0, st>>>(pf.nx, pf.ny, pf.nz, op_a(pf), f.dims,
+        following(k_mg_coarsen<T, OpA<T>>, blocks_for(f.n, 128), 128, 0, st)(pf.nx, pf.ny, pf.nz, op_a(pf), f.dims,
                                                              f.gx, f.gy, f.gz, f.e, 0.5);
       fs_count_launch();
-      k_mg_diag<T><<<blocks_for(f.n, 256), 256, 0, st>>>(f.dims, op_a(f), f.dinv);
+      following(k_mg_diag<T, OpA<T>>, blocks_for(f.n, 256), 256, 0, st)(f.dims, op_a(f), f.dinv);
     } else {
-      k_mg_diag<T><<<blocks_for(f.n, 256), 256, 0, st>>>(f.dims, o0, f.dinv);
+      following(k_mg_diag<T, Op0>, blocks_for(f.n, 256), 256, 0, st)(f.dims, o0, f.dinv);
     }
     fs_count_launch();
   }
   MGLevelT<T>& c = lev[P->nlev - 1];
   if (c.n <= MG_COARSE_MAX) {
-    k_mg_coarse_inverse<T><<<1, 1024, 0, st>>>(c.nx, c.ny, c.nz, c.gx, c.gy, c.gz, c.e, Ainv);
+    following(k_mg_coarse_inverse<T>, 1, 1024, 0, st)(c.nx, c.ny, c.nz, c.gx, c.gy, c.gz, c.e, Ainv);
     fs_count_launch();
   }
 }
@@ -1171,7 +1194,7 @@ int proj_rebuild(void* h, const double* rho, cudaStream_t st) {
   const GridDev& g = P->g;
   const unsigned nb = blocks_for(P->lev[0].n, 256);
   // the FP64 level-0 operator stays the CG's; the FP32 preconditioner has its own
-  k_proj_ir<<<nb, 256, 0, st>>>(g, rho, P->ir, P->tab, g.dx * g.dx, g.dy * g.dy);
+  following(k_proj_ir, nb, 256, 0, st)(g, rho, P->ir, P->tab, g.dx * g.dx, g.dy * g.dy);
   fs_count_launch();
   if (P->fp32) rebuild_levels<float>(P, P->lev32, P->Ainv32, st);
   else rebuild_levels<double>(P, P->lev, P->Ainv, st);
@@ -1238,40 +1261,57 @@ __host__ __device__ inline int64_t tail_smem_elems(const MGLevelT<T>* lev, int n
   return e + (nc <= MG_COARSE_MAX ? nc * nc : 0);
 }
 
+// A level in shared memory: its extents and where its nine arrays begin.  All
+// accesses are the one shared array plus an index, so they are shared-memory
+// instructions with 32-bit addresses.
+struct TailLevel {
+  int nx, ny, nz, n, o;
+  Dims dims;
+  __device__ __forceinline__ int gx() const { return o; }
+  __device__ __forceinline__ int gy() const { return o + n; }
+  __device__ __forceinline__ int gz() const { return o + 2 * n; }
+  __device__ __forceinline__ int e() const { return o + 3 * n; }
+  __device__ __forceinline__ int dinv() const { return o + 4 * n; }
+  __device__ __forceinline__ int b() const { return o + 5 * n; }
+  __device__ __forceinline__ int x() const { return o + 6 * n; }
+  __device__ __forceinline__ int t() const { return o + 7 * n; }
+  __device__ __forceinline__ int s() const { return o + 8 * n; }
+};
+
 template <typename T>
-__device__ __forceinline__ T tail_apply(const MGLevelT<T>& f, const T* x, int64_t c, int i,
-                                        int j, int k) {
-  const int nx = f.nx, ny = f.ny, nz = f.nz;
-  const int64_t sy = nx, sz = (int64_t)nx * ny;
-  const T xc = x[c];
-  T y = f.e[c] * xc;
-  if (i < nx - 1) y += f.gx[c] * (xc - x[c + 1]);
-  if (i > 0) y += f.gx[c - 1] * (xc - x[c - 1]);
+__device__ __forceinline__ T tail_apply(const T* S, const TailLevel& f, int x, int c, int i, int j,
+                                        int k) {
+  const int nx = f.nx, ny = f.ny, nz = f.nz, sz = nx * ny;
+  const T* X = S + x;
+  const T *gx = S + f.gx(), *gy = S + f.gy(), *gz = S + f.gz();
+  const T xc = X[c];
+  T y = S[f.e() + c] * xc;
+  if (i < nx - 1) y += gx[c] * (xc - X[c + 1]);
+  if (i > 0) y += gx[c - 1] * (xc - X[c - 1]);
   if (ny > 1) {
-    int jp = j + 1 < ny ? j + 1 : 0;
-    int jm = j > 0 ? j - 1 : ny - 1;
-    int64_t cp = c - (int64_t)j * sy + (int64_t)jp * sy;
-    int64_t cm = c - (int64_t)j * sy + (int64_t)jm * sy;
-    y += f.gy[c] * (xc - x[cp]);
-    y += f.gy[cm] * (xc - x[cm]);
+    const int cp = j + 1 < ny ? c + nx : c - j * nx;
+    const int cm = j > 0 ? c - nx : c + (ny - 1) * nx;
+    y += gy[c] * (xc - X[cp]);
+    y += gy[cm] * (xc - X[cm]);
   }
-  if (k < nz - 1) y += f.gz[c] * (xc - x[c + sz]);
-  if (k > 0) y += f.gz[c - sz] * (xc - x[c - sz]);
+  if (k < nz - 1) y += gz[c] * (xc - X[c + sz]);
+  if (k > 0) y += gz[c - sz] * (xc - X[c - sz]);
   return y;
 }
 
+// x < 0: from zero
 template <typename T>
-__device__ __forceinline__ void tail_jacobi(const MGLevelT<T>& f, const T* b, const T* x, T* xo,
-                                            T w) {
-  for (int64_t c = threadIdx.x; c < f.n; c += blockDim.x) {
-    if (!x) {
-      xo[c] = w * b[c] * f.dinv[c];
+__device__ __forceinline__ void tail_jacobi(T* S, const TailLevel& f, int x, int xo, T w) {
+  for (int c = threadIdx.x; c < f.n; c += MG_TAIL_THREADS) {
+    const T b = S[f.b() + c], d = S[f.dinv() + c];
+    if (x < 0) {
+      S[xo + c] = w * b * d;
       continue;
     }
     int i, j, k;
     split_cell((uint32_t)c, f.dims.fnx, f.dims.fny, i, j, k);
-    T r = b[c] - tail_apply(f, x, c, i, j, k);
-    xo[c] = x[c] + w * r * f.dinv[c];
+    const T r = b - tail_apply(S, f, x, c, i, j, k);
+    S[xo + c] = S[x + c] + w * r * d;
   }
 }
 
@@ -1280,104 +1320,103 @@ __global__ void __launch_bounds__(MG_TAIL_THREADS, 1)
     k_mg_vcycle_tail(MGTail<T> a, const double* done) {
   PCG_SKIP(done);
   extern __shared__ __align__(16) unsigned char tsh[];
-  T* sp = (T*)tsh;
-  // the levels in shared memory: operator copied in, vectors private
-  MGLevelT<T> L[MG_TAIL_MAX];
-  for (int q = 0; q < a.nl; ++q) {
-    const MGLevelT<T>& g = a.lev[q];
-    const int64_t n = g.n;
-    MGLevelT<T>& f = L[q];
-    f.nx = g.nx; f.ny = g.ny; f.nz = g.nz; f.n = n; f.dims = g.dims;
-    f.gx = sp; f.gy = sp + n; f.gz = sp + 2 * n; f.e = sp + 3 * n; f.dinv = sp + 4 * n;
-    f.b = sp + 5 * n; f.x = sp + 6 * n; f.t = sp + 7 * n; f.s = sp + 8 * n;
-    sp += 9 * n;
-    for (int64_t c = threadIdx.x; c < n; c += blockDim.x) {
-      f.gx[c] = g.gx[c]; f.gy[c] = g.gy[c]; f.gz[c] = g.gz[c]; f.e[c] = g.e[c];
-      f.dinv[c] = g.dinv[c];
-      if (q == 0) f.b[c] = g.b[c];
+  __shared__ TailLevel L[MG_TAIL_MAX];
+  T* const S = (T*)tsh;
+  if (threadIdx.x == 0) {
+    int o = 0;
+    for (int q = 0; q < a.nl; ++q) {
+      const MGLevelT<T>& g = a.lev[q];
+      L[q] = TailLevel{g.nx, g.ny, g.nz, (int)g.n, o, g.dims};
+      o += 9 * (int)g.n;
     }
   }
-  const int64_t ncs = L[a.nl - 1].n;
-  T* Ainv = sp;
+  __syncthreads();
+  // the operators copied in; the vectors are private
+  for (int q = 0; q < a.nl; ++q) {
+    const MGLevelT<T>& g = a.lev[q];
+    const TailLevel f = L[q];
+    for (int c = threadIdx.x; c < f.n; c += MG_TAIL_THREADS) {
+      S[f.gx() + c] = g.gx[c]; S[f.gy() + c] = g.gy[c]; S[f.gz() + c] = g.gz[c];
+      S[f.e() + c] = g.e[c]; S[f.dinv() + c] = g.dinv[c];
+      if (q == 0) S[f.b() + c] = g.b[c];
+    }
+  }
+  const int ncs = L[a.nl - 1].n, Ainv = L[a.nl - 1].o + 9 * ncs;
   if (ncs <= MG_COARSE_MAX)
-    for (int64_t c = threadIdx.x; c < ncs * ncs; c += blockDim.x) Ainv[c] = a.Ainv[c];
+    for (int c = threadIdx.x; c < ncs * ncs; c += MG_TAIL_THREADS) S[Ainv + c] = a.Ainv[c];
   __syncthreads();
   const T w = (T)a.omega;
   const int nu = a.nu;
   // down: pre-smoothing from x = 0 ending in t, residual restricted to the next level's b
   for (int l = 0; l + 1 < a.nl; ++l) {
-    const MGLevelT<T>& f = L[l];
-    const T* src = nullptr;
+    const TailLevel f = L[l], cl = L[l + 1];
+    int src = -1;
     for (int s = 0; s < nu; ++s) {
-      T* dst = ((nu - 1 - s) % 2 == 0) ? f.t : f.s;
-      tail_jacobi(f, f.b, src, dst, w);
+      const int dst = ((nu - 1 - s) % 2 == 0) ? f.t() : f.s();
+      tail_jacobi(S, f, src, dst, w);
       __syncthreads();
       src = dst;
     }
-    const MGLevelT<T>& cl = L[l + 1];
-    const int64_t fsy = f.nx, fsz = (int64_t)f.nx * f.ny;
-    for (int64_t q = threadIdx.x; q < cl.n; q += blockDim.x) {
+    for (int t = threadIdx.x; (t & ~31) < 8 * cl.n; t += MG_TAIL_THREADS) {
+      const int qu = t >> 3, q = min(qu, cl.n - 1);
       int I, J, K;
       split_cell((uint32_t)q, cl.dims.fnx, cl.dims.fny, I, J, K);
-      T sum = 0.0;
-      for (int k = 2 * K; k <= min(2 * K + 1, f.nz - 1); ++k)
-        for (int j = 2 * J; j <= min(2 * J + 1, f.ny - 1); ++j)
-          for (int i = 2 * I; i <= min(2 * I + 1, f.nx - 1); ++i) {
-            int64_t c = (int64_t)k * fsz + (int64_t)j * fsy + i;
-            sum += f.b[c] - tail_apply(f, f.t, c, i, j, k);
-          }
-      cl.b[q] = sum;
+      const int i = 2 * I + (t & 1), j = 2 * J + ((t >> 1) & 1), k = 2 * K + ((t >> 2) & 1);
+      T v = T(0);
+      if (k < f.nz && j < f.ny && i < f.nx) {
+        const int c = (k * f.ny + j) * f.nx + i;
+        v = S[f.b() + c] - tail_apply(S, f, f.t(), c, i, j, k);
+      }
+      const T sum = octet_sum(v);
+      if (qu < cl.n && (t & 7) == 0) S[cl.b() + q] = sum;
     }
     __syncthreads();
   }
   // coarsest level: dense solve, or smoothing only when it is too large for it
   {
-    const MGLevelT<T>& f = L[a.nl - 1];
+    const TailLevel f = L[a.nl - 1];
     if (f.n <= MG_COARSE_MAX) {
-      for (int r = threadIdx.x; r < (int)f.n; r += blockDim.x) {
+      for (int r = threadIdx.x; r < f.n; r += MG_TAIL_THREADS) {
         T sum = 0.0;
-        for (int q = 0; q < (int)f.n; ++q) sum += Ainv[r * f.n + q] * f.b[q];
-        f.x[r] = sum;
+        for (int q = 0; q < f.n; ++q) sum += S[Ainv + r * f.n + q] * S[f.b() + q];
+        S[f.x() + r] = sum;
       }
       __syncthreads();
     } else {
       const T wc = (T)MG_OMEGA;
-      tail_jacobi(f, f.b, (const T*)nullptr, f.x, wc);
+      tail_jacobi(S, f, -1, f.x(), wc);
       __syncthreads();
       for (int s = 0; s < 8; ++s) {
-        const T* src = (s & 1) ? f.t : f.x;
-        T* dst = (s & 1) ? f.x : f.t;
-        tail_jacobi(f, f.b, src, dst, wc);
+        tail_jacobi(S, f, (s & 1) ? f.t() : f.x(), (s & 1) ? f.x() : f.t(), wc);
         __syncthreads();
       }
     }
   }
   // up: prolongation into t, post-smoothing from t ending in the level's x
   for (int l = a.nl - 2; l >= 0; --l) {
-    const MGLevelT<T>& f = L[l];
-    const MGLevelT<T>& cl = L[l + 1];
-    for (int64_t c = threadIdx.x; c < f.n; c += blockDim.x) {
+    const TailLevel f = L[l], cl = L[l + 1];
+    for (int c = threadIdx.x; c < f.n; c += MG_TAIL_THREADS) {
       int i, j, k;
       split_cell((uint32_t)c, f.dims.fnx, f.dims.fny, i, j, k);
-      f.t[c] += cl.x[((int64_t)(k >> 1) * cl.ny + (j >> 1)) * cl.nx + (i >> 1)];
+      S[f.t() + c] += S[cl.x() + ((k >> 1) * cl.ny + (j >> 1)) * cl.nx + (i >> 1)];
     }
     __syncthreads();
-    const T* src = f.t;
+    int src = f.t();
     for (int s = 0; s < nu; ++s) {
-      T* dst = (s == nu - 1) ? f.x : ((s % 2 == 0) ? f.s : f.t);
-      tail_jacobi(f, f.b, src, dst, w);
+      const int dst = (s == nu - 1) ? f.x() : ((s % 2 == 0) ? f.s() : f.t());
+      tail_jacobi(S, f, src, dst, w);
       __syncthreads();
       src = dst;
     }
   }
   // the first tail level's correction back to global memory
-  for (int64_t c = threadIdx.x; c < L[0].n; c += blockDim.x) a.lev[0].x[c] = L[0].x[c];
+  for (int c = threadIdx.x; c < L[0].n; c += MG_TAIL_THREADS) a.lev[0].x[c] = S[L[0].x() + c];
 }
 
 // the sum of the partials that the kernel before left
 static void launch_finish(ProjCtx* P, int nb, int slot, int post, const double* done,
                           cudaStream_t st) {
-  k_finish_sum<<<1, FIN_THREADS, 0, st>>>(P->partial, nb, P->scal, slot, post, done);
+  following(k_finish_sum, 1, FIN_THREADS, 0, st)(P->partial, nb, P->scal, slot, post, done);
 }
 // a sweep and a restriction on level 0 and on the others (returns the launches)
 template <int W, typename T, typename Op, typename V>
@@ -1385,10 +1424,10 @@ static int launch_z_jacobi(ProjCtx* P, const Dims& D, const Op& o, const T* dinv
                            T* xo, double w, bool dot, const double* done, cudaStream_t st) {
   const int nb = z_blocks(D);
   if (!dot) {
-    k_z_jacobi<W, false, T><<<nb, Z_THREADS, 0, st>>>(D, o, dinv, b, x, xo, w, nullptr, nullptr, done);
+    following(k_z_jacobi<W, false, T, Op, V>, nb, Z_THREADS, 0, st)(D, o, dinv, b, x, xo, w, nullptr, nullptr, done);
     return 1;
   }
-  k_z_jacobi<W, true, T><<<nb, Z_THREADS, 0, st>>>(D, o, dinv, b, x, xo, w, P->pc_r, P->partial, done);
+  following(k_z_jacobi<W, true, T, Op, V>, nb, Z_THREADS, 0, st)(D, o, dinv, b, x, xo, w, P->pc_r, P->partial, done);
   launch_finish(P, nb, 2, POST_NONE, done, st);  // rz_new
   return 2;
 }
@@ -1401,14 +1440,15 @@ static int launch_jacobi(ProjCtx* P, const Dims& D, const Op& o, const T* dinv, 
 template <typename T, typename V>
 static int launch_jacobi(ProjCtx*, const Dims& D, const OpA<T>& o, const T* dinv, const T* b, V x,
                           T* xo, double w, bool, const double* done, cudaStream_t st) {
-  k_mg_jacobi<T><<<blocks_for((int64_t)D.nx * D.ny * D.nz, 256), 256, 0, st>>>(D, o, dinv, b, x, xo,
+  following(k_mg_jacobi<T, OpA<T>, V>, blocks_for((int64_t)D.nx * D.ny * D.nz, 256), 256, 0, st)(D, o, dinv, b, x, xo,
                                                                               w, done);
   return 1;
 }
 template <typename T>
 static void launch_restrict(const Dims& D, const OpA<T>& o, const T* b, const T* x, const Dims& DC,
                             T* bc, const double* done, cudaStream_t st) {
-  k_mg_restrict_residual<T><<<blocks_for((int64_t)DC.nx * DC.ny * DC.nz, 128), 128, 0, st>>>(
+  following(k_mg_restrict_residual<T, OpA<T>>, blocks_for(8 * (int64_t)DC.nx * DC.ny * DC.nz, 256), 256,
+            0, st)(
       D, o, b, x, DC, bc, done);
 }
 template <typename T, typename Op>
@@ -1416,9 +1456,10 @@ static void launch_restrict(const Dims& D, const Op& o, const T* b, const T* x, 
                             T* bc, const double* done, cudaStream_t st) {
   const unsigned nc = blocks_for((int64_t)DC.nx * DC.ny * DC.nz, Z_THREADS);
   if (z_width(D) == 2)
-    k_z_restrict<T><<<nc, Z_THREADS, 0, st>>>(D, o, b, x, DC, bc, done);
+    following(k_z_restrict<T, Op>, nc, Z_THREADS, 0, st)(D, o, b, x, DC, bc, done);
   else
-    k_mg_restrict_residual<T><<<nc, Z_THREADS, 0, st>>>(D, o, b, x, DC, bc, done);
+    following(k_mg_restrict_residual<T, Op>, blocks_for(8 * (int64_t)DC.nx * DC.ny * DC.nz, Z_THREADS),
+              Z_THREADS, 0, st)(D, o, b, x, DC, bc, done);
 }
 template <typename Z>
 static void launch_matvec_dir(ProjCtx* P, const Z* z, cudaStream_t st) {
@@ -1426,10 +1467,10 @@ static void launch_matvec_dir(ProjCtx* P, const Z* z, cudaStream_t st) {
   const int nb = z_blocks(D);
   const OpI<double> o = op_0(P, 0.0);
   if (z_width(D) == 2)
-    k_z_matvec_dir<2, Z><<<nb, Z_THREADS, 0, st>>>(D, o, z, P->pc_p, P->pc_p2, P->pc_q, P->scal,
+    following(k_z_matvec_dir<2, Z>, nb, Z_THREADS, 0, st)(D, o, z, P->pc_p, P->pc_p2, P->pc_q, P->scal,
                                                    P->partial);
   else
-    k_z_matvec_dir<1, Z><<<nb, Z_THREADS, 0, st>>>(D, o, z, P->pc_p, P->pc_p2, P->pc_q, P->scal,
+    following(k_z_matvec_dir<1, Z>, nb, Z_THREADS, 0, st)(D, o, z, P->pc_p, P->pc_p2, P->pc_q, P->scal,
                                                    P->partial);
   launch_finish(P, nb, 1, POST_DIR, P->scal + SC_DONE, st);  // p.q
 }
@@ -1439,9 +1480,9 @@ static void launch_residual(ProjCtx* P, const double* x, float* r32, cudaStream_
   const int nb = z_blocks(D);
   const OpI<double> o = op_0(P, 0.0);
   if (z_width(D) == 2)
-    k_z_residual<2><<<nb, Z_THREADS, 0, st>>>(P->g, D, o, P->rhs, x, P->pc_r, r32, P->partial);
+    following(k_z_residual<2>, nb, Z_THREADS, 0, st)(P->g, D, o, P->rhs, x, P->pc_r, r32, P->partial);
   else
-    k_z_residual<1><<<nb, Z_THREADS, 0, st>>>(P->g, D, o, P->rhs, x, P->pc_r, r32, P->partial);
+    following(k_z_residual<1>, nb, Z_THREADS, 0, st)(P->g, D, o, P->rhs, x, P->pc_r, r32, P->partial);
   launch_finish(P, nb, 5, POST_NONE, nullptr, st);
 }
 
@@ -1464,7 +1505,7 @@ static int vcycle_level(ProjCtx* P, MGLevelT<T>* lev, const T* Ainv, int l, Op o
   // pre-smoothing, ending in t: sweep i writes t when (nu-1-i) is even, else s
   const T* src = nullptr;
   if (nu == 1) {
-    k_mg_first<T><<<nb, 256, 0, st>>>(f.n, f.dinv, b, f.t, om, done);
+    following(k_mg_first<T>, nb, 256, 0, st)(f.n, f.dinv, b, f.t, om, done);
     ++nk;
   }
   for (int i = 1; i < nu; ++i) {
@@ -1511,22 +1552,22 @@ static int vcycle(ProjCtx* P, MGLevelT<T>* lev, const T* Ainv, int l, const T* b
     const size_t smem = (size_t)tail_smem_elems(lev + l, ta.nl) * sizeof(T);
     cudaFuncSetAttribute(k_mg_vcycle_tail<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          MG_TAIL_SMEM);
-    k_mg_vcycle_tail<T><<<1, MG_TAIL_THREADS, smem, st>>>(ta, done);
+    following(k_mg_vcycle_tail<T>, 1, MG_TAIL_THREADS, smem, st)(ta, done);
     return 1;
   }
   if (l == P->nlev - 1) {
     if (f.n <= MG_COARSE_MAX) {
-      k_mg_coarse_solve<T><<<1, 64, 0, st>>>((int)f.n, Ainv, b, x, done);
+      following(k_mg_coarse_solve<T>, 1, 64, 0, st)((int)f.n, Ainv, b, x, done);
       ++nk;
     } else {
       // not coarsenable and too large for the dense solve: smoothing only
       const unsigned nb = blocks_for(f.n, 256);
-      k_mg_first<T><<<nb, 256, 0, st>>>(f.n, f.dinv, b, x, MG_OMEGA, done);
+      following(k_mg_first<T>, nb, 256, 0, st)(f.n, f.dinv, b, x, MG_OMEGA, done);
       ++nk;
       for (int s = 0; s < 8; ++s) {
         const T* src = (s & 1) ? f.t : x;
         T* dst = (s & 1) ? x : f.t;
-        k_mg_jacobi<T><<<nb, 256, 0, st>>>(f.dims, op_a(f), f.dinv, b, VecX<T>{src}, dst, MG_OMEGA,
+        following(k_mg_jacobi<T, OpA<T>, VecX<T>>, nb, 256, 0, st)(f.dims, op_a(f), f.dinv, b, VecX<T>{src}, dst, MG_OMEGA,
                                            done);
         ++nk;
       }
@@ -1590,10 +1631,10 @@ static int pcg_iteration(ProjCtx* P, double* x, cudaStream_t st) {
     nk = vcycle<double>(P, P->lev, P->Ainv, 0, P->pc_r, P->pc_z, done, st);
   if (P->nlev == 1) {  // no sweeps: r.z is a pass of its own
     if (P->fp32) {
-      k_cvt_f2d<<<blocks_for(n, 256), 256, 0, st>>>(n, P->z32, P->pc_z, done);
+      following(k_cvt_f2d, blocks_for(n, 256), 256, 0, st)(n, P->z32, P->pc_z, done);
       ++nk;
     }
-    k_dot<<<RED_BLOCKS, RED_THREADS, 0, st>>>(n, P->pc_r, P->pc_z, P->partial, done);
+    following(k_dot, RED_BLOCKS, RED_THREADS, 0, st)(n, P->pc_r, P->pc_z, P->partial, done);
     launch_finish(P, RED_BLOCKS, 2, POST_NONE, done, st);
     nk += 2;
   }
@@ -1601,7 +1642,7 @@ static int pcg_iteration(ProjCtx* P, double* x, cudaStream_t st) {
     launch_matvec_dir(P, P->z32, st);
   else
     launch_matvec_dir(P, P->pc_z, st);
-  k_pcg_update<<<RED_BLOCKS, RED_THREADS, 0, st>>>(P->g, x, P->pc_r, P->fp32 ? P->r32 : nullptr,
+  following(k_pcg_update, RED_BLOCKS, RED_THREADS, 0, st)(P->g, x, P->pc_r, P->fp32 ? P->r32 : nullptr,
                                                    P->pc_p, P->pc_p2, P->pc_q, P->scal, P->partial);
   launch_finish(P, RED_BLOCKS, 5, POST_CHECK, done, st);  // ||r_A||^2
   return nk + 4;
@@ -1669,14 +1710,14 @@ static void lp_presmooth(ProjCtx* P, cudaStream_t st) {
   for (int i = 0; i < P->nu; ++i) {
     float* dst = ((P->nu - 1 - i) % 2 == 0) ? f.t : f.s;
     if (!src)
-      k_mg_first<float><<<nb, 256, 0, st>>>(f.n, f.dinv, P->r32, dst, P->omega, nullptr);
+      following(k_mg_first<float>, nb, 256, 0, st)(f.n, f.dinv, P->r32, dst, P->omega, nullptr);
     else
-      k_mg_jacobi<float><<<nb, 256, 0, st>>>(f.dims, op_0(P, 0.0f), f.dinv, P->r32,
+      following(k_mg_jacobi<float, OpZ<float>, VecX<float>>, nb, 256, 0, st)(f.dims, op_0(P, 0.0f), f.dinv, P->r32,
                                              VecX<float>{src}, dst, P->omega, nullptr);
     src = dst;
     fs_count_launch();
   }
-  k_lp_residual<float><<<nb, 256, 0, st>>>(f.dims, op_0(P, 0.0f), P->r32, f.t, f.b);
+  following(k_lp_residual<float>, nb, 256, 0, st)(f.dims, op_0(P, 0.0f), P->r32, f.t, f.b);
   fs_count_launch();
 }
 
@@ -1689,7 +1730,7 @@ static int learned_precond(ProjCtx* P, cudaStream_t st) {
   MGLevelT<float>& f = P->lev32[0];
   const int64_t n = f.n;
   const unsigned nb = blocks_for(n, 256);
-  k_cvt_d2f<<<nb, 256, 0, st>>>(n, P->pc_r, P->r32, nullptr);
+  following(k_cvt_d2f, nb, 256, 0, st)(n, P->pc_r, P->r32, nullptr);
   fs_count_launch();
   lp_presmooth(P, st);
   int rc = unet_correct(P->net, f.b, f.t, f.s, st);
@@ -1697,12 +1738,12 @@ static int learned_precond(ProjCtx* P, cudaStream_t st) {
   const float* src = f.s;
   for (int i = 0; i < P->nu; ++i) {
     float* dst = (i == P->nu - 1) ? P->z32 : ((i % 2 == 0) ? f.t : f.x);
-    k_mg_jacobi<float><<<nb, 256, 0, st>>>(f.dims, op_0(P, 0.0f), f.dinv, P->r32, VecX<float>{src},
+    following(k_mg_jacobi<float, OpZ<float>, VecX<float>>, nb, 256, 0, st)(f.dims, op_0(P, 0.0f), f.dinv, P->r32, VecX<float>{src},
                                            dst, P->omega, nullptr);
     src = dst;
     fs_count_launch();
   }
-  k_cvt_f2d<<<nb, 256, 0, st>>>(n, P->z32, P->pc_z, nullptr);
+  following(k_cvt_f2d, nb, 256, 0, st)(n, P->z32, P->pc_z, nullptr);
   fs_count_launch();
   return cuda_status();
 }
@@ -1717,11 +1758,11 @@ int proj_smooth_pair(void* h, const double* r0, const double* e0, float* r1, flo
   MGLevelT<float>& f = P->lev32[0];
   const int64_t n = f.n;
   const unsigned nb = blocks_for(n, 256);
-  k_cvt_d2f<<<nb, 256, 0, st>>>(n, r0, P->r32, nullptr);
+  following(k_cvt_d2f, nb, 256, 0, st)(n, r0, P->r32, nullptr);
   fs_count_launch();
   lp_presmooth(P, st);
   cudaMemcpyAsync(r1, f.b, sizeof(float) * n, cudaMemcpyDeviceToDevice, st);
-  k_lp_err<<<nb, 256, 0, st>>>(n, e0, f.t, e1);
+  following(k_lp_err, nb, 256, 0, st)(n, e0, f.t, e1);
   fs_count_launch();
   return cuda_status();
 }
@@ -1735,22 +1776,22 @@ static int fcg_iteration(ProjCtx* P, double* x, int it, cudaStream_t st) {
   int rc = learned_precond(P, st);
   if (rc) return rc;
   if (it > 0) {
-    k_dot<<<RED_BLOCKS, RED_THREADS, 0, st>>>(n, P->pc_z, P->pc_q, P->partial, done);
+    following(k_dot, RED_BLOCKS, RED_THREADS, 0, st)(n, P->pc_z, P->pc_q, P->partial, done);
     launch_finish(P, RED_BLOCKS, 10, POST_NONE, done, st);  // z.q_prev
     fs_count_launch(); fs_count_launch();
   }
-  k_fcg_dir<<<blocks_for(n, 256), 256, 0, st>>>(n, P->scal, P->pc_z, P->pc_p);
+  following(k_fcg_dir, blocks_for(n, 256), 256, 0, st)(n, P->scal, P->pc_z, P->pc_p);
   const int nb = z_blocks(l0.dims);
   if (z_width(l0.dims) == 2)
-    k_z_matvec<2><<<nb, Z_THREADS, 0, st>>>(l0.dims, op_0(P, 0.0), P->pc_p, P->pc_q, P->partial, done);
+    following(k_z_matvec<2>, nb, Z_THREADS, 0, st)(l0.dims, op_0(P, 0.0), P->pc_p, P->pc_q, P->partial, done);
   else
-    k_z_matvec<1><<<nb, Z_THREADS, 0, st>>>(l0.dims, op_0(P, 0.0), P->pc_p, P->pc_q, P->partial, done);
+    following(k_z_matvec<1>, nb, Z_THREADS, 0, st)(l0.dims, op_0(P, 0.0), P->pc_p, P->pc_q, P->partial, done);
   launch_finish(P, nb, 1, POST_NONE, done, st);  // p.q
-  k_dot<<<RED_BLOCKS, RED_THREADS, 0, st>>>(n, P->pc_p, P->pc_r, P->partial, done);
+  following(k_dot, RED_BLOCKS, RED_THREADS, 0, st)(n, P->pc_p, P->pc_r, P->partial, done);
   launch_finish(P, RED_BLOCKS, 12, POST_NONE, done, st);  // p.r
-  k_fcg_alpha<<<1, 1, 0, st>>>(P->scal);  // alpha = p.r / p.q
-  k_set_scal<<<1, 1, 0, st>>>(P->scal, 11, 1);
-  k_pcg_update<<<RED_BLOCKS, RED_THREADS, 0, st>>>(P->g, x, P->pc_r, nullptr, P->pc_p, nullptr,
+  following(k_fcg_alpha, 1, 1, 0, st)(P->scal);  // alpha = p.r / p.q
+  following(k_set_scal, 1, 1, 0, st)(P->scal, 11, 1);
+  following(k_pcg_update, RED_BLOCKS, RED_THREADS, 0, st)(P->g, x, P->pc_r, nullptr, P->pc_p, nullptr,
                                                    P->pc_q, P->scal, P->partial);
   launch_finish(P, RED_BLOCKS, 5, POST_CHECK, done, st);
   for (int k = 0; k < 9; ++k) fs_count_launch();
@@ -1779,7 +1820,7 @@ static int fcg_solve(ProjCtx* P, double* x, int maxiter, int* learned, cudaStrea
     }
     if (fall) {
       launch_residual(P, x, P->r32, st);
-      k_fcg_restart<<<1, 1, 0, st>>>(P->scal);
+      following(k_fcg_restart, 1, 1, 0, st)(P->scal);
       fs_count_launch(); fs_count_launch(); fs_count_launch();
       P->fcg[2] = 1.0;
       P->fcg[3] += 1.0;
@@ -1831,15 +1872,15 @@ int proj_project(void* h, double* u, double* v, double* w, const double* u_in,
   const auto t_start = Clock::now();
   for (int q = 0; q < 8; ++q) P->stats[q] = 0.0;
   *iters = 0;
-  k_proj_rhs<<<RED_BLOCKS, RED_THREADS, 0, st>>>(g, u, v, w, u_in, target, 1.0 / g.dx, 1.0 / g.dy,
+  following(k_proj_rhs, RED_BLOCKS, RED_THREADS, 0, st)(g, u, v, w, u_in, target, 1.0 / g.dx, 1.0 / g.dy,
                                                  1.0 / dt, P->rhs, P->partial);
   launch_finish(P, RED_BLOCKS, 4, POST_NONE, nullptr, st);
   fs_count_launch(); fs_count_launch();
   double* x = P->p_prev;
   launch_residual(P, x, P->fp32 ? P->r32 : nullptr, st);
   fs_count_launch(); fs_count_launch();
-  k_pcg_init<<<1, 1, 0, st>>>(P->scal, rtol * rtol); fs_count_launch();
-  k_zero_if_zero_rhs<<<blocks_for(n, 256), 256, 0, st>>>(n, P->scal, x); fs_count_launch();
+  following(k_pcg_init, 1, 1, 0, st)(P->scal, rtol * rtol); fs_count_launch();
+  following(k_zero_if_zero_rhs, 296, 256, 0, st)(n, P->scal, x); fs_count_launch();
   if (P->log_r0) {
     cudaMemcpyAsync(P->log_r0, P->pc_r, sizeof(double) * n, cudaMemcpyDeviceToDevice, st);
     cudaMemcpyAsync(P->log_x0, x, sizeof(double) * n, cudaMemcpyDeviceToDevice, st);
@@ -1878,7 +1919,8 @@ int proj_project(void* h, double* u, double* v, double* w, const double* u_in,
   P->stats[0] = ms_since(t_start);
   P->have_prev = 1;
   Launch3 L = launch_cells(g);
-  k_proj_correct<<<L.grid, L.block, 0, st>>>(g, u, v, w, x, P->ir, dt); fs_count_launch();
+  following(k_proj_correct, L.grid, L.block, 0, st)(g, u, v, w, x, P->ir, dt, dt / g.dx, dt / g.dy);
+  fs_count_launch();
   return cuda_status();
 }
 
@@ -1889,7 +1931,9 @@ int launch_div_resid_max(const GridDev& g, const double* u, const double* v, con
   int64_t n = ncells(g);
   unsigned nb = blocks_for(n, 256);
   if (nb > 1184) nb = 1184;
-  k_div_resid_max<<<nb, 256, 0, st>>>(g, u, v, w, u_in, target, div_out, out_key); fs_count_launch();
+  following(k_div_resid_max, nb, 256, 0, st)(g, u, v, w, u_in, target, 1.0 / g.dx, 1.0 / g.dy,
+                                            div_out, out_key);
+  fs_count_launch();
   return cuda_status();
 }
 
@@ -1897,7 +1941,7 @@ int launch_div_resid_max(const GridDev& g, const double* u, const double* v, con
 int proj_apply(void* h, const double* x, double* y, cudaStream_t st) {
   ProjCtx* P = (ProjCtx*)h;
   MGLevel& l0 = P->lev[0];
-  k_z_matvec<1><<<blocks_for(l0.n, Z_THREADS), Z_THREADS, 0, st>>>(l0.dims, op_0(P, 0.0), x, y,
+  following(k_z_matvec<1>, blocks_for(l0.n, Z_THREADS), Z_THREADS, 0, st)(l0.dims, op_0(P, 0.0), x, y,
                                                                   nullptr, nullptr);
   fs_count_launch();
   return cuda_status();
