@@ -163,31 +163,10 @@ __device__ __forceinline__ double solid_cond_cell(const GridDev& g, const double
 }
 
 // EDC flag scan tiling: a block of EDC_TPB threads owns EDC_TILE consecutive
-// cells, EDC_CPT per thread (thread t: cells EDC_CPT*t .. EDC_CPT*t + 3 of the
-// tile), so a thread's loads are two 16-byte vectors per FP64 field and the
-// tile's flat order is thread order, then the order within the thread.
+// cells, EDC_CPT per thread.
 #define EDC_TPB 256
 #define EDC_CPT 4
 #define EDC_TILE (EDC_TPB * EDC_CPT)
-
-// Exclusive max-scan over the block's threads of `last` (every thread's
-// largest code, -1 for none): the largest code of the threads before this
-// one.  `sh` holds EDC_TPB / 32 ints; one barrier.
-__device__ __forceinline__ int edc_block_exclusive_max(int last, int* sh) {
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  int v = last;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const int y = __shfl_up_sync(0xffffffffu, v, o);
-    if (lane >= o) v = max(v, y);
-  }
-  if (lane == 31) sh[wid] = v;
-  int ex = __shfl_up_sync(0xffffffffu, v, 1);
-  if (lane == 0) ex = -1;
-  __syncthreads();
-  for (int w = 0; w < wid; ++w) ex = max(ex, sh[w]);
-  return ex;
-}
 
 // Launch geometry helpers: one thread per cell, x fastest.
 struct Launch3 {

@@ -81,16 +81,6 @@ __device__ __forceinline__ void e32_ld4(const float* p, int64_t c0, int64_t n, b
   }
 }
 
-__device__ __forceinline__ void e32_st4(float* p, int64_t c0, int64_t n, bool vec, const float* v) {
-  if (vec) {
-    *reinterpret_cast<float4*>(p + c0) = make_float4(v[0], v[1], v[2], v[3]);
-  } else {
-#pragma unroll
-    for (int q = 0; q < EDC_CPT; ++q)
-      if (c0 + q < n) p[c0 + q] = v[q];
-  }
-}
-
 __global__ void __launch_bounds__(EDC_TPB)
 k_edc_agg32(int64_t n, const float* Yf, const float* YO, const float* YH, int vec_ok,
             signed char* agg) {
@@ -98,10 +88,16 @@ k_edc_agg32(int64_t n, const float* Yf, const float* YO, const float* YH, int ve
   const int t = threadIdx.x;
   const int64_t c0 = (int64_t)blockIdx.x * E32_BLK + EDC_CPT * t;
   const bool vec = vec_ok && c0 + EDC_CPT <= n;
-  float yf[EDC_CPT], yo[EDC_CPT], yh[EDC_CPT];
+  // (O2 and H2O matter where there is fuel: a small part of the domain)
+  float yf[EDC_CPT], yo[EDC_CPT] = {}, yh[EDC_CPT] = {};
   e32_ld4(Yf, c0, n, vec, yf);
-  e32_ld4(YO, c0, n, vec, yo);
-  e32_ld4(YH, c0, n, vec, yh);
+  bool fuel = false;
+#pragma unroll
+  for (int q = 0; q < EDC_CPT; ++q) fuel |= c0 + q < n && !(yf[q] <= 1e-9f);
+  if (fuel) {
+    e32_ld4(YO, c0, n, vec, yo);
+    e32_ld4(YH, c0, n, vec, yh);
+  }
   int v = -1;
 #pragma unroll
   for (int q = 0; q < EDC_CPT; ++q)
@@ -125,8 +121,29 @@ struct Edc32Args {
   const signed char* carry;
   float cp_g, dt, s_stoich, HoC_eff, relax, inv_s, inv_dt;
   int extinction, nsub;
-  int vec_ok;  // every array 16-byte aligned
 };
+
+// A cell without fuel or O2 has no reaction in any substep: the rate is 0 and
+// its mass fractions keep their values, whatever k and epsilon are, as long as
+// 0 / (rho cp) is a zero.
+__device__ __forceinline__ bool edc_idle32(const Edc32Args& a, float Yf, float YO2, float YH, float rho) {
+  const float cp = (1.0f - YH) * a.cp_g + YH * 2000.0f;
+  return (Yf <= 1e-9f || YO2 <= 1e-9f) && fabsf(rho) > 1e-37f && (cp > 0.0f || cp < 0.0f);
+}
+// what the update does to such a cell: the relaxation and the bounds
+__device__ __forceinline__ void edc_idle_cell32(const Edc32Args& a, bool flag, float& Yf, float& YO2,
+                                              float YH, float& Tg) {
+  if (Yf < 0.0f) Yf = 0.0f;
+  if (YO2 < 0.0f) YO2 = 0.0f;
+  for (int sub = 0; sub < a.nsub; ++sub) {
+    if (flag && Tg > 373.15f && YH > 0.0f) {
+      float wb = YH * (1.0f / 0.10f);
+      if (wb > 1.0f) wb = 1.0f;
+      Tg = Tg - (Tg - 373.15f) * a.relax * wb;
+    }
+    if (Tg > 2400.0f) Tg = 2400.0f;
+  }
+}
 
 // One cell's EDC update in float arithmetic (edc_cell's steps); Yf, YO2, Tg
 // in place, the mean reaction rate returned.
@@ -189,42 +206,77 @@ __device__ __forceinline__ float edc_cell32(const Edc32Args& a, bool flag, float
   return a.dt > 0.0f ? acc * a.inv_dt : 0.0f;
 }
 
-__global__ void __launch_bounds__(EDC_TPB)
+// A warp owns EDC_CPT x 32 consecutive cells, 32 of them a pass, so the cells
+// that react (a band of some tens in x) fill its lanes and the passes without
+// any are short.  With four consecutive cells a thread the band kept a few
+// lanes busy four cells deep: 26 us at 301 x 119 x 47, 22 so.
+__global__ void __launch_bounds__(EDC_TPB, 4)
 k_edc_main32(int64_t n, Edc32Args a) {
   __shared__ int sh[EDC_TPB / 32];
-  const int t = threadIdx.x;
-  const int64_t c0 = (int64_t)blockIdx.x * E32_BLK + EDC_CPT * t;
-  const bool vec = a.vec_ok && c0 + EDC_CPT <= n;
-  float yf[EDC_CPT], yo[EDC_CPT], yh[EDC_CPT], tg[EDC_CPT], rh[EDC_CPT], kt[EDC_CPT],
-      et[EDC_CPT];
-  e32_ld4(a.Yf, c0, n, vec, yf);
-  e32_ld4(a.YO, c0, n, vec, yo);
-  e32_ld4(a.YH, c0, n, vec, yh);
-  e32_ld4(a.Tg, c0, n, vec, tg);
-  e32_ld4(a.rho, c0, n, vec, rh);
-  e32_ld4(a.kt, c0, n, vec, kt);
-  e32_ld4(a.et, c0, n, vec, et);
-  const bool carry_in = a.carry[blockIdx.x] > 0;
-  int code[EDC_CPT];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const int64_t c0 = (int64_t)blockIdx.x * EDC_TILE + wid * (32 * EDC_CPT) + lane;
+  float yf[EDC_CPT], yo[EDC_CPT], yh[EDC_CPT], tg[EDC_CPT], rh[EDC_CPT];
+#pragma unroll
+  for (int q = 0; q < EDC_CPT; ++q) {
+    const int64_t c = c0 + 32 * q;
+    const bool in = c < n;
+    yf[q] = in ? a.Yf[c] : 0.0f;
+    yo[q] = in ? a.YO[c] : 0.0f;
+    yh[q] = in ? a.YH[c] : 0.0f;
+    tg[q] = in ? a.Tg[c] : 0.0f;
+    rh[q] = in ? a.rho[c] : 1.0f;
+  }
+  bool cur = a.carry[blockIdx.x] > 0;
+  // k and epsilon only where a cell may react
+  bool idle[EDC_CPT];
+  float kt[EDC_CPT] = {}, et[EDC_CPT] = {};
+#pragma unroll
+  for (int q = 0; q < EDC_CPT; ++q) {
+    const int64_t c = c0 + 32 * q;
+    idle[q] = c >= n || edc_idle32(a, yf[q], yo[q], yh[q], rh[q]);
+    if (!idle[q]) {
+      kt[q] = a.kt[c];
+      et[q] = a.et[c];
+    }
+  }
+  // the cells that set the quench flag, and those that set it to 1
+  unsigned sets[EDC_CPT], ones[EDC_CPT];
   int last = -1;
 #pragma unroll
   for (int q = 0; q < EDC_CPT; ++q) {
-    code[q] = (c0 + q < n) ? edc_flag_code32(yf[q], yo[q], yh[q], EDC_CPT * t + q) : -1;
-    last = max(last, code[q]);
+    const int code = edc_flag_code32(yf[q], yo[q], yh[q], 0);
+    sets[q] = __ballot_sync(0xffffffffu, code >= 0);
+    ones[q] = __ballot_sync(0xffffffffu, code == 1);
+    if (sets[q]) last = (ones[q] >> (31 - __clz(sets[q]))) & 1;
   }
-  int run = edc_block_exclusive_max(last, sh);
-  if (c0 >= n) return;
-  float om[EDC_CPT];
+  if (lane == 0) sh[wid] = last;
+  __syncthreads();
+  for (int w = 0; w < wid; ++w)
+    if (sh[w] >= 0) cur = sh[w] != 0;
 #pragma unroll
   for (int q = 0; q < EDC_CPT; ++q) {
-    run = max(run, code[q]);
-    const bool flag = (run >= 0) ? (run & 1) : carry_in;
-    om[q] = edc_cell32(a, flag, yf[q], yo[q], yh[q], tg[q], rh[q], kt[q], et[q]);
+    const int64_t c = c0 + 32 * q;
+    const unsigned upto = sets[q] & (0xffffffffu >> (31 - lane));
+    const bool flag = upto ? (ones[q] >> (31 - __clz(upto))) & 1 : cur;
+    if (sets[q]) cur = (ones[q] >> (31 - __clz(sets[q]))) & 1;
+    if (c >= n) continue;
+    float om = 0.0f;
+    bool changed = true;
+    if (idle[q]) {
+      const float f0 = yf[q], o0 = yo[q], t0 = tg[q];
+      edc_idle_cell32(a, flag, yf[q], yo[q], yh[q], tg[q]);
+      changed = yf[q] != f0 || yo[q] != o0 || tg[q] != t0;
+    } else {
+      om = edc_cell32(a, flag, yf[q], yo[q], yh[q], tg[q], rh[q], kt[q], et[q]);
+    }
+    // (updated in place: where nothing changed the arrays hold the result)
+    if (changed) {
+      a.Yf[c] = yf[q];
+      a.YO[c] = yo[q];
+      a.Tg[c] = tg[q];
+    }
+    a.omega[c] = om;
   }
-  e32_st4(a.Yf, c0, n, vec, yf);
-  e32_st4(a.YO, c0, n, vec, yo);
-  e32_st4(a.Tg, c0, n, vec, tg);
-  e32_st4(a.omega, c0, n, vec, om);
 }
 
 int64_t edc32_scratch_bytes(int64_t n) { return 2 * ((n + E32_BLK - 1) / E32_BLK) + 16; }
@@ -239,8 +291,7 @@ int launch_edc32(int64_t n, const float* rho, float* Tg, float* Yf, float* YO, c
   const int64_t nb = (n + E32_BLK - 1) / E32_BLK;
   signed char* agg = (signed char*)scratch;
   signed char* carry = agg + nb;
-  const int vec_ok = al16(rho) && al16(Tg) && al16(Yf) && al16(YO) && al16(kt) && al16(et) &&
-                     al16(YH) && al16(omega);
+  const int vec_ok = al16(Yf) && al16(YO) && al16(YH);
   k_edc_agg32<<<(unsigned)nb, EDC_TPB, 0, st>>>(n, Yf, YO, YH, vec_ok, agg);
   fs_count_launch();
   int rc = launch_edc_carry((int)nb, agg, carry, st);
@@ -255,7 +306,6 @@ int launch_edc32(int64_t n, const float* rho, float* Tg, float* Yf, float* YO, c
   a.nsub = n_substeps > 1 ? n_substeps : 1;
   a.relax = (float)(1.0 - exp(-(dt / (double)a.nsub) / 0.5));
   a.extinction = extinction;
-  a.vec_ok = vec_ok;
   k_edc_main32<<<(unsigned)nb, EDC_TPB, 0, st>>>(n, a);
   fs_count_launch();
   return cuda_status();
