@@ -123,8 +123,8 @@ __device__ __forceinline__ double dmax(double a, double b) { return a > b ? a : 
 // harmonic-mean face conductances to the bed cells above and below and the
 // explicit update; cap = 1 clips the result to [lo, hi] (the T_s cap that
 // follows the conduction, spread_3d.py:3193-3196).  T0 = Ts[c].
-__device__ __forceinline__ double solid_cond_cell(const GridDev& g, const double* __restrict__ Ts,
-                                                  const double* __restrict__ as, int k, int64_t c,
+__device__ __forceinline__ double solid_cond_cell(const GridDev& g, const double* Ts,
+                                                  const double* as, int k, int64_t c,
                                                   double T0, double k_solid, double inv_rho_cp,
                                                   double dt, int cap, double lo, double hi) {
   const int64_t sz = (int64_t)g.nx * g.ny;

@@ -52,6 +52,7 @@ __device__ __forceinline__ void edc_ld4(const double* p, int64_t c0, int64_t n, 
 __global__ void __launch_bounds__(EDC_TPB)
 k_edc_agg(int64_t n, const double* Yf, const double* YO, const double* YH, int vec_ok,
           signed char* agg) {
+  FOLLOW();
   __shared__ int sh[EDC_TPB / 32];
   const int t = threadIdx.x;
   const int64_t c0 = (int64_t)blockIdx.x * EDC_TILE + EDC_CPT * t;
@@ -87,6 +88,7 @@ k_edc_agg(int64_t n, const double* Yf, const double* YO, const double* YH, int v
 #define EDC_CARRY_THREADS 1024
 __global__ void __launch_bounds__(EDC_CARRY_THREADS)
 k_edc_carry(int nb, const signed char* agg, signed char* carry, const signed char* carry_in) {
+  FOLLOW();
   __shared__ int incl[EDC_CARRY_THREADS];
   __shared__ int wsum[32];
   const int t = threadIdx.x;
@@ -125,7 +127,7 @@ k_edc_carry(int nb, const signed char* agg, signed char* carry, const signed cha
 }
 
 int launch_edc_carry(int nb, const signed char* agg, signed char* carry, cudaStream_t st) {
-  k_edc_carry<<<1, EDC_CARRY_THREADS, 0, st>>>(nb, agg, carry, nullptr);
+  following(k_edc_carry, 1, EDC_CARRY_THREADS, 0, st)(nb, agg, carry, nullptr);
   fs_count_launch();
   return cuda_status();
 }
@@ -247,6 +249,7 @@ __device__ __forceinline__ double edc_cell(const EdcArgs& a, bool flag, double& 
 // where all inputs and outputs are 253).
 __global__ void __launch_bounds__(EDC_TPB, 3)
 k_edc_main(int64_t n, EdcArgs a) {
+  FOLLOW();
   __shared__ int sh[EDC_TPB / 32];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const int64_t c0 = (int64_t)blockIdx.x * EDC_TILE + wid * (32 * EDC_CPT) + lane;
@@ -329,8 +332,8 @@ int launch_edc(int64_t n, const double* rho, double* Tg, double* Yf, double* YO,
   signed char* agg = (signed char*)scratch;
   signed char* carry = agg + nb;
   const int vec_ok = al16(Yf) && al16(YO) && al16(YH);
-  k_edc_agg<<<(unsigned)nb, EDC_TPB, 0, st>>>(n, Yf, YO, YH, vec_ok, agg); fs_count_launch();
-  k_edc_carry<<<1, EDC_CARRY_THREADS, 0, st>>>((int)nb, agg, carry, nullptr); fs_count_launch();
+  following(k_edc_agg, (unsigned)nb, EDC_TPB, 0, st)(n, Yf, YO, YH, vec_ok, agg); fs_count_launch();
+  following(k_edc_carry, 1, EDC_CARRY_THREADS, 0, st)((int)nb, agg, carry, nullptr); fs_count_launch();
   EdcArgs a{};
   a.rho = rho; a.Tg = Tg; a.Yf = Yf; a.YO = YO; a.kt = kt; a.et = et; a.YH = YH;
   a.omega = omega; a.carry = carry;
@@ -341,7 +344,7 @@ int launch_edc(int64_t n, const double* rho, double* Tg, double* Yf, double* YO,
   a.nsub = n_substeps > 1 ? n_substeps : 1;
   a.relax = 1.0 - exp(-(dt / (double)a.nsub) / 0.5);
   a.extinction = extinction;
-  k_edc_main<<<(unsigned)nb, EDC_TPB, 0, st>>>(n, a); fs_count_launch();
+  following(k_edc_main, (unsigned)nb, EDC_TPB, 0, st)(n, a); fs_count_launch();
   return cuda_status();
 }
 
@@ -396,6 +399,7 @@ __device__ __forceinline__ double gas_update_cell(const GridDev& g, const GasArg
 }
 
 __global__ void k_gas_update(GridDev g, GasArgs a) {
+  FOLLOW();
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   int j = blockIdx.y * blockDim.y + threadIdx.y;
   int k = blockIdx.z;
@@ -419,6 +423,7 @@ struct SolidArgs {
 };
 
 __global__ void k_gas_solid(GridDev g, GasArgs a, SolidArgs b) {
+  FOLLOW();
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   int j = blockIdx.y * blockDim.y + threadIdx.y;
   int k = blockIdx.z;
@@ -449,7 +454,7 @@ int launch_gas_solid(const GridDev& g, double* Tg, const double* rho, const doub
   a.drip_on = drip_on; a.n_z_bed = n_z_bed; a.i_src0 = i_src0; a.i_src1 = i_src1;
   SolidArgs b{as, Ts_out, k_solid, 1.0 / (rho_s * cp_s), lo, hi};
   Launch3 L = launch_cells(g);
-  k_gas_solid<<<L.grid, L.block, 0, st>>>(g, a, b); fs_count_launch();
+  following(k_gas_solid, L.grid, L.block, 0, st)(g, a, b); fs_count_launch();
   return cuda_status();
 }
 
@@ -466,7 +471,7 @@ int launch_gas_update(const GridDev& g, double* Tg, const double* rho, const dou
   a.q_drip_gas = (1.0 - 0.80) * q_drip;
   a.drip_on = drip_on; a.n_z_bed = n_z_bed; a.i_src0 = i_src0; a.i_src1 = i_src1;
   Launch3 L = launch_cells(g);
-  k_gas_update<<<L.grid, L.block, 0, st>>>(g, a); fs_count_launch();
+  following(k_gas_update, L.grid, L.block, 0, st)(g, a); fs_count_launch();
   return cuda_status();
 }
 
@@ -475,8 +480,9 @@ int launch_gas_update(const GridDev& g, double* Tg, const double* rho, const dou
 //   rho_prev = rho; rho = P0 / (R_air max(T_g, T_amb)); Y_O2[:, :, 0] = 0.232
 // and the closing EoS (spread_3d.py:3440) with prev == null.
 // ---------------------------------------------------------------------------
-__global__ void k_eos(GridDev g, double* rho, double* rho_prev, const double* __restrict__ Tg,
+__global__ void k_eos(GridDev g, double* rho, double* rho_prev, const double* Tg,
                       double* YO, double P0, double R_air, double T_amb) {
+  FOLLOW();
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   int j = blockIdx.y * blockDim.y + threadIdx.y;
   int k = blockIdx.z;
@@ -492,7 +498,7 @@ __global__ void k_eos(GridDev g, double* rho, double* rho_prev, const double* __
 int launch_eos(const GridDev& g, double* rho, double* rho_prev, const double* Tg, double* YO,
                double P0, double R_air, double T_amb, cudaStream_t st) {
   Launch3 L = launch_cells(g);
-  k_eos<<<L.grid, L.block, 0, st>>>(g, rho, rho_prev, Tg, YO, P0, R_air, T_amb); fs_count_launch();
+  following(k_eos, L.grid, L.block, 0, st)(g, rho, rho_prev, Tg, YO, P0, R_air, T_amb); fs_count_launch();
   return cuda_status();
 }
 
@@ -500,9 +506,10 @@ int launch_eos(const GridDev& g, double* rho, double* rho_prev, const double* Tg
 // unweighted form): ((S_pyro + S_drying) - (rho - rho_prev)/dt) / max(rho, 0.1),
 // with S_pyro = copy of the bed's pyrolysis source plus its drying source
 // (spread_3d.py:2147-2148).  np.maximum keeps a NaN rho.
-__global__ void k_div_target(int64_t n, const double* __restrict__ rho,
-                             const double* __restrict__ rho_prev, const double* __restrict__ Sp,
-                             const double* __restrict__ Sd, double dt, double* __restrict__ out) {
+__global__ void k_div_target(int64_t n, const double* rho,
+                             const double* rho_prev, const double* Sp,
+                             const double* Sd, double dt, double* out) {
+  FOLLOW();
   int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (c >= n) return;
   const double r = rho[c];
@@ -515,7 +522,7 @@ __global__ void k_div_target(int64_t n, const double* __restrict__ rho,
 int launch_div_target(int64_t n, const double* rho, const double* rho_prev, const double* Sp,
                       const double* Sd, double dt, double* out, cudaStream_t st) {
   if (n == 0) return FS_OK;
-  k_div_target<<<blocks_for(n, 256), 256, 0, st>>>(n, rho, rho_prev, Sp, Sd, dt, out);
+  following(k_div_target, blocks_for(n, 256), 256, 0, st)(n, rho, rho_prev, Sp, Sd, dt, out);
   fs_count_launch();
   return cuda_status();
 }
@@ -670,6 +677,7 @@ int launch_coldiag_keys(const void* scratch, double* out4, cudaStream_t st) {
 
 // clip a field to [lo, hi] (numpy minimum/maximum semantics: NaN stays NaN)
 __global__ void k_clip(int64_t n, double* f, double lo, double hi) {
+  FOLLOW();
   int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (c >= n) return;
   double x = f[c];
@@ -679,7 +687,7 @@ __global__ void k_clip(int64_t n, double* f, double lo, double hi) {
 }
 
 int launch_clip(int64_t n, double* f, double lo, double hi, cudaStream_t st) {
-  k_clip<<<blocks_for(n, 256), 256, 0, st>>>(n, f, lo, hi); fs_count_launch();
+  following(k_clip, blocks_for(n, 256), 256, 0, st)(n, f, lo, hi); fs_count_launch();
   return cuda_status();
 }
 
@@ -689,8 +697,9 @@ int launch_clip(int64_t n, double* f, double lo, double hi, cudaStream_t st) {
 //   mode 2: max f over k in [1,Nz-2], i in [1,Nx-2], starting at 0, NaN ignored
 //           (turbulence_3d.py:894-900)
 // ---------------------------------------------------------------------------
-__global__ void k_max(GridDev g, const double* __restrict__ f, int mode,
+__global__ void k_max(GridDev g, const double* f, int mode,
                       unsigned long long* out) {
+  FOLLOW();
   int64_t n = ncells_dev(g);
   unsigned long long best = dkey(mode == 2 ? 0.0 : -INFINITY);
   for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < n;
@@ -715,6 +724,7 @@ __global__ void k_max(GridDev g, const double* __restrict__ f, int mode,
 }
 
 __global__ void k_init_keys(unsigned long long* out, int n, int mode2_mask) {
+  FOLLOW();
   int t = threadIdx.x;
   if (t < n) out[t] = ((mode2_mask >> t) & 1) ? dkey(0.0) : dkey(-INFINITY);
 }
@@ -724,21 +734,22 @@ int launch_max(const GridDev& g, const double* f, int mode, unsigned long long* 
   int64_t n = ncells(g);
   unsigned nb = blocks_for(n, 256);
   if (nb > 148 * 8) nb = 148 * 8;
-  k_max<<<nb, 256, 0, st>>>(g, f, mode, out_key); fs_count_launch();
+  following(k_max, nb, 256, 0, st)(g, f, mode, out_key); fs_count_launch();
   return cuda_status();
 }
 
 int launch_init_keys(unsigned long long* out, int n, int mode2_mask, cudaStream_t st) {
-  k_init_keys<<<1, 64, 0, st>>>(out, n, mode2_mask); fs_count_launch();
+  following(k_init_keys, 1, 64, 0, st)(out, n, mode2_mask); fs_count_launch();
   return cuda_status();
 }
 
 __global__ void k_keys_to_double(const unsigned long long* in, double* out, int n) {
+  FOLLOW();
   int t = threadIdx.x;
   if (t < n) out[t] = dkey_inv(in[t]);
 }
 
 int launch_keys_to_double(const unsigned long long* in, double* out, int n, cudaStream_t st) {
-  k_keys_to_double<<<1, 64, 0, st>>>(in, out, n); fs_count_launch();
+  following(k_keys_to_double, 1, 64, 0, st)(in, out, n); fs_count_launch();
   return cuda_status();
 }

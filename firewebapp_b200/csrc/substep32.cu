@@ -26,12 +26,14 @@ struct CvArgs {
 };
 
 __global__ void k_to_f32(int64_t n, CvArgs a) {
+  FOLLOW();
   for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < n;
        c += (int64_t)gridDim.x * blockDim.x)
     for (int f = 0; f < a.nf; ++f) ((float*)a.dst[f])[c] = (float)((const double*)a.src[f])[c];
 }
 
 __global__ void k_to_f64(int64_t n, CvArgs a) {
+  FOLLOW();
   for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < n;
        c += (int64_t)gridDim.x * blockDim.x)
     for (int f = 0; f < a.nf; ++f) ((double*)a.dst[f])[c] = (double)((const float*)a.src[f])[c];
@@ -49,8 +51,8 @@ int launch_convert(int64_t n, int nf, const void* const* src, void* const* dst, 
   }
   unsigned nb = blocks_for(n, 256);
   if (nb > 148 * 16) nb = 148 * 16;
-  if (to_f32) k_to_f32<<<nb, 256, 0, st>>>(n, a);
-  else k_to_f64<<<nb, 256, 0, st>>>(n, a);
+  if (to_f32) following(k_to_f32, nb, 256, 0, st)(n, a);
+  else following(k_to_f64, nb, 256, 0, st)(n, a);
   fs_count_launch();
   return cuda_status();
 }
@@ -84,6 +86,7 @@ __device__ __forceinline__ void e32_ld4(const float* p, int64_t c0, int64_t n, b
 __global__ void __launch_bounds__(EDC_TPB)
 k_edc_agg32(int64_t n, const float* Yf, const float* YO, const float* YH, int vec_ok,
             signed char* agg) {
+  FOLLOW();
   __shared__ int sh[EDC_TPB / 32];
   const int t = threadIdx.x;
   const int64_t c0 = (int64_t)blockIdx.x * E32_BLK + EDC_CPT * t;
@@ -212,6 +215,7 @@ __device__ __forceinline__ float edc_cell32(const Edc32Args& a, bool flag, float
 // lanes busy four cells deep: 26 us at 301 x 119 x 47, 22 so.
 __global__ void __launch_bounds__(EDC_TPB, 4)
 k_edc_main32(int64_t n, Edc32Args a) {
+  FOLLOW();
   __shared__ int sh[EDC_TPB / 32];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const int64_t c0 = (int64_t)blockIdx.x * EDC_TILE + wid * (32 * EDC_CPT) + lane;
@@ -292,7 +296,7 @@ int launch_edc32(int64_t n, const float* rho, float* Tg, float* Yf, float* YO, c
   signed char* agg = (signed char*)scratch;
   signed char* carry = agg + nb;
   const int vec_ok = al16(Yf) && al16(YO) && al16(YH);
-  k_edc_agg32<<<(unsigned)nb, EDC_TPB, 0, st>>>(n, Yf, YO, YH, vec_ok, agg);
+  following(k_edc_agg32, (unsigned)nb, EDC_TPB, 0, st)(n, Yf, YO, YH, vec_ok, agg);
   fs_count_launch();
   int rc = launch_edc_carry((int)nb, agg, carry, st);
   if (rc != FS_OK) return rc;
@@ -306,7 +310,7 @@ int launch_edc32(int64_t n, const float* rho, float* Tg, float* Yf, float* YO, c
   a.nsub = n_substeps > 1 ? n_substeps : 1;
   a.relax = (float)(1.0 - exp(-(dt / (double)a.nsub) / 0.5));
   a.extinction = extinction;
-  k_edc_main32<<<(unsigned)nb, EDC_TPB, 0, st>>>(n, a);
+  following(k_edc_main32, (unsigned)nb, EDC_TPB, 0, st)(n, a);
   fs_count_launch();
   return cuda_status();
 }
@@ -359,6 +363,7 @@ struct Gas32Args {
 };
 
 __global__ void k_gas_update32(GridDev g, Gas32Args a) {
+  FOLLOW();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int j = blockIdx.y * blockDim.y + threadIdx.y;
   const int k = blockIdx.z;
@@ -396,13 +401,14 @@ int launch_gas_update32(const GridDev& g, float* Tg, const float* rho, const flo
   a.q_drip_gas = (float)((1.0 - 0.80) * q_drip);
   a.drip_on = drip_on; a.n_z_bed = n_z_bed; a.i_src0 = i_src0; a.i_src1 = i_src1;
   Launch3 L = launch_cells(g);
-  k_gas_update32<<<L.grid, L.block, 0, st>>>(g, a);
+  following(k_gas_update32, L.grid, L.block, 0, st)(g, a);
   fs_count_launch();
   return cuda_status();
 }
 
 // ---- clip ------------------------------------------------------------------------
 __global__ void k_clip32(int64_t n, float* f, float lo, float hi) {
+  FOLLOW();
   const int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (c >= n) return;
   float x = f[c];
@@ -413,7 +419,7 @@ __global__ void k_clip32(int64_t n, float* f, float lo, float hi) {
 
 int launch_clip32(int64_t n, float* f, double lo, double hi, cudaStream_t st) {
   if (n == 0) return FS_OK;
-  k_clip32<<<blocks_for(n, 256), 256, 0, st>>>(n, f, (float)lo, (float)hi);
+  following(k_clip32, blocks_for(n, 256), 256, 0, st)(n, f, (float)lo, (float)hi);
   fs_count_launch();
   return cuda_status();
 }

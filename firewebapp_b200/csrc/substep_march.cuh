@@ -28,6 +28,7 @@ struct SpeciesArgs {
 template <typename T, int NS, bool FUSED>
 __global__ void __launch_bounds__(MR_THREADS, sizeof(T) == 8 ? 3 : 4)
     k_species(GridDev g, SpeciesArgs<T> a, int kz) {
+  FOLLOW();
   typedef PlaneRing<T, NS, 2, 6> Ring;
   extern __shared__ __align__(16) unsigned char mr_raw[];
   T* const ring = (T*)mr_raw;
@@ -115,7 +116,7 @@ static int launch_species_march(const GridDev& g, const SpeciesArgs<T>& a, cudaS
   constexpr int smem = PlaneRing<T, NS, 2, 6>::BYTES + MR_MAXK * MR_RK * (int)sizeof(T);
   const int kz = march_levels(g);
   if (!march_smem((const void*)k_species<T, NS, FUSED>, smem)) return cuda_status();
-  k_species<T, NS, FUSED><<<march_grid(g, kz), dim3(MR_TX, MR_TY), smem, st>>>(g, a, kz);
+  following(k_species<T, NS, FUSED>, march_grid(g, kz), dim3(MR_TX, MR_TY), smem, st)(g, a, kz);
   fs_count_launch();
   return cuda_status();
 }
@@ -140,6 +141,7 @@ struct DiffArgs {
 // neighbours in x and y loaded when they were used.
 template <typename T, int NF>
 __global__ void __launch_bounds__(MR_THREADS, 4) k_turb_diff(GridDev g, DiffArgs<T> a, int kz) {
+  FOLLOW();
   typedef PlaneRing<T, NF, 1, 5> Ring;
   extern __shared__ __align__(16) unsigned char mr_raw[];
   T* const ring = (T*)mr_raw;
@@ -204,7 +206,7 @@ static int launch_turb_march(const GridDev& g, const DiffArgs<T>& a, cudaStream_
   constexpr int smem = PlaneRing<T, NF, 1, 5>::BYTES + MR_MAXK * MR_RK * (int)sizeof(T);
   const int kz = march_levels(g);
   if (!march_smem((const void*)k_turb_diff<T, NF>, smem)) return cuda_status();
-  k_turb_diff<T, NF><<<march_grid(g, kz), dim3(MR_TX, MR_TY), smem, st>>>(g, a, kz);
+  following(k_turb_diff<T, NF>, march_grid(g, kz), dim3(MR_TX, MR_TY), smem, st)(g, a, kz);
   fs_count_launch();
   return cuda_status();
 }

@@ -148,10 +148,11 @@ int launch_advect_scalar(const GridDev& g, const double* phi, const double* u, c
 // instructions a warp, a third of them divisions by spacings; 38 now)
 typedef PlaneRing<double, 1, 2, 6> GasRing;
 __global__ void __launch_bounds__(MR_THREADS, 4)
-    k_gas_energy_adv(GridDev g, const double* __restrict__ T, const double* __restrict__ u,
-                     const double* __restrict__ v, const double* __restrict__ w,
-                     double* __restrict__ To, double dt, double alpha, double T_amb, double inv_dx,
+    k_gas_energy_adv(GridDev g, const double* T, const double* u,
+                     const double* v, const double* w,
+                     double* To, double dt, double alpha, double T_amb, double inv_dx,
                      double inv_dy, int kz) {
+  FOLLOW();
   extern __shared__ __align__(16) unsigned char mr_raw[];
   double* const ring = (double*)mr_raw;
   double* const rks = (double*)(mr_raw + GasRing::BYTES);
@@ -221,7 +222,8 @@ int launch_gas_energy_adv(const GridDev& g, const double* T, const double* u, co
   if (g.nx < 3 || g.nz < 3) return FS_EARG;
   const int kz = march_levels(g);
   if (!march_smem((const void*)k_gas_energy_adv, GasRing::BYTES + MR_RK_BYTES)) return cuda_status();
-  k_gas_energy_adv<<<march_grid(g, kz), dim3(MR_TX, MR_TY), GasRing::BYTES + MR_RK_BYTES, st>>>(
+  following(k_gas_energy_adv, march_grid(g, kz), dim3(MR_TX, MR_TY), GasRing::BYTES + MR_RK_BYTES,
+            st)(
       g, T, u, v, w, To, dt, alpha, T_amb, 1.0 / g.dx, 1.0 / g.dy, kz);
   fs_count_launch();
   return cuda_status();
@@ -310,6 +312,7 @@ struct MomArgs {
 // 400 x 120 x 60; 104 now.
 typedef PlaneRing<double, 3, 2, 6> MomRing;
 __global__ void __launch_bounds__(MR_THREADS, 3) k_momentum(GridDev g, MomArgs a, int kz) {
+  FOLLOW();
   extern __shared__ __align__(16) unsigned char mr_raw[];
   double* const ring = (double*)mr_raw;
   double* const rks = (double*)(mr_raw + MomRing::BYTES);
@@ -418,7 +421,8 @@ int launch_momentum(const GridDev& g, const double* u, const double* v, const do
   a.inv_dx2 = a.inv_dx * a.inv_dx; a.inv_dy2 = a.inv_dy * a.inv_dy;
   const int kz = march_levels(g);
   if (!march_smem((const void*)k_momentum, MomRing::BYTES + MR_RK_BYTES)) return cuda_status();
-  k_momentum<<<march_grid(g, kz), dim3(MR_TX, MR_TY), MomRing::BYTES + MR_RK_BYTES, st>>>(g, a, kz);
+  following(k_momentum, march_grid(g, kz), dim3(MR_TX, MR_TY), MomRing::BYTES + MR_RK_BYTES, st)(
+      g, a, kz);
   fs_count_launch();
   return cuda_status();
 }
@@ -426,9 +430,10 @@ int launch_momentum(const GridDev& g, const double* u, const double* v, const do
 // ---------------------------------------------------------------------------
 // Outflow sponge (momentum_3d.py:293-317), in place
 // ---------------------------------------------------------------------------
-__global__ void k_sponge(GridDev g, double* u, const double* __restrict__ u_t,
-                         const double* __restrict__ sig_x, const double* __restrict__ YF,
+__global__ void k_sponge(GridDev g, double* u, const double* u_t,
+                         const double* sig_x, const double* YF,
                          double skip, double dt) {
+  FOLLOW();
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   int j = blockIdx.y * blockDim.y + threadIdx.y;
   int k = blockIdx.z;
@@ -444,7 +449,7 @@ __global__ void k_sponge(GridDev g, double* u, const double* __restrict__ u_t,
 int launch_sponge(const GridDev& g, double* u, const double* u_t, const double* sig_x,
                   const double* YF, double skip, double dt, cudaStream_t st) {
   Launch3 L = launch_cells(g);
-  k_sponge<<<L.grid, L.block, 0, st>>>(g, u, u_t, sig_x, YF, skip, dt); fs_count_launch();
+  following(k_sponge, L.grid, L.block, 0, st)(g, u, u_t, sig_x, YF, skip, dt); fs_count_launch();
   return cuda_status();
 }
 
@@ -479,6 +484,7 @@ typedef PlaneRing<double, 2, 2, 6> KeRing;
 typedef PlaneRing<double, 3, 1, 4> VelRing;
 #define KEPS_SMEM (KeRing::BYTES + VelRing::BYTES)
 __global__ void __launch_bounds__(MR_THREADS, 2) k_keps(GridDev g, KepsArgs a, int kz) {
+  FOLLOW();
   extern __shared__ __align__(16) unsigned char mr_raw[];
   double* const ring = (double*)mr_raw;
   double* const vring = (double*)(mr_raw + KeRing::BYTES);
@@ -653,7 +659,7 @@ int launch_keps(const GridDev& g, const double* k, const double* e, const double
   if (g.nz < 2) return FS_EARG;
   const int kz = march_levels(g);
   if (!march_smem((const void*)k_keps, KEPS_SMEM + MR_RK_BYTES)) return cuda_status();
-  k_keps<<<march_grid(g, kz), dim3(MR_TX, MR_TY), KEPS_SMEM + MR_RK_BYTES, st>>>(g, a, kz);
+  following(k_keps, march_grid(g, kz), dim3(MR_TX, MR_TY), KEPS_SMEM + MR_RK_BYTES, st)(g, a, kz);
   fs_count_launch();
   return cuda_status();
 }
@@ -663,10 +669,11 @@ int launch_keps(const GridDev& g, const double* k, const double* e, const double
 // ---------------------------------------------------------------------------
 // cap = 1: the result is then clipped to [lo, hi] as k_clip does (the T_s
 // cap that follows the conduction, spread_3d.py:3193-3196)
-__global__ void k_solid_cond(GridDev g, const double* __restrict__ Ts,
-                             const double* __restrict__ as, double* __restrict__ To,
+__global__ void k_solid_cond(GridDev g, const double* Ts,
+                             const double* as, double* To,
                              double k_solid, double inv_rho_cp, double dt, int cap, double lo,
                              double hi) {
+  FOLLOW();
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   int j = blockIdx.y * blockDim.y + threadIdx.y;
   int k = blockIdx.z;
@@ -681,7 +688,7 @@ int launch_solid_cond(const GridDev& g, const double* Ts, const double* as, doub
   GridDev gg = g;
   Launch3 L = launch_cells(g);
   (void)nz_active;
-  k_solid_cond<<<L.grid, L.block, 0, st>>>(gg, Ts, as, To, k_solid, 1.0 / (rho_s * cp_s), dt,
+  following(k_solid_cond, L.grid, L.block, 0, st)(gg, Ts, as, To, k_solid, 1.0 / (rho_s * cp_s), dt,
                                            cap, lo, hi); fs_count_launch();
   return cuda_status();
 }
