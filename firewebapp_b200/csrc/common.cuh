@@ -162,6 +162,24 @@ __device__ __forceinline__ double solid_cond_cell(const GridDev& g, const double
   return x;
 }
 
+// The largest key of a block into *out, by one atomic: one a warp queued at the
+// address (9472 of them, some 20 us of a reduction of 2.9 million cells).
+__device__ __forceinline__ void block_max_to(unsigned long long key, unsigned long long* out) {
+  __shared__ unsigned long long wmax[32];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const unsigned long long y = __shfl_xor_sync(0xffffffffu, key, o);
+    key = y > key ? y : key;
+  }
+  const int warps = (blockDim.x + 31) >> 5;
+  if ((threadIdx.x & 31) == 0) wmax[threadIdx.x >> 5] = key;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int w = 1; w < warps; ++w) key = wmax[w] > key ? wmax[w] : key;
+    atomicMax(out, key);
+  }
+}
+
 // EDC flag scan tiling: a block of EDC_TPB threads owns EDC_TILE consecutive
 // cells, EDC_CPT per thread.
 #define EDC_TPB 256

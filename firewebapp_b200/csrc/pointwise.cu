@@ -702,13 +702,14 @@ __global__ void k_max(GridDev g, const double* f, int mode,
   FOLLOW();
   int64_t n = ncells_dev(g);
   unsigned long long best = dkey(mode == 2 ? 0.0 : -INFINITY);
+#pragma unroll 4
   for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < n;
        c += (int64_t)gridDim.x * blockDim.x) {
     double x = f[c];
     if (mode == 0) x = fabs(x);
     if (mode == 2) {
-      int i = (int)(c % g.nx);
-      int k = (int)(c / ((int64_t)g.nx * g.ny));
+      int i, j, k;
+      split_cell((uint32_t)c, g.fnx, g.fny, i, j, k);
       if (k < 1 || k > g.nz - 2 || i < 1 || i > g.nx - 2) continue;
       if (x != x) continue;
     }
@@ -716,11 +717,7 @@ __global__ void k_max(GridDev g, const double* f, int mode,
     unsigned long long kk = dkey(x);
     if (kk > best) best = kk;
   }
-  for (int o = 16; o > 0; o >>= 1) {
-    unsigned long long y = __shfl_xor_sync(0xffffffffu, best, o);
-    if (y > best) best = y;
-  }
-  if ((threadIdx.x & 31) == 0) atomicMax(out, best);
+  block_max_to(best, out);
 }
 
 __global__ void k_init_keys(unsigned long long* out, int n, int mode2_mask) {

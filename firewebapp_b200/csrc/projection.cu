@@ -991,6 +991,9 @@ __global__ void k_proj_correct(GridDev g, double* u, double* v, double* w,
 }
 
 // max |div(u) - target| (projection_3d.py:847-892 plain branch)
+// (OUT: the divergence is wanted too; without its stores the loads of four cells
+// a thread are in flight together)
+template <bool OUT>
 __global__ void k_div_resid_max(GridDev g, const double* u,
                                 const double* v, const double* w,
                                 const double* u_in, const double* target,
@@ -1002,6 +1005,7 @@ __global__ void k_div_resid_max(GridDev g, const double* u,
   const int64_t sy = nx, sz = (int64_t)nx * ny;
   double best = 0.0;
   bool nan = false;
+#pragma unroll 4
   for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < n;
        c += (int64_t)gridDim.x * blockDim.x) {
     int i, j, k;
@@ -1015,18 +1019,14 @@ __global__ void k_div_resid_max(GridDev g, const double* u,
     }
     if (k > 0) div += (w[c] - w[c - sz]) / g.dz[k];
     else div += (w[c] - 0.0) / g.dz[0];
-    if (div_out) div_out[c] = div;
+    if (OUT) div_out[c] = div;
     if (target) div = div - target[c];
     double a = fabs(div);
     if (a != a) nan = true;
     else if (a > best) best = a;
   }
   unsigned long long key = nan ? 0x7ff8000000000000ull : (unsigned long long)__double_as_longlong(best);
-  for (int o = 16; o > 0; o >>= 1) {
-    unsigned long long y = __shfl_xor_sync(0xffffffffu, key, o);
-    key = y > key ? y : key;
-  }
-  if ((threadIdx.x & 31) == 0) atomicMax(out_key, key);
+  block_max_to(key, out_key);
 }
 
 // ---------------------------------------------------------------------------
@@ -1931,8 +1931,8 @@ int launch_div_resid_max(const GridDev& g, const double* u, const double* v, con
   int64_t n = ncells(g);
   unsigned nb = blocks_for(n, 256);
   if (nb > 1184) nb = 1184;
-  following(k_div_resid_max, nb, 256, 0, st)(g, u, v, w, u_in, target, 1.0 / g.dx, 1.0 / g.dy,
-                                            div_out, out_key);
+  following(div_out ? k_div_resid_max<true> : k_div_resid_max<false>, nb, 256, 0, st)(
+      g, u, v, w, u_in, target, 1.0 / g.dx, 1.0 / g.dy, div_out, out_key);
   fs_count_launch();
   return cuda_status();
 }
