@@ -1567,6 +1567,39 @@ static bool plan_rp(DomCtx* D, int force_C) {
   return found;
 }
 
+static int64_t rp_wrap_elems(const DomCtx* D, size_t ts) {
+  return 8ll * rp_pad((int)ts, D->M / 8) * D->g.nz * (D->g.nx + D->g.nz - 1);
+}
+
+// The register-patch kernel's layouts.  They take more memory than the pencil
+// kernel's (some 500 MB against 300 at 400 x 120 x 60): where they do not fit, that
+// one runs.
+static bool rp_alloc(DomCtx* D, size_t ts) {
+  const GridDev& g = D->g;
+  const int64_t plane = (int64_t)(g.nx + g.ny - 1) * rp_pitch(g.ny);
+  const int64_t all = (int64_t)(g.nx + g.ny + g.nz - 2) * g.nz * rp_pitch(g.ny);
+  bool got = true;
+  auto take = [&](auto** p, size_t bytes) {
+    got = got && cudaMalloc((void**)p, bytes) == cudaSuccess;
+  };
+  for (int q = 0; q < 4; ++q) take(&D->kb4[q], 2 * ts * all);
+  take(&D->igA, ts * plane);
+  take(&D->igB, ts * plane);
+  take(&D->Goct, ts * 8 * g.nz * plane);
+  take(&D->Qoct, ts * 8 * plane);
+  take(&D->wrap, ts * rp_wrap_elems(D, ts));
+  take(&D->om, sizeof(double) * 3 * (D->M / 8));
+  if (got) return true;
+  cudaGetLastError();
+  auto give = [](auto** p) {
+    cudaFree(*p);
+    *p = nullptr;
+  };
+  for (int q = 0; q < 4; ++q) give(&D->kb4[q]);
+  give(&D->igA); give(&D->igB); give(&D->Goct); give(&D->Qoct); give(&D->wrap); give(&D->om);
+  return false;
+}
+
 static int dom_prepare(DomCtx* D, cudaStream_t st) {
   if (D->mode != 0) return FS_OK;
   const GridDev& g = D->g;
@@ -1575,21 +1608,13 @@ static int dom_prepare(DomCtx* D, cudaStream_t st) {
   const size_t ts = D->fp32 ? sizeof(float) : sizeof(double);
   // the register-patch kernel where path and kernel are automatic, or on request
   if ((D->sweep_kernel == 3 && want != 3) || (D->sweep_kernel == 0 && want == 0)) {
-    if (D->force_groups < 2 && octant_grouping(D) && plan_rp(D, D->force_C)) {
+    if (D->force_groups < 2 && octant_grouping(D) && plan_rp(D, D->force_C) && rp_alloc(D, ts)) {
+      const int64_t wn = rp_wrap_elems(D, ts);
       D->mode = 8;
       D->rp = 1;
       D->Mo = D->M / 8;
       int slot = 0;
       for (int o = 0; o < 8; ++o) D->down_slot[o] = D->hoz[o * D->Mo] < 0.0 ? slot++ : -1;
-      const int64_t plane = (int64_t)(g.nx + g.ny - 1) * rp_pitch(g.ny);
-      const int64_t all = (int64_t)(g.nx + g.ny + g.nz - 2) * g.nz * rp_pitch(g.ny);
-      const int64_t wn = 8ll * rp_pad((int)ts, D->Mo) * g.nz * (g.nx + g.nz - 1);
-      for (int q = 0; q < 4; ++q) cudaMalloc(&D->kb4[q], 2 * ts * all);
-      cudaMalloc(&D->igA, ts * plane);
-      cudaMalloc(&D->igB, ts * plane);
-      cudaMalloc(&D->Goct, ts * 8 * g.nz * plane);
-      cudaMalloc(&D->Qoct, ts * 8 * plane);
-      cudaMalloc(&D->wrap, ts * wn);
       cudaMemsetAsync(D->wrap, 0, ts * wn, st);
       std::vector<double> om(3 * D->Mo);
       for (int m = 0; m < D->Mo; ++m) {
@@ -1597,7 +1622,6 @@ static int dom_prepare(DomCtx* D, cudaStream_t st) {
         om[D->Mo + m] = fabs(D->hoy[m]);
         om[2 * D->Mo + m] = fabs(D->hoz[m]);
       }
-      cudaMalloc(&D->om, sizeof(double) * om.size());
       cudaMemcpyAsync(D->om, om.data(), sizeof(double) * om.size(), cudaMemcpyHostToDevice, st);
       // the height the launch constants are for; every CTA compares its levels
       cudaMemcpyAsync(&D->rp_dz0, g.dz, sizeof(double), cudaMemcpyDeviceToHost, st);

@@ -5,9 +5,11 @@
 //   x: Neumann inlet / Dirichlet p=0 outlet face; y periodic;
 //   z: Neumann wall / Dirichlet p=0 top face; non-uniform dz.
 // Row k of A carries 1/dz_k, so S = -diag(dz) A is symmetric positive
-// definite; S is stored as face conductances g (one per interior face) plus
-// a per-cell term e (Dirichlet faces and the -dz_k 1e-6 shift):
-//   (S x)_c = e_c x_c + sum_faces g_f (x_c - x_nb).
+// definite; S is face conductances g (one per interior face) plus a per-cell
+// term e (Dirichlet faces and the -dz_k 1e-6 shift):
+//   (S x)_c = e_c x_c + sum_faces g_f (x_c - x_nb),
+// stored on the coarse levels and on the finest in FP32, formed from 1/rho on the
+// finest in FP64.
 // The reference solves A p = rhs with BiCGSTAB + an FFT preconditioner
 // (projection_3d.py:756-791); here S p = -dz rhs is solved with CG
 // preconditioned by one geometric-multigrid V-cycle:
@@ -1239,7 +1241,7 @@ int proj_set_precision(void* h, int fp32) {
 // each for a few hundred cells).  The first tail level's right-hand side
 // comes from global memory and its correction goes back there.  The order of
 // operations and every per-cell expression are those of vcycle() with
-// k_mg_jacobi, k_mg_restrict_residual, k_mg_coarse_solve and k_mg_prolong, so
+// k_mg_jacobi, k_mg_restrict_residual and k_mg_coarse_solve, so
 // the correction is bit-identical.
 #define MG_TAIL_SMEM (200 * 1024)
 #define MG_TAIL_MAX 10

@@ -22,9 +22,10 @@ struct SpeciesArgs {
 };
 
 // Bound by instructions issued.  With the limiters face by face the three
-// species took 940 a warp and level in FP64: 143 us at 400 x 120 x 60, 101 as
+// species took 940 a warp and level in FP64: 143 us at 400 x 120 x 60, 108 as
 // cell differences; FP32 at 301 x 119 x 47, where every neighbour was loaded from
-// L1, 65 us and now 45.
+// L1, 65 us and now 45.  The expressions keep their order and roundings: cells sit on
+// the EDC's thresholds.
 template <typename T, int NS, bool FUSED>
 __global__ void __launch_bounds__(MR_THREADS, sizeof(T) == 8 ? 3 : 4)
     k_species(GridDev g, SpeciesArgs<T> a, int kz) {
@@ -137,7 +138,7 @@ struct DiffArgs {
 };
 
 // Bound by the loads' latency, so two planes are in flight beyond the three a
-// level reads: three FP64 fields at 400 x 120 x 60 in 43 us; 61 with the
+// level reads: three FP64 fields at 400 x 120 x 60 in 44 us; 61 with the
 // neighbours in x and y loaded when they were used.
 template <typename T, int NF>
 __global__ void __launch_bounds__(MR_THREADS, 4) k_turb_diff(GridDev g, DiffArgs<T> a, int kz) {
