@@ -46,7 +46,7 @@ METRIC = "3D solver cell-steps/s on 1 B200 (plain FP64 Tier-3 step)"
 UNIT = "cell-steps/s"
 WORKLOAD = "tier3_step_400x120x60_S8_fp64"
 # measured DRAM bytes per cell of one launch (see the traffic comment in main)
-TRAFFIC_PER_CELL = {"dom_sweep": (16.780544e6 + 4.06528e6) / 720000.0}
+TRAFFIC_PER_CELL = {"dom_sweep": (465.048576e6 + 189.39392e6) / 2880000.0}
 
 
 def _peaks():
@@ -495,9 +495,9 @@ def kernel_roofline(solver, kt, steps, form, peak, peak_src):
     tot_ms, nl = kt[dom_k]
     avg_ms = tot_ms / max(nl, 1)
     achieved = alg[dom_k] / (avg_ms * 1e-3) / 1e9
-    # DRAM bytes per launch of the dominant kernel from an ncu capture of the
-    # 100x120x60 slice of this workload (dram__bytes_read.sum + write.sum) with
-    # the default sweep (path 8), scaled by the cell count to a full launch
+    # DRAM bytes per launch of the dominant kernel from an ncu capture of this
+    # workload (dram__bytes_read.sum + write.sum) with the default sweep (path 8),
+    # scaled by the cell count
     traffic = (TRAFFIC_PER_CELL.get(dom_k)
                if form == "plain" and (dom_k != "dom_sweep" or dom_mode == 8) else None)
     if traffic is not None:
