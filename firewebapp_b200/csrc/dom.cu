@@ -393,8 +393,9 @@ struct ClArgs {
 // CL_MAX_THREADS_2 (96 registers).
 #define CL_MAX_THREADS_1 768
 #define CL_MAX_THREADS_2 640
-// bounded hand-off waits: try_wait rounds before a thread gives up
-#define CL_WAIT_LIMIT (1 << 20)
+// bounded hand-off waits: try_wait rounds before a thread gives up (4 us each,
+// about a second in all)
+#define CL_WAIT_LIMIT (1 << 18)
 // Shared memory of a CTA: the hyperplane buffers (current and previous,
 // [pencil][ordinate]), the ring of the upstream CTA's last rows
 // ([slot][pencil][ordinate]), the prefetched inputs and the per-ordinate
@@ -2029,18 +2030,32 @@ int dom_solve(void* h, const double* Ts, const double* Tg, const double* as, con
 }
 
 // End of queued source iteration q: the host loop's test on the device.
-// st: [0] done, [1] iterations run, [2] error (2 non-finite G).  A non-finite
+// st: [0] done, [1] iterations run, [2] error (2 non-finite G), [3] a wait of
+// the sweep gave up.  That ends the solve (the sweeps queued behind would wait
+// as long again), and so does a non-finite G.  A non-finite
 // G ends the solve on every iteration, the first included; the convergence
 // ratio, as the reference's (dom_3d.py:450-460), from the second.
 __global__ void k_dom_check(const unsigned long long* __restrict__ keys, double tol, int q,
                             int* st) {
   if (st[0]) return;
+  if (st[3]) { st[1] = q + 1; st[0] = 1; return; }
   double Gmax = __longlong_as_double((long long)keys[0]);
   const double dmax = __longlong_as_double((long long)keys[1]);
   if (Gmax != Gmax || dmax != dmax) { st[2] = 2; st[1] = q + 1; st[0] = 1; return; }
   if (q == 0) return;
   if (Gmax < 1e-12) Gmax = 1e-12;
   if (dmax / Gmax < tol) { st[1] = q + 1; st[0] = 1; }
+}
+
+// A sweep whose wait gave up has left values of rows that never came in what
+// the next solve starts from (the y-inflow rows, and G, whose change the first
+// iteration looks at): back to a new handle's.
+static void dom_forget(DomCtx* D, cudaStream_t st) {
+  const size_t ts = D->fp32 ? sizeof(float) : sizeof(double);
+  const int64_t N = ncells(D->g), rows = (int64_t)D->M * D->g.nz * D->g.nx;
+  cudaMemsetAsync(D->wrap, 0, ts * (D->rp ? rp_wrap_elems(D, ts) : rows), st);
+  cudaMemsetAsync(D->G, 0, sizeof(double) * N, st);
+  cudaMemsetAsync(D->Gp, 0, sizeof(double) * N, st);
 }
 
 // Path 8's source iterations without a host round trip between sweeps: the
@@ -2099,6 +2114,7 @@ static int dom_iterate_dev(DomCtx* D, const ClArgs& base, int nslots, double ref
     cudaMemcpyAsync(D->h_dstate, D->dstate, sizeof(int) * 4, cudaMemcpyDeviceToHost, st);
     if (fs_stream_wait(st) != FS_OK) return FS_ECUDA;
     if (D->h_dstate[3]) {
+      dom_forget(D, st);
       fs_set_error("DOM sweep: a bounded wait for the row hand-off between the cluster's CTAs "
                    "gave up");
       return FS_ETIMEOUT;

@@ -34,8 +34,8 @@
 // the octants are the pencil kernel's, so the results are the same bit for bit.
 //
 // Measured, a sweep of 400 x 120 x 60 with S8 (10 CTAs of 6 rows an octant):
-// FP64 907 us, FP32 641 us (pencil kernel 1810 and 1357); 97 x 41 x 23 with S4:
-// 111 us (167).  What bounds it is latency: a step takes about 3300 cycles, of
+// FP64 890 us, FP32 620 us (pencil kernel 1810 and 1357); 97 x 41 x 23 with S4:
+// 110 us (167).  What bounds it is latency: a step takes about 3300 cycles, of
 // which the busiest scheduler's FP64 pipe works 1300 and issues 1500; a warp by
 // itself needs 1700 (about four cycles an instruction), and the barrier waits
 // for the slowest of twelve.
@@ -112,7 +112,8 @@ __host__ __device__ inline RpLayout rp_layout(int tsize, int Mo, int rows, int n
   const size_t pitch = (size_t)rp_pitch(ny);
   size_t o = 0;
   L.rowb = up16((size_t)ny * Mo * tsize);
-  L.bars = o; o = up16(o + (RP_KS + 2 * RP_ZS_MAX) * sizeof(unsigned long long));
+  // (and two words: the step and the row of the ring whose wait gave up)
+  L.bars = o; o = up16(o + (RP_KS + 2 * RP_ZS_MAX + 1) * sizeof(unsigned long long));
   L.kab = o; o = up16(o + RP_KS * rows * pitch * 2 * tsize);
   L.yin = o; o = up16(o + RP_KS * (size_t)rows * rp_pad(tsize, Mo) * tsize);
   L.ig = o; o = up16(o + RP_KS * pitch * tsize);
@@ -164,9 +165,8 @@ __device__ __forceinline__ void rp_send(uint32_t p, uint32_t bar, const T (&v)[M
 // through the ring is ordered without them: the values arrive by st.async,
 // whose bytes complete the barrier phase, and a slot is released after its
 // values were used.
-__device__ __forceinline__ void rp_wait(uint32_t addr, uint32_t parity, bool& failed, int* err) {
-  if (failed) return;
-  for (int it = 0; it < CL_WAIT_LIMIT; ++it) {
+__device__ __forceinline__ bool rp_poll(uint32_t addr, uint32_t parity, int limit) {
+  for (int it = 0; it < limit; ++it) {
     uint32_t ok;
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
@@ -175,11 +175,28 @@ __device__ __forceinline__ void rp_wait(uint32_t addr, uint32_t parity, bool& fa
         : "=r"(ok)
         : "r"(addr), "r"(parity)
         : "memory");
-    if (ok) return;
+    if (ok) return true;
   }
-  failed = true;
-  if (err) atomicExch(err, 1);
+  return false;
 }
+// Bounded wait.  A thread whose wait gave up does not wait, signal or send
+// again on what it waited for: the row ring (RP_RING) or the inputs (RP_IN).
+// The two are separate, as the thread that waits for the inputs may be one that
+// sends or takes rows: with the ring given up it must go on waiting for its
+// copies, or it would announce new ones on phases that are still open.
+#define RP_RING 1u
+#define RP_IN 2u
+__device__ __forceinline__ bool rp_wait(uint32_t addr, uint32_t parity, unsigned& failed,
+                                        unsigned what, int* err) {
+  if (failed & what) return true;
+  if (rp_poll(addr, parity, CL_WAIT_LIMIT)) return true;
+  failed |= what;
+  if (err) atomicExch(err, 1);
+  return false;  // once
+}
+// try_wait rounds for copies and rows still under way when a CTA leaves, over
+// all the phases it asks about
+#define RP_DRAIN_LIMIT (1 << 16)
 __device__ __forceinline__ void rp_release(uint32_t cluster_addr) {
   asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }
@@ -251,6 +268,7 @@ __global__ void __launch_bounds__(32 * RpShape<MO>::MAXW, 1)
   unsigned long long* bars = (unsigned long long*)(shraw + L.bars);
   const uint32_t full_k = smem_u32(bars), full_z = full_k + 8u * RP_KS,
                  empty_z = full_z + 8u * RP_ZS_MAX;
+  volatile int* const gave_up = (volatile int*)(bars + RP_KS + 2 * RP_ZS_MAX);
   T* igr = (T*)(shraw + L.ig);
   T2* tz = (T2*)(shraw + L.tz);
   const int S = nx + ny - 1;
@@ -276,7 +294,9 @@ __global__ void __launch_bounds__(32 * RpShape<MO>::MAXW, 1)
   // the row handed on to this CTA; empty_z: the next CTA's first row block has
   // read what this CTA sent into its ring
   if (threadIdx.x == 0) {
-    for (int q = 0; q < RP_KS; ++q) cl_mbar_init(bars + q, ground_in ? 3u : 2u);
+    gave_up[0] = steps;
+    gave_up[1] = S;
+    for (int q = 0; q < RP_KS; ++q) cl_mbar_init(bars + q, 3u);
     for (int q = 0; q < RP_ZS_MAX; ++q) {
       cl_mbar_init(bars + RP_KS + q, 1u);
       cl_mbar_init(bars + RP_KS + RP_ZS_MAX + q, (unsigned)nwj);
@@ -293,53 +313,45 @@ __global__ void __launch_bounds__(32 * RpShape<MO>::MAXW, 1)
   const uint32_t a_xb = smem_u32(shraw + L.xb), a_spare = smem_u32(shraw + L.spare);
   const uint32_t a_zin = smem_u32(shraw + L.zin), a_yin = smem_u32(shraw + L.yin);
   const uint32_t a_kab = smem_u32(shraw + L.kab), kstep = (uint32_t)(rows * pitch) * 2 * TS;
-  // The inputs of a step into slot t % RP_KS, one array per loading warp of the
-  // middle row block: all rows of a plane are one run (k ascends in memory).
-  // src steps from plane to plane; a step past last brings nothing.
+  // The inputs of a step into slot t % RP_KS, an array each by the first lanes of
+  // a warp in the middle of the CTA: all rows of a plane are one run (k ascends
+  // in memory), planes are step bytes apart, a step past last brings nothing.
+  // Every one of these lanes waits for the inputs itself, so what it may announce
+  // next is its own knowledge; in lanes of one warp that costs a single wait (in
+  // one lane of three warps each, with a word in shared memory to tell the others
+  // of a wait that gave up: 119 us a sweep at 97 x 41 x 23, S4, against 110).
   const int P = nx + ny + nz - 2, Pw = nx + nz - 1;
-  const int role = lane == 0 ? (warp + nw - (nw / (2 * nwj)) * nwj) % nw : -1;
+  const bool loads = warp == (nw / (2 * nwj)) * nwj + (nwj > 2 ? 1 : 0) && lane < 3;
   struct Load {
     const char* src;
     int64_t step;
     uint32_t dst, size, slot;
     int last;
-  };
-  Load ld[3] = {};
-  int use = 0;  // of which arrays this thread loads
-  if (role == 0) {
+  } ld = {};
+  if (loads && lane == 0) {
     const int64_t plane = (int64_t)nz * pitch * 2 * TS;
-    use |= 1;
-    ld[0] = Load{(const char*)a.kb[rp_class(fx, fy, fz)] + (fx ? r0 : P - 1 - r0) * plane +
-                         (int64_t)(fz ? r0 : nz - r0 - nrows) * pitch * 2 * TS,
-                     fx ? plane : -plane, a_kab, (uint32_t)(nrows * pitch) * 2 * TS, kstep, steps};
-  }
-  if (role == 1 % nw) {
+    ld = Load{(const char*)a.kb[rp_class(fx, fy, fz)] + (fx ? r0 : P - 1 - r0) * plane +
+                  (int64_t)(fz ? r0 : nz - r0 - nrows) * pitch * 2 * TS,
+              fx ? plane : -plane, a_kab, (uint32_t)(nrows * pitch) * 2 * TS, kstep, steps};
+  } else if (loads && lane == 1) {
     const int64_t plane = (int64_t)nz * MOW * TS;
-    use |= 2;
-    ld[1] = Load{(const char*)a.wrap + ((int64_t)oct * Pw + r0) * plane + (int64_t)r0 * MOW * TS,
-                     plane, a_yin, (uint32_t)(nrows * MOW) * TS, (uint32_t)(rows * MOW) * TS,
-                     min(steps, Pw - r0)};
-  }
-  if (role == 2 % nw && ground_in) {
+    ld = Load{(const char*)a.wrap + ((int64_t)oct * Pw + r0) * plane + (int64_t)r0 * MOW * TS,
+              plane, a_yin, (uint32_t)(nrows * MOW) * TS, (uint32_t)(rows * MOW) * TS,
+              min(steps, Pw - r0)};
+  } else if (loads) {
     const int64_t plane = (int64_t)pitch * TS;
-    use |= 4;
-    ld[2] = Load{(const char*)(fx == fy ? a.igA : a.igB) + (fx ? 0 : S - 1) * plane,
-                     fx ? plane : -plane, smem_u32(igr), (uint32_t)plane, (uint32_t)plane,
-                     min(steps, S)};
+    ld = Load{(const char*)(fx == fy ? a.igA : a.igB) + (fx ? 0 : S - 1) * plane,
+              fx ? plane : -plane, smem_u32(igr), (uint32_t)plane, (uint32_t)plane,
+              ground_in ? min(steps, S) : 0};
   }
   auto load = [&](int t) {
     const int sl = t & (RP_KS - 1);
     const uint32_t bar = full_k + 8u * sl;
-#pragma unroll
-    for (int q = 0; q < 3; ++q) {
-      if (!(use & (1 << q))) continue;
-      const bool on = t < ld[q].last;
-      cl_arrive_expect(bar, on ? ld[q].size : 0u);
-      if (on) rp_bulk_in(ld[q].dst + (uint32_t)sl * ld[q].slot, ld[q].src, ld[q].size, bar);
-      ld[q].src += ld[q].step;
-    }
+    const bool on = t < ld.last;
+    cl_arrive_expect(bar, on ? ld.size : 0u);
+    if (on) rp_bulk_in(ld.dst + (uint32_t)sl * ld.slot, ld.src + t * ld.step, ld.size, bar);
   };
-  if (use)
+  if (loads)
     for (int t = 0; t < min(RP_KS, steps); ++t) load(t);
   // the row hand-off: the last row block's warps send, the first one's release
   const int row0 = rb * RK;
@@ -352,7 +364,7 @@ __global__ void __launch_bounds__(32 * RpShape<MO>::MAXW, 1)
   const uint32_t dn_full = sends ? cl_mapa(full_z, (unsigned)(rank + 1)) : 0u;
   const uint32_t up_empty = takes ? cl_mapa(empty_z, (unsigned)(rank - 1)) : 0u;
   const bool own = jb * 32 + lane < ny;  // a doubling lane sends nothing
-  bool failed = false;
+  unsigned failed = 0;  // RP_RING, RP_IN: this thread's wait gave up
   const T I_amb = (T)a.I_amb;
   T I[RK][MO];
 #pragma unroll
@@ -390,7 +402,6 @@ __global__ void __launch_bounds__(32 * RpShape<MO>::MAXW, 1)
   const uint32_t yoff = a_yin + (uint32_t)(min(row0, nrows - 1) * MOW) * TS;
   const int slot = a.slot[oct];
   const bool ground_row = slot >= 0 && r0 + nrows == nz && row0 + RK >= nrows && row0 < nrows;
-  const bool waits_k = role == 0;
   const bool last_col = jb == nwj - 1;
   // every level of the CTA is dz0 high: az and as are launch constants
   bool uni = true;
@@ -414,16 +425,19 @@ __global__ void __launch_bounds__(32 * RpShape<MO>::MAXW, 1)
     uint32_t zslot = 0, kslot = 0, yslot = 0;  // slot offsets of the rings
     for (int t = 0; t < steps; ++t, ++ip) {
       // the inputs of step t are there (one warp waits; the barrier passes it on)
-      if (waits_k)
-        rp_wait(full_k + 8u * (t & (RP_KS - 1)), (uint32_t)((t / RP_KS) & 1), failed, a.err);
+      if (loads && !rp_wait(full_k + 8u * (t & (RP_KS - 1)), (uint32_t)((t / RP_KS) & 1), failed,
+                            RP_IN, a.err))
+        gave_up[0] = t;
       __syncthreads();  // step t - 1 complete in this CTA
-      if (use && t > 0 && t - 1 + RP_KS < steps) load(t - 1 + RP_KS);
+      if (loads && t > 0 && t - 1 + RP_KS < steps && !(failed & RP_IN)) load(t - 1 + RP_KS);
       const int q = t - (rows - 1);  // the item that this step hands on
       if (sends && q > zm && q < S)  // its slot in the next CTA is free again
-        rp_wait(empty_z + 8u * (q & zm), (uint32_t)(((q >> zlog) - 1) & 1), failed, a.err);
+        rp_wait(empty_z + 8u * (q & zm), (uint32_t)(((q >> zlog) - 1) & 1), failed, RP_RING, a.err);
       if (takes && t < S) {
-        rp_wait(full_z + 8u * (t & zm), (uint32_t)((t >> zlog) & 1), failed, a.err);
-        if (jb == 0 && lane == 0 && !failed && t + zm + 1 < S)
+        if (!rp_wait(full_z + 8u * (t & zm), (uint32_t)((t >> zlog) & 1), failed, RP_RING, a.err) &&
+            threadIdx.x == 0)
+          gave_up[1] = t;
+        if (jb == 0 && lane == 0 && !(failed & RP_RING) && t + zm + 1 < S)
           cl_arrive_expect(full_z + 8u * (t & zm), fill_bytes);
       }
       if (t >= t_lo && t <= t_hi) {
@@ -563,7 +577,8 @@ __global__ void __launch_bounds__(32 * RpShape<MO>::MAXW, 1)
       kslot = kwrap ? 0u : kslot + kstep;
       yslot = kwrap ? 0u : yslot + (uint32_t)(rows * MOW) * TS;
       zslot = ((t + 1) & zm) == 0 ? 0u : zslot + row_bytes;
-      if (sends && q >= 0 && q < S && own && !failed && !(rank == 0 && q == a.withhold)) {
+      if (sends && q >= 0 && q < S && own && !(failed & RP_RING) &&
+          !(rank == 0 && q == a.withhold)) {
         const uint32_t dst = dn_zin + (uint32_t)(q & zm) * row_bytes;
         const uint32_t bar = dn_full + 8u * (q & zm);
 #pragma unroll
@@ -572,18 +587,31 @@ __global__ void __launch_bounds__(32 * RpShape<MO>::MAXW, 1)
       }
       if (takes && t < S) {
         __syncwarp();
-        if (lane == 0 && !failed) rp_release(up_empty + 8u * (t & zm));
+        if (lane == 0 && !(failed & RP_RING)) rp_release(up_empty + 8u * (t & zm));
       }
     }
   };
   if (uni) march(std::false_type{});
   else march(std::true_type{});
-  // after a wait that gave up, rows and inputs may still be on their way into
-  // this CTA: give them time to land (their barriers are not waited for)
-  if (__syncthreads_or(failed)) __nanosleep(200000);
   // no CTA leaves while another may still signal its barriers or write its ring
   cluster_arrive_release();
   cluster_wait_acquire();
+  // Nobody sends or loads any more.  Where a wait gave up, copies and rows that
+  // were announced may still be on their way into this CTA: they land before it
+  // leaves (those that were never sent run into the limit).
+  int rounds = RP_DRAIN_LIMIT;
+  auto drain = [&](uint32_t bar, uint32_t parity) {
+    while (rounds > 0 && !rp_poll(bar, parity, 1)) --rounds;
+  };
+  if (loads) {
+    const int t0 = gave_up[0];
+    for (int t = t0; t < min(steps, max(t0 - 1, 0) + RP_KS); ++t)
+      drain(full_k + 8u * (t & (RP_KS - 1)), (uint32_t)((t / RP_KS) & 1));
+  }
+  if (threadIdx.x == 0 && rank > 0) {
+    for (int t = gave_up[1]; t < min(S, gave_up[1] + a.zs); ++t)
+      drain(full_z + 8u * (t & zm), (uint32_t)((t >> zlog) & 1));
+  }
 }
 
 // ---- the arrays in skewed layout ------------------------------------------------

@@ -136,3 +136,64 @@ def test_dom_hand_off_wait_runs_out_with_status_4(fp32, kernel):
         assert np.all(np.isfinite(host(qs))) and np.all(np.isfinite(host(qg)))
     finally:
         lib().fs_dom_destroy(h)
+
+
+@pytest.mark.parametrize("fp32", [0, 1])
+@pytest.mark.parametrize("shape, ctas, threads", [((29, 40, 48), 0, None), ((16, 24, 48), 8, 32),
+                                                  ((6, 40, 21), 3, 64)])
+def test_dom_register_patch_wait_runs_out_and_leaves_nothing(shape, ctas, threads, fp32):
+    """The default sweep kernel's waits end the same way: with a row withheld
+    the solve returns FS_ETIMEOUT, twice in a row, and the next solve on that
+    handle is a new handle's bit for bit (nothing of the abandoned sweep is
+    left in the y-inflow rows or in G).  The second shape's CTAs are one warp
+    that loads, sends and takes rows; the third's two warps."""
+    from gpu_helpers import Grid, call, dev, host, lib, stream
+    from firewebapp_b200._lib import dbl_array, ptr
+    from firewebapp_b200.quadrature import level_symmetric
+    om, wq = level_symmetric(8)
+    nz, ny, nx = shape
+    rng = np.random.default_rng(3)
+    g = Grid(nz, ny, nx, 0.5, 0.5, np.full(nz, 0.1))
+    Ts = dev(300.0 + 900.0 * rng.random(shape) ** 4)
+    Tg = dev(300.0 + 1500.0 * rng.random(shape) ** 6)
+    a = dev(np.where(rng.random(shape) < 0.3, 0.002 * rng.random(shape), 0.0))
+    zero, rho = dev(np.zeros(shape)), dev(np.ones(shape))
+    M = dev(0.05 + 0.1 * rng.random(shape))
+    Tsoil = dev(np.full((ny, nx), 300.0))
+    out = [torch.zeros_like(Ts), torch.zeros_like(Ts), torch.zeros_like(Tsoil)]
+
+    def handle():
+        h = C.c_void_p()
+        call("fs_dom_create", g.ref, om.shape[0], dbl_array(om[:, 0]), dbl_array(om[:, 1]),
+             dbl_array(om[:, 2]), dbl_array(wq), 0.5, C.byref(h))
+        if fp32:
+            call("fs_dom_set_precision", h, 1)
+        call("fs_dom_set_sweep_mode", h, 0, ctas)
+        return h
+
+    def solve(h):
+        return lib().fs_dom_solve(h, ptr(Ts), ptr(Tg), ptr(a), ptr(zero), 5000.0, 300.0,
+                                  ptr(Tsoil), ptr(zero), ptr(rho), ptr(M), ptr(out[0]),
+                                  ptr(out[1]), ptr(out[2]), stream())
+
+    h, new = handle(), handle()
+    try:
+        assert solve(h) == 0
+        assert lib().fs_dom_sweep_kernel(h) == 3
+        s5 = (C.c_int * 5)()
+        call("fs_dom_launch_shape", h, s5)
+        assert threads in (None, s5[2]) and s5[0] > 1
+        call("fs_dom_set_wait_test", h, 5)
+        for _ in range(2):
+            assert solve(h) == 4
+            assert b"gave up" in lib().fs_last_error()
+        call("fs_dom_set_wait_test", h, -1)
+        assert solve(h) == 0
+        got = [host(q).copy() for q in out]
+        assert solve(new) == 0
+        assert lib().fs_dom_iterations(h) == lib().fs_dom_iterations(new)
+        for x, y in zip(got, out):
+            assert np.array_equal(x, host(y))
+    finally:
+        lib().fs_dom_destroy(h)
+        lib().fs_dom_destroy(new)
