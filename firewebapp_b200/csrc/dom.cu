@@ -68,10 +68,10 @@ struct DomCtx {
   int sweep_kernel;           // requested path-8 kernel: 0/1 pencil per thread, 2 lane column
   int cl_lane;                // resolved: 1 = the lane-column kernel
   // the register-patch kernel (resolved: rp = 1): skewed (kappa, kappa*B) and
-  // ground intensity, FP64 or FP32 by fp32; |ordinate components| of an octant
+  // ground intensity, FP64 or FP32 by fp32, with its partials and y-inflow rows
+  // in one allocation (rp_mem); the height that its launch constants are for
   int rp, rp_pair, rp_zs;
-  void *kb4[4], *igA, *igB;
-  double* om;
+  void *rp_mem, *kb4[4], *igA, *igB;
   double rp_dz0;
   int begun;                  // dom_begin done, dom_end due
   double pend_I_amb;          // ambient intensity of the begun solve
@@ -1288,7 +1288,11 @@ void* dom_create(const GridDev& g, int M, const double* ox, const double* oy, co
   D->sweep_kernel = 0; D->cl_lane = 0;
   D->rp = 0; D->rp_pair = 0;
   for (int q = 0; q < 4; ++q) D->kb4[q] = nullptr;
-  D->igA = nullptr; D->igB = nullptr; D->om = nullptr;
+  D->igA = nullptr; D->igB = nullptr; D->rp_mem = nullptr;
+  // (a height that has changed when a sweep runs only costs that sweep the
+  // constants: every CTA compares its levels)
+  D->rp_dz0 = 0.0;
+  cudaMemcpyAsync(&D->rp_dz0, g.dz, sizeof(double), cudaMemcpyDeviceToHost, ss.s);
   cudaMalloc(&D->G, sizeof(double) * N); cudaMalloc(&D->Gp, sizeof(double) * N);
   cudaMemsetAsync(D->G, 0, sizeof(double) * N, ss.s);
   cudaMemsetAsync(D->Gp, 0, sizeof(double) * N, ss.s);
@@ -1319,9 +1323,11 @@ void dom_destroy(void* h) {
   DomCtx* D = (DomCtx*)h;
   if (!D) return;
   cudaFree(D->ox); cudaFree(D->oy); cudaFree(D->oz); cudaFree(D->w); cudaFree(D->I);
-  cudaFree(D->kb); cudaFree(D->Goct); cudaFree(D->Qoct); cudaFree(D->wrap);
-  for (int q = 0; q < 4; ++q) cudaFree(D->kb4[q]);
-  cudaFree(D->igA); cudaFree(D->igB); cudaFree(D->om);
+  if (D->rp_mem) {
+    cudaFree(D->rp_mem);
+  } else {
+    cudaFree(D->kb); cudaFree(D->Goct); cudaFree(D->Qoct); cudaFree(D->wrap);
+  }
   cudaFree(D->G); cudaFree(D->Gp); cudaFree(D->ks); cudaFree(D->kg); cudaFree(D->ksafe);
   cudaFree(D->B); cudaFree(D->Ig_out); cudaFree(D->Isoil); cudaFree(D->qin); cudaFree(D->keys);
   cudaFreeHost(D->h_keys);
@@ -1574,31 +1580,30 @@ static int64_t rp_wrap_elems(const DomCtx* D, size_t ts) {
 
 // The register-patch kernel's layouts.  They take more memory than the pencil
 // kernel's (some 500 MB against 300 at 400 x 120 x 60): where they do not fit, that
-// one runs.
+// one runs.  One allocation, cut up: a new handle's first solve pays for it, and
+// eleven took 2.0 ms (97 x 41 x 23, S4: the first solve 2.8 ms, 1.1 with one, 1.7
+// with the pencil kernel; 400 x 120 x 60, S8: 7.9, 5.5 and 11.1).
 static bool rp_alloc(DomCtx* D, size_t ts) {
   const GridDev& g = D->g;
-  const int64_t plane = (int64_t)(g.nx + g.ny - 1) * rp_pitch(g.ny);
-  const int64_t all = (int64_t)(g.nx + g.ny + g.nz - 2) * g.nz * rp_pitch(g.ny);
-  bool got = true;
-  auto take = [&](auto** p, size_t bytes) {
-    got = got && cudaMalloc((void**)p, bytes) == cudaSuccess;
-  };
-  for (int q = 0; q < 4; ++q) take(&D->kb4[q], 2 * ts * all);
-  take(&D->igA, ts * plane);
-  take(&D->igB, ts * plane);
-  take(&D->Goct, ts * 8 * g.nz * plane);
-  take(&D->Qoct, ts * 8 * plane);
-  take(&D->wrap, ts * rp_wrap_elems(D, ts));
-  take(&D->om, sizeof(double) * 3 * (D->M / 8));
-  if (got) return true;
-  cudaGetLastError();
-  auto give = [](auto** p) {
-    cudaFree(*p);
-    *p = nullptr;
-  };
-  for (int q = 0; q < 4; ++q) give(&D->kb4[q]);
-  give(&D->igA); give(&D->igB); give(&D->Goct); give(&D->Qoct); give(&D->wrap); give(&D->om);
-  return false;
+  const size_t plane = ts * (size_t)(g.nx + g.ny - 1) * rp_pitch(g.ny);
+  const size_t all = 2 * ts * (size_t)(g.nx + g.ny + g.nz - 2) * g.nz * rp_pitch(g.ny);
+  const size_t bytes[9] = {all, all, all, all, plane, plane, 8 * g.nz * plane, 8 * plane,
+                           ts * (size_t)rp_wrap_elems(D, ts)};
+  void** const to[9] = {&D->kb4[0], &D->kb4[1], &D->kb4[2], &D->kb4[3], &D->igA,
+                        &D->igB,    &D->Goct,   &D->Qoct,   &D->wrap};
+  size_t total = 0;
+  for (size_t q : bytes) total += (q + 255) / 256 * 256;
+  if (cudaMalloc(&D->rp_mem, total) != cudaSuccess) {
+    cudaGetLastError();
+    D->rp_mem = nullptr;
+    return false;
+  }
+  char* p = (char*)D->rp_mem;
+  for (int q = 0; q < 9; ++q) {
+    *to[q] = p;
+    p += (bytes[q] + 255) / 256 * 256;
+  }
+  return true;
 }
 
 static int dom_prepare(DomCtx* D, cudaStream_t st) {
@@ -1610,23 +1615,12 @@ static int dom_prepare(DomCtx* D, cudaStream_t st) {
   // the register-patch kernel where path and kernel are automatic, or on request
   if ((D->sweep_kernel == 3 && want != 3) || (D->sweep_kernel == 0 && want == 0)) {
     if (D->force_groups < 2 && octant_grouping(D) && plan_rp(D, D->force_C) && rp_alloc(D, ts)) {
-      const int64_t wn = rp_wrap_elems(D, ts);
       D->mode = 8;
       D->rp = 1;
       D->Mo = D->M / 8;
       int slot = 0;
       for (int o = 0; o < 8; ++o) D->down_slot[o] = D->hoz[o * D->Mo] < 0.0 ? slot++ : -1;
-      cudaMemsetAsync(D->wrap, 0, ts * wn, st);
-      std::vector<double> om(3 * D->Mo);
-      for (int m = 0; m < D->Mo; ++m) {
-        om[m] = fabs(D->hox[m]);
-        om[D->Mo + m] = fabs(D->hoy[m]);
-        om[2 * D->Mo + m] = fabs(D->hoz[m]);
-      }
-      cudaMemcpyAsync(D->om, om.data(), sizeof(double) * om.size(), cudaMemcpyHostToDevice, st);
-      // the height the launch constants are for; every CTA compares its levels
-      cudaMemcpyAsync(&D->rp_dz0, g.dz, sizeof(double), cudaMemcpyDeviceToHost, st);
-      if (fs_stream_wait(st) != FS_OK) return FS_ECUDA;
+      cudaMemsetAsync(D->wrap, 0, ts * rp_wrap_elems(D, ts), st);
       return cuda_status();
     }
     if (D->sweep_kernel == 3) {
@@ -1924,7 +1918,7 @@ static int launch_rp(DomCtx* D, const ClArgs& c, cudaStream_t st) {
   for (int q = 0; q < 4; ++q) a.kb[q] = (const T2*)D->kb4[q];
   a.igA = (const T*)D->igA; a.igB = (const T*)D->igB;
   a.Goct = (T*)D->Goct; a.Qoct = (T*)D->Qoct; a.wrap = (T*)D->wrap;
-  a.om = D->om;
+  a.ox = D->ox; a.oy = D->oy; a.oz = D->oz;
   a.dz0 = D->rp_dz0; a.zs = D->rp_zs;
   a.I_amb = c.I_amb;
   for (int m = 0; m < MO; ++m) {

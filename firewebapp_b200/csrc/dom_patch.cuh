@@ -79,7 +79,7 @@ struct RpArgs {
   const typename Vec2Of<T>::type* kb[4];
   const T *igA, *igB;  // ground intensity, [i + j][j] and [i - j + ny - 1][j]
   T *Goct, *Qoct, *wrap;
-  const double* om;  // |x|, |y|, |z| components, MO each
+  const double *ox, *oy, *oz;  // ordinate components (the first MO: the first octant's)
   double I_amb, dz0;
   // |component| / spacing by level, the denominators' constant part by ordinate,
   // the weights by class; az and as hold for levels of height dz0 (other
@@ -283,8 +283,8 @@ __global__ void __launch_bounds__(32 * RpShape<MO>::MAXW, 1)
   for (int q = threadIdx.x; q < nrows * MO; q += blockDim.x) {
     const int r = q / MO, m = q - r * MO;
     const int kp = r0 + r, k = fz ? kp : nz - 1 - kp;
-    const double axd = a.om[m] / g.dx, ayd = a.om[MO + m] / g.dy;
-    const double azd = a.om[2 * MO + m] / g.dz[k];
+    const double axd = fabs(a.ox[m]) / g.dx, ayd = fabs(a.oy[m]) / g.dy;
+    const double azd = fabs(a.oz[m]) / g.dz[k];
     T2 v;
     v.x = (T)azd;
     v.y = (T)(axd + ayd + azd);

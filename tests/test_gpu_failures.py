@@ -197,3 +197,53 @@ def test_dom_register_patch_wait_runs_out_and_leaves_nothing(shape, ctas, thread
     finally:
         lib().fs_dom_destroy(h)
         lib().fs_dom_destroy(new)
+
+
+def test_dom_begin_of_a_new_handle_does_not_wait_for_its_stream():
+    """fs_dom_begin queues its work and returns, on a handle's first solve too:
+    behind 0.3 s or more of other work on the stream it comes back while that
+    is still running, and the solve's results are a second handle's."""
+    from gpu_helpers import Grid, call, dev, host, lib
+    from firewebapp_b200._lib import dbl_array, ptr
+    from firewebapp_b200.quadrature import level_symmetric
+    om, wq = level_symmetric(4)
+    shape = nz, ny, nx = 20, 24, 64
+    rng = np.random.default_rng(5)
+    g = Grid(nz, ny, nx, 0.5, 0.5, np.full(nz, 0.1))
+    Ts = dev(300.0 + 900.0 * rng.random(shape) ** 4)
+    Tg = dev(300.0 + 1500.0 * rng.random(shape) ** 6)
+    a = dev(np.where(rng.random(shape) < 0.3, 0.002 * rng.random(shape), 0.0))
+    zero, rho, M = dev(np.zeros(shape)), dev(np.ones(shape)), dev(np.full(shape, 0.1))
+    Tsoil = dev(np.full((ny, nx), 300.0))
+    st = torch.cuda.Stream()
+
+    def handle():
+        h = C.c_void_p()
+        call("fs_dom_create", g.ref, om.shape[0], dbl_array(om[:, 0]), dbl_array(om[:, 1]),
+             dbl_array(om[:, 2]), dbl_array(wq), 0.5, C.byref(h))
+        return h
+
+    def solve(h, busy):
+        out = [torch.zeros_like(Ts), torch.zeros_like(Ts), torch.zeros_like(Tsoil)]
+        torch.cuda.synchronize()
+        e = torch.cuda.Event()
+        with torch.cuda.stream(st):
+            if busy:
+                torch.cuda._sleep(600_000_000)  # cycles of at most 1.965 GHz
+            e.record()
+        call("fs_dom_begin", h, ptr(Ts), ptr(Tg), ptr(a), ptr(zero), 5000.0, 300.0, ptr(Tsoil),
+             ptr(zero), ptr(rho), ptr(M), st.cuda_stream)
+        running = not e.query()
+        call("fs_dom_end", h, ptr(out[0]), ptr(out[1]), ptr(out[2]), st.cuda_stream)
+        return [host(q) for q in out], running
+
+    hs = [handle(), handle()]
+    try:
+        want, _ = solve(hs[0], False)
+        got, running = solve(hs[1], True)
+        assert running
+        for x, y in zip(got, want):
+            assert np.array_equal(x, y)
+    finally:
+        for h in hs:
+            lib().fs_dom_destroy(h)
