@@ -1594,9 +1594,8 @@ static bool rp_alloc(DomCtx* D, size_t ts) {
   size_t total = 0;
   for (size_t q : bytes) total += (q + 255) / 256 * 256;
   if (cudaMalloc(&D->rp_mem, total) != cudaSuccess) {
-    cudaGetLastError();
     D->rp_mem = nullptr;
-    return false;
+    return false;  // (with the error, which the caller reports or takes back)
   }
   char* p = (char*)D->rp_mem;
   for (int q = 0; q < 9; ++q) {
@@ -1614,7 +1613,8 @@ static int dom_prepare(DomCtx* D, cudaStream_t st) {
   const size_t ts = D->fp32 ? sizeof(float) : sizeof(double);
   // the register-patch kernel where path and kernel are automatic, or on request
   if ((D->sweep_kernel == 3 && want != 3) || (D->sweep_kernel == 0 && want == 0)) {
-    if (D->force_groups < 2 && octant_grouping(D) && plan_rp(D, D->force_C) && rp_alloc(D, ts)) {
+    const bool fits = D->force_groups < 2 && octant_grouping(D) && plan_rp(D, D->force_C);
+    if (fits && rp_alloc(D, ts)) {
       D->mode = 8;
       D->rp = 1;
       D->Mo = D->M / 8;
@@ -1623,6 +1623,8 @@ static int dom_prepare(DomCtx* D, cudaStream_t st) {
       cudaMemsetAsync(D->wrap, 0, ts * rp_wrap_elems(D, ts), st);
       return cuda_status();
     }
+    if (D->sweep_kernel == 3 && fits) return FS_ECUDA;  // out of memory
+    cudaGetLastError();
     if (D->sweep_kernel == 3) {
       fs_set_error("the register-patch sweep kernel is not built for this shape (3, 6 or 10 "
                    "ordinates per octant, the same in every octant; rows that fit a CTA)");

@@ -247,3 +247,82 @@ def test_dom_begin_of_a_new_handle_does_not_wait_for_its_stream():
     finally:
         for h in hs:
             lib().fs_dom_destroy(h)
+
+
+class _Dom:
+    """A DOM handle on random fields of a 140 x 120 x 60 grid, S8: 48 MB of its
+    own, 275 MB more for the register-patch kernel's first solve and 87 for the
+    pencil kernel's."""
+
+    def __init__(self, kernel=0, shape=(60, 120, 140)):
+        from gpu_helpers import Grid, call, dev
+        from firewebapp_b200._lib import dbl_array
+        from firewebapp_b200.quadrature import level_symmetric
+        om, wq = level_symmetric(8)
+        rng = np.random.default_rng(8)
+        nz, ny, nx = shape
+        self.g = Grid(nz, ny, nx, 0.5, 0.5, np.full(nz, 0.1))
+        self.Ts = dev(300.0 + 900.0 * rng.random(shape) ** 4)
+        self.Tg = dev(300.0 + 1500.0 * rng.random(shape) ** 6)
+        self.a = dev(np.where(rng.random(shape) < 0.3, 0.002 * rng.random(shape), 0.0))
+        self.zero, self.rho = dev(np.zeros(shape)), dev(np.ones(shape))
+        self.Tsoil = dev(np.full((ny, nx), 300.0))
+        self.out = [torch.zeros_like(q) for q in (self.Ts, self.Ts, self.Tsoil)]
+        self.h = C.c_void_p()
+        call("fs_dom_create", self.g.ref, om.shape[0], dbl_array(om[:, 0]), dbl_array(om[:, 1]),
+             dbl_array(om[:, 2]), dbl_array(wq), 0.5, C.byref(self.h))
+        if kernel in (1, 2):
+            call("fs_dom_set_sweep_mode", self.h, 8, 0)
+        call("fs_dom_set_sweep_kernel", self.h, kernel)
+
+    def solve(self):
+        from gpu_helpers import lib, stream
+        from firewebapp_b200._lib import ptr
+        return lib().fs_dom_solve(self.h, ptr(self.Ts), ptr(self.Tg), ptr(self.a), ptr(self.zero),
+                                  5000.0, 300.0, ptr(self.Tsoil), ptr(self.zero), ptr(self.rho),
+                                  ptr(self.zero), *(ptr(q) for q in self.out), stream())
+
+    def close(self):
+        from gpu_helpers import lib
+        lib().fs_dom_destroy(self.h)
+
+
+def _leave_free(mb):
+    """Tensors that hold all of the GPU's memory but some mb MB (untouched)."""
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    held, piece = [], 1 << 36
+    while True:
+        take = min(torch.cuda.mem_get_info()[0] - (mb << 20), piece)
+        if take < (4 << 20):
+            return held
+        try:
+            held.append(torch.empty(take >> 21 << 21, dtype=torch.uint8, device="cuda"))
+        except torch.cuda.OutOfMemoryError:
+            piece = take // 2
+
+
+def test_dom_kernel_3_without_its_memory_says_so():
+    """The register-patch kernel asked for by number where its layouts cannot be
+    had: status 5 and a message about the memory (the shape is one it is built
+    for); left automatic, the pencil kernel runs, with its results."""
+    from gpu_helpers import host, lib
+    small = [_Dom(k, (6, 5, 9)) for k in (1, 3)]
+    assert [q.solve() for q in small] == [0, 0]  # both kernels' code is loaded
+    asked, auto, pencil = _Dom(3), _Dom(0), _Dom(1)
+    held = _leave_free(200)
+    try:
+        assert asked.solve() == 5
+        assert b"out of memory" in lib().fs_last_error()
+        assert auto.solve() == 0
+        assert lib().fs_dom_sweep_kernel(auto.h) == 1
+        held.clear()
+        torch.cuda.empty_cache()
+        assert asked.solve() == 0 and pencil.solve() == 0
+        assert lib().fs_dom_sweep_kernel(asked.h) == 3
+        for x, y, z in zip(auto.out, pencil.out, asked.out):
+            assert np.array_equal(host(x), host(y)) and np.array_equal(host(x), host(z))
+    finally:
+        held.clear()
+        for q in small + [asked, auto, pencil]:
+            q.close()
