@@ -1637,15 +1637,24 @@ static int dom_prepare(DomCtx* D, cudaStream_t st) {
                  "cluster, 4 to 8 k' rows per CTA, ny <= %d)", 32 * LC_MAX_WARPS);
     return FS_EARG;
   }
+  // (without all of its buffers a path is not resolved: the next call tries again)
   if (oct) {
+    const size_t bytes[4] = {2 * ts * N, ts * 8 * D->groups * N, ts * 8 * D->groups * n2,
+                             ts * D->M * g.nz * g.nx};
+    void** const to[4] = {&D->kb, &D->Goct, &D->Qoct, &D->wrap};
+    bool got = true;
+    for (int q = 0; q < 4; ++q) got = got && cudaMalloc(to[q], bytes[q]) == cudaSuccess;
+    if (!got) {
+      for (void** p : to) {
+        cudaFree(*p);
+        *p = nullptr;
+      }
+      return FS_ECUDA;
+    }
     D->mode = 8;
     D->Mo = D->M / 8;
     int slot = 0;
     for (int o = 0; o < 8; ++o) D->down_slot[o] = D->hoz[o * D->Mo] < 0.0 ? slot++ : -1;
-    cudaMalloc(&D->kb, 2 * ts * N);
-    cudaMalloc(&D->Goct, ts * 8 * D->groups * N);
-    cudaMalloc(&D->Qoct, ts * 8 * D->groups * n2);
-    cudaMalloc(&D->wrap, ts * D->M * g.nz * g.nx);
     cudaMemsetAsync(D->wrap, 0, ts * D->M * g.nz * g.nx, st);
     return cuda_status();
   }
@@ -1658,8 +1667,11 @@ static int dom_prepare(DomCtx* D, cudaStream_t st) {
     fs_set_error("octant-cluster sweep not possible for this grid or quadrature");
     return FS_EARG;
   }
+  if (cudaMalloc(&D->I, sizeof(double) * N * D->M) != cudaSuccess) {
+    D->I = nullptr;
+    return FS_ECUDA;
+  }
   D->mode = 3;
-  cudaMalloc(&D->I, sizeof(double) * N * D->M);
   cudaMemsetAsync(D->I, 0, sizeof(double) * N * D->M, st);
   return cuda_status();
 }

@@ -326,3 +326,28 @@ def test_dom_kernel_3_without_its_memory_says_so():
         held.clear()
         for q in small + [asked, auto, pencil]:
             q.close()
+
+
+@pytest.mark.parametrize("mode", [0, 8, 3])
+def test_dom_first_solve_without_memory_can_be_repeated(mode):
+    """No path's buffers can be had: status 5 each time the solve is tried, the
+    handle unresolved, and a solve like a new handle's once there is memory."""
+    from gpu_helpers import call, host, lib
+    q, new = _Dom(), _Dom()
+    for d in (q, new):
+        call("fs_dom_set_sweep_mode", d.h, mode, 0)
+    held = _leave_free(48)
+    try:
+        for _ in range(2):
+            assert q.solve() == 5
+            assert b"out of memory" in lib().fs_last_error()
+            assert lib().fs_dom_sweep_mode(q.h) == 0
+        held.clear()
+        torch.cuda.empty_cache()
+        assert q.solve() == 0 and new.solve() == 0
+        for x, y in zip(q.out, new.out):
+            assert np.array_equal(host(x), host(y))
+    finally:
+        held.clear()
+        q.close()
+        new.close()
