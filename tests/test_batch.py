@@ -91,3 +91,37 @@ def test_tuned_sweep_shapes_agree():
         for k in ("T_g", "q_rad", "u", "T_s"):
             d = np.linalg.norm(st[k] - a[k]) / np.linalg.norm(a[k])
             assert d <= 1e-12, (key, k, d)
+
+
+@pytest.mark.parametrize("fits", [True, False])
+def test_autotune_times_the_default_sweep_kernel(tmp_path, monkeypatch, fits):
+    """The automatic shape is timed with the register-patch kernel, which the
+    automatic choice takes where it fits, and is returned as the automatic
+    choice (valid for any grid); where that kernel does not fit, with the pencil
+    kernel.  A choice cached by a build without that kernel is not used."""
+    import json
+    import firewebapp_b200.autotune as A
+    import firewebapp_b200.batch as B
+    from firewebapp_b200._lib import FireStepError
+    from firewebapp_b200.cases import batch_cases
+    from firewebapp_b200.grid import build_setup
+    path = tmp_path / "tune.json"
+    monkeypatch.setenv("FIREWEBAPP_B200_TUNE_CACHE", str(path))
+    monkeypatch.setattr(A.torch.cuda, "get_device_name", lambda d=None: "fake")
+    cases = batch_cases(2, seed0=0)
+    shapes = sorted({tuple(build_setup(c).grid.shape) for c in cases})
+    old = "fake|plain|conc2|" + ";".join("x".join(map(str, s)) for s in shapes)
+    path.write_text(json.dumps({old: {"key": old, "solver_kw": {"dom_sweep": 8}, "trials": []}}))
+
+    def fake(cases, steps, warmup=3, form="plain", device="cuda", solver_kw=None):
+        kw = (solver_kw["dom_sweep"], solver_kw["dom_cluster_ctas"], solver_kw.get("dom_kernel", 0))
+        if kw == (8, 0, 3) and not fits:
+            raise FireStepError(1, "not built for this shape")
+        return {"value": {(8, 0, 3): 3e8, (8, 0, 0): 1.2e8, (8, 6, 0): 1e8, (8, 15, 0): 1e8}[kw],
+                "wall_s": 1.0}
+
+    monkeypatch.setattr(B, "time_concurrent", fake)
+    out = A.tune_batch(cases, concurrency=2)
+    assert not out["cached"]
+    assert out["solver_kw"] == {"dom_sweep": 0, "dom_cluster_ctas": 0}
+    assert [t["value"] for t in out["trials"]] == [3e8 if fits else 1.2e8, 1e8, 1e8]
