@@ -142,15 +142,16 @@ struct EdcArgs {
   // reciprocals of the constant divisors (1/s_stoich, 1/dt); the divisions
   // by them, by rho and by tau* are multiplications
   double inv_s, inv_dt;
-  int extinction, nsub;
+  int extinction, nsub, idle_ok;
 };
 
 // A cell without fuel or O2 has no reaction in any substep: the rate is 0 and
 // its mass fractions keep their values, whatever k and epsilon are, as long as
-// 0 / (rho cp) is a zero.
+// 0 / (rho cp) is a zero and the substep's length, the heat of combustion and the
+// stoichiometry are finite (idle_ok: else 0 times them is NaN, in every cell).
 __device__ __forceinline__ bool edc_idle(const EdcArgs& a, double Yf, double YO2, double YH, double rho) {
   const double cp = (1.0 - YH) * a.cp_g + YH * 2000.0;
-  return (Yf <= 1e-9 || YO2 <= 1e-9) && fabs(rho) > 1e-300 && (cp > 0.0 || cp < 0.0);
+  return a.idle_ok && (Yf <= 1e-9 || YO2 <= 1e-9) && fabs(rho) > 1e-300 && (cp > 0.0 || cp < 0.0);
 }
 // what the update does to such a cell: the relaxation and the bounds
 __device__ __forceinline__ void edc_idle_cell(const EdcArgs& a, bool flag, double& Yf, double& YO2,
@@ -344,6 +345,7 @@ int launch_edc(int64_t n, const double* rho, double* Tg, double* Yf, double* YO,
   a.nsub = n_substeps > 1 ? n_substeps : 1;
   a.relax = 1.0 - exp(-(dt / (double)a.nsub) / 0.5);
   a.extinction = extinction;
+  a.idle_ok = isfinite(dt) && isfinite(a.HoC_eff) && isfinite(s_stoich);
   following(k_edc_main, (unsigned)nb, EDC_TPB, 0, st)(n, a); fs_count_launch();
   return cuda_status();
 }

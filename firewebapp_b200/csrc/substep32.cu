@@ -123,15 +123,16 @@ struct Edc32Args {
   float* omega;
   const signed char* carry;
   float cp_g, dt, s_stoich, HoC_eff, relax, inv_s, inv_dt;
-  int extinction, nsub;
+  int extinction, nsub, idle_ok;
 };
 
 // A cell without fuel or O2 has no reaction in any substep: the rate is 0 and
 // its mass fractions keep their values, whatever k and epsilon are, as long as
-// 0 / (rho cp) is a zero.
+// 0 / (rho cp) is a zero and the substep's length, the heat of combustion and the
+// stoichiometry are finite (idle_ok: else 0 times them is NaN, in every cell).
 __device__ __forceinline__ bool edc_idle32(const Edc32Args& a, float Yf, float YO2, float YH, float rho) {
   const float cp = (1.0f - YH) * a.cp_g + YH * 2000.0f;
-  return (Yf <= 1e-9f || YO2 <= 1e-9f) && fabsf(rho) > 1e-37f && (cp > 0.0f || cp < 0.0f);
+  return a.idle_ok && (Yf <= 1e-9f || YO2 <= 1e-9f) && fabsf(rho) > 1e-37f && (cp > 0.0f || cp < 0.0f);
 }
 // what the update does to such a cell: the relaxation and the bounds
 __device__ __forceinline__ void edc_idle_cell32(const Edc32Args& a, bool flag, float& Yf, float& YO2,
@@ -310,6 +311,7 @@ int launch_edc32(int64_t n, const float* rho, float* Tg, float* Yf, float* YO, c
   a.nsub = n_substeps > 1 ? n_substeps : 1;
   a.relax = (float)(1.0 - exp(-(dt / (double)a.nsub) / 0.5));
   a.extinction = extinction;
+  a.idle_ok = isfinite(a.dt) && isfinite(a.HoC_eff) && isfinite(a.s_stoich);
   following(k_edc_main32, (unsigned)nb, EDC_TPB, 0, st)(n, a);
   fs_count_launch();
   return cuda_status();

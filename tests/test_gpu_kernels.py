@@ -338,6 +338,36 @@ def test_edc_unaligned_arrays_and_ragged_tail(f32):
     assert not np.array_equal(aligned[0], ins["Tg"].astype(dt_np))
 
 
+@pytest.mark.parametrize("name, value", [("dt", np.nan), ("dt", np.inf), ("hoc_J", np.inf),
+                                         ("s_stoich", np.inf), ("s_stoich", np.nan)])
+def test_edc_non_finite_parameter_reaches_every_cell(name, value):
+    """A step length, heat of combustion or stoichiometry that is not finite makes
+    the same outputs NaN as in the oracle's arithmetic, in the cells without fuel
+    or oxygen too (0 times it), in either precision."""
+    from oracle import kernels as K
+    rng = np.random.default_rng(23)
+    n = 3000
+    ins = [rng.uniform(0.3, 1.2, n), rng.uniform(300.0, 1800.0, n),
+           np.where(rng.random(n) < 0.1, rng.uniform(0.01, 0.2, n), 0.0),
+           np.where(rng.random(n) < 0.9, rng.uniform(0.01, 0.2, n), 0.0),
+           rng.uniform(1e-3, 1.0, n), rng.uniform(1e-3, 1.0, n), rng.uniform(0.0, 0.1, n)]
+    par = dict(dt=2e-3, s_stoich=1.3, hoc_J=17e6)
+    par[name] = value
+    with np.errstate(all="ignore"):
+        want = K.edc(*ins, 0.34, 1100.0, par["dt"], 1, par["s_stoich"], par["hoc_J"], 0)
+    idle = (ins[2] <= 1e-9) | (ins[3] <= 1e-9)
+    assert any(np.isnan(w[idle]).all() for w in want)
+    for fn, dtype in (("fs_edc", torch.float64), ("fs_edc_f32", torch.float32)):
+        rho, Tg, Yf, YO, k, e, YH = (dev(q, dtype) for q in ins)
+        om = torch.zeros_like(Tg)
+        scratch = torch.zeros(int(getattr(lib(), fn + "_scratch_bytes")(n)) + 16,
+                              dtype=torch.uint8, device="cuda")
+        call(fn, n, ptr(rho), ptr(Tg), ptr(Yf), ptr(YO), ptr(k), ptr(e), ptr(YH), ptr(om), 0.34,
+             1100.0, par["dt"], 1, par["s_stoich"], par["hoc_J"], 0, ptr(scratch), stream())
+        for got, w in zip((Tg, Yf, YO, om), want):
+            assert np.array_equal(np.isnan(host(got))[idle], np.isnan(w)[idle]), fn
+
+
 def test_edc_flag_leak_crosses_blocks():
     """Cells without fuel inherit the quench flag of the previous reacting cell
     in flat order, across thread-block boundaries (edc.py:223)."""
