@@ -157,7 +157,9 @@ __global__ void __launch_bounds__(MR_THREADS, 4) k_turb_diff(GridDev g, DiffArgs
   R.init(ring, g);
   for (int q = 0; q < 3; ++q) R.load(g, f, k0 - 1 + q, q);
   copy_commit();
-  R.load(g, f, k0 + 2, 3);
+  // (only if a level reads it: a chunk of one level would leave with the copy
+  // still under way)
+  if (k0 + 2 <= k1) R.load(g, f, k0 + 2, 3);
   copy_commit();
   march_spacings(g, k0, k1, rks);
   const int i = blockIdx.x * MR_TX + threadIdx.x, j = blockIdx.y * MR_TY + threadIdx.y;

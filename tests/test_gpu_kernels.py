@@ -413,6 +413,35 @@ def test_turbulent_diffusion(vectors):
         assert rel_l2(host(f), c["field_out"]) <= TIGHT, name
 
 
+@pytest.mark.parametrize("f32, nf", [(False, 1), (False, 2), (False, 3), (False, 4), (True, 1),
+                                     (True, 3)])
+@pytest.mark.parametrize("shape", [(12, 9, 33), (23, 41, 97), (3, 1, 5), (3, 8, 33)])
+def test_turbulent_diffusion_chunks_of_one_level(shape, f32, nf):
+    """One sub-iteration against the oracle on levels of unequal height, on grids
+    whose blocks march a single level (12 x 9 x 33 and smaller) or whose last
+    chunk has one (23 levels in twos).  Some 20 operations a cell, each within
+    half a unit of terms no larger than 10 times the result: sqrt(20) x 10 x
+    2^-24 = 3e-6 in FP32, and 2^-29 of that in FP64 (asked for: 1e-5, 1e-13)."""
+    from oracle import kernels as K
+    rng = np.random.default_rng(sum(shape) + nf)
+    nz, ny, nx = shape
+    dz = 0.05 + 0.1 * rng.random(nz)
+    mid = 0.5 * (dz[:-1] + dz[1:])
+    da, db = np.append(mid, 0.5 * dz[-1]), np.append(0.5 * dz[0], mid)
+    g = Grid(nz, ny, nx, 0.1, 0.12, dz, da, db)
+    F = [rng.random(shape) for _ in range(nf)]
+    nu, sc = 1e-3 * rng.random(shape), 0.7
+    dt = 0.1 * 0.05 ** 2 * sc / 1e-3
+    dtype = torch.float32 if f32 else torch.float64
+    ins, dnu = [dev(q, dtype) for q in F], dev(nu, dtype)
+    outs = [torch.empty_like(ins[0]) for _ in F]
+    call("fs_turb_diffusion_substep" + ("_f32" if f32 else ""), g.ref, nf, ptr_array(ins),
+         ptr_array(outs), ptr(dnu), sc, dt, 0, None, None, stream())
+    for q, o in zip(F, outs):
+        want = K.turb_diffusion(q, nu, sc, dt, 0.1, 0.12, dz, da, db)
+        assert rel_l2(host(o).astype(np.float64), want) <= (1e-5 if f32 else 1e-13)
+
+
 def test_k_epsilon(vectors):
     for name in vectors.cases("kepsilon"):
         c = vectors.case("kepsilon", name)
