@@ -57,8 +57,13 @@ int launch_species_step(const GridDev& g, const double* const* Y, double* const*
   return launch_species_march<double, 3, true>(g, a, st);
 }
 
-// the stencils wait on their own copies only: nothing to expire
-int stencil_status(int) { return cudaPeekAtLastError() == cudaSuccess ? 0 : -1; }
+// The stencils wait on their own copies only: nothing to expire.  What callers
+// have of it is what a blocking copy from the legacy stream gave: that stream's
+// work has run, or an error of it is reported (one that an earlier call of the
+// thread left is not).
+int stencil_status(int) {
+  return cudaStreamSynchronize(cudaStreamLegacy) == cudaSuccess ? 0 : -1;
+}
 void set_tma(int) {}
 
 // ---------------------------------------------------------------------------

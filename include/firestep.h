@@ -209,9 +209,10 @@ int fs_ignition_pulse(const FsGrid* g, double* q_rad, int k, int i0, int i1, dou
 
 /* Kept for programs that call them.  The stencil kernels stage their planes by
  * asynchronous copies whose completion the copying threads wait for, so no wait
- * of theirs can expire: fs_stencil_status returns 0, or -1 where the thread's
- * last CUDA call failed.  fs_set_tma chose between two forms of the fused
- * species step that gave the same results; there is one form now. */
+ * of theirs can expire: fs_stencil_status waits for the legacy default stream and
+ * returns 0, or -1 on a CUDA error of its work.  fs_set_tma chose between two
+ * forms of the fused species step that gave the same results; there is one form
+ * now. */
 int fs_stencil_status(int clear);
 int fs_set_tma(int on);
 

@@ -351,3 +351,16 @@ def test_dom_first_solve_without_memory_can_be_repeated(mode):
         held.clear()
         q.close()
         new.close()
+
+
+def test_stencil_status_is_synchronous():
+    """fs_stencil_status, kept for programs that check a step with it, returns
+    after the work of the default stream has run."""
+    from gpu_helpers import lib
+    torch.cuda.synchronize()
+    e = torch.cuda.Event()
+    torch.cuda._sleep(200_000_000)
+    e.record()
+    assert not e.query()
+    assert lib().fs_stencil_status(1) == 0
+    assert e.query()
