@@ -2116,8 +2116,9 @@ static int dom_iterate_dev(DomCtx* D, const ClArgs& base, int nslots, double ref
             (int)n2, nslots, (const double*)D->Qoct, D->Isoil, refl, D->relax, D->Ig_out, D->qin,
             D->dstate);
       }
+      if (!D->rp) fs_count_launch();  // the ground exchange (launch_rp_ground counts its own)
       k_dom_check<<<1, 1, 0, st>>>(D->keys, D->tol, queued, D->dstate);
-      fs_count_launch(); fs_count_launch(); fs_count_launch();
+      fs_count_launch(); fs_count_launch();
     }
     cudaMemcpyAsync(D->h_dstate, D->dstate, sizeof(int) * 4, cudaMemcpyDeviceToHost, st);
     if (fs_stream_wait(st) != FS_OK) return FS_ECUDA;

@@ -679,6 +679,18 @@ def test_dom_register_patch_kernel_equals_pencil_kernel(fp32, case):
         assert np.array_equal(qa, qb) and np.array_equal(ga, gb) and np.array_equal(sa, sb)
 
 
+@pytest.mark.parametrize("mode, kernel, begin", [(0, 3, 3), (8, 1, 2)])
+def test_dom_solve_counts_its_launches(mode, kernel, begin):
+    """The launch count of a new handle's solve: set-up and ground (for the
+    register-patch kernel the ground in its layouts too), four kernels a queued
+    iteration (the sweep, G, the ground exchange, the test; at least two are
+    queued), the sources and the ground flux."""
+    n0 = lib().fs_launch_count()
+    (_, _, _, its), = _dom_solves(mode, 0, 13, 7, 21, seed=5, calls=1, want_kernel=kernel,
+                                  want_mode=8)
+    assert lib().fs_launch_count() - n0 == begin + 4 * max(its, 2) + 2
+
+
 @pytest.mark.parametrize("fp32", [0, 1])
 @pytest.mark.parametrize("case", [((29, 40, 48), 8, 10), ((13, 7, 21), 8, 7),
                                   ((60, 120, 24), 8, 10), ((64, 100, 16), 4, 8)])
