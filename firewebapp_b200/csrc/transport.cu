@@ -601,10 +601,10 @@ __global__ void __launch_bounds__(MR_THREADS, 2) k_keps(GridDev g, KepsArgs a, i
       double P_k_lim = nu_t * S2;
       if (P_k_lim > 10.0 * e_loc) P_k_lim = 10.0 * e_loc;
       const double dTdz = (Th - Tl) * idzc;  // (at the ground and the top Tl, Th repeat T0)
-      // buoyant production: none where the gradient is stable or zero (a cell
-      // whose own temperature is NaN, which the gradient does not see, has one)
+      // buoyant production: none where the gradient is stable or zero (it is formed
+      // there too where the temperature that divides it is NaN or infinite)
       double G_k = 0.0, C3 = 0.0;
-      if (!(nu_t * dTdz <= 0.0) || T0 != T0) {
+      if (!(nu_t * dTdz <= 0.0) || !(T0 < INFINITY)) {
         double Tfb = T0;
         if (Tfb < a.T_amb) Tfb = a.T_amb;
         G_k = (nu_t / 0.85) * (9.81 / Tfb) * dTdz;

@@ -500,6 +500,26 @@ def test_k_epsilon(vectors):
         assert rel_l2(host(nuo), c["nu_t_out"]) <= LIBM, name
 
 
+@pytest.mark.parametrize("where", [(0, 0, 0), (6, 4, 10)])
+def test_k_epsilon_of_an_infinite_temperature_at_the_boundary_is_nan(where):
+    """At the ground and at the top the temperature gradient is one-sided: next
+    to an infinite temperature it is infinite, and times 9.81 over that
+    temperature NaN, in the stable direction too (the ground's)."""
+    shape = nz, ny, nx = 7, 5, 11
+    g = Grid(nz, ny, nx, 0.1, 0.1, np.full(nz, 0.1))
+    T = np.full(shape, 300.0)
+    T[where] = np.inf
+    k, e, u = (dev(np.full(shape, q)) for q in (0.1, 0.05, 1.0))
+    v, w, a = (dev(np.zeros(shape)) for _ in range(3))
+    ui, kw, ew = dev(np.ones((nz, ny))), dev(np.full((ny, nx), 0.1)), dev(np.full((ny, nx), 0.05))
+    ko, eo, nuo = (torch.empty_like(k) for _ in range(3))
+    dT = dev(T)
+    call("fs_k_epsilon", g.ref, ptr(k), ptr(e), ptr(u), ptr(v), ptr(w), ptr(dT), ptr(a), ptr(ui),
+         ptr(kw), ptr(ew), ptr(ko), ptr(eo), ptr(nuo), None, None, 2000.0, 1e-3, 300.0, 1.0, 5.0,
+         stream())
+    assert np.isnan(host(ko)[where]) and np.isnan(host(eo)[where])
+
+
 @pytest.mark.parametrize("where", [(3, 2, 5), (0, 0, 0), (6, 4, 10)])
 def test_k_epsilon_of_a_nan_temperature_is_nan(where):
     """Uniform air with one NaN temperature: k and epsilon of that cell are NaN
@@ -513,9 +533,10 @@ def test_k_epsilon_of_a_nan_temperature_is_nan(where):
     v, w, a = (dev(np.zeros(shape)) for _ in range(3))
     ui, kw, ew = dev(np.ones((nz, ny))), dev(np.full((ny, nx), 0.1)), dev(np.full((ny, nx), 0.05))
     ko, eo, nuo = (torch.empty_like(k) for _ in range(3))
-    call("fs_k_epsilon", g.ref, ptr(k), ptr(e), ptr(u), ptr(v), ptr(w), ptr(dev(T)), ptr(a),
-         ptr(ui), ptr(kw), ptr(ew), ptr(ko), ptr(eo), ptr(nuo), None, None, 2000.0, 1e-3, 300.0,
-         1.0, 5.0, stream())
+    dT = dev(T)
+    call("fs_k_epsilon", g.ref, ptr(k), ptr(e), ptr(u), ptr(v), ptr(w), ptr(dT), ptr(a), ptr(ui),
+         ptr(kw), ptr(ew), ptr(ko), ptr(eo), ptr(nuo), None, None, 2000.0, 1e-3, 300.0, 1.0, 5.0,
+         stream())
     assert np.isnan(host(ko)[where]) and np.isnan(host(eo)[where])
     far = tuple((q + n // 2) % n for q, n in zip(where, shape))
     assert np.isfinite(host(ko)[far]) and np.isfinite(host(eo)[far])
