@@ -45,8 +45,9 @@ sys.path.insert(0, str(ROOT))
 METRIC = "3D solver cell-steps/s on 1 B200 (plain FP64 Tier-3 step)"
 UNIT = "cell-steps/s"
 WORKLOAD = "tier3_step_400x120x60_S8_fp64"
-# measured DRAM bytes per cell of one launch (see the traffic comment in main)
-TRAFFIC_PER_CELL = {"dom_sweep": (465.048576e6 + 189.39392e6) / 2880000.0}
+# measured DRAM bytes per cell of one FP64 sweep by path 8's kernel: the
+# register-patch kernel's (the only one captured on this workload)
+SWEEP_TRAFFIC_PER_CELL = {3: (465.048576e6 + 189.39392e6) / 2880000.0}
 
 
 def _peaks():
@@ -496,10 +497,10 @@ def kernel_roofline(solver, kt, steps, form, peak, peak_src):
     avg_ms = tot_ms / max(nl, 1)
     achieved = alg[dom_k] / (avg_ms * 1e-3) / 1e9
     # DRAM bytes per launch of the dominant kernel from an ncu capture of this
-    # workload (dram__bytes_read.sum + write.sum) with the default sweep (path 8),
-    # scaled by the cell count
-    traffic = (TRAFFIC_PER_CELL.get(dom_k)
-               if form == "plain" and (dom_k != "dom_sweep" or dom_mode == 8) else None)
+    # workload (dram__bytes_read.sum + write.sum), where it is of the sweep kernel
+    # in use, scaled by the cell count
+    traffic = (SWEEP_TRAFFIC_PER_CELL.get(int(lib.fs_dom_sweep_kernel(solver.dom)))
+               if form == "plain" and dom_k == "dom_sweep" else None)
     if traffic is not None:
         traffic *= N
     out = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",

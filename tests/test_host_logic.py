@@ -53,6 +53,27 @@ def test_job_totals_single_process():
     assert job_totals(5.0, 2.0) == (5.0, 2.0)
 
 
+@pytest.mark.parametrize("form, kernel, known", [("plain", 3, True), ("plain", 1, False),
+                                                 ("plain", 2, False), ("mixed", 3, False)])
+def test_bench_reports_sweep_traffic_of_the_kernel_it_was_captured_for(monkeypatch, form, kernel,
+                                                                       known):
+    """The bench line's DRAM traffic is a capture of the FP64 register-patch
+    sweep: other sweep kernels and the FP32 form have none."""
+    sys.path.insert(0, str(ROOT))
+    import types
+
+    import firewebapp_b200._lib as L
+    from bench import SWEEP_TRAFFIC_PER_CELL, kernel_roofline
+    fake = types.SimpleNamespace(fs_dom_sweep_mode=lambda h: 8, fs_dom_sweep_kernel=lambda h: kernel,
+                                 fs_dom_launch_shape=lambda h, s: 0)
+    monkeypatch.setattr(L, "lib", lambda: fake)
+    solver = types.SimpleNamespace(n=1000, Omega=np.zeros((80, 3)), dom=None)
+    out = kernel_roofline(solver, {"dom_sweep": (5.0, 5), "edc": (1.0, 10)}, 1, form, 6545.3,
+                          "measured")
+    assert out["kernel"] == "dom_sweep"
+    assert out["traffic"] == (SWEEP_TRAFFIC_PER_CELL[3] * 1000 if known else None)
+
+
 def test_bed_particles_per_cell_matches_loop():
     from firewebapp_b200.api import bed_particles_per_cell
     from firewebapp_b200.grid import build_grid
