@@ -1207,22 +1207,28 @@ int proj_set_precision(void* h, int fp32) {
   ProjCtx* P = (ProjCtx*)h;
   fp32 = fp32 ? 1 : 0;
   if (fp32 == P->fp32) return FS_OK;
-  if (fp32 && !P->lev32[0].t) {
-    for (int l = 0; l < P->nlev; ++l) {
+  // (what is there stays: after a call that ran out of memory the next one asks
+  // for the rest)
+  if (fp32) {
+    bool got = true;
+    auto have = [&](float*& a, int64_t n) {
+      if (!a && cudaMalloc(&a, sizeof(float) * (size_t)(n > 0 ? n : 1)) != cudaSuccess) {
+        a = nullptr;
+        got = false;
+      }
+    };
+    for (int l = 0; l < P->nlev && got; ++l) {
       MGLevelT<float>& lv = P->lev32[l];
       const MGLevel& ld = P->lev[l];
       lv.nx = ld.nx; lv.ny = ld.ny; lv.nz = ld.nz; lv.n = ld.n; lv.dims = ld.dims;
       float** arrs[9] = {&lv.gx, &lv.gy, &lv.gz, &lv.e, &lv.dinv, &lv.x, &lv.b, &lv.t, &lv.s};
-      for (float** a : arrs)
-        if (cudaMalloc(a, sizeof(float) * (size_t)(lv.n > 0 ? lv.n : 1)) != cudaSuccess)
-          return FS_ECUDA;
+      for (float** a : arrs) have(*a, lv.n);
     }
     const int64_t nc = P->lev[P->nlev - 1].n;
-    if (cudaMalloc(&P->Ainv32, sizeof(float) * (size_t)(nc <= MG_COARSE_MAX ? nc * nc : 1)) !=
-            cudaSuccess ||
-        cudaMalloc(&P->r32, sizeof(float) * P->lev[0].n) != cudaSuccess ||
-        cudaMalloc(&P->z32, sizeof(float) * P->lev[0].n) != cudaSuccess)
-      return FS_ECUDA;
+    have(P->Ainv32, nc <= MG_COARSE_MAX ? nc * nc : 1);
+    have(P->r32, P->lev[0].n);
+    have(P->z32, P->lev[0].n);
+    if (!got) return FS_ECUDA;
   }
   P->fp32 = fp32;
   if (P->iter_exec) cudaGraphExecDestroy(P->iter_exec);  // the iteration graph changes

@@ -364,3 +364,41 @@ def test_stencil_status_is_synchronous():
     assert not e.query()
     assert lib().fs_stencil_status(1) == 0
     assert e.query()
+
+
+def test_proj_set_precision_without_memory_can_be_repeated():
+    """Memory for part of the FP32 form only (49 MB at 140 x 120 x 60, of which the
+    finest level's nine arrays take 36 and are the first): status 5 each time,
+    and a solve like a new handle's once there is memory."""
+    from gpu_helpers import Grid, call, dev, host, lib, stream
+    from firewebapp_b200._lib import ptr
+    shape = nz, ny, nx = 60, 120, 140
+    rng = np.random.default_rng(4)
+    g = Grid(nz, ny, nx, 0.5, 0.5, np.full(nz, 0.1))
+    rho, u0, v0, w0 = (dev(0.3 + rng.random(shape)) for _ in range(4))
+    ui = dev(np.full((nz, ny), 1.0))
+    hs = [C.c_void_p(), C.c_void_p()]
+    for h in hs:
+        call("fs_proj_create", g.ref, C.byref(h))
+    held = _leave_free(34)
+    try:
+        for _ in range(2):
+            assert lib().fs_proj_set_precision(hs[0], 1) == 5
+            assert b"out of memory" in lib().fs_last_error()
+        held.clear()
+        torch.cuda.empty_cache()
+        got = []
+        for h in hs:
+            u, v, w = u0.clone(), v0.clone(), w0.clone()
+            its = C.c_int()
+            call("fs_proj_set_precision", h, 1)
+            call("fs_proj_rebuild", h, ptr(rho), stream())
+            call("fs_proj_project", h, ptr(u), ptr(v), ptr(w), ptr(ui), None, 0.01, 1e-8, 200,
+                 C.byref(its), stream())
+            got.append([host(q) for q in (u, v, w)])
+        for x, y in zip(*got):
+            assert np.array_equal(x, y)
+    finally:
+        held.clear()
+        for h in hs:
+            lib().fs_proj_destroy(h)
