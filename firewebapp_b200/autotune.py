@@ -73,7 +73,9 @@ def tune_batch(cases, concurrency: int = 2, form: str = "plain", steps: int = 4,
     trials = []
     for mode, ctas in candidates:
         kw = {"dom_sweep": mode, "dom_cluster_ctas": ctas}
-        # the automatic shape is timed with the kernel the automatic choice takes
+        # the automatic shape is timed with the kernel the automatic choice takes (but
+        # where that kernel would need two waves of clusters it may be the pencil
+        # kernel, up to a fifth faster than what is timed)
         tries = [kw]
         if (mode, ctas) == (8, 0):
             tries = [dict(kw, dom_kernel=REGISTER_PATCH), kw]

@@ -36,6 +36,7 @@
 // orders differ only by rounding).
 #include <vector>
 #include <cstring>
+#include <tuple>
 #include <utility>
 #include <type_traits>
 #include <cooperative_groups.h>
@@ -1508,6 +1509,10 @@ static bool rp_points_match(const DomCtx* D) {
   return true;
 }
 
+static int rp_rows(int Mo) {
+  return Mo == 10 ? RpShape<10>::RK : Mo == 6 ? RpShape<6>::RK : RpShape<3>::RK;
+}
+
 static bool plan_rp(DomCtx* D, int force_C) {
   const GridDev& g = D->g;
   const int Mo = D->M / 8;
@@ -1524,7 +1529,7 @@ static bool plan_rp(DomCtx* D, int force_C) {
                                                              : rp_points_match<3>(D);
   if (!ls) return false;
   D->rp_pair = g.dx == g.dy;
-  const int rk = Mo == 10 ? RpShape<10>::RK : Mo == 6 ? RpShape<6>::RK : RpShape<3>::RK;
+  const int rk = rp_rows(Mo);
   const int maxw = Mo == 10 ? RpShape<10>::MAXW : Mo == 6 ? RpShape<6>::MAXW : RpShape<3>::MAXW;
   const int tsize = D->fp32 ? (int)sizeof(float) : (int)sizeof(double);
   const void* fn = octant_rp_ptr(D->fp32 != 0, Mo, D->rp_pair != 0);
@@ -1574,6 +1579,40 @@ static bool plan_rp(DomCtx* D, int force_C) {
   return found;
 }
 
+// Whether the pencil kernel's sweep is the shorter one where plan_rp's clusters
+// need two waves (more rows than ten CTAs hold; D has that plan, and keeps it).
+// In one wave the register-patch kernel took 0.48 to 0.71 of the pencil kernel's
+// time on every grid tried; in two against the pencil kernel's one it took 0.82 to
+// 1.23.  Cycles of a step, fitted to 60 shapes of each kernel (rows of 40 to 160
+// pencils, 40 to 140 levels): register patch 1000 and 24 (FP32 12) for each
+// ordinate and row of a scheduler's share of the warps; pencils, one a thread,
+// 1435 (1427) and by ordinate 89 + 11.6 a warp (64 + 7.4).  S4, 100 x 100 x 70:
+// 435 us against 355; S6, 100 x 40 x 140: 610 and 561; S8, 100 x 100 x 70: 771 and
+// 738, and 200 x 100 x 64: 913 and 1070.  The choice was at most 5 % slower than
+// the other kernel but for one grid (S6, 150 x 67 x 85: 624 against 577).
+static bool pencils_faster(DomCtx* D) {
+  if (D->cl_waves < 2) return false;
+  const GridDev& g = D->g;
+  const auto plan = [&] {
+    return std::make_tuple(D->cl_C, D->cl_rows, D->cl_threads, D->cl_ppt, D->groups, D->cl_waves,
+                           D->cl_smem);
+  };
+  const auto rp = plan();
+  const int Mo = D->M / 8, rk = rp_rows(Mo);
+  const double rp_cost = D->cl_waves * (g.nx + g.ny + g.nz + 2.0 * D->cl_C) *
+                         (1000.0 + D->cl_threads / 128.0 * rk * Mo * (D->fp32 ? 12 : 24));
+  bool faster = false;
+  if (plan_cl(D, 0) && D->cl_waves == 1 && D->cl_ppt == D->groups) {
+    // (two clusters an octant hold two pencils a thread, half of the ordinates each)
+    const double warps = (D->cl_rows * g.ny + 31) / 32, m = (double)Mo / D->groups;
+    faster = (g.nx + g.ny + g.nz + 2.0 * D->cl_C) *
+                 (D->fp32 ? 1427.0 + m * (64.0 + 7.4 * warps) : 1435.0 + m * (89.0 + 11.6 * warps)) <
+             rp_cost;
+  }
+  std::tie(D->cl_C, D->cl_rows, D->cl_threads, D->cl_ppt, D->groups, D->cl_waves, D->cl_smem) = rp;
+  return faster;
+}
+
 static int64_t rp_wrap_elems(const DomCtx* D, size_t ts) {
   return 8ll * rp_pad((int)ts, D->M / 8) * D->g.nz * (D->g.nx + D->g.nz - 1);
 }
@@ -1611,10 +1650,12 @@ static int dom_prepare(DomCtx* D, cudaStream_t st) {
   const int64_t N = ncells(g), n2 = (int64_t)g.nx * g.ny;
   const int want = D->mode_req;
   const size_t ts = D->fp32 ? sizeof(float) : sizeof(double);
-  // the register-patch kernel where path and kernel are automatic, or on request
+  // the register-patch kernel where path and kernel are automatic and it is the
+  // faster one, or on request
   if ((D->sweep_kernel == 3 && want != 3) || (D->sweep_kernel == 0 && want == 0)) {
     const bool fits = D->force_groups < 2 && octant_grouping(D) && plan_rp(D, D->force_C);
-    if (fits && rp_alloc(D, ts)) {
+    const bool take = fits && (D->sweep_kernel == 3 || D->force_C > 0 || !pencils_faster(D));
+    if (take && rp_alloc(D, ts)) {
       D->mode = 8;
       D->rp = 1;
       D->Mo = D->M / 8;

@@ -435,7 +435,9 @@ int fs_dom_set_octant_groups(void* handle, int groups);
 /* The path in use (0 before the first solve or intensity load). */
 int fs_dom_sweep_mode(void* handle);
 /* Path 8's kernel: 0 automatic: 3 where the sweep path is automatic too (mode
- * 0, one cluster per octant) and its shape fits, else 1; 1 one pencil per
+ * 0, one cluster per octant), its shape fits and kernel 1 is not the faster one
+ * (it is on some grids of more than 60 levels, whose clusters kernel 3 would
+ * run in two waves), else 1; 1 one pencil per
  * thread (a hyperplane's intensities pass through shared memory, one barrier
  * over all pencil warps); 3 register patch (a thread keeps its pencils'
  * intensities in registers, inputs and outputs lie by hyperplane; 3, 6 or 10

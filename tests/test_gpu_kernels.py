@@ -739,6 +739,23 @@ def test_dom_register_patch_kernel_equals_pencil_kernel(fp32, case):
         assert np.array_equal(qa, qb) and np.array_equal(ga, gb) and np.array_equal(sa, sb)
 
 
+@pytest.mark.parametrize("fp32", [0, 1])
+@pytest.mark.parametrize("case, faster", [((70, 100, 40), (4, 1)), ((66, 100, 20), (4, 1)),
+                                          ((140, 40, 30), (6, 1)), ((60, 100, 40), (4, 3)),
+                                          ((64, 100, 20), (8, 3)), ((72, 120, 20), (6, 3))],
+                         ids=str)
+def test_dom_kernel_on_more_levels_than_one_wave_holds(fp32, case, faster):
+    """Where the register-patch kernel's clusters need two waves and the pencil
+    kernel's one, the automatic choice is the kernel that was measured faster;
+    asked for, the register-patch kernel runs there too, with the same results."""
+    order, kernel = faster
+    (a,) = _dom_solves(0, fp32, *case, seed=3, calls=1, order=order, want_kernel=kernel, want_mode=8)
+    (b,) = _dom_solves(0, fp32, *case, seed=3, calls=1, order=order, kernel=4 - kernel,
+                       want_kernel=4 - kernel, want_mode=8, groups=1)
+    for x, y in zip(a, b):
+        assert np.array_equal(x, y)
+
+
 @pytest.mark.parametrize("mode, kernel, begin", [(0, 3, 3), (8, 1, 2)])
 def test_dom_solve_counts_its_launches(mode, kernel, begin):
     """The launch count of a new handle's solve: set-up and ground (for the
