@@ -877,7 +877,7 @@ __global__ void __launch_bounds__(PPT == 1 ? CL_MAX_THREADS_1 : CL_MAX_THREADS_2
 // independent updates per hyperplane, where the pencil-per-thread form moves
 // every intensity through shared memory and waits at a barrier over 24 warps
 // that each have ten.  Measured on the 400 x 120 x 60 S8 workload it is the
-// slower of the two (3.85 ms per FP64 sweep, twice the other): with one warp per
+// slower of the two (3.85 ms per FP64 sweep, twice that one): with one warp per
 // scheduler a lane's updates do not overlap enough to cover the latency of
 // the reciprocal and its corrections, which the other form hides with six
 // warps per scheduler.  It is built for comparison and chosen only on request.
@@ -1481,8 +1481,8 @@ static bool plan_lc(DomCtx* D) {
 // shared memory, the update's dependency chain) and the busiest scheduler's
 // arithmetic, and every CTA of the chain adds the steps by which it trails the
 // one before it.  Measured at 97 x 41 x 23, S4: 158, 117, 114 and 111 us a sweep
-// with 2, 4, 6 and 8 CTAs; 400 x 120 x 60, S8: 907 us with 10, 1514 with 15 (two
-// waves of clusters).
+// with 2, 4, 6 and 8 CTAs (an earlier build; 110 with 6 now); 400 x 120 x 60, S8:
+// 890 us with 10, 1514 with 15 (two waves of clusters).
 static const void* octant_rp_ptr(bool fp32, int Mo, bool pair) {
 #define RPP(T, M, P) (const void*)k_dom_octant_rp<T, M, P>
   switch (Mo) {

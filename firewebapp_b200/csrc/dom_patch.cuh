@@ -44,7 +44,12 @@
 #define RP_KS 4      // steps of prefetched inputs
 #define RP_ZS_MAX 8  // slots of the row hand-off ring (4 where shared memory is short)
 template <int MO> struct RpShape;
-// rows per thread and warps at most (168 and 80 registers a thread)
+// Rows per thread and warps at most: 6 rows of 97 to 128 pencils, what a CTA has to
+// hold for 60 levels to run in one wave of clusters.  Ten ordinates: two rows a
+// thread at 168 registers.  Six and three: one row at 80, which the FP64 form of six
+// exceeds by 36 bytes of spill loads; with them its sweep takes 790 us at
+// 400 x 120 x 60 (FP32 528), the pencil kernel's 1359 (1051), and at 133 x 45 x 37
+// 168 (147) against 301 (242).  Three: 542 (451) against 857 (736).
 template <> struct RpShape<10> { static constexpr int RK = 2, MAXW = 12; };
 template <> struct RpShape<6> { static constexpr int RK = 1, MAXW = 24; };
 template <> struct RpShape<3> { static constexpr int RK = 1, MAXW = 24; };

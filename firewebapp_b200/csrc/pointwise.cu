@@ -16,9 +16,10 @@
 //   pass 1: per tile, the last assigned flag (or none);
 //   pass 2: one block carries the flag across tiles;
 //   pass 3: in-tile scan + carry, then the EDC update itself.
-// Passes 1 and 3 give each thread EDC_CPT consecutive cells and issue all of
-// a thread's loads before the scan's barrier, so the block's memory requests
-// are in flight together instead of after it.
+// Pass 1 gives each thread EDC_CPT consecutive cells, pass 3 as many that lie a
+// warp's width apart (k_edc_main says why); both issue a thread's loads before the
+// scan's barrier, so the block's memory requests are in flight together instead
+// of after it.
 // ---------------------------------------------------------------------------
 #define EDC_BLK EDC_TILE
 

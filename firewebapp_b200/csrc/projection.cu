@@ -486,9 +486,10 @@ __device__ __forceinline__ double warp_sum(double v) {
 }
 
 // A kernel's sum: every block leaves its partial, and one small block adds them
-// in block order and does the scalar work that follows (post).  (Adding them in
-// the kernel's own last block, found by a ticket, took 25 us more at the 5850
-// blocks of level 0's tiles: the tickets queue at one address.)
+// (a thread every FIN_THREADS-th, then a tree: the same order each time) and does
+// the scalar work that follows (post).  (Adding them in the kernel's own last
+// block, found by a ticket, took 25 us more at the 5850 blocks of level 0's tiles:
+// the tickets queue at one address.)
 #define POST_NONE 0
 #define POST_DIR 1    // rz of this iteration becomes the old one (slot 0 = slot 2)
 #define POST_CHECK 2  // end of a PCG iteration: count it, ||r_A|| < rtol ||b_A||

@@ -59,7 +59,8 @@ int launch_convert(int64_t n, int nf, const void* const* src, void* const* dst, 
 
 // ---- EDC -----------------------------------------------------------------------
 // The FP64 kernels' tiling: EDC_TPB threads own EDC_TILE consecutive cells,
-// EDC_CPT (four) per thread, one 16-byte load per field and thread.
+// EDC_CPT (four) per thread: consecutive in the flags' aggregate (one 16-byte load
+// per field), a warp's width apart in the update.
 #define E32_BLK EDC_TILE
 
 __device__ __forceinline__ int edc_flag_code32(float Yf, float YO2, float YH, int t) {

@@ -97,7 +97,8 @@ class Tier3Solver:
     ``dom_cluster_ctas`` its CTAs per octant (0: automatic; a nonzero value
     alone selects path 8) and ``dom_kernel`` path 8's kernel
     (``fs_dom_set_sweep_kernel``: 0 automatic, 1 pencil per thread, 2 lane
-    column, 3 register patch)."""
+    column, 3 register patch).  With a path or a cluster size named the
+    automatic kernel is 1; the fastest, 3, is what all three at 0 take."""
 
     FIELDS = ("rho", "u", "v", "w", "T_g", "Y_fuel", "Y_O2", "Y_H2O", "T_s", "alpha_s",
               "k_turb", "eps_turb", "nu_t", "phi")

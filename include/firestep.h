@@ -442,7 +442,7 @@ int fs_dom_sweep_mode(void* handle);
  * over all pencil warps); 3 register patch (a thread keeps its pencils'
  * intensities in registers, inputs and outputs lie by hyperplane; 3, 6 or 10
  * ordinates per octant, the same level-symmetric set in every octant; FS_EARG at
- * the first solve for other shapes): 0.91 ms per FP64 sweep of the S8 workload
+ * the first solve for other shapes): 0.89 ms per FP64 sweep of the S8 workload
  * at 400 x 120 x 60 against kernel 1's 1.81; 2 lane column (a lane owns one y
  * column of all of the CTA's k' rows and keeps their intensities in registers,
  * y-neighbours by warp shuffles; built for ten ordinates per cluster, 4 to 8 rows per CTA and ny <= 128;
