@@ -1,5 +1,5 @@
-// The sub-step's marching stencils in either precision: species transport and
-// turbulent diffusion (march.cuh has the scheme).
+// The sub-step's marching stencils in either precision: species transport
+// (march.cuh has the scheme) and turbulent diffusion.
 #pragma once
 #include "march.cuh"
 
@@ -137,79 +137,79 @@ struct DiffArgs {
   int clip;
 };
 
-// Bound by the loads' latency, so two planes are in flight beyond the three a
-// level reads: three FP64 fields at 400 x 120 x 60 in 44 us; 61 with the
-// neighbours in x and y loaded when they were used.
+// A thread marches up its column with the levels below and above in registers, one
+// more level requested, and takes the neighbours in x and y from L1.  A level reads
+// one plane's halo only, so the ring of planes that the other stencils use did not
+// pay for its copies: three FP64 fields at 400 x 120 x 60 43 us with the ring, 40 so
+// (FP32 31 and 24), one field 21 and 17 (17 and 11); at 133 x 45 x 37 10.2 and 5.8
+// (9.0 and 4.4), 5.4 and 3.7 (4.8 and 3.6).  (Three FP64 fields spill 72 bytes at
+// four blocks an SM; at three they took 44 and 6.2.)
 template <typename T, int NF>
-__global__ void __launch_bounds__(MR_THREADS, 4) k_turb_diff(GridDev g, DiffArgs<T> a, int kz) {
+__global__ void __launch_bounds__(MR_THREADS, sizeof(T) == 4 || NF < 4 ? 4 : 2)
+    k_turb_diff(GridDev g, DiffArgs<T> a, int kz) {
   FOLLOW();
-  typedef PlaneRing<T, NF, 1, 5> Ring;
-  extern __shared__ __align__(16) unsigned char mr_raw[];
-  T* const ring = (T*)mr_raw;
-  T* const rks = (T*)(mr_raw + Ring::BYTES);
+  __shared__ T rks[MR_MAXK * MR_RK];
   const int nx = g.nx, ny = g.ny, nz = g.nz;
   const int64_t sz = (int64_t)nx * ny;
   const int k0 = blockIdx.z * kz, k1 = min(nz, k0 + kz);
-  const T* f[NF];
-#pragma unroll
-  for (int s = 0; s < NF; ++s) f[s] = a.f[s];
-  Ring R;
-  R.init(ring, g);
-  for (int q = 0; q < 3; ++q) R.load(g, f, k0 - 1 + q, q);
-  copy_commit();
-  // (only if a level reads it: a chunk of one level would leave with the copy
-  // still under way)
-  if (k0 + 2 <= k1) R.load(g, f, k0 + 2, 3);
-  copy_commit();
   march_spacings(g, k0, k1, rks);
+  __syncthreads();
   const int i = blockIdx.x * MR_TX + threadIdx.x, j = blockIdx.y * MR_TY + threadIdx.y;
-  const bool inside = i < nx && j < ny;
-  const int64_t col = (int64_t)min(j, ny - 1) * nx + min(i, nx - 1);
-  T nu0 = a.nu_t[k0 * sz + col], nu1 = a.nu_t[min(k0 + 1, nz - 1) * sz + col];
-  int sl = 1;
-  for (int k = k0; k < k1; ++k, sl = Ring::slot(sl, 1)) {
-    copy_wait<1>();
-    __syncthreads();
-    if (k + 3 <= k1) R.load(g, f, k + 3, Ring::slot(sl, 3));
-    copy_commit();
-    const int64_t c = k * sz + col;
+  if (i >= nx || j >= ny) return;
+  int64_t c = k0 * sz + (int64_t)j * nx + i;
+  // zero gradient at the inlet, the outlet, the ground and the top
+  const int oL = i == 0 ? 0 : -1, oR = i == nx - 1 ? 0 : 1;
+  const int oB = (j > 0 ? -1 : ny - 1) * nx, oF = (j < ny - 1 ? 1 : 1 - ny) * nx;
+  T zL[NF], C[NF], zR[NF];
+#pragma unroll
+  for (int s = 0; s < NF; ++s) {
+    C[s] = a.f[s][c];
+    zL[s] = k0 == 0 ? C[s] : a.f[s][c - sz];
+    zR[s] = k0 == nz - 1 ? C[s] : a.f[s][c + sz];
+  }
+  T nu = a.nu_t[c];
+  for (int k = k0; k < k1; ++k, c += sz) {
+    const bool more = k + 1 < k1;
+    const T nu_n = more ? a.nu_t[c + sz] : T(0);
+    T far[NF], xL[NF], xR[NF], yL[NF], yR[NF];
+#pragma unroll
+    for (int s = 0; s < NF; ++s) {
+      const T* const f = a.f[s] + c;
+      far[s] = more && k + 2 < nz ? f[2 * sz] : zR[s];
+      xL[s] = f[oL];
+      xR[s] = f[oR];
+      yL[s] = f[oB];
+      yR[s] = f[oF];
+    }
     // (each precision as it has always rounded: a cell on an extinction threshold
     // must not change sides)
-    const T D_t = sizeof(T) == 8 ? nu0 / a.sc_t : nu0 * a.inv_sc;
-    nu0 = nu1;
-    nu1 = a.nu_t[min(k + 2, nz - 1) * sz + col];
-    if (!inside) continue;
-    const T* const p0 = Ring::at(ring, sl);
-    const T* const pl = Ring::at(ring, Ring::slot(sl, -1));
-    const T* const ph = Ring::at(ring, Ring::slot(sl, 1));
+    const T D_t = sizeof(T) == 8 ? nu / a.sc_t : nu * a.inv_sc;
+    nu = nu_n;
     const T* rk = rks + (k - k0) * MR_RK;
     const T ida = rk[0], idb = rk[1], idz = rk[2];
 #pragma unroll
     for (int s = 0; s < NF; ++s) {
-      const T* const P = p0 + s * Ring::PLANE;
-      const T C = P[0];
-      // zero gradient at the inlet, the outlet, the ground and the top
-      const T xL = i == 0 ? C : P[-1], xR = i == nx - 1 ? C : P[1];
-      const T zL = k == 0 ? C : pl[s * Ring::PLANE], zR = k == nz - 1 ? C : ph[s * Ring::PLANE];
-      const T d2x = (xR - T(2) * C + xL) * a.inv_dx2;
-      const T d2y = (P[Ring::HX] - T(2) * C + P[-Ring::HX]) * a.inv_dy2;
-      const T d2z = ((zR - C) * ida - (C - zL) * idb) * idz;
-      T nv = C + D_t * (d2x + d2y + d2z) * a.dt;
+      const T c0 = C[s];
+      const T d2x = (xR[s] - T(2) * c0 + xL[s]) * a.inv_dx2;
+      const T d2y = (yR[s] - T(2) * c0 + yL[s]) * a.inv_dy2;
+      const T d2z = ((zR[s] - c0) * ida - (c0 - zL[s]) * idb) * idz;
+      T nv = c0 + D_t * (d2x + d2y + d2z) * a.dt;
       if (a.clip) {
         if (nv < a.lo[s]) nv = a.lo[s];
         if (nv > a.hi[s]) nv = a.hi[s];
       }
       a.fo[s][c] = nv;
+      zL[s] = c0;
+      C[s] = zR[s];
+      zR[s] = far[s];
     }
   }
 }
 
 template <typename T, int NF>
 static int launch_turb_march(const GridDev& g, const DiffArgs<T>& a, cudaStream_t st) {
-  constexpr int smem = PlaneRing<T, NF, 1, 5>::BYTES + MR_MAXK * MR_RK * (int)sizeof(T);
   const int kz = march_levels(g);
-  if (!march_smem((const void*)k_turb_diff<T, NF>, smem)) return cuda_status();
-  following(k_turb_diff<T, NF>, march_grid(g, kz), dim3(MR_TX, MR_TY), smem, st)(g, a, kz);
+  following(k_turb_diff<T, NF>, march_grid(g, kz), dim3(MR_TX, MR_TY), 0, st)(g, a, kz);
   fs_count_launch();
   return cuda_status();
 }
