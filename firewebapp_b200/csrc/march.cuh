@@ -70,18 +70,22 @@ struct PlaneRing {
   }
 };
 
-// Levels a block marches.  A block alone on its SM takes about twice the time
-// a level that it takes of a full one's, and two levels' worth before the first:
-// the chunk count with the least (blocks an SM + 1) x (levels + 2).  At
-// 400 x 120 x 60 that is 10 levels (momentum 104 us; 106 with 5, 110 with 15, 119
-// with 30), at 64 x 24 x 20 one.
+// Levels a block marches.  Few tiles: one, as long as that gives no more than
+// MR_FLAT blocks (an SM's blocks overlap each other's copies and barriers, a block
+// alone pays two levels' worth before its first; 97 x 41 x 23: momentum 14.9 us
+// with one level, 16.2 with two, 22 with five; 48 x 120 x 12: 10.7, 13.9, 15.6).
+// Then the chunk count with the least (blocks an SM + 2) x (levels + 2).  At
+// 400 x 120 x 60 that is 10 levels (momentum 99 us; 101 with 5, 105 with 15, 114
+// with 30).  Over 23 grids and all kernels the choice is 1.7 % above the best one.
+#define MR_FLAT 800
 inline int march_levels(const GridDev& g) {
   const int tiles = ((g.nx + MR_TX - 1) / MR_TX) * ((g.ny + MR_TY - 1) / MR_TY);
+  if ((int64_t)tiles * g.nz <= MR_FLAT) return 1;
   int best = 1;
   int64_t least = INT64_MAX;
   for (int kz = 1; kz <= g.nz && kz <= MR_MAXK; ++kz) {
     const int64_t blocks = (int64_t)tiles * ((g.nz + kz - 1) / kz);
-    const int64_t cost = ((blocks + 147) / 148 + 1) * (kz + 2);
+    const int64_t cost = ((blocks + 147) / 148 + 2) * (kz + 2);
     if (cost < least) {
       least = cost;
       best = kz;
