@@ -8,6 +8,7 @@
 // Planes below the ground or above the top repeat the nearest one, columns
 // outside in x the nearest column (the stencils do not use them).
 #pragma once
+#include <type_traits>
 #include "common.cuh"
 
 #define MR_TX 32
@@ -70,13 +71,50 @@ struct PlaneRing {
   }
 };
 
+// The kernels' second form, DIRECT, for grids of few tile levels, where a ring would
+// bring five planes for a level or two: a block has one level and a thread takes
+// its neighbours from memory.  Offsets of a cell's neighbours in x and y there; at
+// an end in x the cell itself (not used).
+struct NearCells {
+  int xl, xr, yl, yr, yl2, yr2;
+  __device__ __forceinline__ void init(const GridDev& g, int i, int j) {
+    xl = i > 0 ? -1 : 0;
+    xr = i < g.nx - 1 ? 1 : 0;
+    yl = (wrapj(j - 1, g.ny) - j) * g.nx;
+    yr = (wrapj(j + 1, g.ny) - j) * g.nx;
+    yl2 = (wrapj(j - 2, g.ny) - j) * g.nx;
+    yr2 = (wrapj(j + 2, g.ny) - j) * g.nx;
+  }
+};
+// the same in a ring's plane
+template <int HX>
+struct NearSlots {
+  static constexpr int xl = -1, xr = 1, yl = -HX, yr = HX, yl2 = -2 * HX, yr2 = 2 * HX;
+  __device__ __forceinline__ void init(const GridDev&, int, int) {}
+};
+template <bool DIRECT, int HX>
+using Near = std::conditional_t<DIRECT, NearCells, NearSlots<HX>>;
+
+// Whether a grid takes the DIRECT form of momentum, k-epsilon and species
+// transport.  us with the ring and direct: 97 x 41 x 23 (552 tile levels) 14.7 and
+// 9.9, 18.0 and 10.8, 15.3 and 10.0 (FP32 14.0 and 6.5); 133 x 45 x 37 (1110) 19.1 and
+// 15.4, 23.3 and 19.8, 19.1 and 15.6 (16.5 and 10.6); 48 x 120 x 60 (1800) 26.4 and
+// 22.7, 34.0 and 33.1, 26.9 and 23.3 (18.6 and 16.4); 600 x 60 x 12 (1824) 19.5 and
+// 22.9, 27.5 and 29.7, 20.3 and 22.1 (14.7 and 15.6); 301 x 119 x 47 (7050) 64 and 102,
+// 88 and 149, 68 and 107 (43 and 60).
+#define MR_DIRECT 1800
+inline bool march_direct(const GridDev& g) {
+  const int tiles = ((g.nx + MR_TX - 1) / MR_TX) * ((g.ny + MR_TY - 1) / MR_TY);
+  return (int64_t)tiles * g.nz <= MR_DIRECT;
+}
+
 // Levels a block marches.  Few tiles: one, as long as that gives no more than
-// MR_FLAT blocks (an SM's blocks overlap each other's copies and barriers, a block
-// alone pays two levels' worth before its first; 97 x 41 x 23: momentum 14.9 us
-// with one level, 16.2 with two, 22 with five; 48 x 120 x 12: 10.7, 13.9, 15.6).
-// Then the chunk count with the least (blocks an SM + 2) x (levels + 2).  At
-// 400 x 120 x 60 that is 10 levels (momentum 99 us; 101 with 5, 105 with 15, 114
-// with 30).  Over 23 grids and all kernels the choice is 1.7 % above the best one.
+// MR_FLAT blocks (an SM's blocks overlap each other's loads and barriers, a block
+// alone pays two levels' worth before its first; 130 x 100 x 9: gas advection 6.3 us
+// with one level, 7.3 with two, 9.1 with five).  Then the chunk count with the least
+// (blocks an SM + 2) x (levels + 2).  At 400 x 120 x 60 that is 10 levels (momentum
+// 99 us; 101 with 5, 105 with 15, 114 with 30).  Over 23 grids and all kernels the
+// choice is 1.7 % above the best one.
 #define MR_FLAT 800
 inline int march_levels(const GridDev& g) {
   const int tiles = ((g.nx + MR_TX - 1) / MR_TX) * ((g.ny + MR_TY - 1) / MR_TY);

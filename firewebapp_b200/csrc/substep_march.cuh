@@ -26,14 +26,14 @@ struct SpeciesArgs {
 // cell differences; FP32 at 301 x 119 x 47, where every neighbour was loaded from
 // L1, 65 us and now 45.  The expressions keep their order and roundings: cells sit on
 // the EDC's thresholds.
-template <typename T, int NS, bool FUSED>
+template <typename T, int NS, bool FUSED, bool DIRECT>
 __global__ void __launch_bounds__(MR_THREADS, sizeof(T) == 8 ? 3 : 4)
     k_species(GridDev g, SpeciesArgs<T> a, int kz) {
   FOLLOW();
   typedef PlaneRing<T, NS, 2, 6> Ring;
   extern __shared__ __align__(16) unsigned char mr_raw[];
   T* const ring = (T*)mr_raw;
-  T* const rks = (T*)(mr_raw + Ring::BYTES);
+  T* const rks = (T*)(mr_raw + (DIRECT ? 0 : Ring::BYTES));
   const int nx = g.nx, ny = g.ny, nz = g.nz;
   const int64_t sz = (int64_t)nx * ny;
   const int k0 = blockIdx.z * kz, k1 = min(nz, k0 + kz);
@@ -41,9 +41,11 @@ __global__ void __launch_bounds__(MR_THREADS, sizeof(T) == 8 ? 3 : 4)
 #pragma unroll
   for (int s = 0; s < NS; ++s) f[s] = a.Y[s];
   Ring R;
-  R.init(ring, g);
-  for (int q = 0; q < 5; ++q) R.load(g, f, k0 - 2 + q, q);
-  copy_commit();
+  if constexpr (!DIRECT) {
+    R.init(ring, g);
+    for (int q = 0; q < 5; ++q) R.load(g, f, k0 - 2 + q, q);
+    copy_commit();
+  }
   march_spacings(g, k0, k1, rks);
   const int i = blockIdx.x * MR_TX + threadIdx.x, j = blockIdx.y * MR_TY + threadIdx.y;
   const bool inside = i < nx && j < ny;
@@ -55,12 +57,16 @@ __global__ void __launch_bounds__(MR_THREADS, sizeof(T) == 8 ? 3 : 4)
   };
   centre(k0 * sz + col);
   const bool mx = i >= 2 && i <= nx - 3;
+  Near<DIRECT, Ring::HX> N;
+  N.init(g, i, min(j, ny - 1));
   int sl = 2;  // the slot of plane k
   for (int k = k0; k < k1; ++k, sl = Ring::slot(sl, 1)) {
-    copy_wait<0>();
+    if constexpr (!DIRECT) copy_wait<0>();
     __syncthreads();
-    if (k + 3 <= k1 + 1) R.load(g, f, k + 3, Ring::slot(sl, 3));
-    copy_commit();
+    if constexpr (!DIRECT) {
+      if (k + 3 <= k1 + 1) R.load(g, f, k + 3, Ring::slot(sl, 3));
+      copy_commit();
+    }
     const T ui = n_u, vi = n_v, wi = n_w, rho_c = n_r, sp = n_p, sd = n_d;
     const int64_t c = k * sz + col;
     if (k + 1 < k1) centre(c + sz);
@@ -70,7 +76,7 @@ __global__ void __launch_bounds__(MR_THREADS, sizeof(T) == 8 ? 3 : 4)
     const T* const ph = Ring::at(ring, Ring::slot(sl, 1));
     const bool ux = ui >= T(0), uy = vi >= T(0), uz = wi >= T(0);
     const T* const pf = Ring::at(ring, Ring::slot(sl, uz ? -2 : 2));
-    const int ox = ux ? -2 : 2, oy = uy ? -2 * Ring::HX : 2 * Ring::HX;
+    const int ox = ux ? -2 : 2, oy = uy ? N.yl2 : N.yr2;
     const T* rk = rks + (k - k0) * MR_RK;
     const T ida = rk[0], idb = rk[1], idz = rk[2], ihz = rk[3];
     const bool mz = k >= 2 && k <= nz - 3;
@@ -78,17 +84,20 @@ __global__ void __launch_bounds__(MR_THREADS, sizeof(T) == 8 ? 3 : 4)
     const T stot = sp + sd;
 #pragma unroll
     for (int s = 0; s < NS; ++s) {
-      const T* const P = p0 + s * Ring::PLANE;
+      const T* const P = DIRECT ? f[s] + c : p0 + s * Ring::PLANE;
       const T C = P[0];
-      const T xL = i == 0 ? a.Y_inlet[s] : P[-1], xR = i == nx - 1 ? C : P[1];
-      const T yL = P[-Ring::HX], yR = P[Ring::HX];
-      const T zL = k == 0 ? C : pl[s * Ring::PLANE], zR = k == nz - 1 ? C : ph[s * Ring::PLANE];
+      const T xL = i == 0 ? a.Y_inlet[s] : P[N.xl], xR = i == nx - 1 ? C : P[N.xr];
+      const T yL = P[N.yl], yR = P[N.yr];
+      const T zL = k == 0 ? C : *(DIRECT ? P - sz : pl + s * Ring::PLANE);
+      const T zR = k == nz - 1 ? C : *(DIRECT ? P + sz : ph + s * Ring::PLANE);
       T fx, fz;
       if (mx) fx = fabs(ui) * muscl_diff(xR - C, C - xL, C, ux ? xL : xR, P[ox], ux) * a.inv_dx;
       else fx = ux ? ui * (C - xL) * a.inv_dx : ui * (xR - C) * a.inv_dx;
       const T fy = fabs(vi) * muscl_diff(yR - C, C - yL, C, uy ? yL : yR, P[oy], uy) * a.inv_dy;
       if (mz)
-        fz = fabs(wi) * muscl_diff(zR - C, C - zL, C, uz ? zL : zR, pf[s * Ring::PLANE], uz) * ihz;
+        fz = fabs(wi) * muscl_diff(zR - C, C - zL, C, uz ? zL : zR,
+                                  *(DIRECT ? P + (uz ? -2 * sz : 2 * sz) : pf + s * Ring::PLANE), uz) *
+             ihz;
       else
         fz = uz ? wi * (C - zL) * idb : wi * (zR - C) * ida;
       const T adv = -(fx + fy + fz);
@@ -114,10 +123,16 @@ __global__ void __launch_bounds__(MR_THREADS, sizeof(T) == 8 ? 3 : 4)
 
 template <typename T, int NS, bool FUSED>
 static int launch_species_march(const GridDev& g, const SpeciesArgs<T>& a, cudaStream_t st) {
-  constexpr int smem = PlaneRing<T, NS, 2, 6>::BYTES + MR_MAXK * MR_RK * (int)sizeof(T);
+  constexpr int spacings = MR_MAXK * MR_RK * (int)sizeof(T);
+  constexpr int smem = PlaneRing<T, NS, 2, 6>::BYTES + spacings;
+  if (march_direct(g)) {
+    following(k_species<T, NS, FUSED, true>, march_grid(g, 1), dim3(MR_TX, MR_TY), spacings, st)(g, a, 1);
+    fs_count_launch();
+    return cuda_status();
+  }
   const int kz = march_levels(g);
-  if (!march_smem((const void*)k_species<T, NS, FUSED>, smem)) return cuda_status();
-  following(k_species<T, NS, FUSED>, march_grid(g, kz), dim3(MR_TX, MR_TY), smem, st)(g, a, kz);
+  if (!march_smem((const void*)k_species<T, NS, FUSED, false>, smem)) return cuda_status();
+  following(k_species<T, NS, FUSED, false>, march_grid(g, kz), dim3(MR_TX, MR_TY), smem, st)(g, a, kz);
   fs_count_launch();
   return cuda_status();
 }

@@ -316,19 +316,22 @@ struct MomArgs {
 // bound: 1200 instructions a warp, 98 registers, 12 warps an SM, 268 us at
 // 400 x 120 x 60; 104 now.
 typedef PlaneRing<double, 3, 2, 6> MomRing;
+template <bool DIRECT>
 __global__ void __launch_bounds__(MR_THREADS, 3) k_momentum(GridDev g, MomArgs a, int kz) {
   FOLLOW();
   extern __shared__ __align__(16) unsigned char mr_raw[];
   double* const ring = (double*)mr_raw;
-  double* const rks = (double*)(mr_raw + MomRing::BYTES);
+  double* const rks = (double*)(mr_raw + (DIRECT ? 0 : MomRing::BYTES));
   const int nx = g.nx, ny = g.ny, nz = g.nz;
   const int64_t sz = (int64_t)nx * ny;
   const int k0 = blockIdx.z * kz, k1 = min(nz, k0 + kz);
   const double* const f[3] = {a.u, a.v, a.w};
   MomRing R;
-  R.init(ring, g);
-  for (int q = 0; q < 5; ++q) R.load(g, f, k0 - 2 + q, q);
-  copy_commit();
+  if constexpr (!DIRECT) {
+    R.init(ring, g);
+    for (int q = 0; q < 5; ++q) R.load(g, f, k0 - 2 + q, q);
+    copy_commit();
+  }
   march_spacings(g, k0, k1, rks);
   const int i = blockIdx.x * MR_TX + threadIdx.x, j = blockIdx.y * MR_TY + threadIdx.y;
   const bool inside = i < nx && j < ny;
@@ -337,12 +340,16 @@ __global__ void __launch_bounds__(MR_THREADS, 3) k_momentum(GridDev g, MomArgs a
   double n_as = a.Fx ? 0.0 : a.alpha_s[k0 * sz + col];
   const bool mx = i >= 2 && i <= nx - 3;
   const double g_T = 9.81 / a.T_amb;
+  Near<DIRECT, MomRing::HX> N;
+  N.init(g, i, min(j, ny - 1));
   int s = 2;  // the slot of plane k
   for (int k = k0; k < k1; ++k, s = MomRing::slot(s, 1)) {
-    copy_wait<0>();
+    if constexpr (!DIRECT) copy_wait<0>();
     __syncthreads();
-    if (k + 3 <= k1 + 1) R.load(g, f, k + 3, MomRing::slot(s, 3));
-    copy_commit();
+    if constexpr (!DIRECT) {
+      if (k + 3 <= k1 + 1) R.load(g, f, k + 3, MomRing::slot(s, 3));
+      copy_commit();
+    }
     const double rho_i = n_rho, T = n_T, as = n_as;
     const int64_t c = k * sz + col;
     if (k + 1 < k1) {
@@ -354,10 +361,12 @@ __global__ void __launch_bounds__(MR_THREADS, 3) k_momentum(GridDev g, MomArgs a
     const double* const p0 = MomRing::at(ring, s);
     const double* const pl = MomRing::at(ring, MomRing::slot(s, -1));
     const double* const ph = MomRing::at(ring, MomRing::slot(s, 1));
-    const double vel[3] = {p0[0], p0[MomRing::PLANE], p0[2 * MomRing::PLANE]};
+    double vel[3];
+#pragma unroll
+    for (int q = 0; q < 3; ++q) vel[q] = *(DIRECT ? f[q] + c : p0 + q * MomRing::PLANE);
     const bool ux = vel[0] >= 0.0, uy = vel[1] >= 0.0, uz = vel[2] >= 0.0;
     const double* const pf = MomRing::at(ring, MomRing::slot(s, uz ? -2 : 2));
-    const int fx = ux ? -2 : 2, fy = uy ? -2 * MomRing::HX : 2 * MomRing::HX;
+    const int fx = ux ? -2 : 2, fy = uy ? N.yl2 : N.yr2;
     const double* rk = rks + (k - k0) * MR_RK;
     const double ida = rk[0], idb = rk[1], idz = rk[2], ihz = rk[3];
     const bool mz = k >= 2 && k <= nz - 3;
@@ -373,9 +382,9 @@ __global__ void __launch_bounds__(MR_THREADS, 3) k_momentum(GridDev g, MomArgs a
     }
 #pragma unroll
     for (int q = 0; q < 3; ++q) {
-      const double* const P = p0 + q * MomRing::PLANE;
+      const double* const P = DIRECT ? f[q] + c : p0 + q * MomRing::PLANE;
       const double C = vel[q];
-      double L = P[-1], H = P[1];
+      double L = P[N.xl], H = P[N.xr];
       if (i == 0) {
         const double* in = q == 0 ? a.u_in : (q == 1 ? a.v_in : a.w_in);
         L = in ? in[(int64_t)k * ny + j] : 0.0;
@@ -385,19 +394,22 @@ __global__ void __launch_bounds__(MR_THREADS, 3) k_momentum(GridDev g, MomArgs a
       double n = ux ? L : H;
       const double dx = mx ? muscl_diff(dp, dm, C, n, P[fx], ux) : C - n;
       double d2 = (dp - dm) * a.inv_dx2;
-      L = P[-MomRing::HX];
-      H = P[MomRing::HX];
+      L = P[N.yl];
+      H = P[N.yr];
       dp = H - C;
       dm = C - L;
       const double dy = muscl_diff(dp, dm, C, uy ? L : H, P[fy], uy);
       d2 += (dp - dm) * a.inv_dy2;
-      L = k == 0 ? 0.0 : pl[q * MomRing::PLANE];
-      H = k == nz - 1 ? C : ph[q * MomRing::PLANE];
+      L = k == 0 ? 0.0 : *(DIRECT ? P - sz : pl + q * MomRing::PLANE);
+      H = k == nz - 1 ? C : *(DIRECT ? P + sz : ph + q * MomRing::PLANE);
       dp = H - C;
       dm = C - L;
       n = uz ? L : H;
-      const double dz = mz ? muscl_diff(dp, dm, C, n, pf[q * MomRing::PLANE], uz) * ihz
-                           : (C - n) * (uz ? idb : ida);
+      const double dz =
+          mz ? muscl_diff(dp, dm, C, n,
+                          *(DIRECT ? P + (uz ? -2 * sz : 2 * sz) : pf + q * MomRing::PLANE), uz) *
+                   ihz
+             : (C - n) * (uz ? idb : ida);
       d2 += (dp * ida - dm * idb) * idz;
       const double adv =
           -(fabs(vel[0]) * (dx * a.inv_dx) + fabs(vel[1]) * (dy * a.inv_dy) + fabs(vel[2]) * dz);
@@ -424,9 +436,14 @@ int launch_momentum(const GridDev& g, const double* u, const double* v, const do
   a.dt = dt; a.T_amb = T_amb;
   a.inv_dx = 1.0 / g.dx; a.inv_dy = 1.0 / g.dy;
   a.inv_dx2 = a.inv_dx * a.inv_dx; a.inv_dy2 = a.inv_dy * a.inv_dy;
+  if (march_direct(g)) {
+    following(k_momentum<true>, march_grid(g, 1), dim3(MR_TX, MR_TY), MR_RK_BYTES, st)(g, a, 1);
+    fs_count_launch();
+    return cuda_status();
+  }
   const int kz = march_levels(g);
-  if (!march_smem((const void*)k_momentum, MomRing::BYTES + MR_RK_BYTES)) return cuda_status();
-  following(k_momentum, march_grid(g, kz), dim3(MR_TX, MR_TY), MomRing::BYTES + MR_RK_BYTES, st)(
+  if (!march_smem((const void*)k_momentum<false>, MomRing::BYTES + MR_RK_BYTES)) return cuda_status();
+  following(k_momentum<false>, march_grid(g, kz), dim3(MR_TX, MR_TY), MomRing::BYTES + MR_RK_BYTES, st)(
       g, a, kz);
   fs_count_launch();
   return cuda_status();
@@ -488,12 +505,13 @@ struct KepsTransport {
 typedef PlaneRing<double, 2, 2, 6> KeRing;
 typedef PlaneRing<double, 3, 1, 4> VelRing;
 #define KEPS_SMEM (KeRing::BYTES + VelRing::BYTES)
+template <bool DIRECT>
 __global__ void __launch_bounds__(MR_THREADS, 2) k_keps(GridDev g, KepsArgs a, int kz) {
   FOLLOW();
   extern __shared__ __align__(16) unsigned char mr_raw[];
   double* const ring = (double*)mr_raw;
   double* const vring = (double*)(mr_raw + KeRing::BYTES);
-  double* const rks = (double*)(mr_raw + KEPS_SMEM);
+  double* const rks = (double*)(mr_raw + (DIRECT ? 0 : KEPS_SMEM));
   const int nx = g.nx, ny = g.ny, nz = g.nz;
   const int64_t sz = (int64_t)nx * ny;
   const int k0 = blockIdx.z * kz, k1 = min(nz, k0 + kz);
@@ -501,11 +519,13 @@ __global__ void __launch_bounds__(MR_THREADS, 2) k_keps(GridDev g, KepsArgs a, i
   const double* const fv[3] = {a.u, a.v, a.w};
   KeRing R;
   VelRing V;
-  R.init(ring, g);
-  V.init(vring, g);
-  for (int q = 0; q < 5; ++q) R.load(g, f, k0 - 2 + q, q);
-  for (int q = 0; q < 3; ++q) V.load(g, fv, k0 - 1 + q, q);
-  copy_commit();
+  if constexpr (!DIRECT) {
+    R.init(ring, g);
+    V.init(vring, g);
+    for (int q = 0; q < 5; ++q) R.load(g, f, k0 - 2 + q, q);
+    for (int q = 0; q < 3; ++q) V.load(g, fv, k0 - 1 + q, q);
+    copy_commit();
+  }
   march_spacings(g, k0, k1, rks);
   const int i = blockIdx.x * MR_TX + threadIdx.x, j = blockIdx.y * MR_TY + threadIdx.y;
   const bool inside = i < nx && j < ny;
@@ -515,13 +535,19 @@ __global__ void __launch_bounds__(MR_THREADS, 2) k_keps(GridDev g, KepsArgs a, i
   double n_as = a.alpha_s[k0 * sz + col];
   const bool mx = i >= 2 && i <= nx - 3;
   constexpr int VP = VelRing::PLANE;
+  Near<DIRECT, KeRing::HX> N;
+  Near<DIRECT, VelRing::HX> NV;
+  N.init(g, i, min(j, ny - 1));
+  NV.init(g, i, min(j, ny - 1));
   int s = 2, sv = 1;
   for (int k = k0; k < k1; ++k, s = KeRing::slot(s, 1), sv = VelRing::slot(sv, 1)) {
-    copy_wait<0>();
+    if constexpr (!DIRECT) copy_wait<0>();
     __syncthreads();
-    if (k + 3 <= k1 + 1) R.load(g, f, k + 3, KeRing::slot(s, 3));
-    if (k + 2 <= k1) V.load(g, fv, k + 2, VelRing::slot(sv, 2));
-    copy_commit();
+    if constexpr (!DIRECT) {
+      if (k + 3 <= k1 + 1) R.load(g, f, k + 3, KeRing::slot(s, 3));
+      if (k + 2 <= k1) V.load(g, fv, k + 2, VelRing::slot(sv, 2));
+      copy_commit();
+    }
     const int64_t c = k * sz + col;
     const double as = n_as;
     const double Tn = a.T[min(k + 2, nz - 1) * sz + col];
@@ -532,17 +558,20 @@ __global__ void __launch_bounds__(MR_THREADS, 2) k_keps(GridDev g, KepsArgs a, i
       const double* const v0 = VelRing::at(vring, sv);
       const double* const vl = VelRing::at(vring, VelRing::slot(sv, -1));
       const double* const vh = VelRing::at(vring, VelRing::slot(sv, 1));
-      const double vel[3] = {v0[0], v0[VP], v0[2 * VP]};
+      double vel[3];
+#pragma unroll
+      for (int q = 0; q < 3; ++q) vel[q] = *(DIRECT ? fv[q] + c : v0 + q * VP);
       // the velocity gradient D[q][x, y, z]
       double D[3][3];
 #pragma unroll
       for (int q = 0; q < 3; ++q) {
-        const double* const P = v0 + q * VP;
-        const double xL = i == 0 ? (q == 0 ? a.u_in[(int64_t)k * ny + j] : 0.0) : P[-1];
-        const double xH = i == nx - 1 ? vel[q] : P[1];
-        const double zL = k == 0 ? 0.0 : vl[q * VP], zH = k == nz - 1 ? vel[q] : vh[q * VP];
+        const double* const P = DIRECT ? fv[q] + c : v0 + q * VP;
+        const double xL = i == 0 ? (q == 0 ? a.u_in[(int64_t)k * ny + j] : 0.0) : P[NV.xl];
+        const double xH = i == nx - 1 ? vel[q] : P[NV.xr];
+        const double zL = k == 0 ? 0.0 : *(DIRECT ? P - sz : vl + q * VP);
+        const double zH = k == nz - 1 ? vel[q] : *(DIRECT ? P + sz : vh + q * VP);
         D[q][0] = (xH - xL) * 0.5 * a.inv_dx;
-        D[q][1] = (P[VelRing::HX] - P[-VelRing::HX]) * 0.5 * a.inv_dy;
+        D[q][1] = (P[NV.yr] - P[NV.yl]) * 0.5 * a.inv_dy;
         D[q][2] = (zH - zL) * idzc;
       }
       const double S12 = 0.5 * (D[0][1] + D[1][0]), S13 = 0.5 * (D[0][2] + D[2][0]),
@@ -560,34 +589,37 @@ __global__ void __launch_bounds__(MR_THREADS, 2) k_keps(GridDev g, KepsArgs a, i
       const bool ux = vel[0] >= 0.0, uy = vel[1] >= 0.0, uz = vel[2] >= 0.0;
       const double* const pf = KeRing::at(ring, KeRing::slot(s, uz ? -2 : 2));
       const bool mz = k >= 2 && k <= nz - 3;
-      double loc[2] = {p0[0], p0[KeRing::PLANE]};
+      double loc[2] = {*(DIRECT ? f[0] + c : p0), *(DIRECT ? f[1] + c : p0 + KeRing::PLANE)};
       if (loc[0] < K_MIN) loc[0] = K_MIN;
       if (loc[1] < EPS_MIN) loc[1] = EPS_MIN;
       KepsTransport tr[2];
 #pragma unroll
       for (int q = 0; q < 2; ++q) {
-        const double* const P = p0 + q * KeRing::PLANE;
+        const double* const P = DIRECT ? f[q] + c : p0 + q * KeRing::PLANE;
         const double C = loc[q];
-        double L = i == 0 ? (q == 0 ? K_MIN : EPS_MIN) : P[-1], H = i == nx - 1 ? C : P[1];
+        double L = i == 0 ? (q == 0 ? K_MIN : EPS_MIN) : P[N.xl], H = i == nx - 1 ? C : P[N.xr];
         double dp = H - C, dm = C - L, n = ux ? L : H;
         double adv = fabs(vel[0]) *
                      (mx ? muscl_diff(dp, dm, C, n, P[ux ? -2 : 2], ux) : C - n) * a.inv_dx;
         double d2 = (dp - dm) * a.inv_dx2;
-        L = P[-KeRing::HX];
-        H = P[KeRing::HX];
+        L = P[N.yl];
+        H = P[N.yr];
         dp = H - C;
         dm = C - L;
         adv += fabs(vel[1]) *
-               muscl_diff(dp, dm, C, uy ? L : H, P[uy ? -2 * KeRing::HX : 2 * KeRing::HX], uy) *
-               a.inv_dy;
+               muscl_diff(dp, dm, C, uy ? L : H, P[uy ? N.yl2 : N.yr2], uy) * a.inv_dy;
         d2 += (dp - dm) * a.inv_dy2;
-        L = k == 0 ? (q == 0 ? a.kwall : a.ewall)[col] : pl[q * KeRing::PLANE];
-        H = k == nz - 1 ? C : ph[q * KeRing::PLANE];
+        L = k == 0 ? (q == 0 ? a.kwall : a.ewall)[col] : *(DIRECT ? P - sz : pl + q * KeRing::PLANE);
+        H = k == nz - 1 ? C : *(DIRECT ? P + sz : ph + q * KeRing::PLANE);
         dp = H - C;
         dm = C - L;
         n = uz ? L : H;
-        adv += fabs(vel[2]) * (mz ? muscl_diff(dp, dm, C, n, pf[q * KeRing::PLANE], uz) * ihz
-                                  : (C - n) * (uz ? idb : ida));
+        adv += fabs(vel[2]) *
+               (mz ? muscl_diff(dp, dm, C, n,
+                                *(DIRECT ? P + (uz ? -2 * sz : 2 * sz) : pf + q * KeRing::PLANE),
+                                uz) *
+                         ihz
+                   : (C - n) * (uz ? idb : ida));
         d2 += (dp * ida - dm * idb) * idz;
         tr[q].adv = adv;
         tr[q].d2 = d2;
@@ -663,9 +695,14 @@ int launch_keps(const GridDev& g, const double* k, const double* e, const double
   a.inv_dx = 1.0 / g.dx; a.inv_dy = 1.0 / g.dy;
   a.inv_dx2 = 1.0 / (g.dx * g.dx); a.inv_dy2 = 1.0 / (g.dy * g.dy);
   if (g.nz < 2) return FS_EARG;
+  if (march_direct(g)) {
+    following(k_keps<true>, march_grid(g, 1), dim3(MR_TX, MR_TY), MR_RK_BYTES, st)(g, a, 1);
+    fs_count_launch();
+    return cuda_status();
+  }
   const int kz = march_levels(g);
-  if (!march_smem((const void*)k_keps, KEPS_SMEM + MR_RK_BYTES)) return cuda_status();
-  following(k_keps, march_grid(g, kz), dim3(MR_TX, MR_TY), KEPS_SMEM + MR_RK_BYTES, st)(g, a, kz);
+  if (!march_smem((const void*)k_keps<false>, KEPS_SMEM + MR_RK_BYTES)) return cuda_status();
+  following(k_keps<false>, march_grid(g, kz), dim3(MR_TX, MR_TY), KEPS_SMEM + MR_RK_BYTES, st)(g, a, kz);
   fs_count_launch();
   return cuda_status();
 }

@@ -1060,6 +1060,16 @@ def test_marching_stencils_against_exact_forms(nx, ny, nz, form):
             assert err <= (1e-12 if form == "plain" else 3e-5), (kind, name, err)
 
 
+@pytest.mark.parametrize("form", ["plain", "mixed"])
+@pytest.mark.parametrize("nx, ny, nz", [(33, 9, 450), (33, 9, 451), (289, 17, 61), (65, 2, 601),
+                                        (250, 40, 46)])
+def test_marching_stencils_either_side_of_the_direct_form(nx, ny, nz, form):
+    """As above with as many levels of tiles (1800) as the form without a ring
+    takes, and with a few more: the ring, on ragged tiles and wrapped rows, in
+    chunks of several levels and a shorter last one."""
+    test_marching_stencils_against_exact_forms(nx, ny, nz, form)
+
+
 def test_level_set(vectors):
     for name in vectors.cases("flame_front"):
         c = vectors.case("flame_front", name)
