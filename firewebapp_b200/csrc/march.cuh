@@ -96,12 +96,13 @@ template <bool DIRECT, int HX>
 using Near = std::conditional_t<DIRECT, NearCells, NearSlots<HX>>;
 
 // Whether a grid takes the DIRECT form of momentum, k-epsilon and species
-// transport.  us with the ring and direct: 97 x 41 x 23 (552 tile levels) 14.7 and
-// 9.9, 18.0 and 10.8, 15.3 and 10.0 (FP32 14.0 and 6.5); 133 x 45 x 37 (1110) 19.1 and
-// 15.4, 23.3 and 19.8, 19.1 and 15.6 (16.5 and 10.6); 48 x 120 x 60 (1800) 26.4 and
-// 22.7, 34.0 and 33.1, 26.9 and 23.3 (18.6 and 16.4); 600 x 60 x 12 (1824) 19.5 and
-// 22.9, 27.5 and 29.7, 20.3 and 22.1 (14.7 and 15.6); 301 x 119 x 47 (7050) 64 and 102,
-// 88 and 149, 68 and 107 (43 and 60).
+// transport, by its tile levels (tiles times levels).  us with the ring and direct,
+// momentum, k-epsilon, species (FP32 species): 97 x 41 x 23 (552) 14.7 and 9.9, 18.0
+// and 10.8, 15.3 and 10.0 (14.0 and 6.5); 133 x 45 x 37 (1110) 19.1 and 15.4, 23.3 and
+// 19.8, 19.1 and 15.6 (16.5 and 10.6); 48 x 120 x 60 (1800) 26.4 and 22.7, 34.0 and
+// 33.1, 26.9 and 23.3 (18.6 and 16.4); 600 x 60 x 12 (1824) 19.5 and 22.9, 27.5 and
+// 29.7, 20.3 and 22.1 (14.7 and 15.6); 301 x 119 x 47 (7050) 64 and 102, 88 and 149, 68
+// and 107 (43 and 60).
 #define MR_DIRECT 1800
 inline bool march_direct(const GridDev& g) {
   const int tiles = ((g.nx + MR_TX - 1) / MR_TX) * ((g.ny + MR_TY - 1) / MR_TY);
