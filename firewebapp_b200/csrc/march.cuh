@@ -96,17 +96,25 @@ template <bool DIRECT, int HX>
 using Near = std::conditional_t<DIRECT, NearCells, NearSlots<HX>>;
 
 // Whether a grid takes the DIRECT form of momentum, k-epsilon and species
-// transport, by its tile levels (tiles times levels).  us with the ring and direct,
-// momentum, k-epsilon, species (FP32 species): 97 x 41 x 23 (552) 14.7 and 9.9, 18.0
-// and 10.8, 15.3 and 10.0 (14.0 and 6.5); 133 x 45 x 37 (1110) 19.1 and 15.4, 23.3 and
-// 19.8, 19.1 and 15.6 (16.5 and 10.6); 48 x 120 x 60 (1800) 26.4 and 22.7, 34.0 and
-// 33.1, 26.9 and 23.3 (18.6 and 16.4); 600 x 60 x 12 (1824) 19.5 and 22.9, 27.5 and
-// 29.7, 20.3 and 22.1 (14.7 and 15.6); 301 x 119 x 47 (7050) 64 and 102, 88 and 149, 68
-// and 107 (43 and 60).
-#define MR_DIRECT 1800
+// transport, by its tile levels (tiles times levels): up to six blocks an SM it was
+// the faster one on all of 23 grids, beyond that the ring except on odd rows, whose
+// copies touch more sectors, and a little longer in FP32.  us with the ring and
+// direct, momentum, k-epsilon, species (FP32 species): 131 x 47 x 14 (420 tile levels)
+// 12.8 and 6.7, 15.2 and 10.2, 12.8 and 6.8 (12.6 and 6.3); 128 x 64 x 24 (768) 12.2 and
+// 11.4, 16.1 and 15.1, 12.3 and 11.4 (9.1 and 8.9); 90 x 90 x 25 (900) 12.3 and 13.4, 18.6
+// and 18.1, 12.6 and 13.5 (11.1 and 9.7); 133 x 45 x 37 (1110) 18.9 and 15.3, 23.2 and
+// 19.8, 19.1 and 15.6 (16.3 and 10.6); 224 x 56 x 24 (1176) 14.9 and 15.8, 17.8 and 19.9,
+// 14.8 and 15.6 (9.6 and 10.8); 301 x 119 x 47 (7050) 64 and 102, 88 and 149, 68 and 107
+// (43 and 60).
+#define MR_DIRECT 888
+#define MR_DIRECT_F32 1000
+#define MR_DIRECT_ODD 1200
+template <typename T>
 inline bool march_direct(const GridDev& g) {
   const int tiles = ((g.nx + MR_TX - 1) / MR_TX) * ((g.ny + MR_TY - 1) / MR_TY);
-  return (int64_t)tiles * g.nz <= MR_DIRECT;
+  return (int64_t)tiles * g.nz <= (g.nx % 2      ? MR_DIRECT_ODD
+                                   : sizeof(T) == 4 ? MR_DIRECT_F32
+                                                    : MR_DIRECT);
 }
 
 // Levels a block marches.  Few tiles: one, as long as that gives no more than

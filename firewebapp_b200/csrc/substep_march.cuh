@@ -125,7 +125,7 @@ template <typename T, int NS, bool FUSED>
 static int launch_species_march(const GridDev& g, const SpeciesArgs<T>& a, cudaStream_t st) {
   constexpr int spacings = MR_MAXK * MR_RK * (int)sizeof(T);
   constexpr int smem = PlaneRing<T, NS, 2, 6>::BYTES + spacings;
-  if (march_direct(g)) {
+  if (march_direct<T>(g)) {
     following(k_species<T, NS, FUSED, true>, march_grid(g, 1), dim3(MR_TX, MR_TY), spacings, st)(g, a, 1);
     fs_count_launch();
     return cuda_status();

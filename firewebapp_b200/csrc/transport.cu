@@ -436,7 +436,7 @@ int launch_momentum(const GridDev& g, const double* u, const double* v, const do
   a.dt = dt; a.T_amb = T_amb;
   a.inv_dx = 1.0 / g.dx; a.inv_dy = 1.0 / g.dy;
   a.inv_dx2 = a.inv_dx * a.inv_dx; a.inv_dy2 = a.inv_dy * a.inv_dy;
-  if (march_direct(g)) {
+  if (march_direct<double>(g)) {
     following(k_momentum<true>, march_grid(g, 1), dim3(MR_TX, MR_TY), MR_RK_BYTES, st)(g, a, 1);
     fs_count_launch();
     return cuda_status();
@@ -695,7 +695,7 @@ int launch_keps(const GridDev& g, const double* k, const double* e, const double
   a.inv_dx = 1.0 / g.dx; a.inv_dy = 1.0 / g.dy;
   a.inv_dx2 = 1.0 / (g.dx * g.dx); a.inv_dy2 = 1.0 / (g.dy * g.dy);
   if (g.nz < 2) return FS_EARG;
-  if (march_direct(g)) {
+  if (march_direct<double>(g)) {
     following(k_keps<true>, march_grid(g, 1), dim3(MR_TX, MR_TY), MR_RK_BYTES, st)(g, a, 1);
     fs_count_launch();
     return cuda_status();

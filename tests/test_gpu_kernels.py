@@ -1061,12 +1061,14 @@ def test_marching_stencils_against_exact_forms(nx, ny, nz, form):
 
 
 @pytest.mark.parametrize("form", ["plain", "mixed"])
-@pytest.mark.parametrize("nx, ny, nz", [(33, 9, 450), (33, 9, 451), (289, 17, 61), (65, 2, 601),
-                                        (250, 40, 46)])
+@pytest.mark.parametrize("nx, ny, nz", [(33, 9, 300), (33, 9, 301), (34, 9, 222), (34, 9, 223),
+                                        (40, 10, 250), (40, 10, 251), (289, 17, 61),
+                                        (65, 2, 601), (250, 40, 46)])
 def test_marching_stencils_either_side_of_the_direct_form(nx, ny, nz, form):
-    """As above with as many levels of tiles (1800) as the form without a ring
-    takes, and with a few more: the ring, on ragged tiles and wrapped rows, in
-    chunks of several levels and a shorter last one."""
+    """As above with as many levels of tiles as the form without a ring takes
+    (1200 on odd rows, else 888 in FP64 and 1000 in FP32) and with a few more: the
+    ring, on ragged tiles and wrapped rows, in chunks of several levels and a
+    shorter last one."""
     test_marching_stencils_against_exact_forms(nx, ny, nz, form)
 
 
