@@ -4,7 +4,8 @@
 // a block by cp.async while the levels before it compute.
 //
 // The copies are of single elements: rows need no alignment, the periodic wrap
-// in y is part of a thread's fixed offset, and any grid size takes this path.
+// in y is part of a thread's fixed offset, and any grid size can take this path
+// (march_direct says which do).
 // Planes below the ground or above the top repeat the nearest one, columns
 // outside in x the nearest column (the stencils do not use them).
 #pragma once
